@@ -124,7 +124,7 @@ namespace b200
         return clamp_cast<Q>(q);
     }
 
-    // Fast path of round-to-nearest-even Quantize to 8 bits (see quantize_rows_rne8_kernel): is the scale one for
+    // Fast path of round-to-nearest-even Quantize to 8 bits (see quantize4 in quantize.cu): is the scale one for
     // which y = RN(1/s), q0 = RN(x*y), e = fma(-q0,s,x), q = fma(e,y,q0) is the correctly rounded x / s.
     __device__ __forceinline__ bool scale_allows_fast_division(float s)
     {

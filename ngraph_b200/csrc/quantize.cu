@@ -5,19 +5,22 @@
 // the iteration order does not matter because every element is independent.
 //
 // Two launch shapes:
-//   rows    - the tensor is viewed as [rows, inner] where every row has ONE scale /
-//             zero point (per-tensor: a single row; per-axis on axis a: rows =
-//             prod(shape[0..a]), inner = prod(shape[a+1..])).  128-bit loads,
-//             packed 32-bit (or 128-bit) stores, 4 independent loads in flight per thread.
+//   stream  - the tensor is viewed as [rows, inner] where every row has ONE scale / zero point (per-tensor: a single
+//             row; per-axis on axis a: rows = prod(shape[0..a]), inner = prod(shape[a+1..])) but is walked as one flat
+//             run of 16-byte vectors, wherever the rows start and end: 128-bit loads, packed 32-bit (or 128-bit) stores,
+//             4 independent loads in flight per thread.  The scales of the rows a block touches are looked up once per
+//             block into a small shared-memory table while its loads are under way.
 //   generic - one element per thread with the scale index recomputed from the
 //             coordinates; any axis set, any alignment.
 #include "common.cuh"
 
 namespace b200
 {
-    constexpr int QT = 256;         // threads per block
-    constexpr int QU = 4;           // independent 4-element vectors per thread
-    constexpr int QCHUNK = QT * QU * 4; // elements per block
+    constexpr int QT = 256;                // threads per block
+    constexpr int QU = 4;                  // independent 4-element vectors per thread (1 for small tensors)
+    constexpr int QBLOCKS = 6;             // blocks an SM should hold (registers are kept below 42 for it)
+    constexpr int MIN_INNER = 16;          // shortest row the streaming kernels take
+    constexpr int MAX_ROWS = QT * QU * 4 / MIN_INNER + 2; // rows a block can touch
 
     struct ProjDims
     {
@@ -59,142 +62,179 @@ namespace b200
         *reinterpret_cast<int4*>(p) = make_int4(a, b, c, d);
     }
 
-    template <typename Q, int MODE, bool FAST>
-    __global__ void __launch_bounds__(QT) quantize_rows_kernel(const float* __restrict__ x,
-                                                               const float* __restrict__ scale,
-                                                               const Q* __restrict__ zp,
-                                                               Q* __restrict__ out,
-                                                               int64_t inner,
-                                                               uint32_t chunks_per_row,
-                                                               int64_t n_scales)
+    // The [rows, inner] view of a tensor, with what replaces divisions by `inner` (see make_rows).
+    struct RowMap
     {
-        const int64_t row = blockIdx.x / chunks_per_row;
-        const uint32_t chunk = blockIdx.x - uint32_t(row) * chunks_per_row;
-        const int64_t sidx = row % n_scales;
-        const float s = scale[sidx];
-        const float z = static_cast<float>(zp[sidx]);
-        const int64_t row_off = int64_t(chunk) * QCHUNK;
-        const int64_t rem = inner - row_off; // elements of this row from the chunk start
-        const float* xp = x + row * inner + row_off;
-        Q* op = out + row * inner + row_off;
-        // one scale per block: the division becomes two multiply-adds where that is exact (8-bit outputs only; an
-        // int32 output can be large enough for the last bit of a quotient beyond 2^24 to matter)
-        const bool fast = FAST && sizeof(Q) == 1 && scale_allows_fast_division(s);
-        const float y = __frcp_rn(s);
-        const float s_low = __fmul_rn(fabsf(s), 5.9604644775390625e-8f); // |s| * 2^-24 (quantize4_directed_fast)
-        const int zi = static_cast<int>(zp[sidx]);
-        const int lo = sizeof(Q) == 1 ? int(QLimits<Q>::lo) - zi : 0, hi = sizeof(Q) == 1 ? int(QLimits<Q>::hi) - zi : 0; // 8-bit path only
+        int64_t total;
+        uint32_t inner, n_scales, rows;
+        uint64_t inner_inv64;  // ceil(2^64 / inner): row of a block's first element
+        uint32_t inner_inv32;  // ceil(2^32 / inner): rows inside a block, for inner < the block's elements
+    };
 
-        float4 v[QU];
-#pragma unroll
-        for (int u = 0; u < QU; ++u)
+    // Where a block's first element lies: its row, and its offset inside that row.
+    __device__ __forceinline__ void block_row(const RowMap& m, int64_t base, uint32_t& row, uint32_t& r0)
+    {
+        row = uint32_t(__umul64hi(uint64_t(base), m.inner_inv64));
+        r0 = uint32_t(base - int64_t(row) * m.inner);
+    }
+
+    // Row (counted from the block's first) of the element `off` = r0 + local, and the elements left in that row.
+    template <int CHUNK>
+    __device__ __forceinline__ uint32_t local_row(const RowMap& m, uint32_t off, uint32_t& left)
+    {
+        const uint32_t r = m.inner >= CHUNK ? (off >= m.inner ? 1u : 0u) : __umulhi(off, m.inner_inv32);
+        left = (r + 1) * m.inner - off;
+        return r;
+    }
+
+    // Four elements with one scale.  FAST (8-bit outputs): the row's scale s is uniform, so y = RN(1/s) is computed once
+    // (correctly rounded reciprocal) and each quotient is  q0 = RN(x*y);  e = x - q0*s (exact in one FMA);
+    // q = RN(q0 + e*y), which is the correctly rounded x/s (Markstein's division theorem) whenever s is a normal number
+    // whose significand is not all ones and nothing over/underflows.  y == 0 marks a scale that fails that test (or the
+    // switched-off path): its row takes the IEEE division.  Quotients of magnitude >= 2^24, whose 8-bit result saturates
+    // regardless of the last bit, skip the correction (see common.cuh).  Every output byte equals the plain
+    // x / s -> rounding -> +zero_point -> clamp sequence of the reference.  An int32 output can be large enough for
+    // the last bit of a quotient beyond 2^24 to matter, so it always divides.
+    template <typename Q, int MODE, bool FAST>
+    __device__ __forceinline__ void quantize4(const float4& v, float s, float y, int zi, Q (&r)[4])
+    {
+        if (FAST && y != 0.0f)
         {
-            int64_t off = (int64_t(u) * QT + threadIdx.x) * 4;
-            if (off + 4 <= rem)
-                v[u] = *reinterpret_cast<const float4*>(xp + off);
-        }
-#pragma unroll
-        for (int u = 0; u < QU; ++u)
-        {
-            int64_t off = (int64_t(u) * QT + threadIdx.x) * 4;
-            if (off + 4 <= rem && fast)
+            const int lo = int(QLimits<Q>::lo) - zi, hi = int(QLimits<Q>::hi) - zi;
+            constexpr bool directed = MODE == B200_ROUND_TOWARD_INFINITY || MODE == B200_ROUND_TOWARD_ZERO || MODE == B200_ROUND_UP ||
+                                      MODE == B200_ROUND_DOWN;
+            int i[4];
+            if (directed)
+                quantize4_directed_fast<MODE>(v, s, y, __fmul_rn(fabsf(s), 5.9604644775390625e-8f) /* |s| * 2^-24 */, lo, hi, zi, i);
+            else if (MODE == B200_ROUND_NEAREST_TOWARD_EVEN)
             {
-                constexpr bool directed = MODE == B200_ROUND_TOWARD_INFINITY || MODE == B200_ROUND_TOWARD_ZERO ||
-                                          MODE == B200_ROUND_UP || MODE == B200_ROUND_DOWN;
-                if (directed)
-                {
-                    int r[4];
-                    quantize4_directed_fast<MODE>(v[u], s, y, s_low, lo, hi, zi, r);
-                    store4<Q>(op + off, static_cast<Q>(r[0]), static_cast<Q>(r[1]), static_cast<Q>(r[2]), static_cast<Q>(r[3]));
-                }
-                else
-                    store4<Q>(op + off,
-                              static_cast<Q>(quantize_int_fast<Q, MODE>(v[u].x, s, y, lo, hi, zi)),
-                              static_cast<Q>(quantize_int_fast<Q, MODE>(v[u].y, s, y, lo, hi, zi)),
-                              static_cast<Q>(quantize_int_fast<Q, MODE>(v[u].z, s, y, lo, hi, zi)),
-                              static_cast<Q>(quantize_int_fast<Q, MODE>(v[u].w, s, y, lo, hi, zi)));
-            }
-            else if (off + 4 <= rem)
-            {
-                store4<Q>(op + off,
-                          quantize_one<Q, MODE>(v[u].x, s, z),
-                          quantize_one<Q, MODE>(v[u].y, s, z),
-                          quantize_one<Q, MODE>(v[u].z, s, z),
-                          quantize_one<Q, MODE>(v[u].w, s, z));
+                i[0] = quantize_rne_fast<Q>(v.x, s, y, lo, hi, zi), i[1] = quantize_rne_fast<Q>(v.y, s, y, lo, hi, zi);
+                i[2] = quantize_rne_fast<Q>(v.z, s, y, lo, hi, zi), i[3] = quantize_rne_fast<Q>(v.w, s, y, lo, hi, zi);
             }
             else
             {
-                for (int64_t e = off; e < rem && e < off + 4; ++e)
-                    op[e] = quantize_one<Q, MODE>(xp[e], s, z);
+                i[0] = quantize_int_fast<Q, MODE>(v.x, s, y, lo, hi, zi), i[1] = quantize_int_fast<Q, MODE>(v.y, s, y, lo, hi, zi);
+                i[2] = quantize_int_fast<Q, MODE>(v.z, s, y, lo, hi, zi), i[3] = quantize_int_fast<Q, MODE>(v.w, s, y, lo, hi, zi);
             }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                r[j] = static_cast<Q>(i[j]);
+        }
+        else
+        {
+            const float z = static_cast<float>(static_cast<Q>(zi));
+            r[0] = quantize_one<Q, MODE>(v.x, s, z), r[1] = quantize_one<Q, MODE>(v.y, s, z);
+            r[2] = quantize_one<Q, MODE>(v.z, s, z), r[3] = quantize_one<Q, MODE>(v.w, s, z);
         }
     }
 
-    // Round-to-nearest-even Quantize to 8 bits with the division strength-reduced per row.
-    //
-    // The row's scale s is uniform, so y = RN(1/s) is computed once (correctly rounded reciprocal)
-    // and each quotient is  q0 = RN(x*y);  e = x - q0*s (exact in one FMA);  q = RN(q0 + e*y),
-    // which is the correctly rounded x/s (Markstein's division theorem) whenever s is a normal
-    // number whose significand is not all ones and nothing over/underflows.  Blocks whose scale
-    // fails that test, and quotients of magnitude >= 2^24 (whose result saturates regardless of
-    // the last bit), take the other branches below, so every output byte equals the plain
-    // x / s -> floor(q+0.5)/ceil(q-0.5)/parity -> +zero_point -> clamp sequence of the reference.
-    // (For |q| < 2^23 that rounding sequence is round-half-even, i.e. one cvt.rni; beyond it clamps.)
-    template <typename Q>
-    __global__ void __launch_bounds__(QT) quantize_rows_rne8_kernel(const float* __restrict__ x,
-                                                                   const float* __restrict__ scale,
-                                                                   const Q* __restrict__ zp,
-                                                                   Q* __restrict__ out,
-                                                                   int64_t inner,
-                                                                   uint32_t chunks_per_row,
-                                                                   int64_t n_scales)
+    // A row's scale as the kernels use it: {scale, reciprocal or 0, zero point}.
+    struct RowScale
     {
-        const int64_t row = blockIdx.x / chunks_per_row;
-        const uint32_t chunk = blockIdx.x - uint32_t(row) * chunks_per_row;
-        const int64_t sidx = row % n_scales;
-        const float s = scale[sidx];
-        const int zi = static_cast<int>(zp[sidx]);
-        const float z = static_cast<float>(zi);
-        const int64_t row_off = int64_t(chunk) * QCHUNK;
-        const int64_t rem = inner - row_off;
-        const float* xp = x + row * inner + row_off;
-        Q* op = out + row * inner + row_off;
-        const bool fast = scale_allows_fast_division(s);
-        const float y = __frcp_rn(s);
-        const int lo = int(QLimits<Q>::lo) - zi, hi = int(QLimits<Q>::hi) - zi;
+        float s, y;
+        int zp;
+    };
+    template <typename Q, bool FAST>
+    __device__ __forceinline__ RowScale row_scale(const float* scale, const Q* zp, uint32_t i, bool fast)
+    {
+        RowScale e;
+        e.s = __ldg(scale + i);
+        e.zp = static_cast<int>(zp[i]);
+        e.y = FAST && fast && scale_allows_fast_division(e.s) ? __frcp_rn(e.s) : 0.0f;
+        return e;
+    }
 
-        float4 v[QU];
+    // The scales of the rows a block touches, looked up by as many threads.
+    template <typename Q, bool FAST, int CHUNK>
+    __device__ __forceinline__ void fill_table(RowScale* table, const float* scale, const Q* zp, const RowMap& m, uint32_t row, uint32_t r0, bool fast)
+    {
+        const uint32_t n = min((r0 + uint32_t(CHUNK) - 1) / m.inner + 1, m.rows - row);
+        for (uint32_t i = threadIdx.x; i < n; i += QT)
+            table[i] = row_scale<Q, FAST>(scale, zp, (row + i) % m.n_scales, fast);
+    }
+
+    // ROWS: more than one row.  U vectors of four elements per thread.  A block that lies inside one row (every block of a
+    // per-tensor call, nearly every block of a call with long rows) keeps its scale in registers; only the others pay for
+    // the table, its barrier and the test for vectors that run into the next row.
+    // Bound by HBM for large tensors (f32 -> u8, round to even, 1 GB per tensor: 6.5 TB/s, a plain copy's rate; the half-way
+    // modes 6.2, the directed ones 6.1-6.3; per channel 6.2) and by load latency below some 100 MB.  Walking the tensor flat
+    // instead of row by row is what keeps odd row lengths on 128-bit accesses: [24, 64, 113, 113] per channel 182 -> 24 us,
+    // [128, 64, 28, 28] 16 us.  Six blocks per SM (40 registers) measured best: at eight the spills of the division's slow
+    // path cost 10 %.
+    template <typename Q, int MODE, bool FAST, bool ROWS, int U>
+    __global__ void __launch_bounds__(QT, QBLOCKS) quantize_stream_kernel(const float* __restrict__ x, const float* __restrict__ scale,
+                                                                          const Q* __restrict__ zp, Q* __restrict__ out, RowMap m, bool fast)
+    {
+        constexpr int CHUNK = QT * U * 4;
+        __shared__ RowScale table[ROWS ? MAX_ROWS : 1];
+        const int64_t base = int64_t(blockIdx.x) * CHUNK;
+        const uint32_t rem = uint32_t(min(m.total - base, int64_t(CHUNK)));
+        x += base;
+        out += base;
+        float4 v[U];
 #pragma unroll
-        for (int u = 0; u < QU; ++u)
+        for (int u = 0; u < U; ++u)
         {
-            int64_t off = (int64_t(u) * QT + threadIdx.x) * 4;
+            const uint32_t off = (u * QT + threadIdx.x) * 4;
             if (off + 4 <= rem)
-                v[u] = *reinterpret_cast<const float4*>(xp + off);
+                v[u] = *reinterpret_cast<const float4*>(x + off);
         }
-#pragma unroll
-        for (int u = 0; u < QU; ++u)
+        uint32_t row = 0, r0 = 0;
+        if (ROWS)
+            block_row(m, base, row, r0);
+        if (!ROWS || r0 + rem <= m.inner)
         {
-            int64_t off = (int64_t(u) * QT + threadIdx.x) * 4;
+            const RowScale e = row_scale<Q, FAST>(scale, zp, ROWS ? row % m.n_scales : 0, fast);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+            {
+                const uint32_t off = (u * QT + threadIdx.x) * 4;
+                if (off + 4 <= rem)
+                {
+                    Q r[4];
+                    quantize4<Q, MODE, FAST>(v[u], e.s, e.y, e.zp, r);
+                    store4<Q>(out + off, r[0], r[1], r[2], r[3]);
+                }
+                else // the last, partial vector of the tensor
+                    for (uint32_t i = off; i < rem; ++i)
+                        out[i] = quantize_one<Q, MODE>(x[i], e.s, static_cast<float>(static_cast<Q>(e.zp)));
+            }
+            return;
+        }
+        fill_table<Q, FAST, CHUNK>(table, scale, zp, m, row, r0, fast);
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+        {
+            const uint32_t off = (u * QT + threadIdx.x) * 4;
+            if (off >= rem)
+                break;
+            uint32_t left, lr = local_row<CHUNK>(m, r0 + off, left);
             if (off + 4 <= rem)
             {
-                if (fast)
+                // four elements with the vector's row; where it runs into the next row, once more with that row's scale
+                Q r[4];
+                uint32_t done = 0;
+#pragma unroll 1
+                do
                 {
-                    const int a = quantize_rne_fast<Q>(v[u].x, s, y, lo, hi, zi), b = quantize_rne_fast<Q>(v[u].y, s, y, lo, hi, zi);
-                    const int c = quantize_rne_fast<Q>(v[u].z, s, y, lo, hi, zi), d = quantize_rne_fast<Q>(v[u].w, s, y, lo, hi, zi);
-                    *reinterpret_cast<uint32_t*>(op + off) =
-                        uint32_t(a & 0xFF) | (uint32_t(b & 0xFF) << 8) | (uint32_t(c & 0xFF) << 16) | (uint32_t(d & 0xFF) << 24);
-                }
-                else
-                {
-                    store4<Q>(op + off, quantize_one<Q, 4>(v[u].x, s, z), quantize_one<Q, 4>(v[u].y, s, z),
-                              quantize_one<Q, 4>(v[u].z, s, z), quantize_one<Q, 4>(v[u].w, s, z));
-                }
+                    Q t[4];
+                    const RowScale e = table[lr++];
+                    quantize4<Q, MODE, FAST>(v[u], e.s, e.y, e.zp, t);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        r[j] = j >= int(done) ? t[j] : r[j];
+                    done = left;
+                    left = 4;
+                } while (done < 4);
+                store4<Q>(out + off, r[0], r[1], r[2], r[3]);
             }
             else
-            {
-                for (int64_t e = off; e < rem && e < off + 4; ++e)
-                    op[e] = quantize_one<Q, 4>(xp[e], s, z);
-            }
+                for (uint32_t i = off; i < rem; ++i)
+                {
+                    const RowScale e = table[i - off >= left ? lr + 1 : lr];
+                    out[i] = quantize_one<Q, MODE>(x[i], e.s, static_cast<float>(static_cast<Q>(e.zp)));
+                }
         }
     }
 
@@ -250,51 +290,63 @@ namespace b200
         __device__ __forceinline__ int32_t get(int i) const { return i == 0 ? w.x : i == 1 ? w.y : i == 2 ? w.z : w.w; }
     };
 
-    template <typename Q>
-    __global__ void __launch_bounds__(QT) dequantize_rows_kernel(const Q* __restrict__ in,
-                                                                 const float* __restrict__ scale,
-                                                                 const Q* __restrict__ zp,
-                                                                 float* __restrict__ out,
-                                                                 int64_t inner,
-                                                                 uint32_t chunks_per_row,
-                                                                 int64_t n_scales)
+    // The same walk as quantize_stream_kernel.
+    template <typename Q, bool ROWS, int U>
+    __global__ void __launch_bounds__(QT, QBLOCKS) dequantize_stream_kernel(const Q* __restrict__ in, const float* __restrict__ scale,
+                                                                            const Q* __restrict__ zp, float* __restrict__ out, RowMap m)
     {
-        const int64_t row = blockIdx.x / chunks_per_row;
-        const uint32_t chunk = blockIdx.x - uint32_t(row) * chunks_per_row;
-        const int64_t sidx = row % n_scales;
-        const float s = scale[sidx];
-        const int z = static_cast<int>(zp[sidx]);
-        const int64_t row_off = int64_t(chunk) * QCHUNK;
-        const int64_t rem = inner - row_off;
-        const Q* ip = in + row * inner + row_off;
-        float* op = out + row * inner + row_off;
-
-        Vec4<Q> v[QU];
+        constexpr int CHUNK = QT * U * 4;
+        __shared__ RowScale table[ROWS ? MAX_ROWS : 1];
+        const int64_t base = int64_t(blockIdx.x) * CHUNK;
+        const uint32_t rem = uint32_t(min(m.total - base, int64_t(CHUNK)));
+        in += base;
+        out += base;
+        Vec4<Q> v[U];
 #pragma unroll
-        for (int u = 0; u < QU; ++u)
+        for (int u = 0; u < U; ++u)
         {
-            int64_t off = (int64_t(u) * QT + threadIdx.x) * 4;
+            const uint32_t off = (u * QT + threadIdx.x) * 4;
             if (off + 4 <= rem)
-                v[u].load(ip + off);
+                v[u].load(in + off);
+        }
+        uint32_t row = 0, r0 = 0;
+        if (ROWS)
+            block_row(m, base, row, r0);
+        const bool one_row = !ROWS || r0 + rem <= m.inner;
+        RowScale e;
+        if (one_row)
+            e = row_scale<Q, false>(scale, zp, ROWS ? row % m.n_scales : 0, false);
+        else
+        {
+            fill_table<Q, false, CHUNK>(table, scale, zp, m, row, r0, false);
+            __syncthreads();
         }
 #pragma unroll
-        for (int u = 0; u < QU; ++u)
+        for (int u = 0; u < U; ++u)
         {
-            int64_t off = (int64_t(u) * QT + threadIdx.x) * 4;
+            const uint32_t off = (u * QT + threadIdx.x) * 4;
+            if (off >= rem)
+                break;
+            uint32_t left = 4;
+            RowScale e2 = e;
+            if (!one_row)
+            {
+                const uint32_t lr = local_row<CHUNK>(m, r0 + off, left);
+                e = table[lr];
+                e2 = left < min(4u, rem - off) ? table[lr + 1] : e;
+            }
             if (off + 4 <= rem)
             {
                 float4 r;
-                r.x = dequantize_one<Q>(v[u].get(0), z, s);
-                r.y = dequantize_one<Q>(v[u].get(1), z, s);
-                r.z = dequantize_one<Q>(v[u].get(2), z, s);
-                r.w = dequantize_one<Q>(v[u].get(3), z, s);
-                *reinterpret_cast<float4*>(op + off) = r;
+                r.x = dequantize_one<Q>(v[u].get(0), e.zp, e.s);
+                r.y = dequantize_one<Q>(v[u].get(1), left > 1 ? e.zp : e2.zp, left > 1 ? e.s : e2.s);
+                r.z = dequantize_one<Q>(v[u].get(2), left > 2 ? e.zp : e2.zp, left > 2 ? e.s : e2.s);
+                r.w = dequantize_one<Q>(v[u].get(3), left > 3 ? e.zp : e2.zp, left > 3 ? e.s : e2.s);
+                *reinterpret_cast<float4*>(out + off) = r;
             }
             else
-            {
-                for (int64_t e = off; e < rem && e < off + 4; ++e)
-                    op[e] = dequantize_one<Q>(ip[e], z, s);
-            }
+                for (uint32_t i = off; i < rem; ++i)
+                    out[i] = i - off < left ? dequantize_one<Q>(in[i], e.zp, e.s) : dequantize_one<Q>(in[i], e2.zp, e2.s);
         }
     }
 
@@ -373,17 +425,28 @@ namespace b200
         return B200_OK;
     }
 
-    static bool use_rows(const QuantPlan& p, const void* a, const void* b)
+    // The streaming kernels take 16-byte aligned tensors whose rows are at least MIN_INNER long (shorter ones would need
+    // more table entries per block than there are threads to fill them in one go).
+    static bool make_rows(const QuantPlan& p, const void* a, const void* b, RowMap& m)
     {
-        if (!p.rows_ok || p.total == 0)
+        if (!p.rows_ok || ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15))
             return false;
-        if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15)
+        if (p.rows > 1 && (p.inner < MIN_INNER || p.inner > (int64_t(1) << 30) || p.rows > (int64_t(1) << 31) || p.total > (int64_t(1) << 33)))
+            return false; // beyond these the 64-bit reciprocal below is no longer exact (total * inner < 2^64)
+        if (p.total / (QT * 4) >= (int64_t(1) << 31) - 1)
             return false;
-        if (p.rows > 1 && ((p.inner & 3) || p.inner < 512))
-            return false;
-        int64_t chunks = (p.inner + QCHUNK - 1) / QCHUNK;
-        return chunks * p.rows < (int64_t(1) << 31) && chunks < (int64_t(1) << 31);
+        m.total = p.total;
+        m.rows = uint32_t(p.rows);
+        m.n_scales = uint32_t(p.n_scales);
+        m.inner = p.rows > 1 ? uint32_t(p.inner) : 0;
+        m.inner_inv64 = p.rows > 1 ? ~uint64_t(0) / uint64_t(p.inner) + 1 : 0;
+        m.inner_inv32 = p.rows > 1 ? uint32_t(0xFFFFFFFFull / uint64_t(p.inner) + 1) : 0;
+        return true;
     }
+
+    // Vectors per thread: one while that is what it takes to give every SM two blocks, else four.
+    static bool small_tensor(int64_t total) { return total < int64_t(sm_count()) * 2 * QT * QU * 4; }
+    static unsigned stream_grid(int64_t total, int u) { return unsigned((total + QT * u * 4 - 1) / (QT * u * 4)); }
 
     static unsigned generic_grid(int64_t total)
     {
@@ -394,43 +457,29 @@ namespace b200
 
     std::atomic<int> g_fast_division{1};
 
-    template <typename Q>
-    static void launch_rne8(const float* x, const float* scale, const void* zp, void* out, const QuantPlan& p,
-                            uint32_t chunks, cudaStream_t st)
-    {
-        quantize_rows_rne8_kernel<Q><<<unsigned(chunks * p.rows), QT, 0, st>>>(
-            x, scale, static_cast<const Q*>(zp), static_cast<Q*>(out), p.inner, chunks, p.n_scales);
-    }
-    template <>
-    void launch_rne8<int32_t>(const float*, const float*, const void*, void*, const QuantPlan&, uint32_t, cudaStream_t)
-    {
-    }
-
     template <typename Q, int MODE>
     static int launch_quantize(const float* x, const float* scale, const void* zp, void* out,
                                const QuantPlan& p, cudaStream_t st)
     {
-        if (use_rows(p, x, out) && MODE == B200_ROUND_NEAREST_TOWARD_EVEN && sizeof(Q) == 1 &&
-            g_fast_division.load(std::memory_order_relaxed))
+        constexpr bool FAST = sizeof(Q) == 1;
+        const Q* z = static_cast<const Q*>(zp);
+        Q* o = static_cast<Q*>(out);
+        RowMap m;
+        if (make_rows(p, x, out, m))
         {
-            uint32_t chunks = uint32_t((p.inner + QCHUNK - 1) / QCHUNK);
-            launch_rne8<Q>(x, scale, zp, out, p, chunks, st);
-        }
-        else if (use_rows(p, x, out))
-        {
-            uint32_t chunks = uint32_t((p.inner + QCHUNK - 1) / QCHUNK);
-            if (sizeof(Q) == 1 && g_fast_division.load(std::memory_order_relaxed))
-                quantize_rows_kernel<Q, MODE, true><<<unsigned(chunks * p.rows), QT, 0, st>>>(
-                    x, scale, static_cast<const Q*>(zp), static_cast<Q*>(out), p.inner, chunks, p.n_scales);
+            const bool fast = g_fast_division.load(std::memory_order_relaxed) != 0, small = small_tensor(p.total);
+            const unsigned grid = stream_grid(p.total, small ? 1 : QU);
+            if (p.rows > 1 && small)
+                quantize_stream_kernel<Q, MODE, FAST, true, 1><<<grid, QT, 0, st>>>(x, scale, z, o, m, fast);
+            else if (p.rows > 1)
+                quantize_stream_kernel<Q, MODE, FAST, true, QU><<<grid, QT, 0, st>>>(x, scale, z, o, m, fast);
+            else if (small)
+                quantize_stream_kernel<Q, MODE, FAST, false, 1><<<grid, QT, 0, st>>>(x, scale, z, o, m, fast);
             else
-                quantize_rows_kernel<Q, MODE, false><<<unsigned(chunks * p.rows), QT, 0, st>>>(
-                    x, scale, static_cast<const Q*>(zp), static_cast<Q*>(out), p.inner, chunks, p.n_scales);
+                quantize_stream_kernel<Q, MODE, FAST, false, QU><<<grid, QT, 0, st>>>(x, scale, z, o, m, fast);
         }
         else
-        {
-            quantize_generic_kernel<Q, MODE><<<generic_grid(p.total), QT, 0, st>>>(
-                x, scale, static_cast<const Q*>(zp), static_cast<Q*>(out), p.total, p.dims);
-        }
+            quantize_generic_kernel<Q, MODE><<<generic_grid(p.total), QT, 0, st>>>(x, scale, z, o, p.total, p.dims);
         return after_launch("b200_quantize");
     }
 
@@ -457,17 +506,23 @@ namespace b200
     static int launch_dequantize(const void* in, const float* scale, const void* zp, float* out,
                                  const QuantPlan& p, cudaStream_t st)
     {
-        if (use_rows(p, in, out))
+        const Q *q = static_cast<const Q*>(in), *z = static_cast<const Q*>(zp);
+        RowMap m;
+        if (make_rows(p, in, out, m))
         {
-            uint32_t chunks = uint32_t((p.inner + QCHUNK - 1) / QCHUNK);
-            dequantize_rows_kernel<Q><<<unsigned(chunks * p.rows), QT, 0, st>>>(
-                static_cast<const Q*>(in), scale, static_cast<const Q*>(zp), out, p.inner, chunks, p.n_scales);
+            const bool small = small_tensor(p.total);
+            const unsigned grid = stream_grid(p.total, small ? 1 : QU);
+            if (p.rows > 1 && small)
+                dequantize_stream_kernel<Q, true, 1><<<grid, QT, 0, st>>>(q, scale, z, out, m);
+            else if (p.rows > 1)
+                dequantize_stream_kernel<Q, true, QU><<<grid, QT, 0, st>>>(q, scale, z, out, m);
+            else if (small)
+                dequantize_stream_kernel<Q, false, 1><<<grid, QT, 0, st>>>(q, scale, z, out, m);
+            else
+                dequantize_stream_kernel<Q, false, QU><<<grid, QT, 0, st>>>(q, scale, z, out, m);
         }
         else
-        {
-            dequantize_generic_kernel<Q><<<generic_grid(p.total), QT, 0, st>>>(
-                static_cast<const Q*>(in), scale, static_cast<const Q*>(zp), out, p.total, p.dims);
-        }
+            dequantize_generic_kernel<Q><<<generic_grid(p.total), QT, 0, st>>>(q, scale, z, out, p.total, p.dims);
         return after_launch("b200_dequantize");
     }
 }

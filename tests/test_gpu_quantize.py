@@ -215,3 +215,23 @@ def test_bandwidth_sweep_tool_runs():
     rows = quantize_sweep.sweep(max_mb=4, iters=2, out=lines.append)
     assert len(rows) == 2 * 2 * 2 + 9 and all(r[4] > 0 for r in rows)
     assert any("ROUND_DOWN" in l for l in lines)
+
+
+@pytest.mark.parametrize("rows,inner,axes", [(1200, 1025, (0,)), (83, 17011, (0,)), (700, 4095, (0,)), (700, 4097, (0,)), (90000, 16, (0,)), (90001, 17, (0,)),
+                                             (7001, 211, (0,)), (60, 16, (0,)), (61, 1023, (0,)), (1, 1300003, ()), (100000, 15, (0,))])
+def test_rows_that_start_anywhere(ops, rows, inner, axes):
+    """Per-axis rows of any length through the streaming kernels (four vectors per thread for the larger tensors, one for the
+    smaller): row boundaries inside vectors, blocks inside one row, over two and over the most rows a block can touch."""
+    for lead in (1, 2):  # the scales repeat along a leading axis
+        shape = (rows, inner) if lead == 1 else (lead, rows, inner)
+        ax = tuple(a + lead - 1 for a in axes)
+        rng = np.random.default_rng(rows + inner)
+        scale = (np.exp(rng.uniform(np.log(1e-3), np.log(1e-1), size=rows)) if axes else np.array(0.05)).astype(np.float32)
+        x = rng.standard_normal(shape).astype(np.float32)
+        for qname, mode in (("u8", 4), ("i8", 0), ("u8", 7), ("i32", 4)):
+            zp = rng.integers(0, 100, size=scale.shape).astype(NP[qname])
+            want = ref.quantize(x, scale, zp, ax, mode)
+            got = ops.quantize(dev(x), dev(scale), dev(zp), ax, mode)
+            np.testing.assert_array_equal(got.cpu().numpy(), want, err_msg="%s mode %d" % (qname, mode))
+            back = ops.dequantize(got, dev(scale), dev(zp), ax).cpu().numpy()
+            np.testing.assert_array_equal(back.view(np.uint32), ref.dequantize(want, scale, zp, ax).view(np.uint32), err_msg=qname)
