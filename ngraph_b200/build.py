@@ -51,6 +51,25 @@ def build_kernels(force=False, verbose=False):
     return KERNEL_LIB
 
 
+TORCH_OPS = os.path.join(HERE, "_torch_ops.so")
+
+
+def build_torch_ops(force=False):
+    """g++ the native half of ngraph_b200/ops.py (a CPython extension over torch's C++ tensors)."""
+    src = os.path.join(CSRC, "torch_ops.cpp")
+    if not force and _newer(TORCH_OPS, [src, os.path.join(ROOT, "include", "b200_kernels.h")]):
+        return TORCH_OPS
+    import sysconfig
+    import torch
+    base = os.path.dirname(torch.__file__)
+    libs = os.path.join(base, "lib")
+    cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-w", "-shared", "-fvisibility=hidden", "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch.compiled_with_cxx11_abi()), "-I" + os.path.join(ROOT, "include"),
+           "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(base, "include"), "-I" + os.path.join(base, "include", "torch", "csrc", "api", "include"),
+           "-I/usr/local/cuda/include", src, "-o", TORCH_OPS, "-L" + libs, "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+    subprocess.check_call(cmd)
+    return TORCH_OPS
+
+
 PLUGIN_LIB = os.path.join(HERE, "libb200_backend.so")
 NGRAPH_LIB_DIR = os.path.join(ROOT, "oracle", "_ref", "lib")
 
@@ -129,5 +148,6 @@ def build_capi(force=False):
 
 if __name__ == "__main__":
     print(build_kernels(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    print(build_torch_ops(force="--force" in sys.argv))
     print(build_plugin(force="--force" in sys.argv))
     print(build_capi(force="--force" in sys.argv))

@@ -3,6 +3,8 @@
 torch supplies device memory and streams; every computation below is one call into
 ``libb200_kernels.so``.  Names and argument meaning follow the nGraph ops they run
 (``op::v0::Quantize``, ``Dequantize``, ``QuantizedDotBias``, ``QuantizedConvolutionBias`` ...).
+Argument checks, output allocation and the call itself are native code (csrc/torch_ops.cpp): a small
+layer's call is bound by the host.
 """
 import ctypes
 
@@ -10,6 +12,16 @@ import torch
 
 from . import lib
 from .lib import F32, I8, I32, LIB, U8, ConvParams, Epilogue, check
+
+try:
+    from . import _torch_ops as _native
+except ImportError as e:
+    raise ImportError("ngraph_b200/_torch_ops.so is missing or does not match this torch: run `python -m ngraph_b200.build`; "
+                      "there is no Python fallback") from e
+
+_native.bind(check, {name: ctypes.cast(getattr(LIB, name), ctypes.c_void_p).value for name in (
+    "b200_quantize", "b200_dequantize", "b200_qgemm", "b200_qconv", "b200_qconv_packed", "b200_qconv_out_shape", "b200_nchw_to_nhwc_u8",
+    "b200_nhwc_to_nchw_u8", "b200_transpose_u8", "b200_maxpool_nhwc_u8", "b200_global_avgpool_q_nhwc_u8")})
 
 _DT = {torch.uint8: U8, torch.int8: I8, torch.int32: I32, torch.float32: F32}
 _TORCH = {U8: torch.uint8, I8: torch.int8, I32: torch.int32, F32: torch.float32}
@@ -23,10 +35,6 @@ def _ptr(t):
     return None if t is None else ctypes.c_void_p(t.data_ptr())
 
 
-def _i64(v):
-    return (ctypes.c_int64 * max(len(v), 1))(*[int(x) for x in v])
-
-
 def _dev(t, dtype=None):
     assert t.is_cuda, "b200 ops take CUDA tensors"
     if dtype is not None:
@@ -36,23 +44,12 @@ def _dev(t, dtype=None):
 
 def quantize(x, scale, zero_point, axes=(), round_mode=4, out=None):
     """op::v0::Quantize(x, scale, zero_point, type=zero_point.dtype, axes, round_mode)."""
-    x, scale, zero_point = _dev(x, torch.float32), _dev(scale, torch.float32), _dev(zero_point)
-    out = torch.empty(x.shape, dtype=zero_point.dtype, device=x.device) if out is None else out
-    axes = sorted(int(a) for a in axes)
-    check(LIB.b200_quantize(_ptr(x), _ptr(scale), _ptr(zero_point), _ptr(out), _DT[zero_point.dtype], _i64(x.shape),
-                            x.dim(), _i64(axes), len(axes), int(round_mode), _stream()), "b200_quantize")
-    return out
+    return _native.quantize(x, scale, zero_point, axes, round_mode, out)
 
 
 def dequantize(x, scale, zero_point, axes=(), out=None):
     """op::v0::Dequantize(x, scale, zero_point, f32, axes)."""
-    x, scale, zero_point = _dev(x), _dev(scale, torch.float32), _dev(zero_point)
-    assert zero_point.dtype == x.dtype
-    out = torch.empty(x.shape, dtype=torch.float32, device=x.device) if out is None else out
-    axes = sorted(int(a) for a in axes)
-    check(LIB.b200_dequantize(_ptr(x), _ptr(scale), _ptr(zero_point), _ptr(out), _DT[x.dtype], _i64(x.shape), x.dim(),
-                              _i64(axes), len(axes), _stream()), "b200_dequantize")
-    return out
+    return _native.dequantize(x, scale, zero_point, axes, out)
 
 
 WEIGHTS_U8 = 0x100
@@ -101,6 +98,8 @@ def qgemm(a, w, scale, out_dtype, bias=None, relu=False, sum_in=None, sum_scale=
           packed=False):
     """out[M,N] = epilogue(a[M,K] @ w[N,K]^T): QuantizedDotBias (fused contract) or, with core=True,
     QuantizedDot's requantisation on a pre-transposed B.  packed=True sends the weights through the packed image."""
+    if not packed:
+        return _native.qgemm(a, w, out, scale, out_dtype, bias, relu, sum_in, sum_scale, core, out_zp)
     a, w = _dev(a), _dev(w)
     assert w.dtype in (torch.int8, torch.uint8)
     m, k = a.shape
@@ -108,13 +107,10 @@ def qgemm(a, w, scale, out_dtype, bias=None, relu=False, sum_in=None, sum_scale=
     assert k == k2
     e, keep = _epilogue(n, scale, out_dtype, bias, relu, sum_in, sum_scale, core, out_zp)
     out = torch.empty((m, n), dtype=out_dtype, device=a.device) if out is None else out
-    if packed:
-        pw = pack_weights(w, 128)
-        check(LIB.b200_qgemm_packed(_ptr(a), _operands(a, w), _ptr(pw), _ptr(out), m, n, k, ctypes.byref(e), _stream()),
-              "b200_qgemm_packed")
-        torch.cuda.current_stream().synchronize()  # pw is released on return
-        return out
-    check(LIB.b200_qgemm(_ptr(a), _operands(a, w), _ptr(w), _ptr(out), m, n, k, ctypes.byref(e), _stream()), "b200_qgemm")
+    pw = pack_weights(w, 128)
+    check(LIB.b200_qgemm_packed(_ptr(a), _operands(a, w), _ptr(pw), _ptr(out), m, n, k, ctypes.byref(e), _stream()),
+          "b200_qgemm_packed")
+    torch.cuda.current_stream().synchronize()  # pw is released on return
     return out
 
 
@@ -136,21 +132,13 @@ def conv_out_hw(cp):
 def qconv(data, filters, scale, out_dtype, cp, bias=None, relu=False, sum_in=None, sum_scale=None, core=False, out_zp=0,
           out=None, packed=False):
     """Channels-last int8 convolution with the fused epilogue: data [N,H,W,C], filters [K,R,S,C] -> [N,P,Q,K]."""
-    data, filters = _dev(data), _dev(filters)
-    assert filters.dtype in (torch.int8, torch.uint8)
-    e, keep = _epilogue(cp.K, scale, out_dtype, bias, relu, sum_in, sum_scale, core, out_zp)
-    p, q = conv_out_hw(cp)
-    out = torch.empty((cp.N, p, q, cp.K), dtype=out_dtype, device=data.device) if out is None else out
-    if packed:
-        pw = filters if packed == "prepacked" else pack_weights(filters.reshape(cp.K, -1), LIB.b200_qconv_weight_block(cp.C))
-        check(LIB.b200_qconv_packed(_ptr(data), _operands(data, filters), _ptr(pw), _ptr(out), ctypes.byref(cp), ctypes.byref(e),
-                                    _stream()), "b200_qconv_packed")
-        if packed != "prepacked":
-            torch.cuda.current_stream().synchronize()  # pw is released on return
+    if packed and packed != "prepacked":
+        assert filters.dtype in (torch.int8, torch.uint8)
+        pw = pack_weights(filters.reshape(cp.K, -1), LIB.b200_qconv_weight_block(cp.C)).view(filters.dtype)
+        out = _native.qconv(data, pw, cp, True, out, scale, out_dtype, bias, relu, sum_in, sum_scale, core, out_zp)
+        torch.cuda.current_stream().synchronize()  # pw is released on return
         return out
-    check(LIB.b200_qconv(_ptr(data), _operands(data, filters), _ptr(filters), _ptr(out), ctypes.byref(cp), ctypes.byref(e),
-                         _stream()), "b200_qconv")
-    return out
+    return _native.qconv(data, filters, cp, bool(packed), out, scale, out_dtype, bias, relu, sum_in, sum_scale, core, out_zp)
 
 
 def stem_geometry(h, w, r, s, pad_below, pad_above):
@@ -186,52 +174,20 @@ def qconv_stem(data_nchw, filters_kcrs, scale, out_dtype, pad_below, pad_above=N
 
 
 def nchw_to_nhwc(x, c_pad=None):
-    x = _dev(x)
-    assert x.element_size() == 1
-    n, c, h, w = x.shape
-    c_pad = c if c_pad is None else c_pad
-    out = torch.empty((n, h, w, c_pad), dtype=x.dtype, device=x.device)
-    check(LIB.b200_nchw_to_nhwc_u8(_ptr(x), _ptr(out), n, c, h, w, c_pad, _stream()), "b200_nchw_to_nhwc_u8")
-    return out
+    return _native.nchw_to_nhwc(x, c_pad)
 
 
 def nhwc_to_nchw(x, c=None):
-    x = _dev(x)
-    assert x.element_size() == 1
-    n, h, w, c_pad = x.shape
-    c = c_pad if c is None else c
-    out = torch.empty((n, c, h, w), dtype=x.dtype, device=x.device)
-    check(LIB.b200_nhwc_to_nchw_u8(_ptr(x), _ptr(out), n, c, h, w, c_pad, _stream()), "b200_nhwc_to_nchw_u8")
-    return out
+    return _native.nhwc_to_nchw(x, c)
 
 
 def transpose_u8(x):
-    x = _dev(x)
-    assert x.element_size() == 1 and x.dim() == 2
-    r, c = x.shape
-    out = torch.empty((c, r), dtype=x.dtype, device=x.device)
-    check(LIB.b200_transpose_u8(_ptr(x), _ptr(out), r, c, _stream()), "b200_transpose_u8")
-    return out
+    return _native.transpose(x)
 
 
 def maxpool_nhwc(x, window, stride, pad_below=(0, 0), pad_above=None):
-    x = _dev(x, torch.uint8)
-    pad_above = pad_below if pad_above is None else pad_above
-    n, h, w, c = x.shape
-    p = (h + pad_below[0] + pad_above[0] - window[0]) // stride[0] + 1
-    q = (w + pad_below[1] + pad_above[1] - window[1]) // stride[1] + 1
-    out = torch.empty((n, p, q, c), dtype=torch.uint8, device=x.device)
-    check(LIB.b200_maxpool_nhwc_u8(_ptr(x), _ptr(out), n, h, w, c, window[0], window[1], stride[0], stride[1],
-                                   pad_below[0], pad_below[1], pad_above[0], pad_above[1], _stream()),
-          "b200_maxpool_nhwc_u8")
-    return out
+    return _native.maxpool(x, window, stride, pad_below, pad_below if pad_above is None else pad_above)
 
 
 def global_avgpool_q(x, scale_in, scale_out):
-    x = _dev(x, torch.uint8)
-    n, h, w, c = x.shape
-    out = torch.empty((n, c), dtype=torch.uint8, device=x.device)
-    check(LIB.b200_global_avgpool_q_nhwc_u8(_ptr(x), _ptr(out), _ptr(_dev(scale_in, torch.float32)),
-                                            _ptr(_dev(scale_out, torch.float32)), n, h, w, c, _stream()),
-          "b200_global_avgpool_q_nhwc_u8")
-    return out
+    return _native.global_avgpool(x, scale_in, scale_out)

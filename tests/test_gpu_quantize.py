@@ -235,3 +235,24 @@ def test_rows_that_start_anywhere(ops, rows, inner, axes):
             np.testing.assert_array_equal(got.cpu().numpy(), want, err_msg="%s mode %d" % (qname, mode))
             back = ops.dequantize(got, dev(scale), dev(zp), ax).cpu().numpy()
             np.testing.assert_array_equal(back.view(np.uint32), ref.dequantize(want, scale, zp, ax).view(np.uint32), err_msg=qname)
+
+
+def test_wrapper_arguments(ops):
+    """what the torch-facing wrappers do with tensors and arguments before the C ABI sees them"""
+    x = torch.randn((6, 10, 8), device="cuda")
+    s, z = torch.full((10,), 0.05, device="cuda"), torch.zeros(10, dtype=torch.int8, device="cuda")
+    want = ops.quantize(x, s, z, axes=[1])
+    assert torch.equal(ops.quantize(x.transpose(0, 1).contiguous().transpose(0, 1), s, z, axes=(1,)), want)  # not contiguous: copied first
+    out = torch.empty_like(want)
+    assert ops.quantize(x, s, z, axes=(np.int64(1),), out=out) is out and torch.equal(out, want)
+    two = torch.rand(60, device="cuda").view(6, 10) * 0.1 + 0.01
+    z2 = torch.zeros((6, 10), dtype=torch.uint8, device="cuda")
+    assert torch.equal(ops.quantize(x, two, z2, axes=(1, 0)), ops.quantize(x, two, z2, axes=(0, 1)))  # axes in any order
+    for call in (lambda: ops.quantize(x.cpu(), s, z, (1,)), lambda: ops.quantize(x.double(), s, z, (1,)),
+                 lambda: ops.dequantize(want, s, z.view(torch.uint8), (1,)), lambda: ops.qgemm(want[0], want[0][:, :4], s, torch.int8)):
+        with pytest.raises(AssertionError):
+            call()
+    with pytest.raises(KeyError):
+        ops.quantize(x, s, z.double(), (1,))
+    with pytest.raises(TypeError):
+        ops.quantize(x.cpu().numpy(), s, z, (1,))
