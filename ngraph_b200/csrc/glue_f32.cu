@@ -589,167 +589,179 @@ namespace b200
         return (bits & 15) == 0;
     }
 
-    // out[b, m, n] = float(sum_k double(a[b, m, k]) * double(b[b, k, n])), k ascending.  One thread owns a 4 x 4 block
-    // of outputs, each with its own double accumulator walked in k order (so every output sees exactly the reference's
-    // sequence of additions); the block shares 4 + 4 operand loads per 16 multiply-adds.
-    __global__ void __launch_bounds__(128) bmm_f32_kernel(const float* __restrict__ a, const float* __restrict__ bm,
-                                                          float* __restrict__ out, int64_t B, int M, int K, int N)
+    // out[b, m, n] = float(sum_k double(a[b, m, k]) * double(b[b, k, n])), k ascending, on the double-precision matrix
+    // instruction (m8n8k4: each output receives its four exact products in ascending k, one rounding each, like the
+    // reference's loop; B200 has no tcgen05 form of it).  A warp owns MT x NT tiles of 8 x 8 outputs, a block WM x WN warps.
+    //
+    // Bound by the double-precision pipe, 64 multiply-adds per clock and SM.  A matrix instruction issues 256 of them, so
+    // the issue slots that scalar multiply-adds needed are free for the operands: panels of f32 in shared memory (filled by
+    // cp.async while the previous panel is multiplied), converted to double as a warp picks up its fragments.  Scalar
+    // multiply-adds on panels of doubles, 8 x 4 per thread, kept the pipe 49 % busy; measured before / after at
+    // 768 x [384, 64] x [64, 384]: 756 -> 478 us, 768 x [384, 384] x [384, 64]: 725 -> 458 us (81-85 % of that pipe).
+    constexpr int BMM_KC = 32;
+    __device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src, bool ok)
     {
-        const int tiles_n = (N + 3) / 4, tiles_m = (M + 3) / 4;
-        const int64_t total = B * tiles_m * tiles_n;
-        for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x)
-        {
-            const int tn = int(i % tiles_n);
-            const int64_t t = i / tiles_n;
-            const int tm = int(t % tiles_m);
-            const int64_t b = t / tiles_m;
-            const int m0 = tm * 4, n0 = tn * 4;
-            const float* ap = a + (b * M + m0) * K;
-            const float* bp = bm + b * K * N + n0;
-            // rows / columns beyond the matrix read the last valid one (their results are not stored)
-            const int r1 = m0 + 1 < M ? 1 : 0, r2 = m0 + 2 < M ? 2 : r1, r3 = m0 + 3 < M ? 3 : r2;
-            const int c1 = n0 + 1 < N ? 1 : 0, c2 = n0 + 2 < N ? 2 : c1, c3 = n0 + 3 < N ? 3 : c2;
-            double acc[4][4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    acc[r][c] = 0.0;
-            for (int k = 0; k < K; ++k)
-            {
-                const double x0 = ap[k], x1 = ap[int64_t(r1) * K + k], x2 = ap[int64_t(r2) * K + k], x3 = ap[int64_t(r3) * K + k];
-                const float* brow = bp + int64_t(k) * N;
-                const double y0 = brow[0], y1 = brow[c1], y2 = brow[c2], y3 = brow[c3];
-                const double xs[4] = {x0, x1, x2, x3}, ys[4] = {y0, y1, y2, y3};
-#pragma unroll
-                for (int r = 0; r < 4; ++r)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-                        acc[r][c] = fma(xs[r], ys[c], acc[r][c]); // a product of two floats is exact in double: one rounding, like mul + add
-            }
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    if (m0 + r < M && n0 + c < N)
-                        out[(b * M + m0 + r) * N + n0 + c] = static_cast<float>(acc[r][c]);
-        }
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(ok ? 4 : 0) : "memory");
+    }
+    __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, bool ok)
+    {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+    }
+    __device__ __forceinline__ void dmma(double (&c)[2], double a, double b)
+    {
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
     }
 
-    // The same product for large matrices: a block of 256 threads owns a TM x TN tile of one batch entry.  Operands are
-    // converted to double ONCE per block and K chunk into shared memory (the conversion, not the multiply-add, limits
-    // the register-only kernel above), and every thread keeps (TM/16) x (TN/16) double accumulators for the outputs
-    // (ty + 16 i, tx + 16 j).  Each accumulator still receives its products in ascending k, one rounding each, so the
-    // result is bit-identical to the kernel above.  Zero-filled padding beyond M, N or K adds fma(0, 0, acc) = acc.
-    template <int TM, int TN, int KC>
-    __global__ void __launch_bounds__(256) bmm_f32_tiled_kernel(const float* __restrict__ a, const float* __restrict__ bm,
-                                                                float* __restrict__ out, int M, int K, int N, int tiles_m, int tiles_n)
+    template <int WM, int WN, int MT, int NT, bool VEC>
+    __global__ void __launch_bounds__(WM* WN * 32) bmm_f32_kernel(const float* __restrict__ a, const float* __restrict__ bm, float* __restrict__ out,
+                                                                  int M, int K, int N, uint32_t tiles_m, uint32_t tiles_n)
     {
-        constexpr int RM = TM / 16, RN = TN / 16;
-        constexpr int LDA = TM + 2, LDB = TN; // LDA: the transposing store of the A panel spreads over the banks
-        extern __shared__ double panels[];
-        double* As = panels;            // [KC][LDA]  As[k][m]
-        double* Bs = panels + KC * LDA; // [KC][LDB]  Bs[k][n]
-        const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-        const int tile = blockIdx.x;
-        const int tn = tile % tiles_n, tm = (tile / tiles_n) % tiles_m;
-        const int64_t batch = tile / (tiles_n * tiles_m);
-        const int m0 = tm * TM, n0 = tn * TN;
+        constexpr int TM = WM * MT * 8, TN = WN * NT * 8, KC = BMM_KC, THREADS = WM * WN * 32;
+        constexpr int LDA = KC + 4, LDB = TN + 8; // fragment loads then touch 32 different banks
+        extern __shared__ __align__(16) float panels[]; // two of { A [TM][LDA], B [KC][LDB] }
+        const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+        const uint32_t tn = blockIdx.x % tiles_n, rest = blockIdx.x / tiles_n;
+        const int m0 = int(rest % tiles_m) * TM, n0 = int(tn) * TN;
+        const int64_t batch = rest / tiles_m;
         const float* ab = a + batch * int64_t(M) * K;
         const float* bb = bm + batch * int64_t(K) * N;
-        double acc[RM][RN];
-#pragma unroll
-        for (int i = 0; i < RM; ++i)
-#pragma unroll
-            for (int j = 0; j < RN; ++j)
-                acc[i][j] = 0.0;
-        // the panels of chunk c + 1 travel from memory into registers while chunk c is multiplied out of shared memory
-        constexpr int A_PER = TM * KC / 256, B_PER = KC * TN / 256;
-        float ra[A_PER], rb[B_PER];
-        auto fetch = [&](int k0) {
-#pragma unroll
-            for (int j = 0; j < A_PER; ++j)
+        const uint32_t base = uint32_t(__cvta_generic_to_shared(panels));
+        auto fetch = [&](int k0, int buf) {
+            // what lies beyond M, N or K is filled with zeros: fma(0, 0, acc) = acc
+            const uint32_t as = base + uint32_t(buf) * (TM * LDA + KC * LDB) * 4, bs = as + TM * LDA * 4;
+            if (VEC)
             {
-                const int i = tid + j * 256, m = i / KC, k = i % KC; // consecutive threads along k (contiguous in memory)
-                ra[j] = (m0 + m < M && k0 + k < K) ? ab[int64_t(m0 + m) * K + k0 + k] : 0.0f;
+                for (int i = tid; i < TM * KC / 4; i += THREADS)
+                {
+                    const int m = i / (KC / 4), k = (i % (KC / 4)) * 4;
+                    const bool ok = m0 + m < M && k0 + k < K;
+                    cp_async_16(as + (m * LDA + k) * 4, ok ? ab + int64_t(m0 + m) * K + k0 + k : ab, ok);
+                }
+                for (int i = tid; i < KC * TN / 4; i += THREADS)
+                {
+                    const int k = i / (TN / 4), n = (i % (TN / 4)) * 4;
+                    const bool ok = k0 + k < K && n0 + n < N;
+                    cp_async_16(bs + (k * LDB + n) * 4, ok ? bb + int64_t(k0 + k) * N + n0 + n : bb, ok);
+                }
             }
-#pragma unroll
-            for (int j = 0; j < B_PER; ++j)
+            else
             {
-                const int i = tid + j * 256, k = i / TN, n = i % TN; // consecutive threads along n
-                rb[j] = (k0 + k < K && n0 + n < N) ? bb[int64_t(k0 + k) * N + n0 + n] : 0.0f;
+                for (int i = tid; i < TM * KC; i += THREADS)
+                {
+                    const int m = i / KC, k = i % KC;
+                    const bool ok = m0 + m < M && k0 + k < K;
+                    cp_async_4(as + (m * LDA + k) * 4, ok ? ab + int64_t(m0 + m) * K + k0 + k : ab, ok);
+                }
+                for (int i = tid; i < KC * TN; i += THREADS)
+                {
+                    const int k = i / TN, n = i % TN;
+                    const bool ok = k0 + k < K && n0 + n < N;
+                    cp_async_4(bs + (k * LDB + n) * 4, ok ? bb + int64_t(k0 + k) * N + n0 + n : bb, ok);
+                }
             }
+            asm volatile("cp.async.commit_group;" ::: "memory");
         };
-        auto stash = [&]() {
+        double acc[MT][NT][2];
 #pragma unroll
-            for (int j = 0; j < A_PER; ++j)
-            {
-                const int i = tid + j * 256;
-                As[(i % KC) * LDA + i / KC] = double(ra[j]);
-            }
+        for (int i = 0; i < MT; ++i)
 #pragma unroll
-            for (int j = 0; j < B_PER; ++j)
-            {
-                const int i = tid + j * 256;
-                Bs[(i / TN) * LDB + i % TN] = double(rb[j]);
-            }
-        };
-        fetch(0);
-        stash();
-        __syncthreads();
-        for (int k0 = 0; k0 < K; k0 += KC)
+            for (int j = 0; j < NT; ++j)
+                acc[i][j][0] = acc[i][j][1] = 0.0;
+        const int wm = (warp / WN) * MT * 8, wn = (warp % WN) * NT * 8;
+        if (K > 0)
+            fetch(0, 0);
+        for (int k0 = 0, buf = 0; k0 < K; k0 += KC, buf ^= 1)
         {
-            const bool more = k0 + KC < K;
-            if (more)
-                fetch(k0 + KC);
-#pragma unroll 4
-            for (int k = 0; k < KC; ++k)
+            if (k0 + KC < K)
             {
-                double x[RM], y[RN];
-#pragma unroll
-                for (int i = 0; i < RM; ++i)
-                    x[i] = As[k * LDA + ty + 16 * i];
-#pragma unroll
-                for (int j = 0; j < RN; ++j)
-                    y[j] = Bs[k * LDB + tx + 16 * j];
-#pragma unroll
-                for (int i = 0; i < RM; ++i)
-#pragma unroll
-                    for (int j = 0; j < RN; ++j)
-                        acc[i][j] = fma(x[i], y[j], acc[i][j]);
+                fetch(k0 + KC, buf ^ 1);
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
             }
+            else
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
             __syncthreads();
-            if (more)
+            const float* as = panels + buf * (TM * LDA + KC * LDB) + (wm + g) * LDA + t;
+            const float* bs = panels + buf * (TM * LDA + KC * LDB) + TM * LDA + t * LDB + wn + g;
+#pragma unroll
+            for (int k = 0; k < KC; k += 4)
             {
-                stash();
-                __syncthreads();
+                double x[MT], y[NT];
+#pragma unroll
+                for (int i = 0; i < MT; ++i)
+                    x[i] = double(as[i * 8 * LDA + k]);
+#pragma unroll
+                for (int j = 0; j < NT; ++j)
+                    y[j] = double(bs[k * LDB + 8 * j]);
+#pragma unroll
+                for (int i = 0; i < MT; ++i)
+#pragma unroll
+                    for (int j = 0; j < NT; ++j)
+                        dmma(acc[i][j], x[i], y[j]);
             }
+            __syncthreads(); // this panel's buffer is filled again in the next step
         }
         float* ob = out + batch * int64_t(M) * N;
 #pragma unroll
-        for (int i = 0; i < RM; ++i)
+        for (int i = 0; i < MT; ++i)
 #pragma unroll
-            for (int j = 0; j < RN; ++j)
+            for (int j = 0; j < NT; ++j)
             {
-                const int m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
-                if (m < M && n < N)
-                    ob[int64_t(m) * N + n] = static_cast<float>(acc[i][j]);
+                const int m = m0 + wm + 8 * i + g, n = n0 + wn + 8 * j + 2 * t;
+                if (m < M)
+                {
+                    float* o = ob + int64_t(m) * N + n;
+                    if (VEC && n + 1 < N) // N even: the pair is 8-byte aligned
+                        *reinterpret_cast<float2*>(o) = make_float2(static_cast<float>(acc[i][j][0]), static_cast<float>(acc[i][j][1]));
+                    else
+                    {
+                        if (n < N)
+                            o[0] = static_cast<float>(acc[i][j][0]);
+                        if (n + 1 < N)
+                            o[1] = static_cast<float>(acc[i][j][1]);
+                    }
+                }
             }
     }
 
-    template <int TM, int TN, int KC>
-    bool launch_bmm_tiled(const float* a, const float* b, float* out, int64_t batch, int M, int K, int N, cudaStream_t st)
+    // One tile shape of the product: what it would cost, and its launch.
+    template <int WM, int WN, int MT, int NT>
+    struct BmmShape
     {
-        constexpr size_t bytes = size_t(KC) * (TM + 2 + TN) * sizeof(double);
-        if (cudaFuncSetAttribute(bmm_f32_tiled_kernel<TM, TN, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)) != cudaSuccess)
-            return false;
-        const int tiles_m = (M + TM - 1) / TM, tiles_n = (N + TN - 1) / TN;
-        const int64_t tiles = batch * tiles_m * tiles_n;
-        if (tiles > 0x7FFFFFFF)
-            return false;
-        bmm_f32_tiled_kernel<TM, TN, KC><<<unsigned(tiles), 256, bytes, st>>>(a, b, out, M, K, N, tiles_m, tiles_n);
-        return true;
-    }
+        static constexpr int TM = WM * MT * 8, TN = WN * NT * 8;
+        static int64_t tiles(int64_t batch, int64_t M, int64_t N) { return batch * ((M + TM - 1) / TM) * ((N + TN - 1) / TN); }
+        // time in units of one 8 x 8 tile's walk over K: rounds of warps over the 4 x 148 scheduler partitions, each warp's
+        // MT * NT tiles in turn (its operand loads weigh more the fewer tiles share them)
+        static double cost(int64_t batch, int64_t M, int64_t N)
+        {
+            const double slots = 4.0 * sm_count(), warps = double(tiles(batch, M, N)) * WM * WN;
+            const double rounds = warps <= slots ? 1.0 : warps / slots;
+            return rounds * (MT * NT + 0.25 * (MT + NT));
+        }
+        static bool launch(const float* a, const float* b, float* out, int64_t batch, int M, int K, int N, cudaStream_t st)
+        {
+            constexpr size_t bytes = 2 * sizeof(float) * (TM * (BMM_KC + 4) + BMM_KC * (TN + 8));
+            const int64_t blocks = tiles(batch, M, N);
+            if (blocks > 0x7FFFFFFF)
+                return false;
+            const uint32_t tiles_m = uint32_t((M + TM - 1) / TM), tiles_n = uint32_t((N + TN - 1) / TN);
+            const bool vec = K % 4 == 0 && N % 4 == 0 && all_aligned16({a, b, out});
+            static std::atomic<uint64_t> told{0};
+            int dev = 0;
+            cudaGetDevice(&dev);
+            if (bytes > 48 * 1024 && !((told.load(std::memory_order_relaxed) >> (dev & 63)) & 1))
+            {
+                if (cudaFuncSetAttribute(bmm_f32_kernel<WM, WN, MT, NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)) != cudaSuccess ||
+                    cudaFuncSetAttribute(bmm_f32_kernel<WM, WN, MT, NT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)) != cudaSuccess)
+                    return false;
+                told.fetch_or(uint64_t(1) << (dev & 63), std::memory_order_relaxed);
+            }
+            if (vec)
+                bmm_f32_kernel<WM, WN, MT, NT, true><<<unsigned(blocks), WM * WN * 32, bytes, st>>>(a, b, out, M, K, N, tiles_m, tiles_n);
+            else
+                bmm_f32_kernel<WM, WN, MT, NT, false><<<unsigned(blocks), WM * WN * 32, bytes, st>>>(a, b, out, M, K, N, tiles_m, tiles_n);
+            return true;
+        }
+    };
 
     template <typename I>
     __global__ void __launch_bounds__(256) gather_rows_kernel(const uint32_t* __restrict__ table, const I* __restrict__ idx,
@@ -1086,14 +1098,17 @@ extern "C" int b200_bmm_f32(const float* a, const float* b, float* out, int64_t 
     if (!out || (K > 0 && (!a || !b)))
         return B200_ERR_INVALID_ARGUMENT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // large products go through the shared-memory kernel; both kernels give the same bits
-    // the wide tile pays off once there are enough K chunks to prefetch behind (measured: K = 64 runs 7 % faster on the narrow one)
-    if (M >= 64 && N >= 96 && K >= 256 && launch_bmm_tiled<128, 128, 16>(a, b, out, batch, int(M), int(K), int(N), st))
-        return after_launch("b200_bmm_f32");
-    if (M >= 64 && N >= 48 && K >= 16 && launch_bmm_tiled<128, 64, 32>(a, b, out, batch, int(M), int(K), int(N), st))
-        return after_launch("b200_bmm_f32");
-    const int64_t blocks4 = batch * ((M + 3) / 4) * ((N + 3) / 4);
-    bmm_f32_kernel<<<grid_for(blocks4, 128), 128, 0, st>>>(a, b, out, batch, int(M), int(K), int(N));
+    // the largest tile that spreads over the scheduler partitions: smaller ones load their operands more often, larger ones
+    // leave partitions idle on small products (12 x [128, 128] x [128, 128] is 24 tiles of 128 x 64 for 148 SMs)
+    using Big = BmmShape<4, 2, 4, 4>;
+    using Mid = BmmShape<2, 2, 4, 4>;
+    using Small = BmmShape<2, 2, 2, 2>;
+    const double big = Big::cost(batch, M, N), mid = Mid::cost(batch, M, N), small = Small::cost(batch, M, N);
+    const bool ok = big <= mid && big <= small ? Big::launch(a, b, out, batch, int(M), int(K), int(N), st)
+                    : mid <= small             ? Mid::launch(a, b, out, batch, int(M), int(K), int(N), st)
+                                               : Small::launch(a, b, out, batch, int(M), int(K), int(N), st);
+    if (!ok)
+        return B200_ERR_TOO_LARGE;
     return after_launch("b200_bmm_f32");
 }
 

@@ -268,3 +268,18 @@ def test_gather_rows(L):
         td, idxd = dev(table), dev(idx)
         L.check(L.LIB.b200_gather_rows_b32(td.data_ptr(), 50, 24, idxd.data_ptr(), code, 77, out.data_ptr(), stream()), "gather")
         np.testing.assert_array_equal(out.cpu().numpy(), table[idx])
+
+
+@pytest.mark.parametrize("batch,m,k,n", [(1, 1, 1, 1), (2, 31, 3, 33), (1, 64, 32, 64), (1, 65, 33, 65), (150, 128, 64, 64), (40, 129, 36, 100), (3, 7, 0, 5)])
+def test_bmm_tile_edges(L, batch, m, k, n):
+    """one tile, one more than a tile and many of the three tile shapes, panels that end early, rows that are not 16-byte aligned"""
+    rng = np.random.default_rng(40)
+    a = (rng.standard_normal((batch, m, k)) * 50).astype(np.float32)
+    b = (rng.standard_normal((batch, k, n)) * 50).astype(np.float32)
+    acc = np.zeros((batch, m, n), np.float64)
+    for kk in range(k):
+        acc += a[:, :, kk, None].astype(np.float64) * b[:, kk, None, :].astype(np.float64)
+    out = torch.full((batch, m, n), 7.0, device="cuda")
+    ad, bd = dev(a), dev(b)
+    L.check(L.LIB.b200_bmm_f32(ad.data_ptr(), bd.data_ptr(), out.data_ptr(), batch, m, k, n, stream()), "bmm")
+    np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(acc.astype(np.float32)))
