@@ -17,6 +17,7 @@
 // reference's summation order so that results are identical, not merely close).
 #include <cuda_runtime.h>
 #include <math.h>
+#include <algorithm>
 #include <initializer_list>
 #include "common.cuh"
 
@@ -204,6 +205,20 @@ namespace b200
             z = __fadd_rn(z, x);
     }
 
+    // Max, Min and Max over Abs.  The result does not depend on the order the inputs are taken in (a NaN never wins the strict
+    // comparison, in any order), so these equal the sequential reference loops (max.hpp:32-58, min.hpp).
+    template <int OP>
+    __device__ __forceinline__ float extreme_of(float m, float x)
+    {
+        if (OP == B200_REDUCE_MAX_ABS)
+            x = fabsf(x);
+        return (OP == B200_REDUCE_MIN ? x < m : x > m) ? x : m;
+    }
+    template <int OP>
+    __device__ __forceinline__ float extreme_start()
+    {
+        return OP == B200_REDUCE_MIN ? INFINITY : -INFINITY;
+    }
     template <int OP> // b200_reduce_op
     __global__ void __launch_bounds__(128) reduce_kernel(const float* __restrict__ in, float* __restrict__ out, Dims keep, Dims red,
                                                          int64_t n_out, int64_t n_red)
@@ -220,88 +235,116 @@ namespace b200
             }
             else
             {
-                // max.hpp:32-58 / min.hpp: start from -inf / +inf, replace on a strict comparison (a NaN never wins)
-                float m = OP == B200_REDUCE_MIN ? INFINITY : -INFINITY;
+                float m = extreme_start<OP>();
                 for (int64_t r = 0; r < n_red; ++r)
-                {
-                    float x = base[mapped_offset(red, r)];
-                    if (OP == B200_REDUCE_MAX_ABS)
-                        x = fabsf(x);
-                    if (OP == B200_REDUCE_MIN ? x < m : x > m)
-                        m = x;
-                }
+                    m = extreme_of<OP>(m, base[mapped_offset(red, r)]);
                 out[o] = m;
             }
         }
     }
 
-    // Max with few outputs and long reductions (a whole-tensor max for a dynamic activation scale): one block per
-    // output.  The result of a max does not depend on the order the inputs are taken in (NaNs never win the
-    // x > max test, in any order), so this equals the sequential reference loop.
-    __global__ void __launch_bounds__(256) reduce_max_block_kernel(const float* __restrict__ in, float* __restrict__ out, Dims keep,
-                                                                   Dims red, int64_t n_red)
+    // of all threads of the block, in thread 0 (partial results meet without the absolute value: -inf is "nothing yet")
+    template <int ELEMENT_OP>
+    __device__ __forceinline__ float extreme_of_block(float m, float* partial)
+    {
+        constexpr int OP = ELEMENT_OP == B200_REDUCE_MAX_ABS ? int(B200_REDUCE_MAX) : ELEMENT_OP;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1)
+            m = extreme_of<OP>(m, __shfl_xor_sync(0xffffffffu, m, d));
+        if ((threadIdx.x & 31) == 0)
+            partial[threadIdx.x >> 5] = m;
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 1; w < int(blockDim.x >> 5); ++w)
+                m = extreme_of<OP>(m, partial[w]);
+        return m;
+    }
+    // of a contiguous run, thread `t` of `threads`: 16-byte loads, four in flight
+    template <int OP>
+    __device__ __forceinline__ float extreme_of_run(const float* __restrict__ in, int64_t n, int64_t t, int64_t threads)
+    {
+        float m = extreme_start<OP>();
+        const int64_t head = min(n, int64_t((16 - (reinterpret_cast<uintptr_t>(in) & 15)) & 15) / 4), n4 = (n - head) / 4;
+        const float4* in4 = reinterpret_cast<const float4*>(in + head);
+        for (int64_t i = t; i < n4; i += 4 * threads)
+        {
+            float4 v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                v[j] = in4[min(i + j * threads, n4 - 1)]; // past the end: the last vector again
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                m = extreme_of<OP>(extreme_of<OP>(extreme_of<OP>(extreme_of<OP>(m, v[j].x), v[j].y), v[j].z), v[j].w);
+        }
+        if (t < head)
+            m = extreme_of<OP>(m, in[t]);
+        if (t < n - head - 4 * n4)
+            m = extreme_of<OP>(m, in[head + 4 * n4 + t]);
+        return m;
+    }
+
+    // few outputs, long reductions: one block per output
+    template <int OP>
+    __global__ void __launch_bounds__(256) reduce_extreme_block_kernel(const float* __restrict__ in, float* __restrict__ out, Dims keep,
+                                                                       Dims red, int64_t n_red)
     {
         __shared__ float partial[8];
         const float* base = in + mapped_offset(keep, blockIdx.x);
-        float m = -INFINITY;
+        float m = extreme_start<OP>();
         for (int64_t r = threadIdx.x; r < n_red; r += blockDim.x)
-        {
-            const float x = base[mapped_offset(red, r)];
-            if (x > m)
-                m = x;
-        }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1)
-        {
-            const float o = __shfl_xor_sync(0xffffffffu, m, d);
-            if (o > m)
-                m = o;
-        }
-        if ((threadIdx.x & 31) == 0)
-            partial[threadIdx.x >> 5] = m;
-        __syncthreads();
+            m = extreme_of<OP>(m, base[mapped_offset(red, r)]);
+        m = extreme_of_block<OP>(m, partial);
+        if (threadIdx.x == 0)
+            out[blockIdx.x] = m;
+    }
+
+    // The whole of a tensor of up to a million elements (the dynamic activation scale of a layer): one cluster of eight
+    // blocks, whose partial results meet in the first block's shared memory: one launch, no scratch, no atomics.
+    // [128, 768]: 2.2 us, where the two launches of the form below took 4; fewer than 65536 elements used to run in one thread.
+    constexpr int EXTREME_CLUSTER = 8;
+    template <int OP>
+    __global__ void __cluster_dims__(EXTREME_CLUSTER, 1, 1) __launch_bounds__(1024)
+        reduce_extreme_cluster_kernel(const float* __restrict__ in, float* __restrict__ out, int64_t n)
+    {
+        __shared__ float partial[32];
+        __shared__ float of_block[EXTREME_CLUSTER];
+        asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); // this block runs: its shared memory may be written
+        const float m = extreme_of_block<OP>(extreme_of_run<OP>(in, n, int64_t(blockIdx.x) * 1024 + threadIdx.x, EXTREME_CLUSTER * 1024), partial);
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
         if (threadIdx.x == 0)
         {
-            for (int w = 1; w < 8; ++w)
-                if (partial[w] > m)
-                    m = partial[w];
-            out[blockIdx.x] = m;
+            uint32_t dst;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(dst) : "r"(uint32_t(__cvta_generic_to_shared(&of_block[blockIdx.x]))));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(m) : "memory");
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (blockIdx.x == 0 && threadIdx.x == 0)
+        {
+            float r = of_block[0];
+#pragma unroll
+            for (int b = 1; b < EXTREME_CLUSTER; ++b)
+                r = extreme_of<OP == B200_REDUCE_MAX_ABS ? int(B200_REDUCE_MAX) : OP>(r, of_block[b]);
+            out[0] = r;
         }
     }
 
-    // Whole-tensor max (one output): many blocks, each over a contiguous slice, combined with an atomic on the ordered
-    // integer image of the float (non-negative floats order like signed ints, negative ones like reversed unsigned
-    // ints).  NaNs never win, as in the reference loop; the output must hold -inf on entry.
-    template <bool ABS> // the max of |x|: op::v0::Max over op::v0::Abs without the tensor in between
-    __global__ void __launch_bounds__(256) reduce_max_all_kernel(const float* __restrict__ in, float* __restrict__ out, int64_t n)
+    // Larger tensors: many blocks, each over a slice, combined with an atomic on the ordered integer image of the float
+    // (non-negative floats order like signed ints, negative ones like reversed unsigned ints); the output must hold the
+    // starting value on entry.  Bound by HBM.
+    template <int OP>
+    __global__ void __launch_bounds__(256) reduce_extreme_all_kernel(const float* __restrict__ in, float* __restrict__ out, int64_t n)
     {
         __shared__ float partial[8];
-        float m = -INFINITY;
-        for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-        {
-            const float x = ABS ? fabsf(in[i]) : in[i];
-            if (x > m)
-                m = x;
-        }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1)
-        {
-            const float o = __shfl_xor_sync(0xffffffffu, m, d);
-            if (o > m)
-                m = o;
-        }
-        if ((threadIdx.x & 31) == 0)
-            partial[threadIdx.x >> 5] = m;
-        __syncthreads();
+        const float m = extreme_of_block<OP>(extreme_of_run<OP>(in, n, int64_t(blockIdx.x) * 256 + threadIdx.x, int64_t(gridDim.x) * 256), partial);
         if (threadIdx.x == 0)
         {
-            for (int w = 1; w < 8; ++w)
-                if (partial[w] > m)
-                    m = partial[w];
-            if (m >= 0.0f)
-                atomicMax(reinterpret_cast<int*>(out), __float_as_int(m));
-            else if (m > -INFINITY)
-                atomicMin(reinterpret_cast<unsigned int*>(out), __float_as_uint(m));
+            int* const as_int = reinterpret_cast<int*>(out);
+            unsigned int* const as_uint = reinterpret_cast<unsigned int*>(out);
+            if (__float_as_int(m) < 0) // -0.0 included: below +0.0 in the image, equal as a value
+                OP == B200_REDUCE_MIN ? atomicMax(as_uint, __float_as_uint(m)) : atomicMin(as_uint, __float_as_uint(m));
+            else
+                OP == B200_REDUCE_MIN ? atomicMin(as_int, __float_as_int(m)) : atomicMax(as_int, __float_as_int(m));
         }
     }
 
@@ -979,19 +1022,41 @@ extern "C" int b200_reduce_f32(int op, const float* in, float* out, const int64_
     if (!out || (!in && n_red > 0))
         return B200_ERR_INVALID_ARGUMENT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const bool any_max = op == B200_REDUCE_MAX || op == B200_REDUCE_MAX_ABS;
-    if (any_max && n_out == 1 && n_red >= (int64_t(1) << 16))
+    if (op != B200_REDUCE_SUM && n_out == 1 && n_red > 0)
     {
-        // every axis reduced: the input is one contiguous run
-        fill_f32_kernel<<<1, 32, 0, st>>>(out, -INFINITY, 1);
-        if (op == B200_REDUCE_MAX_ABS)
-            reduce_max_all_kernel<true><<<grid_for(n_red / 4, 256), 256, 0, st>>>(in, out, n_red);
-        else
-            reduce_max_all_kernel<false><<<grid_for(n_red / 4, 256), 256, 0, st>>>(in, out, n_red);
-        g_launches.fetch_add(1, std::memory_order_relaxed);
+        // every axis reduced: the input is one contiguous run.  Up to a million elements one cluster reads it about as fast
+        // as the extra launch of the atomic form takes.
+        const bool small = n_red <= (int64_t(1) << 20);
+        if (!small)
+        {
+            fill_f32_kernel<<<1, 32, 0, st>>>(out, op == B200_REDUCE_MIN ? INFINITY : -INFINITY, 1);
+            g_launches.fetch_add(1, std::memory_order_relaxed);
+        }
+        const unsigned grid = small ? EXTREME_CLUSTER : unsigned(std::min<int64_t>((n_red + 8191) / 8192, sm_count() * 8));
+        switch (op)
+        {
+        case B200_REDUCE_MAX:
+            small ? reduce_extreme_cluster_kernel<B200_REDUCE_MAX><<<grid, 1024, 0, st>>>(in, out, n_red)
+                  : reduce_extreme_all_kernel<B200_REDUCE_MAX><<<grid, 256, 0, st>>>(in, out, n_red);
+            break;
+        case B200_REDUCE_MIN:
+            small ? reduce_extreme_cluster_kernel<B200_REDUCE_MIN><<<grid, 1024, 0, st>>>(in, out, n_red)
+                  : reduce_extreme_all_kernel<B200_REDUCE_MIN><<<grid, 256, 0, st>>>(in, out, n_red);
+            break;
+        default:
+            small ? reduce_extreme_cluster_kernel<B200_REDUCE_MAX_ABS><<<grid, 1024, 0, st>>>(in, out, n_red)
+                  : reduce_extreme_all_kernel<B200_REDUCE_MAX_ABS><<<grid, 256, 0, st>>>(in, out, n_red);
+        }
     }
-    else if (op == B200_REDUCE_MAX && n_out <= 4096 && n_red >= 1024)
-        reduce_max_block_kernel<<<unsigned(n_out), 256, 0, st>>>(in, out, keep, red, n_red);
+    else if (op != B200_REDUCE_SUM && n_out <= 4096 && n_red >= 1024)
+    {
+        if (op == B200_REDUCE_MAX)
+            reduce_extreme_block_kernel<B200_REDUCE_MAX><<<unsigned(n_out), 256, 0, st>>>(in, out, keep, red, n_red);
+        else if (op == B200_REDUCE_MIN)
+            reduce_extreme_block_kernel<B200_REDUCE_MIN><<<unsigned(n_out), 256, 0, st>>>(in, out, keep, red, n_red);
+        else
+            reduce_extreme_block_kernel<B200_REDUCE_MAX_ABS><<<unsigned(n_out), 256, 0, st>>>(in, out, keep, red, n_red);
+    }
     else if (op == B200_REDUCE_SUM && n_axes == 1 && axes[0] == rank - 1 && n_out >= 64)
     {
         // the last axis of a matrix with many rows: panels staged through shared memory

@@ -283,3 +283,27 @@ def test_bmm_tile_edges(L, batch, m, k, n):
     ad, bd = dev(a), dev(b)
     L.check(L.LIB.b200_bmm_f32(ad.data_ptr(), bd.data_ptr(), out.data_ptr(), batch, m, k, n, stream()), "bmm")
     np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(acc.astype(np.float32)))
+
+
+@pytest.mark.parametrize("n", [1, 3, 1023, 65535, 65536, (1 << 20) - 1, 1 << 20, (1 << 20) + 1, 3000001])
+def test_extremes_of_a_whole_tensor(L, n):
+    """Max, Min and Max over Abs of every element: the cluster form and the atomic form, runs that do not start on 16 bytes,
+    negative results, NaNs that never win"""
+    rng = np.random.default_rng(n)
+    buf = torch.empty(n + 1, device="cuda")
+    out = torch.empty(1, device="cuda")
+    for off in (0, 1):
+        for sign in (0, 1, -1):
+            x = rng.standard_normal(n).astype(np.float32)
+            x = x if sign == 0 else np.float32(sign) * (np.abs(x) + np.float32(0.5))
+            if n > 2:
+                x[n // 2] = np.nan
+            xd = buf[off:off + n]
+            xd.copy_(dev(x))
+            for op, want in ((1, np.nanmax(x)), (2, np.nanmin(x)), (3, np.nanmax(np.abs(x)))):
+                L.check(L.LIB.b200_reduce_f32(op, xd.data_ptr(), out.data_ptr(), i64([n]), 1, i64([0]), 1, stream()), "reduce")
+                assert out.item() == want, (op, off, sign)
+    buf.fill_(float("nan"))
+    for op, want in ((1, -np.inf), (2, np.inf), (3, -np.inf)):
+        L.check(L.LIB.b200_reduce_f32(op, buf.data_ptr(), out.data_ptr(), i64([n]), 1, i64([0]), 1, stream()), "reduce")
+        assert out.item() == want
