@@ -4,7 +4,8 @@
 //   elementwise +, -, *, /, max, min, abs, neg, sqrt, relu   IEEE single, one rounding each, nothing contracted
 //   exp, erf                                                   reference: std::exp / std::erf on float; here the double
 //                                                              routine rounded to float (differs from a given libm in
-//                                                              the last bit on a small share of inputs)
+//                                                              the last bit on a small share of inputs), computed in
+//                                                              single precision with a rounding test (rounded_math.cuh)
 //   Sum          runtime/reference/sum.hpp:56-90     Kahan-compensated, inputs taken in row-major order
 //   Max          runtime/reference/max.hpp:32-58     start at -inf, replace when x > max
 //   Broadcast    runtime/reference/broadcast.hpp     output coordinate with the broadcast axes dropped
@@ -20,6 +21,7 @@
 #include <algorithm>
 #include <initializer_list>
 #include "common.cuh"
+#include "rounded_math.cuh"
 
 namespace b200
 {
@@ -355,136 +357,209 @@ namespace b200
     }
 
     // Softmax and LayerNorm over the LAST axis of a [rows, L] matrix.  Their compensated sums have to walk a row in
-    // order, so a row belongs to one thread; reading it straight from memory would make the 32 lanes of a warp touch 32
-    // different rows per load.  A block therefore stages 32 rows in shared memory, lets all its threads do the
-    // order-free parts (max, exp, normalise, divide) and one warp the 32 ordered sums, one row per lane.
-    // VEC: L is a multiple of 4 and the pointers are 16-byte aligned, so rows move as float4 with eight loads in flight
-    // per thread (row stride L + 4: the ordered walks then meet 4-way bank conflicts, hidden behind the dependent
-    // additions); otherwise element by element with an odd row stride.
-    constexpr int ROWS_PER_TILE = 32;
+    // order, so a row belongs to one thread; reading it straight from memory would make the lanes of a warp touch as many
+    // different rows per load.  A block therefore stages R rows in shared memory, lets all its threads do the order-free
+    // parts (max, exp, normalise, divide) and the first R lanes of one warp the ordered sums, one row per lane.
+    //
+    // What bounds them is the chain of a compensated sum, four dependent additions (16 clocks) per element, against the rows
+    // an SM can hold: so the tiles are small (many blocks per SM, one block's chain under another's loads and stores), the
+    // walk reads four elements ahead, and the test for infinities is made once per row on the result (see kahan_row).
+    // VEC: L is a multiple of 4 and the pointers are 16-byte aligned, so rows move as float4 (row stride L + 4: for the
+    // usual lengths the lanes' 16-byte walks meet no bank twice); otherwise element by element with an odd row stride.
     __host__ __device__ inline int staged_row_stride(int L, bool vec) { return vec ? L + 4 : (L | 1); }
 
-    // The elementwise op that produced the rows can be applied while they are staged (one rounding, the same value the
-    // op's own kernel would have written): factor != nullptr multiplies by the scalar *factor (op::v1::Multiply by a
-    // broadcast scalar), addend != nullptr adds the rows of a second tensor (op::v1::Add).
-    template <bool VEC>
-    __device__ __forceinline__ void stage_rows(const float* __restrict__ src, float* tile, int n_rows, int L, int stride,
-                                               const float* __restrict__ factor, const float* __restrict__ addend)
+    // The compensated sum of f(row[0]), f(row[1]), ...  The reference leaves the compensation out wherever an element or the
+    // running sum is not finite; such a sum never becomes finite again, so a finite result of the plain chain means that no
+    // such element was met, and only the others are walked a second time with the test.
+    template <bool VEC, typename F>
+    __device__ __forceinline__ float kahan_row(const float* row, int L, F f)
     {
-        const float f = factor ? __ldg(factor) : 1.0f;
+        float z = 0.0f, c = 0.0f;
+        auto step = [&](float x) {
+            const float y = __fsub_rn(x, c), t = __fadd_rn(z, y);
+            c = __fsub_rn(__fsub_rn(t, z), y);
+            z = t;
+        };
         if (VEC)
         {
-            const int L4 = L >> 2, total = n_rows * L4;
-            const float4* src4 = reinterpret_cast<const float4*>(src);
-            const float4* add4 = reinterpret_cast<const float4*>(addend);
-            for (int i0 = threadIdx.x; i0 < total; i0 += blockDim.x * 8)
+            const float4* row4 = reinterpret_cast<const float4*>(row);
+            float4 v = row4[0];
+#pragma unroll 4
+            for (int k = 0; k < L / 4; ++k)
             {
-                float4 v[8], w[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                {
-                    const int i = i0 + j * blockDim.x;
-                    if (i < total)
-                    {
-                        v[j] = __ldg(src4 + i);
-                        if (addend)
-                            w[j] = __ldg(add4 + i);
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                {
-                    const int i = i0 + j * blockDim.x;
-                    if (i < total)
-                    {
-                        float4 r = v[j];
-                        if (factor)
-                            r = make_float4(__fmul_rn(r.x, f), __fmul_rn(r.y, f), __fmul_rn(r.z, f), __fmul_rn(r.w, f));
-                        if (addend)
-                            r = make_float4(__fadd_rn(r.x, w[j].x), __fadd_rn(r.y, w[j].y), __fadd_rn(r.z, w[j].z), __fadd_rn(r.w, w[j].w));
-                        *reinterpret_cast<float4*>(tile + (i / L4) * stride + 4 * (i % L4)) = r;
-                    }
-                }
+                const float4 next = row4[k + 1]; // the row's padding at the end
+                step(f(v.x)), step(f(v.y)), step(f(v.z)), step(f(v.w));
+                v = next;
             }
         }
         else
-            for (int i = threadIdx.x; i < n_rows * L; i += blockDim.x)
-            {
-                float r = src[i];
-                if (factor)
-                    r = __fmul_rn(r, f);
-                if (addend)
-                    r = __fadd_rn(r, addend[i]);
-                tile[(i / L) * stride + i % L] = r;
-            }
+        {
+#pragma unroll 8
+            for (int k = 0; k < L; ++k)
+                step(f(row[k]));
+        }
+        if (!isfinite(z))
+        {
+            z = 0.0f, c = 0.0f;
+            for (int k = 0; k < L; ++k)
+                kahan_step(z, c, f(row[k]));
+        }
+        return z;
     }
 
-    template <bool VEC>
-    __global__ void __launch_bounds__(128) softmax_rows_kernel(const float* __restrict__ in, const float* __restrict__ factor, float* __restrict__ out,
-                                                               int64_t rows, int L)
+    // x / d where y = RN(1 / d) if d admits it (scale_allows_fast_division), else y = 0: the correctly rounded quotient, by two
+    // multiply-adds unless x is so small that a step could underflow.
+    __device__ __forceinline__ float divide_by(float x, float d, float y)
     {
+        const float q0 = __fmul_rn(x, y), q = __fmaf_rn(__fmaf_rn(-q0, d, x), y, q0);
+        // the admitted divisors lie in [2^-40, 2^41): nothing overflows below 2^80
+        return (y != 0.0f && fabsf(x) > 8.673617379884035e-19f && fabsf(x) < 1.2089258e24f) ? q : __fdiv_rn(x, d);
+    }
+    __device__ __forceinline__ float4 divide4_by(const float4& x, float d, float y)
+    {
+        const float lo = fminf(fminf(fabsf(x.x), fabsf(x.y)), fminf(fabsf(x.z), fabsf(x.w)));
+        const float hi = fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w)));
+        auto quotient = [d, y](float v) {
+            const float q0 = __fmul_rn(v, y);
+            return __fmaf_rn(__fmaf_rn(-q0, d, v), y, q0);
+        };
+        if (y != 0.0f && lo > 8.673617379884035e-19f && hi < 1.2089258e24f) // a NaN beside usable neighbours stays one
+            return make_float4(quotient(x.x), quotient(x.y), quotient(x.z), quotient(x.w));
+        return make_float4(__fdiv_rn(x.x, d), __fdiv_rn(x.y, d), __fdiv_rn(x.z, d), __fdiv_rn(x.w, d));
+    }
+    __device__ __forceinline__ float reciprocal_if_exact(float d) { return scale_allows_fast_division(d) ? __frcp_rn(d) : 0.0f; }
+
+    // The elementwise op that produced the rows can be applied while they are staged (one rounding, the same value the
+    // op's own kernel would have written): factor multiplies by the scalar *factor (op::v1::Multiply by a broadcast
+    // scalar), addend adds the rows of a second tensor (op::v1::Add).
+    constexpr int SOFTMAX_ROWS = 16, SOFTMAX_THREADS = 256, NORM_ROWS = 8, ROW_THREADS = 128;
+
+    // NV > 0 (VEC only): rows of at most 128 * NV elements stay in registers between the steps, NV float4 per lane and row,
+    // and shared memory holds only what the ordered sums walk; NV == 0: any length, in shared memory throughout.
+    // 294912 rows of 384: 602 -> 266 us (906 MB: 139 us at the copy rate), bound by the chains and the instructions of exp.
+    template <bool VEC, bool FACTOR, int NV>
+    __global__ void __launch_bounds__(SOFTMAX_THREADS) softmax_rows_kernel(const float* __restrict__ in, const float* __restrict__ factor,
+                                                                           float* __restrict__ out, int64_t rows, int L)
+    {
+        constexpr int R = SOFTMAX_ROWS, WARPS = SOFTMAX_THREADS / 32, OWN = R / WARPS;
         extern __shared__ __align__(16) float tile[];
-        __shared__ float row_max[ROWS_PER_TILE], row_sum[ROWS_PER_TILE];
-        const int stride = staged_row_stride(L, VEC);
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int64_t n_tiles = (rows + ROWS_PER_TILE - 1) / ROWS_PER_TILE;
-        for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x)
+        __shared__ double exp_table[rounded::EXP_STEPS];
+        __shared__ float row_sum[R];
+        rounded::load_exp_table(exp_table);
+        const int stride = staged_row_stride(L, VEC), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int64_t row0 = int64_t(blockIdx.x) * R;
+        const int n_rows = int(min(rows - row0, int64_t(R)));
+        const float f = FACTOR ? __ldg(factor) : 1.0f;
+        in += row0 * L;
+        out += row0 * L;
+        // a warp owns rows warp, warp + 8 of the tile: their loads are under way together, their maxima stay in registers.
+        // Rows beyond the last one of the matrix read that one again and store nothing.
+        const float* src[OWN];
+        float* row[OWN];
+        float row_max[OWN];
+        float4 v[OWN][NV > 0 ? NV : 1];
+#pragma unroll
+        for (int i = 0; i < OWN; ++i)
         {
-            const int64_t row0 = t * ROWS_PER_TILE;
-            const int n_rows = int(rows - row0 < ROWS_PER_TILE ? rows - row0 : ROWS_PER_TILE);
-            stage_rows<VEC>(in + row0 * L, tile, n_rows, L, stride, factor, nullptr);
-            __syncthreads();
-            // softmax.hpp: max over the axis (the largest value whatever the order), then exp(x - max)
-            for (int r = warp; r < n_rows; r += 4)
+            src[i] = in + int64_t(min(warp + i * WARPS, n_rows - 1)) * L;
+            row[i] = tile + (warp + i * WARPS) * stride;
+            row_max[i] = -INFINITY;
+        }
+        auto scaled = [f](float4 x) {
+            return FACTOR ? make_float4(__fmul_rn(x.x, f), __fmul_rn(x.y, f), __fmul_rn(x.z, f), __fmul_rn(x.w, f)) : x;
+        };
+        auto max4 = [](float m, const float4& x) { return fmaxf(fmaxf(m, fmaxf(x.x, x.y)), fmaxf(x.z, x.w)); }; // a NaN never wins
+        if (NV > 0)
+        {
+#pragma unroll
+            for (int i = 0; i < OWN; ++i)
+#pragma unroll
+                for (int j = 0; j < NV; ++j)
+                    if (4 * lane + 128 * j < L)
+                        v[i][j] = __ldg(reinterpret_cast<const float4*>(src[i] + 4 * lane + 128 * j));
+#pragma unroll
+            for (int i = 0; i < OWN; ++i)
+#pragma unroll
+                for (int j = 0; j < NV; ++j)
+                    if (4 * lane + 128 * j < L)
+                        row_max[i] = max4(row_max[i], v[i][j] = scaled(v[i][j]));
+        }
+        else if (VEC)
+            for (int c = 4 * lane; c < L; c += 128)
             {
-                float m = -INFINITY;
-                for (int c = lane; c < L; c += 32)
+                float4 x[OWN];
+#pragma unroll
+                for (int i = 0; i < OWN; ++i)
+                    x[i] = __ldg(reinterpret_cast<const float4*>(src[i] + c));
+#pragma unroll
+                for (int i = 0; i < OWN; ++i)
                 {
-                    const float x = tile[r * stride + c];
-                    m = x > m ? x : m;
-                }
-                for (int d = 16; d; d >>= 1)
-                {
-                    const float o = __shfl_xor_sync(0xFFFFFFFFu, m, d);
-                    m = o > m ? o : m;
-                }
-                // the same warp owns the row in the next step too, so no block-wide barrier is needed in between
-                for (int c = lane; c < L; c += 32)
-                {
-                    float& v = tile[r * stride + c];
-                    v = static_cast<float>(exp(static_cast<double>(__fsub_rn(v, m))));
+                    *reinterpret_cast<float4*>(row[i] + c) = x[i] = scaled(x[i]);
+                    row_max[i] = max4(row_max[i], x[i]);
                 }
             }
-            __syncthreads();
-            if (warp == 0 && lane < n_rows)
-            {
-                const float* row = tile + lane * stride;
-                float z = 0.0f, c = 0.0f;
-                for (int k = 0; k < L; ++k)
-                    kahan_step(z, c, row[k]);
-                row_sum[lane] = z;
-            }
-            __syncthreads();
-            float* dst = out + row0 * L;
-            if (VEC)
-            {
-                const int L4 = L >> 2, total = n_rows * L4;
-                for (int i = threadIdx.x; i < total; i += blockDim.x)
+        else
+            for (int c = lane; c < L; c += 32)
+#pragma unroll
+                for (int i = 0; i < OWN; ++i)
                 {
-                    const int r = i / L4;
-                    float4 v = *reinterpret_cast<const float4*>(tile + r * stride + 4 * (i % L4));
-                    const float sum = row_sum[r];
-                    v.x = __fdiv_rn(v.x, sum), v.y = __fdiv_rn(v.y, sum), v.z = __fdiv_rn(v.z, sum), v.w = __fdiv_rn(v.w, sum);
-                    reinterpret_cast<float4*>(dst)[i] = v;
+                    const float x = FACTOR ? __fmul_rn(src[i][c], f) : src[i][c];
+                    row[i][c] = x;
+                    row_max[i] = fmaxf(row_max[i], x);
                 }
+#pragma unroll
+        for (int i = 0; i < OWN; ++i)
+#pragma unroll
+            for (int d = 16; d; d >>= 1)
+                row_max[i] = fmaxf(row_max[i], __shfl_xor_sync(0xFFFFFFFFu, row_max[i], d));
+        __syncthreads(); // the exp table
+        // softmax.hpp: exp(x - max); every element is read back by the lane that stored it
+#pragma unroll
+        for (int i = 0; i < OWN; ++i)
+        {
+            const float m = row_max[i];
+            auto exp4 = [&](const float4& x) {
+                return make_float4(rounded::exp_rounded(__fsub_rn(x.x, m), exp_table), rounded::exp_rounded(__fsub_rn(x.y, m), exp_table),
+                                   rounded::exp_rounded(__fsub_rn(x.z, m), exp_table), rounded::exp_rounded(__fsub_rn(x.w, m), exp_table));
+            };
+            if (NV > 0)
+            {
+#pragma unroll
+                for (int j = 0; j < NV; ++j)
+                    if (4 * lane + 128 * j < L)
+                        *reinterpret_cast<float4*>(row[i] + 4 * lane + 128 * j) = v[i][j] = exp4(v[i][j]);
             }
+            else if (VEC)
+                for (int c = 4 * lane; c < L; c += 128)
+                    *reinterpret_cast<float4*>(row[i] + c) = exp4(*reinterpret_cast<float4*>(row[i] + c));
             else
-                for (int i = threadIdx.x; i < n_rows * L; i += blockDim.x)
-                {
-                    const int r = i / L;
-                    dst[i] = __fdiv_rn(tile[r * stride + i % L], row_sum[r]);
-                }
-            __syncthreads();
+                for (int c = lane; c < L; c += 32)
+                    row[i][c] = rounded::exp_rounded(__fsub_rn(row[i][c], m), exp_table);
+        }
+        __syncthreads();
+        if (threadIdx.x < R)
+            row_sum[threadIdx.x] = kahan_row<VEC>(tile + threadIdx.x * stride, L, [](float x) { return x; });
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < OWN; ++i)
+        {
+            if (warp + i * WARPS >= n_rows)
+                break;
+            const float sum = row_sum[warp + i * WARPS], y = reciprocal_if_exact(sum);
+            float* dst = out + int64_t(warp + i * WARPS) * L;
+            if (NV > 0)
+            {
+#pragma unroll
+                for (int j = 0; j < NV; ++j)
+                    if (4 * lane + 128 * j < L)
+                        *reinterpret_cast<float4*>(dst + 4 * lane + 128 * j) = divide4_by(v[i][j], sum, y);
+            }
+            else if (VEC)
+                for (int c = 4 * lane; c < L; c += 128)
+                    *reinterpret_cast<float4*>(dst + c) = divide4_by(*reinterpret_cast<const float4*>(row[i] + c), sum, y);
+            else
+                for (int c = lane; c < L; c += 32)
+                    dst[c] = divide_by(row[i][c], sum, y);
         }
     }
 
@@ -493,78 +568,128 @@ namespace b200
     // src/ngraph/builder/reduce_ops.cpp:68-127), in that order:
     //   mean = KahanSum(x) / N;  var = KahanSum((x - mean) * (x - mean)) / N;  sd = sqrt(var + eps);
     //   y = ((x - mean) / sd) * gamma + beta          (every operation a separate IEEE rounding, no fused multiply-add)
-    template <bool VEC>
-    __global__ void __launch_bounds__(128) layer_norm_rows_kernel(const float* __restrict__ in, const float* __restrict__ addend,
-                                                                  const float* __restrict__ gamma, const float* __restrict__ beta,
-                                                                  float* __restrict__ out, int64_t rows, int L, float count, float eps)
+    // 24576 rows of 768: 197 -> 88 us (226 MB: 35 us); 128 rows: 60 -> 21 us, of which the two chains are 13.
+    template <bool VEC, bool ADDEND>
+    __global__ void __launch_bounds__(ROW_THREADS) layer_norm_rows_kernel(const float* __restrict__ in, const float* __restrict__ addend,
+                                                                          const float* __restrict__ gamma, const float* __restrict__ beta,
+                                                                          float* __restrict__ out, int64_t rows, int L, float count, float eps,
+                                                                          int64_t ahead)
     {
+        constexpr int R = NORM_ROWS, WARPS = ROW_THREADS / 32;
         extern __shared__ __align__(16) float tile[];
-        __shared__ float row_mean[ROWS_PER_TILE], row_sd[ROWS_PER_TILE];
-        const int stride = staged_row_stride(L, VEC);
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int64_t n_tiles = (rows + ROWS_PER_TILE - 1) / ROWS_PER_TILE;
-        for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x)
+        __shared__ float row_mean[R], row_sd[R];
+        const int stride = staged_row_stride(L, VEC), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int64_t row0 = int64_t(blockIdx.x) * R;
+        const int n_rows = int(min(rows - row0, int64_t(R)));
+        in += row0 * L;
+        out += row0 * L;
+        if (ADDEND)
+            addend += row0 * L;
+        for (int r = warp; r < n_rows; r += WARPS)
         {
-            const int64_t row0 = t * ROWS_PER_TILE;
-            const int n_rows = int(rows - row0 < ROWS_PER_TILE ? rows - row0 : ROWS_PER_TILE);
-            stage_rows<VEC>(in + row0 * L, tile, n_rows, L, stride, nullptr, addend ? addend + row0 * L : nullptr);
-            __syncthreads();
-            if (warp == 0 && lane < n_rows)
-            {
-                const float* row = tile + lane * stride;
-                float z = 0.0f, c = 0.0f;
-                for (int k = 0; k < L; ++k)
-                    kahan_step(z, c, row[k]);
-                const float mean = __fdiv_rn(z, count);
-                z = 0.0f, c = 0.0f;
-                for (int k = 0; k < L; ++k)
-                {
-                    const float d = __fsub_rn(row[k], mean);
-                    kahan_step(z, c, __fmul_rn(d, d));
-                }
-                row_mean[lane] = mean;
-                row_sd[lane] = __fsqrt_rn(__fadd_rn(__fdiv_rn(z, count), eps));
-            }
-            __syncthreads();
-            float* dst = out + row0 * L;
             if (VEC)
             {
-                const int L4 = L >> 2, total = n_rows * L4;
-                for (int i = threadIdx.x; i < total; i += blockDim.x)
+                const float4* x4 = reinterpret_cast<const float4*>(in + int64_t(r) * L);
+                const float4* a4 = reinterpret_cast<const float4*>(addend + int64_t(r) * L);
+#pragma unroll 4
+                for (int c = lane; c < L / 4; c += 32)
                 {
-                    const int r = i / L4, k4 = i % L4;
-                    float4 v = *reinterpret_cast<const float4*>(tile + r * stride + 4 * k4);
-                    const float4 g = __ldg(reinterpret_cast<const float4*>(gamma) + k4), b = __ldg(reinterpret_cast<const float4*>(beta) + k4);
-                    const float mean = row_mean[r], sd = row_sd[r];
-                    v.x = __fadd_rn(__fmul_rn(__fdiv_rn(__fsub_rn(v.x, mean), sd), g.x), b.x);
-                    v.y = __fadd_rn(__fmul_rn(__fdiv_rn(__fsub_rn(v.y, mean), sd), g.y), b.y);
-                    v.z = __fadd_rn(__fmul_rn(__fdiv_rn(__fsub_rn(v.z, mean), sd), g.z), b.z);
-                    v.w = __fadd_rn(__fmul_rn(__fdiv_rn(__fsub_rn(v.w, mean), sd), g.w), b.w);
-                    reinterpret_cast<float4*>(dst)[i] = v;
+                    float4 v = __ldg(x4 + c);
+                    if (ADDEND)
+                    {
+                        const float4 w = __ldg(a4 + c);
+                        v = make_float4(__fadd_rn(v.x, w.x), __fadd_rn(v.y, w.y), __fadd_rn(v.z, w.z), __fadd_rn(v.w, w.w));
+                    }
+                    *reinterpret_cast<float4*>(tile + r * stride + 4 * c) = v;
                 }
             }
             else
-                for (int i = threadIdx.x; i < n_rows * L; i += blockDim.x)
+                for (int c = lane; c < L; c += 32)
+                    tile[r * stride + c] = ADDEND ? __fadd_rn(in[int64_t(r) * L + c], addend[int64_t(r) * L + c]) : in[int64_t(r) * L + c];
+        }
+        __syncthreads();
+        if (threadIdx.x < n_rows)
+        {
+            const float* row = tile + threadIdx.x * stride;
+            const float mean = __fdiv_rn(kahan_row<VEC>(row, L, [](float x) { return x; }), count);
+            const float var = __fdiv_rn(kahan_row<VEC>(row, L,
+                                                       [mean](float x) {
+                                                           const float d = __fsub_rn(x, mean);
+                                                           return __fmul_rn(d, d);
+                                                       }),
+                                        count);
+            row_mean[threadIdx.x] = mean;
+            row_sd[threadIdx.x] = __fsqrt_rn(__fadd_rn(var, eps));
+        }
+        else if (warp > 0)
+        {
+            // the other warps have nothing to do: they bring the rows of the tile that follows this one on the SM into L2, whose
+            // loads would otherwise all start when the chains of a whole wave of blocks have ended
+            const int64_t first = row0 + ahead, last = min(first + R, rows);
+            const char* p[2] = {reinterpret_cast<const char*>(in + ahead * L), reinterpret_cast<const char*>(ADDEND ? addend + ahead * L : nullptr)};
+            for (int64_t i = int64_t(threadIdx.x - 32) * 128; first < last && i < (last - first) * L * 4; i += (ROW_THREADS - 32) * 128)
+            {
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(p[0] + i));
+                if (ADDEND)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(p[1] + i));
+            }
+        }
+        __syncthreads();
+        for (int r = warp; r < n_rows; r += WARPS)
+        {
+            const float mean = row_mean[r], sd = row_sd[r], y = reciprocal_if_exact(sd);
+            if (VEC)
+#pragma unroll 2
+                for (int c = lane; c < L / 4; c += 32)
                 {
-                    const int r = i / L, k = i % L;
-                    const float norm = __fdiv_rn(__fsub_rn(tile[r * stride + k], row_mean[r]), row_sd[r]);
-                    dst[i] = __fadd_rn(__fmul_rn(norm, __ldg(gamma + k)), __ldg(beta + k));
+                    float4 v = *reinterpret_cast<const float4*>(tile + r * stride + 4 * c);
+                    const float4 g = __ldg(reinterpret_cast<const float4*>(gamma) + c), b = __ldg(reinterpret_cast<const float4*>(beta) + c);
+                    v = divide4_by(make_float4(__fsub_rn(v.x, mean), __fsub_rn(v.y, mean), __fsub_rn(v.z, mean), __fsub_rn(v.w, mean)), sd, y);
+                    v.x = __fadd_rn(__fmul_rn(v.x, g.x), b.x), v.y = __fadd_rn(__fmul_rn(v.y, g.y), b.y);
+                    v.z = __fadd_rn(__fmul_rn(v.z, g.z), b.z), v.w = __fadd_rn(__fmul_rn(v.w, g.w), b.w);
+                    reinterpret_cast<float4*>(out + int64_t(r) * L)[c] = v;
                 }
-            __syncthreads();
+            else
+                for (int c = lane; c < L; c += 32)
+                    out[int64_t(r) * L + c] =
+                        __fadd_rn(__fmul_rn(divide_by(__fsub_rn(tile[r * stride + c], mean), sd, y), __ldg(gamma + c)), __ldg(beta + c));
         }
     }
 
     // op::v0::Gelu with the rounding steps of its decomposition (src/ngraph/op/gelu.cpp:46-60):
     //   (0.5 * x) * (1 + erf(x / float(sqrt(2.0))))
-    __global__ void __launch_bounds__(256) gelu_kernel(const float* __restrict__ x, float* __restrict__ out, int64_t n)
+    // 75 million elements: 358 -> 130 us (604 MB: 92 us), bound by the table lookups' bank conflicts beside HBM.
+    // The quotient by the constant is two multiply-adds (see divide_by; where they underflow, erf vanishes against 1).
+    __device__ __forceinline__ float gelu_of(float v, const rounded::ErfPoint* table)
     {
-        const float sqrt_two = static_cast<float>(1.4142135623730951);
-        for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
+        constexpr float sqrt_two = 1.4142135623730951f, inv = 0.70710677f; // RN(1 / sqrt_two)
+        const float q0 = __fmul_rn(v, inv), q = __fmaf_rn(__fmaf_rn(-q0, sqrt_two, v), inv, q0);
+        const float e = copysignf(rounded::erf_abs(fabsf(q), table), v);
+        return __fmul_rn(__fmul_rn(0.5f, v), __fadd_rn(1.0f, e));
+    }
+    template <bool VEC>
+    __global__ void __launch_bounds__(256, 6) gelu_kernel(const float* __restrict__ x, float* __restrict__ out, int64_t n)
+    {
+        __shared__ __align__(16) rounded::ErfPoint table[rounded::ERF_ENTRIES];
+        rounded::load_erf_table(table);
+        __syncthreads();
+        const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, threads = int64_t(gridDim.x) * blockDim.x;
+        if (VEC)
         {
-            const float v = x[i];
-            const float e = static_cast<float>(erf(static_cast<double>(__fdiv_rn(v, sqrt_two))));
-            out[i] = __fmul_rn(__fmul_rn(0.5f, v), __fadd_rn(1.0f, e));
+            const float4* x4 = reinterpret_cast<const float4*>(x);
+            float4 next = t < n / 4 ? x4[t] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            for (int64_t i = t; i < n / 4; i += threads)
+            {
+                const float4 v = next;
+                next = x4[min(i + threads, n / 4 - 1)]; // under way while this vector is computed
+                reinterpret_cast<float4*>(out)[i] = make_float4(gelu_of(v.x, table), gelu_of(v.y, table), gelu_of(v.z, table), gelu_of(v.w, table));
+            }
+            for (int64_t i = (n / 4) * 4 + t; i < n; i += threads)
+                out[i] = gelu_of(x[i], table);
         }
+        else
+            for (int64_t i = t; i < n; i += threads)
+                out[i] = gelu_of(x[i], table);
     }
 
     // Sum over the last axis for rows of any length: a warp owns 32 rows, one per lane, and walks them 64 columns at a
@@ -610,17 +735,18 @@ namespace b200
         }
     }
 
-    // Grid and shared memory of the two staged kernels: as many 32-row tiles per SM as fit.
+    // Shared memory of the two staged kernels; above 48 KB a kernel has to be told once per device.
     template <typename Kernel>
-    bool staged_launch_shape(Kernel kernel, int64_t rows, int L, bool vec, unsigned& grid, size_t& bytes)
+    bool staged_bytes(Kernel kernel, std::atomic<uint64_t>& told, int rows, int L, bool vec, size_t& bytes)
     {
-        bytes = size_t(ROWS_PER_TILE) * staged_row_stride(L, vec) * sizeof(float);
-        if (bytes > 48 * 1024 && // the attribute belongs to the current device's copy of the kernel: set it on each use
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
+        bytes = size_t(rows) * staged_row_stride(L, vec) * sizeof(float);
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (bytes <= 44 * 1024 /* and the static arrays */ || ((told.load(std::memory_order_relaxed) >> (dev & 63)) & 1))
+            return true;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) != cudaSuccess)
             return false;
-        const int64_t tiles = (rows + ROWS_PER_TILE - 1) / ROWS_PER_TILE;
-        const int64_t per_sm = (200 * 1024) / int64_t(bytes) < 8 ? (200 * 1024) / int64_t(bytes) : 8;
-        grid = unsigned(tiles < b200::sm_count() * per_sm ? tiles : b200::sm_count() * per_sm);
+        told.fetch_or(uint64_t(1) << (dev & 63), std::memory_order_relaxed);
         return true;
     }
 
@@ -1094,15 +1220,33 @@ extern "C" int b200_softmax_rows_scaled_f32(const float* x, const float* factor,
     const int L = int(row_elements);
     const bool vec = L % 4 == 0 && all_aligned16({x, out});
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    unsigned grid;
-    size_t bytes;
-    if (!(vec ? staged_launch_shape(softmax_rows_kernel<true>, rows, L, vec, grid, bytes)
-              : staged_launch_shape(softmax_rows_kernel<false>, rows, L, vec, grid, bytes)))
+    const int64_t grid = (rows + SOFTMAX_ROWS - 1) / SOFTMAX_ROWS;
+    if (grid > 0x7FFFFFFF)
+        return B200_ERR_TOO_LARGE;
+    auto launch = [&](auto kernel, std::atomic<uint64_t>& told) {
+        size_t bytes;
+        if (!staged_bytes(kernel, told, SOFTMAX_ROWS, L, vec, bytes))
+            return false;
+        kernel<<<unsigned(grid), SOFTMAX_THREADS, bytes, st>>>(x, factor, out, rows, L);
+        return true;
+    };
+    static std::atomic<uint64_t> told[2][6];
+    auto pick = [&](auto with_factor) {
+        constexpr bool F = decltype(with_factor)::value;
+        if (!vec)
+            return launch(softmax_rows_kernel<false, F, 0>, told[F][5]);
+        switch ((L + 127) / 128)
+        {
+        case 1: return launch(softmax_rows_kernel<true, F, 1>, told[F][1]);
+        case 2: return launch(softmax_rows_kernel<true, F, 2>, told[F][2]);
+        case 3: return launch(softmax_rows_kernel<true, F, 3>, told[F][3]);
+        case 4: return launch(softmax_rows_kernel<true, F, 4>, told[F][4]);
+        default: return launch(softmax_rows_kernel<true, F, 0>, told[F][0]);
+        }
+    };
+    const bool ok = factor ? pick(std::true_type()) : pick(std::false_type());
+    if (!ok)
         return B200_ERR_CUDA;
-    if (vec)
-        softmax_rows_kernel<true><<<grid, 128, bytes, st>>>(x, factor, out, rows, L);
-    else
-        softmax_rows_kernel<false><<<grid, 128, bytes, st>>>(x, factor, out, rows, L);
     return after_launch("b200_softmax_rows_f32");
 }
 
@@ -1128,15 +1272,23 @@ extern "C" int b200_layer_norm_rows_sum_f32(const float* x, const float* addend,
     const bool vec = L % 4 == 0 && all_aligned16({x, addend, gamma, beta, out});
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const float count = static_cast<float>(row_elements);
-    unsigned grid;
-    size_t bytes;
-    if (!(vec ? staged_launch_shape(layer_norm_rows_kernel<true>, rows, L, vec, grid, bytes)
-              : staged_launch_shape(layer_norm_rows_kernel<false>, rows, L, vec, grid, bytes)))
+    const int64_t grid = (rows + NORM_ROWS - 1) / NORM_ROWS;
+    if (grid > 0x7FFFFFFF)
+        return B200_ERR_TOO_LARGE;
+    auto launch = [&](auto kernel, std::atomic<uint64_t>& told) {
+        size_t bytes;
+        if (!staged_bytes(kernel, told, NORM_ROWS, L, vec, bytes))
+            return false;
+        // rows that run at the same time: what follows a tile on its SM starts that much further on
+        const int64_t resident = std::min<int64_t>(200 * 1024 / int64_t(bytes + 1024), 2048 / ROW_THREADS);
+        kernel<<<unsigned(grid), ROW_THREADS, bytes, st>>>(x, addend, gamma, beta, out, rows, L, count, epsilon, resident * sm_count() * NORM_ROWS);
+        return true;
+    };
+    static std::atomic<uint64_t> told[4];
+    const bool ok = vec ? (addend ? launch(layer_norm_rows_kernel<true, true>, told[0]) : launch(layer_norm_rows_kernel<true, false>, told[1]))
+                        : (addend ? launch(layer_norm_rows_kernel<false, true>, told[2]) : launch(layer_norm_rows_kernel<false, false>, told[3]));
+    if (!ok)
         return B200_ERR_CUDA;
-    if (vec)
-        layer_norm_rows_kernel<true><<<grid, 128, bytes, st>>>(x, addend, gamma, beta, out, rows, L, count, epsilon);
-    else
-        layer_norm_rows_kernel<false><<<grid, 128, bytes, st>>>(x, addend, gamma, beta, out, rows, L, count, epsilon);
     return after_launch("b200_layer_norm_rows_f32");
 }
 
@@ -1149,7 +1301,14 @@ extern "C" int b200_gelu_f32(const float* x, float* out, int64_t n, void* stream
         return B200_OK;
     if (!x || !out)
         return B200_ERR_INVALID_ARGUMENT;
-    gelu_kernel<<<grid_for(n, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(x, out, n);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const bool vec = all_aligned16({x, out});
+    // blocks that stay (each copies the table first); short tensors get about two vectors per thread
+    const unsigned grid = unsigned(std::min<int64_t>((n + 2047) / 2048, int64_t(sm_count()) * 6));
+    if (vec)
+        gelu_kernel<true><<<grid, 256, 0, st>>>(x, out, n);
+    else
+        gelu_kernel<false><<<grid, 256, 0, st>>>(x, out, n);
     return after_launch("b200_gelu_f32");
 }
 

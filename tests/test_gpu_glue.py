@@ -307,3 +307,49 @@ def test_extremes_of_a_whole_tensor(L, n):
     for op, want in ((1, -np.inf), (2, np.inf), (3, -np.inf)):
         L.check(L.LIB.b200_reduce_f32(op, buf.data_ptr(), out.data_ptr(), i64([n]), 1, i64([0]), 1, stream()), "reduce")
         assert out.item() == want
+
+
+@pytest.mark.parametrize("rows,n", [(33, 4), (17, 128), (16, 132), (15, 256), (31, 260), (64, 384), (5, 388), (18, 512), (9, 516), (1, 1532), (40, 127)])
+def test_row_kernels_at_the_edges_of_their_forms(L, rows, n):
+    """Softmax keeps rows of up to 512 elements in registers (one, two, three, four vectors per lane), longer ones and odd
+    lengths in shared memory; tiles of 16 (Softmax) and 8 (LayerNorm) rows that are not full; values whose quotient or exp
+    is 0, denormal or NaN"""
+    from oracle import glue
+    rng = np.random.default_rng(rows * n)
+    x = (rng.standard_normal((rows, n)) * 5).astype(np.float32)
+    x[0] -= np.linspace(0, 120, n).astype(np.float32)
+    xd, out = dev(x), torch.empty((rows, n), device="cuda")
+    L.check(L.LIB.b200_softmax_rows_f32(xd.data_ptr(), out.data_ptr(), rows, n, stream()), "softmax")
+    want = glue.softmax(x)
+    np.testing.assert_allclose(out.cpu().numpy(), want, rtol=2.4e-7, atol=1.5e-45)
+    assert (bits(out.cpu().numpy()) != bits(want)).mean() < 0.05
+    g, b = rng.standard_normal(n).astype(np.float32), rng.standard_normal(n).astype(np.float32)
+    y = x.copy()
+    y[-1] = 0.5  # every element equals the mean: 0 / sd
+    yd, gd, bd = dev(y), dev(g), dev(b)
+    L.check(L.LIB.b200_layer_norm_rows_f32(yd.data_ptr(), gd.data_ptr(), bd.data_ptr(), out.data_ptr(), rows, n, ctypes.c_float(1e-5), stream()), "ln")
+    np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(glue.layer_norm(y, g, b, 1e-5)))
+    z = x.copy()
+    z[0, n // 2] = np.nan
+    zd = dev(z)
+    L.check(L.LIB.b200_softmax_rows_f32(zd.data_ptr(), out.data_ptr(), rows, n, stream()), "softmax")
+    got = out.cpu().numpy()
+    assert np.isnan(got[0]).all() and not np.isnan(got[1:]).any()
+
+
+def test_exp_and_erf_are_the_rounded_double_values(L):
+    """all but about one result in a million equal the double routine's value rounded to float, denormal results included"""
+    rng = np.random.default_rng(77)
+    for op, fn, x in ((9, math.exp, np.concatenate([rng.uniform(-104, 88.7, 200000), rng.uniform(-1e-3, 1e-3, 20000)])),
+                      (10, math.erf, np.concatenate([rng.uniform(-4.5, 4.5, 200000), rng.normal(0, 1e-3, 20000), rng.normal(0, 1e-20, 1000)]))):
+        x = x.astype(np.float32)
+        want = np.array([fn(float(v)) for v in x]).astype(np.float32)
+        xd, out = dev(x), torch.empty(x.size, device="cuda")
+        L.check(L.LIB.b200_f32_unary(op, xd.data_ptr(), out.data_ptr(), x.size, stream()), "unary")
+        assert (bits(out.cpu().numpy()) != bits(want)).sum() <= 2
+    special = np.float32([np.inf, -np.inf, np.nan, 0.0, -0.0, 200.0, -200.0, 3e38, -3e38])
+    xd, out = dev(special), torch.empty(special.size, device="cuda")
+    L.check(L.LIB.b200_f32_unary(9, xd.data_ptr(), out.data_ptr(), special.size, stream()), "exp")
+    np.testing.assert_array_equal(out.cpu().numpy(), np.float32([np.inf, 0, np.nan, 1, 1, np.inf, 0, np.inf, 0]))
+    L.check(L.LIB.b200_f32_unary(10, xd.data_ptr(), out.data_ptr(), special.size, stream()), "erf")
+    np.testing.assert_array_equal(bits(np.nan_to_num(out.cpu().numpy())), bits(np.float32([1, -1, 0, 0.0, -0.0, 1, -1, 1, -1])))
