@@ -25,9 +25,17 @@ namespace b200
     // which is also the answer if the query fails.
     inline int sm_count()
     {
+        static std::atomic<int> of_device[64]; // asked once per device: the query costs a noticeable part of a small launch
         int dev = 0, n = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
-            n = 148;
+        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64)
+            return 148;
+        n = of_device[dev].load(std::memory_order_relaxed);
+        if (n == 0)
+        {
+            if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+                n = 148;
+            of_device[dev].store(n, std::memory_order_relaxed);
+        }
         return n;
     }
 

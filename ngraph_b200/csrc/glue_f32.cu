@@ -71,16 +71,16 @@ namespace b200
     // One operand is a small tensor that op::v0::Broadcast would repeat along new leading axes (a bias row, a scalar
     // factor): element i of the large operand meets v[i % period] instead of a materialised copy.  V_LEFT: v is the
     // left-hand operand.  Four neighbours at a time when `period` allows it.
-    template <int OP, bool V_LEFT, bool VEC>
+    template <int OP, bool V_LEFT, bool VEC, typename IDX>
     __global__ void __launch_bounds__(256) binary_periodic_kernel(const float* __restrict__ a, const float* __restrict__ v,
-                                                                  float* __restrict__ out, int64_t n, int64_t period)
+                                                                  float* __restrict__ out, IDX n, IDX period)
     {
         if (VEC)
         {
-            const int64_t n4 = n >> 2, p4 = period >> 2; // period == 1: p4 == 0
+            const IDX n4 = n >> 2, p4 = period >> 2; // period == 1: p4 == 0
             const float4* a4 = reinterpret_cast<const float4*>(a);
             const float s = p4 == 0 ? __ldg(v) : 0.0f;
-            for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n4; i += int64_t(gridDim.x) * blockDim.x)
+            for (IDX i = IDX(blockIdx.x) * blockDim.x + threadIdx.x; i < n4; i += IDX(gridDim.x) * blockDim.x)
             {
                 const float4 x = a4[i];
                 const float4 y = p4 == 0 ? make_float4(s, s, s, s) : __ldg(reinterpret_cast<const float4*>(v) + i % p4);
@@ -93,24 +93,33 @@ namespace b200
             }
         }
         else
-            for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
+            for (IDX i = IDX(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += IDX(gridDim.x) * blockDim.x)
             {
                 const float x = a[i], y = __ldg(v + i % period);
                 out[i] = V_LEFT ? binary_op<OP>(y, x) : binary_op<OP>(x, y);
             }
     }
 
-    template <int OP>
-    void launch_binary_periodic(const float* a, const float* v, float* out, int64_t n, int64_t period, bool v_left, cudaStream_t st)
+    template <int OP, typename IDX>
+    void launch_binary_periodic_as(const float* a, const float* v, float* out, IDX n, IDX period, bool v_left, cudaStream_t st)
     {
         const bool vec = n % 4 == 0 && (period == 1 || period % 4 == 0) &&
                          ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(out) | (period == 1 ? 0 : reinterpret_cast<uintptr_t>(v))) & 15) == 0;
         const int64_t work = vec ? n / 4 : n, blocks = (work + 255) / 256, cap = b200::sm_count() * 16;
         const unsigned g = unsigned(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
-        if (vec && v_left) binary_periodic_kernel<OP, true, true><<<g, 256, 0, st>>>(a, v, out, n, period);
-        else if (vec) binary_periodic_kernel<OP, false, true><<<g, 256, 0, st>>>(a, v, out, n, period);
-        else if (v_left) binary_periodic_kernel<OP, true, false><<<g, 256, 0, st>>>(a, v, out, n, period);
-        else binary_periodic_kernel<OP, false, false><<<g, 256, 0, st>>>(a, v, out, n, period);
+        if (vec && v_left) binary_periodic_kernel<OP, true, true, IDX><<<g, 256, 0, st>>>(a, v, out, n, period);
+        else if (vec) binary_periodic_kernel<OP, false, true, IDX><<<g, 256, 0, st>>>(a, v, out, n, period);
+        else if (v_left) binary_periodic_kernel<OP, true, false, IDX><<<g, 256, 0, st>>>(a, v, out, n, period);
+        else binary_periodic_kernel<OP, false, false, IDX><<<g, 256, 0, st>>>(a, v, out, n, period);
+    }
+    // 32-bit indices wherever they reach: the modulo by the period is a division per vector
+    template <int OP>
+    void launch_binary_periodic(const float* a, const float* v, float* out, int64_t n, int64_t period, bool v_left, cudaStream_t st)
+    {
+        if (n < (int64_t(1) << 31))
+            launch_binary_periodic_as<OP, uint32_t>(a, v, out, uint32_t(n), uint32_t(period), v_left, st);
+        else
+            launch_binary_periodic_as<OP, int64_t>(a, v, out, n, period, v_left, st);
     }
 
     template <int OP>
@@ -121,8 +130,6 @@ namespace b200
         case B200_F32_ABS: return fabsf(x);
         case B200_F32_NEG: return -x;
         case B200_F32_SQRT: return __fsqrt_rn(x);
-        case B200_F32_EXP: return static_cast<float>(exp(static_cast<double>(x)));
-        case B200_F32_ERF: return static_cast<float>(erf(static_cast<double>(x)));
         default: return x > 0.0f ? x : 0.0f; // reference::relu
         }
     }
@@ -134,32 +141,109 @@ namespace b200
             out[i] = unary_op<OP>(x[i]);
     }
 
+    // Exp and Erf.  A block copies the function's table once and then strides over the tensor.
+    template <int OP>
+    __global__ void __launch_bounds__(256) unary_table_kernel(const float* __restrict__ x, float* __restrict__ out, int64_t n)
+    {
+        __shared__ double exp_table[OP == B200_F32_EXP ? rounded::EXP_STEPS : 1];
+        __shared__ __align__(16) rounded::ErfPoint erf_table[OP == B200_F32_ERF ? rounded::ERF_ENTRIES : 1];
+        if (OP == B200_F32_EXP)
+            rounded::load_exp_table(exp_table);
+        else
+            rounded::load_erf_table(erf_table);
+        __syncthreads();
+        for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
+            out[i] = OP == B200_F32_EXP ? rounded::exp_rounded(x[i], exp_table) : rounded::erf_rounded(x[i], erf_table);
+    }
+
+    // n / d for 0 <= n < 2^31 by a multiplication: ceil(2^(31 + l) / d) with l = ceil(log2 d) is exact over that range.
+    struct FastDiv
+    {
+        uint32_t d, mul, shift;
+        FastDiv() = default;
+        explicit FastDiv(uint32_t divisor) : d(divisor), mul(0), shift(0)
+        {
+            while ((uint64_t(1) << shift) < d)
+                ++shift;
+            mul = d > 1 ? uint32_t(((uint64_t(1) << (31 + shift)) + d - 1) / d) : 0;
+        }
+        __device__ __forceinline__ uint32_t div(uint32_t n) const { return d > 1 ? __umulhi(n, mul) >> (shift - 1) : n; }
+    };
+
     // out[idx] = in[mapped(idx)] for 4-byte elements: Broadcast (stride 0 on the new axes) and axis permutations.
-    // T: one element (uint32_t) or four neighbours along a last axis that both tensors share (uint4); IDX: 32-bit index
-    // arithmetic when every index and offset fits (a 64-bit division costs several times a 32-bit one).
-    template <typename T, typename IDX>
+    // T: one element (uint32_t) or four neighbours along a last axis that both tensors share (uint4).  The general form
+    // divides 64-bit indices; remap_small_kernel serves whatever has fewer than 2^31 elements, RANK axes after merging.
+    template <typename T>
     __global__ void __launch_bounds__(256) remap_kernel(const T* __restrict__ in, T* __restrict__ out, Dims d, int64_t n)
     {
-        IDX dim[MAX_RANK], stride[MAX_RANK];
-#pragma unroll
-        for (int a = 0; a < MAX_RANK; ++a)
-        {
-            dim[a] = a < d.rank ? IDX(d.out_dim[a]) : IDX(1);
-            stride[a] = a < d.rank ? IDX(d.in_stride[a]) : IDX(0);
-        }
         for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-        {
-            IDX idx = IDX(i), off = 0;
+            out[i] = in[mapped_offset(d, i)];
+    }
+    struct SmallDims
+    {
+        FastDiv dim[MAX_RANK];      // innermost first
+        uint32_t stride[MAX_RANK];
+    };
+    template <typename T, int RANK>
+    __global__ void __launch_bounds__(256) remap_small_kernel(const T* __restrict__ in, T* __restrict__ out, SmallDims d, uint32_t n)
+    {
+        auto source = [&](uint32_t i) {
+            uint32_t off = 0;
 #pragma unroll
-            for (int a = MAX_RANK - 1; a >= 0; --a)
-                if (a < d.rank)
-                {
-                    const IDX q = idx / dim[a];
-                    off += (idx - q * dim[a]) * stride[a];
-                    idx = q;
-                }
-            out[i] = in[off];
+            for (int a = 0; a < RANK - 1; ++a)
+            {
+                const uint32_t q = d.dim[a].div(i);
+                off += (i - q * d.dim[a].d) * d.stride[a];
+                i = q;
+            }
+            return off + i * d.stride[RANK - 1];
+        };
+        const uint32_t threads = gridDim.x * blockDim.x;
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 2 * threads)
+        {
+            const bool two = i + threads < n;
+            const T x = in[source(i)], y = in[two ? source(i + threads) : 0];
+            out[i] = x;
+            if (two)
+                out[i + threads] = y;
         }
+    }
+
+    // Axis permutations that move the last axis: 32 x 32 tiles through shared memory, so that both the loads (along the
+    // input's last axis) and the stores (along the output's) are whole 128-byte lines.
+    struct TileDims
+    {
+        FastDiv tiles_x, tiles_y, outer[MAX_RANK]; // tiles along the input's / the output's last axis, the remaining axes (innermost first)
+        uint32_t outer_in[MAX_RANK], outer_out[MAX_RANK];
+        uint32_t nx, ny;       // extents of the input's last axis (x) and of the output's (y)
+        uint32_t in_y, out_x;  // stride of y in the input, of x in the output (the other two strides are 1)
+        int n_outer;
+    };
+    __global__ void __launch_bounds__(256) permute_tiles_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, TileDims d)
+    {
+        __shared__ uint32_t tile[32][33];
+        uint32_t t = blockIdx.x;
+        const uint32_t ty = d.tiles_x.div(t), tx = t - ty * d.tiles_x.d;
+        t = d.tiles_y.div(ty);
+        const uint32_t y0 = (ty - t * d.tiles_y.d) * 32, x0 = tx * 32;
+        uint32_t in_off = 0, out_off = 0;
+        for (int a = 0; a < d.n_outer; ++a)
+        {
+            const uint32_t q = d.outer[a].div(t), c = t - q * d.outer[a].d;
+            in_off += c * d.outer_in[a];
+            out_off += c * d.outer_out[a];
+            t = q;
+        }
+        const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+        for (uint32_t j = 0; j < 32; j += 8)
+            if (x0 + lane < d.nx && y0 + w + j < d.ny)
+                tile[w + j][lane] = in[in_off + (y0 + w + j) * d.in_y + x0 + lane];
+        __syncthreads();
+#pragma unroll
+        for (uint32_t j = 0; j < 32; j += 8)
+            if (y0 + lane < d.ny && x0 + w + j < d.nx)
+                out[out_off + (x0 + w + j) * d.out_x + y0 + lane] = tile[lane][w + j];
     }
 
     // Picks the widest form the tensors allow.  `d` describes the output axes and the input stride of each.
@@ -181,14 +265,83 @@ namespace b200
         const bool small = n < (int64_t(1) << 31) && in_elements < (int64_t(1) << 31);
         const int64_t blocks = (n + 255) / 256, cap = b200::sm_count() * 16;
         const unsigned grid = unsigned(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
-        if (wide && small)
-            remap_kernel<uint4, uint32_t><<<grid, 256, 0, st>>>(static_cast<const uint4*>(in), static_cast<uint4*>(out), d, n);
-        else if (wide)
-            remap_kernel<uint4, int64_t><<<grid, 256, 0, st>>>(static_cast<const uint4*>(in), static_cast<uint4*>(out), d, n);
-        else if (small)
-            remap_kernel<uint32_t, uint32_t><<<grid, 256, 0, st>>>(static_cast<const uint32_t*>(in), static_cast<uint32_t*>(out), d, n);
+        if (!small)
+        {
+            if (wide)
+                remap_kernel<uint4><<<grid, 256, 0, st>>>(static_cast<const uint4*>(in), static_cast<uint4*>(out), d, n);
+            else
+                remap_kernel<uint32_t><<<grid, 256, 0, st>>>(static_cast<const uint32_t*>(in), static_cast<uint32_t*>(out), d, n);
+            return;
+        }
+        // axes innermost first; neighbours that are one run in both tensors count as one, and so do axes of one element
+        SmallDims sd = {};
+        uint32_t extent[MAX_RANK] = {1};
+        int r = 0;
+        for (int a = d.rank - 1; a >= 0; --a)
+        {
+            if (d.out_dim[a] == 1)
+                continue;
+            if (r > 0 && d.in_stride[a] == int64_t(sd.stride[r - 1]) * extent[r - 1])
+            {
+                extent[r - 1] *= uint32_t(d.out_dim[a]);
+                continue;
+            }
+            extent[r] = uint32_t(d.out_dim[a]);
+            sd.stride[r++] = uint32_t(d.in_stride[a]);
+        }
+        for (int a = 0; a < MAX_RANK; ++a)
+            sd.dim[a] = FastDiv(a < r ? extent[a] : 1);
+        auto launch = [&](auto element) {
+            using T = decltype(element);
+            const T* i = static_cast<const T*>(in);
+            T* o = static_cast<T*>(out);
+            if (r <= 2)
+                remap_small_kernel<T, 2><<<grid, 256, 0, st>>>(i, o, sd, uint32_t(n));
+            else if (r <= 4)
+                remap_small_kernel<T, 4><<<grid, 256, 0, st>>>(i, o, sd, uint32_t(n));
+            else
+                remap_small_kernel<T, MAX_RANK><<<grid, 256, 0, st>>>(i, o, sd, uint32_t(n));
+        };
+        if (wide)
+            launch(uint4());
         else
-            remap_kernel<uint32_t, int64_t><<<grid, 256, 0, st>>>(static_cast<const uint32_t*>(in), static_cast<uint32_t*>(out), d, n);
+            launch(uint32_t());
+    }
+
+    // The tile form, where it pays: fewer than 2^31 elements and both last axes long enough to fill most of a tile.
+    static bool launch_permute_tiles(const void* in, void* out, const Dims& d, int64_t n, cudaStream_t st)
+    {
+        const int last = d.rank - 1;
+        if (d.rank < 2 || n >= (int64_t(1) << 31) || d.in_stride[last] == 1)
+            return false;
+        int xa = -1; // the output axis that is the input's last
+        for (int a = 0; a < last; ++a)
+            if (d.in_stride[a] == 1 && d.out_dim[a] > 1)
+                xa = a;
+        if (xa < 0 || d.out_dim[xa] < 24 || d.out_dim[last] < 24)
+            return false;
+        TileDims t = {};
+        t.nx = uint32_t(d.out_dim[xa]);
+        t.ny = uint32_t(d.out_dim[last]);
+        t.in_y = uint32_t(d.in_stride[last]);
+        int64_t out_stride = 1, outer = 1;
+        for (int a = last; a >= 0; --a)
+        {
+            if (a == xa)
+                t.out_x = uint32_t(out_stride);
+            else if (a != last)
+            {
+                t.outer[t.n_outer] = FastDiv(uint32_t(d.out_dim[a]));
+                t.outer_in[t.n_outer] = uint32_t(d.in_stride[a]);
+                t.outer_out[t.n_outer++] = uint32_t(out_stride);
+                outer *= d.out_dim[a];
+            }
+            out_stride *= d.out_dim[a];
+        }
+        t.tiles_x = FastDiv((t.nx + 31) / 32);
+        t.tiles_y = FastDiv((t.ny + 31) / 32);
+        permute_tiles_kernel<<<unsigned(outer * t.tiles_x.d * t.tiles_y.d), 256, 0, st>>>(static_cast<const uint32_t*>(in), static_cast<uint32_t*>(out), t);
+        return true;
     }
 
     // One thread per output element; the reduced coordinates are walked in row-major order, as the reference does.
@@ -1017,8 +1170,8 @@ extern "C" int b200_f32_unary(int op, const float* x, float* out, int64_t n, voi
     case B200_F32_ABS: unary_kernel<B200_F32_ABS><<<g, 256, 0, st>>>(x, out, n); break;
     case B200_F32_NEG: unary_kernel<B200_F32_NEG><<<g, 256, 0, st>>>(x, out, n); break;
     case B200_F32_SQRT: unary_kernel<B200_F32_SQRT><<<g, 256, 0, st>>>(x, out, n); break;
-    case B200_F32_EXP: unary_kernel<B200_F32_EXP><<<g, 256, 0, st>>>(x, out, n); break;
-    case B200_F32_ERF: unary_kernel<B200_F32_ERF><<<g, 256, 0, st>>>(x, out, n); break;
+    case B200_F32_EXP: unary_table_kernel<B200_F32_EXP><<<g, 256, 0, st>>>(x, out, n); break;
+    case B200_F32_ERF: unary_table_kernel<B200_F32_ERF><<<g, 256, 0, st>>>(x, out, n); break;
     default: unary_kernel<B200_F32_RELU><<<g, 256, 0, st>>>(x, out, n); break;
     }
     return after_launch("b200_f32_unary");
@@ -1107,7 +1260,9 @@ extern "C" int b200_permute_b32(const void* in, void* out, const int64_t* in_sha
         d.out_dim[a] = in_shape[order[a]];
         d.in_stride[a] = in_stride[order[a]];
     }
-    launch_remap(in, out, d, n, n, static_cast<cudaStream_t>(stream));
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (!launch_permute_tiles(in, out, d, n, st))
+        launch_remap(in, out, d, n, n, st);
     return after_launch("b200_permute_b32");
 }
 

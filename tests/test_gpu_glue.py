@@ -353,3 +353,15 @@ def test_exp_and_erf_are_the_rounded_double_values(L):
     np.testing.assert_array_equal(out.cpu().numpy(), np.float32([np.inf, 0, np.nan, 1, 1, np.inf, 0, np.inf, 0]))
     L.check(L.LIB.b200_f32_unary(10, xd.data_ptr(), out.data_ptr(), special.size, stream()), "erf")
     np.testing.assert_array_equal(bits(np.nan_to_num(out.cpu().numpy())), bits(np.float32([1, -1, 0, 0.0, -0.0, 1, -1, 1, -1])))
+
+
+@pytest.mark.parametrize("shape", [(3, 33, 5, 40), (2, 24, 25), (1, 65, 2, 64), (64, 31), (2, 3, 1, 30, 1, 31), (5, 24, 3, 2, 32)])
+def test_permutes_that_move_the_last_axis(L, shape):
+    """32 x 32 tiles through shared memory (both last axes 24 or longer) beside the element-wise form, axes that merge and
+    axes of one element"""
+    import itertools
+    x = np.arange(int(np.prod(shape)), dtype=np.float32).reshape(shape)
+    xd, o = dev(x), torch.empty(x.size, device="cuda")
+    for order in itertools.islice(itertools.permutations(range(len(shape))), 0, None, 1 if len(shape) < 5 else 7):
+        L.check(L.LIB.b200_permute_b32(xd.data_ptr(), o.data_ptr(), i64(shape), len(shape), i64(order), stream()), "permute")
+        np.testing.assert_array_equal(o.cpu().numpy(), np.transpose(x, order).ravel(), err_msg=str(order))
