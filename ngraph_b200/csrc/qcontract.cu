@@ -526,12 +526,29 @@ namespace b200
             ptx::cluster_sync(); // the peer's barriers exist before anything arrives on them from here
         ptx::tc_fence_after_sync();
         const uint32_t tmem_base = tmem_base_slot;
+        // the tensor maps are launch parameters: fetching them need not wait for the previous kernel either
+        if (threadIdx.x == 32)
+        {
+            if (!p.a_cells)
+                ptx::prefetch_tmap(&maps.a[0]);
+            if (!p.b_packed)
+                ptx::prefetch_tmap(&maps.b);
+            if (p.tma_store)
+                ptx::prefetch_tmap(&maps.out);
+            if (p.tma_sum)
+                ptx::prefetch_tmap(&maps.sum);
+        }
         // everything above touched only this CTA's own state; from here on global memory of earlier kernels is read
         // and their inputs are overwritten (no-ops when the launch is not a programmatic dependent one)
         asm volatile("griddepcontrol.wait;" ::: "memory");
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
         const int num_tiles = p.tiles_m * p.tiles_n;
+        // naps between polls spare the epilogue's issue slots in a steady state; a CTA with one unit of work has none, and every
+        // hand-over is on its critical path
+        const bool naps = num_tiles > int(gridDim.x) * p.pair;
+        const uint32_t nap_empty = naps ? BACKOFF_EMPTY_NS : 0, nap_full = naps ? BACKOFF_FULL_NS : 0, nap_tempty = naps ? BACKOFF_TEMPTY_NS : 0,
+                       nap_tfull = naps ? BACKOFF_TFULL_NS : 0;
         int fail = 0;
 #ifdef B200_PROFILE_WAITS
         const long long prof_kernel_t0 = clock64();
@@ -549,8 +566,6 @@ namespace b200
             const int pw = warp - 1;
             if (ptx::elect_one())
             {
-                ptx::prefetch_tmap(&maps.b);
-                ptx::prefetch_tmap(&maps.a[0]);
                 if (p.smem.b_resident && pw == 0)
                 {
                     // the single column tile's weights, all k-blocks, once
@@ -642,7 +657,7 @@ namespace b200
                     for (; j < nkb; j += NUM_PRODUCERS)
                     {
                         PROF_T0();
-                        if (!ptx::mbar_wait(empty_bar(s), ph ^ 1, abortp, BACKOFF_EMPTY_NS))
+                        if (!ptx::mbar_wait(empty_bar(s), ph ^ 1, abortp, nap_empty))
                         {
                             fail = 1001;
                             break;
@@ -738,7 +753,7 @@ namespace b200
                 for (int unit = worker; unit < num_units && !fail; unit += nworkers)
                     for (int kb = 0; kb < num_kblocks; ++kb)
                     {
-                        if (!ptx::mbar_wait(full_bar(s), ph, abortp, BACKOFF_FULL_NS))
+                        if (!ptx::mbar_wait(full_bar(s), ph, abortp, nap_full))
                         {
                             fail = 2004;
                             break;
@@ -772,7 +787,7 @@ namespace b200
                 // CTA pairs: the hardware reads the other 128 rows of A and the other half of B at the same offsets of the odd CTA
                 // descriptor address fields count 16-byte units
                 const uint32_t b_step = p.smem.b_resident ? (C::B_BYTES >> 4) : (stage_bytes >> 4);
-                if (p.smem.b_resident && !ptx::mbar_wait(bres_bar, 0, abortp, BACKOFF_FULL_NS))
+                if (p.smem.b_resident && !ptx::mbar_wait(bres_bar, 0, abortp, nap_full))
                     fail = 2003;
                 // one unit per iteration: a tile, or the two row tiles of a pair (accumulators acc and acc + 1; NACC is even)
                 const int num_units = CTA2 ? num_tiles / 2 : num_tiles / pair;
@@ -782,8 +797,8 @@ namespace b200
                     const uint32_t acc_ph = (tile_it / NACC) & 1;
                     {
                         PROF_T0();
-                        if (!ptx::mbar_wait<CTA2>(tempty_bar(acc), acc_ph ^ 1, abortp, BACKOFF_TEMPTY_NS) ||
-                            (pair == 2 && !ptx::mbar_wait(tempty_bar(acc + 1), acc_ph ^ 1, abortp, BACKOFF_TEMPTY_NS)))
+                        if (!ptx::mbar_wait<CTA2>(tempty_bar(acc), acc_ph ^ 1, abortp, nap_tempty) ||
+                            (pair == 2 && !ptx::mbar_wait(tempty_bar(acc + 1), acc_ph ^ 1, abortp, nap_tempty)))
                         {
                             fail = 2001;
                             break;
@@ -801,7 +816,7 @@ namespace b200
                         {
                             {
                                 PROF_T0();
-                                if (!ptx::mbar_wait(full_bar(s), ph, abortp, BACKOFF_FULL_NS))
+                                if (!ptx::mbar_wait(full_bar(s), ph, abortp, nap_full))
                                 {
                                     fail = 2002;
                                     break;
@@ -843,7 +858,7 @@ namespace b200
                         // instructions, one commit
                         {
                             PROF_T0();
-                            if (!ptx::mbar_wait(full_bar(s), ph, abortp, BACKOFF_FULL_NS))
+                            if (!ptx::mbar_wait(full_bar(s), ph, abortp, nap_full))
                             {
                                 fail = 2002;
                                 break;
@@ -873,7 +888,7 @@ namespace b200
                     {
                         {
                             PROF_T0();
-                            if (!ptx::mbar_wait(full_bar(s), ph, abortp, BACKOFF_FULL_NS))
+                            if (!ptx::mbar_wait(full_bar(s), ph, abortp, nap_full))
                             {
                                 fail = 2002;
                                 break;
@@ -1146,9 +1161,9 @@ namespace b200
                     {
                         PROF_T0();
                         // the verdict is made warp-uniform: the loop body uses full-mask shuffles and warp syncs
-                        bool ok = ptx::mbar_wait(tfull_bar(acc), acc_ph, abortp, BACKOFF_TFULL_NS);
+                        bool ok = ptx::mbar_wait(tfull_bar(acc), acc_ph, abortp, nap_tfull);
                         if (F_SUM)
-                            ok = ok && ptx::mbar_wait(sum_bar(ew, blk), sum_ph, abortp, BACKOFF_TFULL_NS);
+                            ok = ok && ptx::mbar_wait(sum_bar(ew, blk), sum_ph, abortp, nap_tfull);
                         if (!__all_sync(0xffffffffu, ok))
                         {
                             fail = 3001;
@@ -1381,9 +1396,9 @@ namespace b200
             case 8: epilogue_loop(std::integral_constant<int, 8>{}); break;
             default: epilogue_loop(std::integral_constant<int, -1>{}); break;
             }
-            // stores must be complete (not just read) before the CTA exits
+            // the staging blocks must have been read before the CTA exits (the end of the grid waits for the writes themselves)
             if (ptx::elect_one())
-                asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+                asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         }
 
         // ------------------------------------------------------------ common tail
