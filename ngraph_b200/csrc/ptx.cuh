@@ -96,6 +96,9 @@ namespace b200
             asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
             asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         }
+        // the two halves of a cluster-wide barrier; the relaxed arrival orders no memory
+        __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+        __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
         // the address, in the cluster's shared window, of this CTA's shared-memory address `addr` in CTA `rank`
         __device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank)
         {
@@ -138,6 +141,14 @@ namespace b200
                 }
             }
             return true;
+        }
+
+        // 16 bytes into the shared memory of a CTA of the cluster, completing on an mbarrier there (both addresses from mapa)
+        __device__ __forceinline__ void store_async(uint32_t dst, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t bar)
+        {
+            asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst), "r"(a), "r"(b), "r"(c),
+                         "r"(d), "r"(bar)
+                         : "memory");
         }
 
         // ---- TMA tiled loads (global -> shared, completion on an mbarrier) ---------------
@@ -260,6 +271,17 @@ namespace b200
                   "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]),
                   "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]),
                   "=r"(r[30]), "=r"(r[31])
+                : "r"(taddr)
+                : "memory");
+        }
+        // 32 lanes x 16 columns -> 16 registers per thread
+        __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
+        {
+            asm volatile(
+                "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                 : "r"(taddr)
                 : "memory");
         }

@@ -124,6 +124,7 @@ namespace b200
                              // (8192^3: 1.5 against 3.0 POP/s): with the same bytes in flight per SM the stage loop is twice
                              // as long (free -> landed takes 3 us per 32 KB stage, six stages per 4 us).  Never chosen; the
                              // variant is compiled into instrumented builds only, which can force it.
+        int split;           // CTAs that share one tile's reduction (a thread-block cluster), 1: none
         void* out;
         uint32_t idesc;
         SmemPlan smem;
@@ -438,16 +439,155 @@ namespace b200
         }
     }
 
-    template <int BN, int BK, bool CTA2 = false>
-    __global__ void __launch_bounds__(NUM_THREADS, 1)
+    // Split reductions (SPLITK, 64-wide tiles): a product with few tiles and a long reduction leaves most SMs idle and pays for
+    // every k-block in turn (0.2 us each).  A cluster of p.split CTAs then shares a tile: each multiplies its range of
+    // k-blocks, hands its int32 partial sums to the CTAs that finish them - CTA r the columns 64 / split * r and up - by
+    // asynchronous stores into distributed shared memory that complete on one barrier of the receiving CTA (a cluster barrier
+    // with its release fence took 1.1 us), and that CTA adds the parts - exact integers, any order - and runs the epilogue, four
+    // columns of a row per thread.  This code runs once per launch: it is kept short, unrolled over 16 columns of a warp it
+    // spent 2.6 us, mostly on fetching instructions.
+    constexpr int MAX_SPLIT = 8;
+    constexpr int SPLIT_EXCHANGE_BYTES = BM * 64 * 4;  // the parts a CTA receives: split x (64 / split) columns x 128 rows
+    constexpr int SPLIT_SMEM_LIMIT = 112 * 1024;       // two CTAs per SM
+
+    __device__ __forceinline__ void split_epilogue(const ContractParams& p, int tile, int rank, int warp, int lane, uint32_t tmem_base, uint32_t exchange,
+                                                   uint32_t tfull, uint32_t landed, volatile int* abortp, int& fail)
+    {
+        const int quarter = warp & 3, group = (warp - 4) >> 2; // accumulator rows 32 * quarter .. + 31, columns 16 * group .. + 15
+        const int row = quarter * 32 + lane, split_log2 = __ffs(p.split) - 1;
+        const int quads = 16 >> split_log2; // groups of four columns this CTA finishes; thread: quads group, group + 4, ...
+        const uint32_t remote0 = exchange + uint32_t(rank) * uint32_t(quads) * (BM * 16) + uint32_t(row) * 16;
+        if (!__all_sync(0xffffffffu, ptx::mbar_wait(tfull, 0, abortp, 0)))
+            fail = 3001;
+        ptx::tc_fence_after_sync();
+        {
+            uint32_t v[16];
+            ptx::tmem_ld_32x16(tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(group) * 16, v);
+            ptx::tmem_ld_wait();
+            ptx::cluster_wait(); // every CTA of the cluster runs, its barrier is initialised
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+            {
+                // [part's rank][quad][row], 16 bytes each: a warp's store is 512 contiguous bytes
+                const int quad = group * 4 + j, owner = quad / quads;
+                const uint32_t dst = remote0 + uint32_t(quad - owner * quads) * (BM * 16);
+                ptx::store_async(ptx::mapa(dst, uint32_t(owner)), v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3], ptx::mapa(landed, uint32_t(owner)));
+            }
+        }
+        int tm, tn, q0, p0, n0;
+        decode_tile(p, tile, tm, tn, q0, p0, n0);
+        bool valid;
+        int64_t off;
+        if (p.conv) // the patch's extents are powers of two
+        {
+            const int w = __ffs(p.RW) - 1, h = __ffs(p.TH) - 1;
+            const int q = q0 + (row & (p.RW - 1)), pp = p0 + ((row >> w) & (p.TH - 1)), n = n0 + (row >> (w + h));
+            valid = q < p.Q && pp < p.P && n < p.NB;
+            off = ((int64_t(n) * p.P + pp) * p.Q + q) * p.N;
+        }
+        else
+        {
+            valid = tm * BM + row < p.M;
+            off = int64_t(tm * BM + row) * p.N;
+        }
+        const int first = tn * 64 + rank * quads * 4; // first column finished here
+        const bool one_byte = p.out_type == B200_U8 || p.out_type == B200_I8;
+        const bool aligned = p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out) & (one_byte ? 3 : 15)) == 0;
+        const float sum_scale = p.sum_in ? __ldg(p.sum_scale) : 0.0f;
+        bool waited = false;
+#pragma unroll 1
+        for (int quad = group; quad < quads; quad += 4)
+        {
+            const int col = first + 4 * quad, cols = p.N - col; // may be <= 0
+            float scale[4];
+            int bias[4];
+            uint32_t sum[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+            {
+                scale[i] = i < cols && p.scale ? __ldg(p.scale + (p.scale_per_channel ? col + i : 0)) : 0.0f;
+                bias[i] = i < cols && p.bias ? __ldg(p.bias + col + i) : 0;
+                sum[i] = i < cols && valid && p.sum_in ? static_cast<const uint8_t*>(p.sum_in)[off + col + i] : 0;
+            }
+            if (!waited && !__all_sync(0xffffffffu, ptx::mbar_wait(landed, 0, abortp, 0)))
+                fail = 3002;
+            waited = true;
+            const uint32_t part = exchange + uint32_t(quad * BM + row) * 16;
+            int v[4] = {0, 0, 0, 0};
+#pragma unroll 1
+            for (int r = 0; r < p.split; ++r)
+            {
+                const int4 w = lds_i4(part + uint32_t(r) * uint32_t(quads) * (BM * 16));
+                v[0] += w.x, v[1] += w.y, v[2] += w.z, v[3] += w.w;
+            }
+            uint32_t bytes = 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+            {
+                if (p.half_away == 1)
+                    v[i] = int(epilogue_core(p, v[i], scale[i]));
+                else if (p.half_away == 0)
+                {
+                    float f = __fmul_rn(__int2float_rn(v[i] + bias[i]), scale[i]);
+                    if (p.sum_in)
+                        f = __fadd_rn(f, __fmul_rn(sum_scale, p.sum_type == B200_U8 ? float(sum[i]) : float(int8_t(sum[i]))));
+                    if (p.relu)
+                        f = fmaxf(f, 0.0f);
+                    if (p.out_type == B200_F32)
+                        v[i] = __float_as_int(f);
+                    else if (p.out_type == B200_I32)
+                        v[i] = clamp_cast<int32_t>(round_quant<B200_ROUND_NEAREST_TOWARD_EVEN>(f));
+                    else
+                        v[i] = min(max(__float2int_rn(f), p.out_type == B200_U8 ? 0 : -128), p.out_type == B200_U8 ? 255 : 127);
+                }
+                bytes |= (uint32_t(v[i]) & 0xFFu) << (8 * i);
+            }
+            if (!valid)
+                continue;
+            if (one_byte)
+            {
+                uint8_t* o = static_cast<uint8_t*>(p.out) + off + col;
+                if (aligned && cols >= 4)
+                    *reinterpret_cast<uint32_t*>(o) = bytes;
+                else
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (i < cols)
+                            o[i] = uint8_t(bytes >> (8 * i));
+            }
+            else
+            {
+                int* o = static_cast<int*>(p.out) + off + col;
+                if (aligned && cols >= 4)
+                    *reinterpret_cast<int4*>(o) = make_int4(v[0], v[1], v[2], v[3]);
+                else
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (i < cols)
+                            o[i] = v[i];
+            }
+        }
+        // a warp without a quad of its own leaves only when every part has landed: the senders' stores need this CTA's memory
+        if (!waited && !__all_sync(0xffffffffu, ptx::mbar_wait(landed, 0, abortp, 0)))
+            fail = 3002;
+    }
+
+    template <int BN, int BK, bool CTA2 = false, bool SPLITK = false>
+    __global__ void __launch_bounds__(NUM_THREADS, SPLITK ? 2 : 1)
         qcontract_kernel(const __grid_constant__ TensorMaps maps, const __grid_constant__ ContractParams p)
     {
         using C = Cfg<BN, BK>;
         constexpr int SPLIT = C::SPLIT, GROUPS = C::GROUPS, NACC = C::NACC;
+        // a split tile has one accumulator: two of these CTAs, of one launch or of consecutive ones, share an SM
+        constexpr uint32_t TMEM_COLS = SPLITK ? BN : C::TMEM_COLS;
         // CTA pairs: rank 0 issues the pair's MMAs; a "worker" is what takes units of work in turn (a CTA, or a pair)
         const uint32_t cta_rank = CTA2 ? ptx::cluster_ctarank() : 0u;
-        const int worker = CTA2 ? int(blockIdx.x >> 1) : int(blockIdx.x);
-        const int nworkers = CTA2 ? int(gridDim.x >> 1) : int(gridDim.x);
+        const int worker = CTA2 ? int(blockIdx.x >> 1) : SPLITK ? int(blockIdx.x) / p.split : int(blockIdx.x);
+        const int nworkers = CTA2 ? int(gridDim.x >> 1) : SPLITK ? int(gridDim.x) / p.split : int(gridDim.x);
+        // this CTA's share of the tile's k-blocks
+        const int split_rank = SPLITK ? int(ptx::cluster_ctarank()) : 0;
+        const int kb_total = p.ntaps * p.cblocks;
+        const int kb_begin = SPLITK ? kb_total * split_rank / p.split : 0, kb_end = SPLITK ? kb_total * (split_rank + 1) / p.split : kb_total;
         // bytes of B one CTA stages per k-block: the whole column tile, or this CTA's half of it
         constexpr uint32_t B_STAGE_BYTES = CTA2 ? uint32_t(C::B_BYTES) / 2 : uint32_t(C::B_BYTES);
 #ifdef B200_PROFILE_WAITS
@@ -504,6 +644,8 @@ namespace b200
                 ptx::mbar_init(sum_bar((t - 96) / 3, (t - 96) % 3), 1);
             else if (CTA2 && t >= 160 && t < 160 + STAGES)
                 ptx::mbar_init(peer_full_bar(t - 160), 1);
+            if (SPLITK && t == 96)
+                ptx::mbar_expect_tx(sum_bar(0, 0), SPLIT_EXCHANGE_BYTES); // the partial sums of the columns finished here
             if (t >= 0 && t < 224)
                 ptx::fence_barrier_init();
         }
@@ -516,7 +658,7 @@ namespace b200
             }
             else
             {
-                ptx::tmem_alloc(ptx::smem_u32(&tmem_base_slot), C::TMEM_COLS);
+                ptx::tmem_alloc(ptx::smem_u32(&tmem_base_slot), TMEM_COLS);
                 ptx::tmem_relinquish();
             }
         }
@@ -524,6 +666,8 @@ namespace b200
         __syncthreads();
         if (CTA2)
             ptx::cluster_sync(); // the peer's barriers exist before anything arrives on them from here
+        if (SPLITK)
+            ptx::cluster_arrive_relaxed(); // this CTA runs: its shared memory may be written from now on
         ptx::tc_fence_after_sync();
         const uint32_t tmem_base = tmem_base_slot;
         // the tensor maps are launch parameters: fetching them need not wait for the previous kernel either
@@ -592,13 +736,13 @@ namespace b200
             }
             // pipeline stages one tile consumes: one per (tap, channel block), or one per channel block in halo mode
             // (the stem's cell runs: every tap of a tile in ONE stage - per-stage bookkeeping, not bytes, bounds that path)
-            const int nkb = p.halo ? p.cblocks : p.a_cells ? 1 : p.ntaps * p.cblocks;
+            const int nkb = p.halo ? p.cblocks : p.a_cells ? 1 : kb_end;
             int info_a = 0, info_b = 0, info_c = 0, info_d = 0;
             int info_a2 = 0, info_b2 = 0, info_c2 = 0; // paired mode: the second row tile of the unit (same column tile)
             int idx = 32;
             // this producer's next k-block, as (offset inside the current tile, pipeline stage, stage parity); it advances
             // by NUM_PRODUCERS k-blocks at a time and carries over from tile to tile
-            int j = pw, s = pw;
+            int j = kb_begin + pw, s = pw;
             int use_p = pw; // running index of this producer's k-block over the whole launch (instrumentation)
             (void)use_p;
             uint32_t ph = 0;
@@ -786,7 +930,7 @@ namespace b200
                 int use_m = 0;
                 (void)use_m;
                 uint32_t ph = 0, tile_it = 0;
-                const int num_kblocks = p.ntaps * p.cblocks;
+                const int num_kblocks = kb_end - kb_begin;
                 // stem cells: row m of the A tile is the 64 bytes starting at cell m of a linear run, so rows overlap:
                 // 16-byte K pieces 16 bytes apart, rows 16 bytes apart, 8-row groups 128 bytes apart, no swizzle
                 const uint64_t a_desc0 = p.a_cells ? ptx::smem_desc_overlapping_rows(smem_base) : ptx::smem_desc_kmajor(smem_base, BK);
@@ -963,6 +1107,13 @@ namespace b200
         else
         {
             // ------------------------------------------------------------ epilogue (warps 4..19)
+            if constexpr (SPLITK)
+            {
+                wait_for_earlier_kernels();
+                split_epilogue(p, worker, split_rank, warp, lane, tmem_base, out_base, tfull_bar(0), sum_bar(0, 0), abortp, fail);
+            }
+            else
+            {
             // The TMEM lane quarter a warp may read (warp id % 4) is fixed by the hardware.  Every warp owns 32 rows x
             // 64 columns of a tile, so a tile takes 4 * SPLIT warps; the GROUPS warp groups work on different tiles
             // at the same time (tile_it % GROUPS), each with two of the NACC accumulator buffers.
@@ -1408,6 +1559,7 @@ namespace b200
             // the staging blocks must have been read before the CTA exits (the end of the grid waits for the writes themselves)
             if (ptx::elect_one())
                 asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            } // !SPLITK
         }
 
         // ------------------------------------------------------------ common tail
@@ -1418,6 +1570,10 @@ namespace b200
         if (fail)
             atomicCAS(&g_contract_status, 0, fail);
         __syncwarp();
+        if (SPLITK && warp < 4)
+        {
+            ptx::cluster_wait(); // the barrier that the epilogue warps waited on counts every thread of the cluster
+        }
         ptx::tc_fence_before_sync();
         __syncthreads();
         if (abort_flag)
@@ -1435,7 +1591,7 @@ namespace b200
             if (CTA2)
                 ptx::tmem_dealloc_pair(tmem_base, C::TMEM_COLS);
             else
-                ptx::tmem_dealloc(tmem_base, C::TMEM_COLS);
+                ptx::tmem_dealloc(tmem_base, TMEM_COLS);
         }
 #ifdef B200_PROFILE_WAITS
         if (threadIdx.x == 0)
@@ -1583,6 +1739,26 @@ namespace b200
         return uint64_t(uint32_t(dev));
     }
 
+    // CTAs that share a tile's reduction.  Measured here (launches in a row): 3.5 us + 0.19 us per k-block of a 64-wide tile
+    // whole, 1.9 us more and the k-blocks divided when split; clusters of eight fit 128 of the 148 SMs at a time.
+    // [1, 512, 7, 7] 3x3 -> 512: 10.5 -> 6.3 us, 128 x 1000 x 2048: 17.4 -> 6.4 us, [1, 256, 14, 14] 3x3 -> 256: 7.0 -> 5.8 us.
+    static int pick_split(int64_t tiles, int64_t nkb)
+    {
+        int best = 1;
+        double best_us = 1e30;
+        for (int s = 1; s <= MAX_SPLIT && s <= nkb; s *= 2)
+        {
+            const int64_t room = s == 1 ? num_sms() : s == MAX_SPLIT ? num_sms() * 7 / 8 : num_sms() * 15 / 16;
+            const double us = double((tiles * s + room - 1) / room) * double((nkb + s - 1) / s) * 0.19 + (s > 1 ? 1.9 : 0.0);
+            if (us < best_us - 0.15)
+            {
+                best = s;
+                best_us = us;
+            }
+        }
+        return best;
+    }
+
     template <int BN, int BK>
     static int fire_contract(const TensorMaps& maps, const ContractParams& p, int grid, cudaStream_t st)
     {
@@ -1608,10 +1784,10 @@ namespace b200
             attr[nattr].val.programmaticStreamSerializationAllowed = 1;
             ++nattr;
         }
-        if (p.cta2)
+        if (p.cta2 || p.split > 1)
         {
-            attr[nattr].id = cudaLaunchAttributeClusterDimension; // CTAs 2i and 2i + 1 form a pair
-            attr[nattr].val.clusterDim.x = 2;
+            attr[nattr].id = cudaLaunchAttributeClusterDimension; // CTAs 2i and 2i + 1 form a pair; split i, split i + 1, ... share a tile
+            attr[nattr].val.clusterDim.x = p.cta2 ? 2 : unsigned(p.split);
             attr[nattr].val.clusterDim.y = 1;
             attr[nattr].val.clusterDim.z = 1;
             ++nattr;
@@ -1620,12 +1796,14 @@ namespace b200
         cfg.numAttrs = unsigned(nattr);
 #ifdef B200_PROFILE_WAITS
         // the CTA-pair variant is compiled into instrumented builds only (see ContractParams::cta2)
-        cudaError_t le = p.cta2 ? cudaLaunchKernelEx(&cfg, qcontract_kernel<BN, BK, (BN == 256)>, maps, p)
+        cudaError_t le = p.split > 1 ? cudaLaunchKernelEx(&cfg, qcontract_kernel<BN, BK, false, (BN == 64)>, maps, p)
+                         : p.cta2 ? cudaLaunchKernelEx(&cfg, qcontract_kernel<BN, BK, (BN == 256)>, maps, p)
                                 : cudaLaunchKernelEx(&cfg, qcontract_kernel<BN, BK>, maps, p);
 #else
         if (p.cta2)
             return B200_ERR_UNSUPPORTED;
-        cudaError_t le = cudaLaunchKernelEx(&cfg, qcontract_kernel<BN, BK>, maps, p);
+        cudaError_t le = p.split > 1 ? cudaLaunchKernelEx(&cfg, qcontract_kernel<BN, BK, false, (BN == 64)>, maps, p)
+                                     : cudaLaunchKernelEx(&cfg, qcontract_kernel<BN, BK>, maps, p);
 #endif
         if (le != cudaSuccess)
             return cuda_status(le, "cudaLaunchKernelEx(qcontract_kernel)");
@@ -1661,6 +1839,8 @@ namespace b200
             if (e == cudaSuccess && BN == 256)
                 e = cudaFuncSetAttribute(qcontract_kernel<BN, BK, (BN == 256)>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
 #endif
+            if (e == cudaSuccess && BN == 64)
+                e = cudaFuncSetAttribute(qcontract_kernel<BN, BK, false, (BN == 64)>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
             if (e != cudaSuccess)
                 return cuda_status(e, "cudaFuncSetAttribute(qcontract)");
             attr_set[dev] = true;
@@ -1674,7 +1854,10 @@ namespace b200
             return B200_ERR_TOO_LARGE;
         const int nkb = p.ntaps * p.cblocks;
         SmemPlan& sp = p.smem;
-        sp.b_resident = (p.tiles_n == 1 && nkb * C::B_BYTES <= B_RESIDENT_MAX) ? 1 : 0;
+        p.split = (BN == 64 && !p.a_cells && !p.halo && p.pair != 2 && !p.cta2) ? pick_split(int64_t(p.tiles_m) * p.tiles_n, nkb) : 1;
+        sp.b_resident = (p.tiles_n == 1 && nkb * C::B_BYTES <= B_RESIDENT_MAX && p.split == 1) ? 1 : 0;
+        if (p.split > 1) // results are written from registers; the staging area holds the partial sums on their way
+            p.tma_store = p.tma_sum = p.f32_staged = 0;
         if (p.cta2)
         {
             // CTA pairs: the plain tile pipeline with 256-wide column tiles, an even number of row tiles (the caller pads)
@@ -1705,7 +1888,7 @@ namespace b200
             // the patch plus the rows the last taps read past it for the junk positions of the last tile row
             sp.stage_bytes = ((p.halo_bytes + 64 * BK + 1023) / 1024) * 1024;
         }
-        const int room = SMEM_LIMIT - C::FIXED - sp.b_res_bytes - 64;
+        const int room = (p.split > 1 ? SPLIT_SMEM_LIMIT : SMEM_LIMIT) - C::FIXED - sp.b_res_bytes - 64;
         if (p.tma_store && nkb >= 16 && (room - 2 * C::OUT_BYTES) / sp.stage_bytes < (p.cta2 ? 7 : 4))
         {
             // long reductions are MMA-bound: pipeline depth matters more than store efficiency, so the
@@ -1717,7 +1900,7 @@ namespace b200
         if (p.tma_sum && (room - 3 * C::OUT_BYTES) / sp.stage_bytes < 2)
             p.tma_sum = 0;
         sp.out_bufs = p.tma_store ? (p.tma_sum ? 3 : 2) : (p.f32_staged ? 2 : 0);
-        sp.out_bytes = sp.out_bufs * C::OUT_BYTES;
+        sp.out_bytes = p.split > 1 ? SPLIT_EXCHANGE_BYTES : sp.out_bufs * C::OUT_BYTES;
         int fit = (room - sp.out_bytes) / sp.stage_bytes;
         sp.stages = fit > MAX_STAGES ? MAX_STAGES : fit;
         if (p.pair == 2 && sp.stages < 3)
@@ -1733,7 +1916,7 @@ namespace b200
             return B200_ERR_UNSUPPORTED;
         sp.total_bytes = sp.b_res_bytes + sp.stages * sp.stage_bytes + sp.out_bytes + C::FIXED;
         int tiles = p.tiles_m * p.tiles_n / p.pair; // units of work: tiles, or pairs of row tiles
-        int grid = tiles < num_sms() ? tiles : num_sms();
+        int grid = p.split > 1 ? tiles * p.split : tiles < num_sms() ? tiles : num_sms();
         if (p.cta2) // two CTAs per unit of two row tiles
             grid = 2 * std::min(tiles / 2, num_sms() / 2);
         if (t_capture)

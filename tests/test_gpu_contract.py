@@ -484,3 +484,48 @@ def test_repeated_calls_reuse_the_launch_plan_not_the_data(ops):
     again = run_conv(ops, data, filt, bias, scale[:64], cs, np.uint8, True)
     np.testing.assert_array_equal(first, again)
     np.testing.assert_array_equal(first, ref.qconv_fused(data, filt, bias, scale[:64], cs, np.uint8, relu=True))
+
+
+# ---------------------------------------------------------------- one tile's reduction shared by a cluster of CTAs
+@pytest.mark.parametrize("m,n,k", [(1, 16, 4096), (130, 75, 3072), (64, 1000, 2048), (128, 250, 8192), (300, 64, 2560), (5, 3, 16384)])
+def test_qgemm_split_reductions(ops, m, n, k):
+    """Few tiles and a long K: clusters of two, four and eight CTAs, shares of unequal length, widths that end inside a CTA's
+    columns or leave CTAs of the cluster without any, every output type and contract"""
+    rng = np.random.default_rng(m + n + k)
+    a = rng.integers(0, 256, size=(m, k)).astype(np.uint8)
+    w = rng.integers(-127, 128, size=(n, k)).astype(np.int8)
+    bias = rng.integers(-1000, 1001, size=n).astype(np.int32)
+    scale = (np.exp(rng.uniform(np.log(0.5), np.log(2.0), size=n)) * 40.0 / (np.sqrt(k) * 74 * 147)).astype(np.float32)
+    s = rng.integers(-128, 128, size=(m, n)).astype(np.int8)
+    for packed in (True, False):
+        for out_dt, relu, sum_in in ((np.uint8, True, None), (np.int8, False, s), (np.uint8, False, s.view(np.uint8)), (np.float32, True, None), (np.int32, False, None)):
+            kw = {} if sum_in is None else {"sum_in": sum_in, "sum_scale": np.float32(0.37)}
+            dkw = {} if sum_in is None else {"sum_in": dev(sum_in), "sum_scale": dev(np.array([0.37], np.float32))}
+            exp = ref.qgemm_fused(a, w, bias, scale, out_dt, relu=relu, **kw)
+            got = ops.qgemm(dev(a), dev(w), dev(scale), TDT[np.dtype(out_dt)], bias=dev(bias), relu=relu, packed=packed, **dkw).cpu().numpy()
+            if out_dt == np.float32:
+                same_f32(got, exp)
+            else:
+                np.testing.assert_array_equal(got, exp, err_msg="%s packed=%d" % (out_dt, packed))
+        for out_dt, zp in ((np.int8, 3), (np.int32, -5)):
+            got = ops.qgemm(dev(a), dev(w), dev(scale[:1]), TDT[np.dtype(out_dt)], core=True, out_zp=zp, packed=packed).cpu().numpy()
+            np.testing.assert_array_equal(got, ref.qgemm_core(a, w, scale[0], zp, out_dt), err_msg="core %s" % out_dt)
+
+
+@pytest.mark.parametrize("cfg", [(1, 512, 7, 7, 512, 3, 3, (1, 1)), (2, 512, 9, 11, 72, 3, 3, (2, 2)), (1, 2048, 7, 7, 130, 1, 1, (1, 1)), (3, 64, 6, 5, 24, 7, 7, (1, 1))])
+def test_qconv_split_reductions(ops, cfg):
+    n, c, h, w, k, r, s, stride = cfg
+    rng = np.random.default_rng(sum(cfg[:7]))
+    data = rng.integers(0, 256, size=(n, c, h, w)).astype(np.uint8)
+    filt = rng.integers(-127, 128, size=(k, c, r, s)).astype(np.int8)
+    bias = rng.integers(-1000, 1001, size=k).astype(np.int32)
+    pad = (r // 2, s // 2)
+    cs = ref.conv_shape(data.shape, filt.shape, stride, pad, pad, (1, 1))
+    p, q = ref.conv_out_hw(cs)
+    scale = (np.exp(rng.uniform(np.log(0.5), np.log(2.0), size=k)) * 60.0 / (np.sqrt(c * r * s) * 74 * 147)).astype(np.float32)
+    sum_u8 = rng.integers(0, 256, size=(n, k, p, q)).astype(np.uint8)
+    for packed in (True, False):
+        np.testing.assert_array_equal(run_conv(ops, data, filt, bias, scale, cs, np.uint8, True, packed=packed),
+                                      ref.qconv_fused(data, filt, bias, scale, cs, np.uint8, relu=True))
+        np.testing.assert_array_equal(run_conv(ops, data, filt, bias, scale, cs, np.uint8, True, sum_in=sum_u8, sum_scale=0.61, packed=packed),
+                                      ref.qconv_fused(data, filt, bias, scale, cs, np.uint8, relu=True, sum_in=sum_u8, sum_scale=np.float32(0.61)))
