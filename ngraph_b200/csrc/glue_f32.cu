@@ -64,6 +64,7 @@ namespace b200
     __global__ void __launch_bounds__(256) binary_kernel(const float* __restrict__ a, const float* __restrict__ b,
                                                          float* __restrict__ out, int64_t n)
     {
+        after_earlier_kernels(a, b, out);
         for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
             out[i] = binary_op<OP>(a[i], b[i]);
     }
@@ -75,6 +76,7 @@ namespace b200
     __global__ void __launch_bounds__(256) binary_periodic_kernel(const float* __restrict__ a, const float* __restrict__ v,
                                                                   float* __restrict__ out, IDX n, IDX period)
     {
+        after_earlier_kernels(a, v, out);
         if (VEC)
         {
             const IDX n4 = n >> 2, p4 = period >> 2; // period == 1: p4 == 0
@@ -107,10 +109,10 @@ namespace b200
                          ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(out) | (period == 1 ? 0 : reinterpret_cast<uintptr_t>(v))) & 15) == 0;
         const int64_t work = vec ? n / 4 : n, blocks = (work + 255) / 256, cap = b200::sm_count() * 16;
         const unsigned g = unsigned(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
-        if (vec && v_left) binary_periodic_kernel<OP, true, true, IDX><<<g, 256, 0, st>>>(a, v, out, n, period);
-        else if (vec) binary_periodic_kernel<OP, false, true, IDX><<<g, 256, 0, st>>>(a, v, out, n, period);
-        else if (v_left) binary_periodic_kernel<OP, true, false, IDX><<<g, 256, 0, st>>>(a, v, out, n, period);
-        else binary_periodic_kernel<OP, false, false, IDX><<<g, 256, 0, st>>>(a, v, out, n, period);
+        if (vec && v_left) launch(binary_periodic_kernel<OP, true, true, IDX>, g, 256, 0, st, a, v, out, n, period);
+        else if (vec) launch(binary_periodic_kernel<OP, false, true, IDX>, g, 256, 0, st, a, v, out, n, period);
+        else if (v_left) launch(binary_periodic_kernel<OP, true, false, IDX>, g, 256, 0, st, a, v, out, n, period);
+        else launch(binary_periodic_kernel<OP, false, false, IDX>, g, 256, 0, st, a, v, out, n, period);
     }
     // 32-bit indices wherever they reach: the modulo by the period is a division per vector
     template <int OP>
@@ -187,6 +189,7 @@ namespace b200
     template <typename T, int RANK>
     __global__ void __launch_bounds__(256) remap_small_kernel(const T* __restrict__ in, T* __restrict__ out, SmallDims d, uint32_t n)
     {
+        after_earlier_kernels(in, out);
         auto source = [&](uint32_t i) {
             uint32_t off = 0;
 #pragma unroll
@@ -221,6 +224,7 @@ namespace b200
     };
     __global__ void __launch_bounds__(256) permute_tiles_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, TileDims d)
     {
+        after_earlier_kernels(in, out);
         __shared__ uint32_t tile[32][33];
         uint32_t t = blockIdx.x;
         const uint32_t ty = d.tiles_x.div(t), tx = t - ty * d.tiles_x.d;
@@ -235,10 +239,13 @@ namespace b200
             t = q;
         }
         const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+        uint32_t v[4];
 #pragma unroll
-        for (uint32_t j = 0; j < 32; j += 8)
-            if (x0 + lane < d.nx && y0 + w + j < d.ny)
-                tile[w + j][lane] = in[in_off + (y0 + w + j) * d.in_y + x0 + lane];
+        for (uint32_t j = 0; j < 4; ++j)
+            v[j] = __ldg(in + in_off + min(y0 + w + 8 * j, d.ny - 1) * d.in_y + min(x0 + lane, d.nx - 1)); // all four under way
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j)
+            tile[w + 8 * j][lane] = v[j];
         __syncthreads();
 #pragma unroll
         for (uint32_t j = 0; j < 32; j += 8)
@@ -291,21 +298,21 @@ namespace b200
         }
         for (int a = 0; a < MAX_RANK; ++a)
             sd.dim[a] = FastDiv(a < r ? extent[a] : 1);
-        auto launch = [&](auto element) {
+        auto launch_as = [&](auto element) {
             using T = decltype(element);
             const T* i = static_cast<const T*>(in);
             T* o = static_cast<T*>(out);
             if (r <= 2)
-                remap_small_kernel<T, 2><<<grid, 256, 0, st>>>(i, o, sd, uint32_t(n));
+                launch(remap_small_kernel<T, 2>, grid, 256, 0, st, i, o, sd, uint32_t(n));
             else if (r <= 4)
-                remap_small_kernel<T, 4><<<grid, 256, 0, st>>>(i, o, sd, uint32_t(n));
+                launch(remap_small_kernel<T, 4>, grid, 256, 0, st, i, o, sd, uint32_t(n));
             else
-                remap_small_kernel<T, MAX_RANK><<<grid, 256, 0, st>>>(i, o, sd, uint32_t(n));
+                launch(remap_small_kernel<T, MAX_RANK>, grid, 256, 0, st, i, o, sd, uint32_t(n));
         };
         if (wide)
-            launch(uint4());
+            launch_as(uint4());
         else
-            launch(uint32_t());
+            launch_as(uint32_t());
     }
 
     // The tile form, where it pays: fewer than 2^31 elements and both last axes long enough to fill most of a tile.
@@ -340,7 +347,7 @@ namespace b200
         }
         t.tiles_x = FastDiv((t.nx + 31) / 32);
         t.tiles_y = FastDiv((t.ny + 31) / 32);
-        permute_tiles_kernel<<<unsigned(outer * t.tiles_x.d * t.tiles_y.d), 256, 0, st>>>(static_cast<const uint32_t*>(in), static_cast<uint32_t*>(out), t);
+        launch(permute_tiles_kernel, unsigned(outer * t.tiles_x.d * t.tiles_y.d), 256, 0, st, static_cast<const uint32_t*>(in), static_cast<uint32_t*>(out), t);
         return true;
     }
 
@@ -461,6 +468,7 @@ namespace b200
     __global__ void __cluster_dims__(EXTREME_CLUSTER, 1, 1) __launch_bounds__(1024)
         reduce_extreme_cluster_kernel(const float* __restrict__ in, float* __restrict__ out, int64_t n)
     {
+        after_earlier_kernels(in, out);
         __shared__ float partial[32];
         __shared__ float of_block[EXTREME_CLUSTER];
         asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); // this block runs: its shared memory may be written
@@ -490,6 +498,7 @@ namespace b200
     template <int OP>
     __global__ void __launch_bounds__(256) reduce_extreme_all_kernel(const float* __restrict__ in, float* __restrict__ out, int64_t n)
     {
+        after_earlier_kernels(in, out);
         __shared__ float partial[8];
         const float m = extreme_of_block<OP>(extreme_of_run<OP>(in, n, int64_t(blockIdx.x) * 256 + threadIdx.x, int64_t(gridDim.x) * 256), partial);
         if (threadIdx.x == 0)
@@ -505,6 +514,7 @@ namespace b200
 
     __global__ void fill_f32_kernel(float* out, float value, int64_t n)
     {
+        after_earlier_kernels(out);
         for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
             out[i] = value;
     }
@@ -599,6 +609,7 @@ namespace b200
         __shared__ double exp_table[rounded::EXP_STEPS];
         __shared__ float row_sum[R];
         rounded::load_exp_table(exp_table);
+        after_earlier_kernels(in, factor, out);
         const int stride = staged_row_stride(L, VEC), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
         const int64_t row0 = int64_t(blockIdx.x) * R;
         const int n_rows = int(min(rows - row0, int64_t(R)));
@@ -728,6 +739,7 @@ namespace b200
                                                                           float* __restrict__ out, int64_t rows, int L, float count, float eps,
                                                                           int64_t ahead)
     {
+        after_earlier_kernels(in, addend, gamma, beta, out);
         constexpr int R = NORM_ROWS, WARPS = ROW_THREADS / 32;
         extern __shared__ __align__(16) float tile[];
         __shared__ float row_mean[R], row_sd[R];
@@ -825,6 +837,7 @@ namespace b200
     {
         __shared__ __align__(16) rounded::ErfPoint table[rounded::ERF_ENTRIES];
         rounded::load_erf_table(table);
+        after_earlier_kernels(x, out);
         __syncthreads();
         const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, threads = int64_t(gridDim.x) * blockDim.x;
         if (VEC)
@@ -938,6 +951,7 @@ namespace b200
     __global__ void __launch_bounds__(WM* WN * 32) bmm_f32_kernel(const float* __restrict__ a, const float* __restrict__ bm, float* __restrict__ out,
                                                                   int M, int K, int N, uint32_t tiles_m, uint32_t tiles_n)
     {
+        after_earlier_kernels(a, bm, out);
         constexpr int TM = WM * MT * 8, TN = WN * NT * 8, KC = BMM_KC, THREADS = WM * WN * 32;
         constexpr int LDA = KC + 4, LDB = TN + 8; // fragment loads then touch 32 different banks
         extern __shared__ __align__(16) float panels[]; // two of { A [TM][LDA], B [KC][LDB] }
@@ -1078,9 +1092,9 @@ namespace b200
                 told.fetch_or(uint64_t(1) << (dev & 63), std::memory_order_relaxed);
             }
             if (vec)
-                bmm_f32_kernel<WM, WN, MT, NT, true><<<unsigned(blocks), WM * WN * 32, bytes, st>>>(a, b, out, M, K, N, tiles_m, tiles_n);
+                b200::launch(bmm_f32_kernel<WM, WN, MT, NT, true>, unsigned(blocks), WM * WN * 32, bytes, st, a, b, out, M, K, N, tiles_m, tiles_n);
             else
-                bmm_f32_kernel<WM, WN, MT, NT, false><<<unsigned(blocks), WM * WN * 32, bytes, st>>>(a, b, out, M, K, N, tiles_m, tiles_n);
+                b200::launch(bmm_f32_kernel<WM, WN, MT, NT, false>, unsigned(blocks), WM * WN * 32, bytes, st, a, b, out, M, K, N, tiles_m, tiles_n);
             return true;
         }
     };
@@ -1120,12 +1134,12 @@ extern "C" int b200_f32_binary(int op, const float* a, const float* b, float* ou
     const unsigned g = grid_for(n, 256);
     switch (op)
     {
-    case B200_F32_ADD: binary_kernel<B200_F32_ADD><<<g, 256, 0, st>>>(a, b, out, n); break;
-    case B200_F32_SUB: binary_kernel<B200_F32_SUB><<<g, 256, 0, st>>>(a, b, out, n); break;
-    case B200_F32_MUL: binary_kernel<B200_F32_MUL><<<g, 256, 0, st>>>(a, b, out, n); break;
-    case B200_F32_DIV: binary_kernel<B200_F32_DIV><<<g, 256, 0, st>>>(a, b, out, n); break;
-    case B200_F32_MAX: binary_kernel<B200_F32_MAX><<<g, 256, 0, st>>>(a, b, out, n); break;
-    default: binary_kernel<B200_F32_MIN><<<g, 256, 0, st>>>(a, b, out, n); break;
+    case B200_F32_ADD: launch(binary_kernel<B200_F32_ADD>, g, 256, 0, st, a, b, out, n); break;
+    case B200_F32_SUB: launch(binary_kernel<B200_F32_SUB>, g, 256, 0, st, a, b, out, n); break;
+    case B200_F32_MUL: launch(binary_kernel<B200_F32_MUL>, g, 256, 0, st, a, b, out, n); break;
+    case B200_F32_DIV: launch(binary_kernel<B200_F32_DIV>, g, 256, 0, st, a, b, out, n); break;
+    case B200_F32_MAX: launch(binary_kernel<B200_F32_MAX>, g, 256, 0, st, a, b, out, n); break;
+    default: launch(binary_kernel<B200_F32_MIN>, g, 256, 0, st, a, b, out, n); break;
     }
     return after_launch("b200_f32_binary");
 }
@@ -1310,23 +1324,23 @@ extern "C" int b200_reduce_f32(int op, const float* in, float* out, const int64_
         const bool small = n_red <= (int64_t(1) << 20);
         if (!small)
         {
-            fill_f32_kernel<<<1, 32, 0, st>>>(out, op == B200_REDUCE_MIN ? INFINITY : -INFINITY, 1);
+            launch(fill_f32_kernel, 1, 32, 0, st, out, op == B200_REDUCE_MIN ? INFINITY : -INFINITY, 1);
             g_launches.fetch_add(1, std::memory_order_relaxed);
         }
         const unsigned grid = small ? EXTREME_CLUSTER : unsigned(std::min<int64_t>((n_red + 8191) / 8192, sm_count() * 8));
         switch (op)
         {
         case B200_REDUCE_MAX:
-            small ? reduce_extreme_cluster_kernel<B200_REDUCE_MAX><<<grid, 1024, 0, st>>>(in, out, n_red)
-                  : reduce_extreme_all_kernel<B200_REDUCE_MAX><<<grid, 256, 0, st>>>(in, out, n_red);
+            small ? launch(reduce_extreme_cluster_kernel<B200_REDUCE_MAX>, grid, 1024, 0, st, in, out, n_red)
+                  : launch(reduce_extreme_all_kernel<B200_REDUCE_MAX>, grid, 256, 0, st, in, out, n_red);
             break;
         case B200_REDUCE_MIN:
-            small ? reduce_extreme_cluster_kernel<B200_REDUCE_MIN><<<grid, 1024, 0, st>>>(in, out, n_red)
-                  : reduce_extreme_all_kernel<B200_REDUCE_MIN><<<grid, 256, 0, st>>>(in, out, n_red);
+            small ? launch(reduce_extreme_cluster_kernel<B200_REDUCE_MIN>, grid, 1024, 0, st, in, out, n_red)
+                  : launch(reduce_extreme_all_kernel<B200_REDUCE_MIN>, grid, 256, 0, st, in, out, n_red);
             break;
         default:
-            small ? reduce_extreme_cluster_kernel<B200_REDUCE_MAX_ABS><<<grid, 1024, 0, st>>>(in, out, n_red)
-                  : reduce_extreme_all_kernel<B200_REDUCE_MAX_ABS><<<grid, 256, 0, st>>>(in, out, n_red);
+            small ? launch(reduce_extreme_cluster_kernel<B200_REDUCE_MAX_ABS>, grid, 1024, 0, st, in, out, n_red)
+                  : launch(reduce_extreme_all_kernel<B200_REDUCE_MAX_ABS>, grid, 256, 0, st, in, out, n_red);
         }
     }
     else if (op != B200_REDUCE_SUM && n_out <= 4096 && n_red >= 1024)
@@ -1382,7 +1396,7 @@ extern "C" int b200_softmax_rows_scaled_f32(const float* x, const float* factor,
         size_t bytes;
         if (!staged_bytes(kernel, told, SOFTMAX_ROWS, L, vec, bytes))
             return false;
-        kernel<<<unsigned(grid), SOFTMAX_THREADS, bytes, st>>>(x, factor, out, rows, L);
+        b200::launch(kernel, unsigned(grid), SOFTMAX_THREADS, bytes, st, x, factor, out, rows, L);
         return true;
     };
     static std::atomic<uint64_t> told[2][6];
@@ -1436,7 +1450,7 @@ extern "C" int b200_layer_norm_rows_sum_f32(const float* x, const float* addend,
             return false;
         // rows that run at the same time: what follows a tile on its SM starts that much further on
         const int64_t resident = std::min<int64_t>(200 * 1024 / int64_t(bytes + 1024), 2048 / ROW_THREADS);
-        kernel<<<unsigned(grid), ROW_THREADS, bytes, st>>>(x, addend, gamma, beta, out, rows, L, count, epsilon, resident * sm_count() * NORM_ROWS);
+        b200::launch(kernel, unsigned(grid), ROW_THREADS, bytes, st, x, addend, gamma, beta, out, rows, L, count, epsilon, resident * sm_count() * NORM_ROWS);
         return true;
     };
     static std::atomic<uint64_t> told[4];
@@ -1461,9 +1475,9 @@ extern "C" int b200_gelu_f32(const float* x, float* out, int64_t n, void* stream
     // blocks that stay (each copies the table first); short tensors get about two vectors per thread
     const unsigned grid = unsigned(std::min<int64_t>((n + 2047) / 2048, int64_t(sm_count()) * 6));
     if (vec)
-        gelu_kernel<true><<<grid, 256, 0, st>>>(x, out, n);
+        launch(gelu_kernel<true>, grid, 256, 0, st, x, out, n);
     else
-        gelu_kernel<false><<<grid, 256, 0, st>>>(x, out, n);
+        launch(gelu_kernel<false>, grid, 256, 0, st, x, out, n);
     return after_launch("b200_gelu_f32");
 }
 

@@ -165,6 +165,7 @@ namespace b200
     __global__ void __launch_bounds__(QT, QBLOCKS) quantize_stream_kernel(const float* __restrict__ x, const float* __restrict__ scale,
                                                                           const Q* __restrict__ zp, Q* __restrict__ out, RowMap m, bool fast)
     {
+        after_earlier_kernels(x, scale, zp, out);
         constexpr int CHUNK = QT * U * 4;
         __shared__ RowScale table[ROWS ? MAX_ROWS : 1];
         const int64_t base = int64_t(blockIdx.x) * CHUNK;
@@ -295,6 +296,7 @@ namespace b200
     __global__ void __launch_bounds__(QT, QBLOCKS) dequantize_stream_kernel(const Q* __restrict__ in, const float* __restrict__ scale,
                                                                             const Q* __restrict__ zp, float* __restrict__ out, RowMap m)
     {
+        after_earlier_kernels(in, scale, zp, out);
         constexpr int CHUNK = QT * U * 4;
         __shared__ RowScale table[ROWS ? MAX_ROWS : 1];
         const int64_t base = int64_t(blockIdx.x) * CHUNK;
@@ -470,13 +472,13 @@ namespace b200
             const bool fast = g_fast_division.load(std::memory_order_relaxed) != 0, small = small_tensor(p.total);
             const unsigned grid = stream_grid(p.total, small ? 1 : QU);
             if (p.rows > 1 && small)
-                quantize_stream_kernel<Q, MODE, FAST, true, 1><<<grid, QT, 0, st>>>(x, scale, z, o, m, fast);
+                launch(quantize_stream_kernel<Q, MODE, FAST, true, 1>, grid, QT, 0, st, x, scale, z, o, m, fast);
             else if (p.rows > 1)
-                quantize_stream_kernel<Q, MODE, FAST, true, QU><<<grid, QT, 0, st>>>(x, scale, z, o, m, fast);
+                launch(quantize_stream_kernel<Q, MODE, FAST, true, QU>, grid, QT, 0, st, x, scale, z, o, m, fast);
             else if (small)
-                quantize_stream_kernel<Q, MODE, FAST, false, 1><<<grid, QT, 0, st>>>(x, scale, z, o, m, fast);
+                launch(quantize_stream_kernel<Q, MODE, FAST, false, 1>, grid, QT, 0, st, x, scale, z, o, m, fast);
             else
-                quantize_stream_kernel<Q, MODE, FAST, false, QU><<<grid, QT, 0, st>>>(x, scale, z, o, m, fast);
+                launch(quantize_stream_kernel<Q, MODE, FAST, false, QU>, grid, QT, 0, st, x, scale, z, o, m, fast);
         }
         else
             quantize_generic_kernel<Q, MODE><<<generic_grid(p.total), QT, 0, st>>>(x, scale, z, o, p.total, p.dims);
@@ -513,13 +515,13 @@ namespace b200
             const bool small = small_tensor(p.total);
             const unsigned grid = stream_grid(p.total, small ? 1 : QU);
             if (p.rows > 1 && small)
-                dequantize_stream_kernel<Q, true, 1><<<grid, QT, 0, st>>>(q, scale, z, out, m);
+                launch(dequantize_stream_kernel<Q, true, 1>, grid, QT, 0, st, q, scale, z, out, m);
             else if (p.rows > 1)
-                dequantize_stream_kernel<Q, true, QU><<<grid, QT, 0, st>>>(q, scale, z, out, m);
+                launch(dequantize_stream_kernel<Q, true, QU>, grid, QT, 0, st, q, scale, z, out, m);
             else if (small)
-                dequantize_stream_kernel<Q, false, 1><<<grid, QT, 0, st>>>(q, scale, z, out, m);
+                launch(dequantize_stream_kernel<Q, false, 1>, grid, QT, 0, st, q, scale, z, out, m);
             else
-                dequantize_stream_kernel<Q, false, QU><<<grid, QT, 0, st>>>(q, scale, z, out, m);
+                launch(dequantize_stream_kernel<Q, false, QU>, grid, QT, 0, st, q, scale, z, out, m);
         }
         else
             dequantize_generic_kernel<Q><<<generic_grid(p.total), QT, 0, st>>>(q, scale, z, out, p.total, p.dims);
