@@ -52,22 +52,25 @@ def build_kernels(force=False, verbose=False):
 
 
 TORCH_OPS = os.path.join(HERE, "_torch_ops.so")
+FASTCALL = os.path.join(HERE, "_fastcall.so")
 
 
-def build_torch_ops(force=False):
-    """g++ the native half of ngraph_b200/ops.py (a CPython extension over torch's C++ tensors)."""
-    src = os.path.join(CSRC, "torch_ops.cpp")
-    if not force and _newer(TORCH_OPS, [src, os.path.join(ROOT, "include", "b200_kernels.h")]):
-        return TORCH_OPS
+def build_python(force=False):
+    """g++ the two CPython extensions: the native callables of lib.py, and the native half of ops.py over torch's C++ tensors."""
     import sysconfig
-    import torch
-    base = os.path.dirname(torch.__file__)
-    libs = os.path.join(base, "lib")
-    cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-w", "-shared", "-fvisibility=hidden", "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch.compiled_with_cxx11_abi()), "-I" + os.path.join(ROOT, "include"),
-           "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(base, "include"), "-I" + os.path.join(base, "include", "torch", "csrc", "api", "include"),
-           "-I/usr/local/cuda/include", src, "-o", TORCH_OPS, "-L" + libs, "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
-    subprocess.check_call(cmd)
-    return TORCH_OPS
+    common = ["g++", "-std=c++17", "-O2", "-fPIC", "-w", "-shared", "-fvisibility=hidden", "-I" + os.path.join(ROOT, "include"), "-I" + sysconfig.get_paths()["include"]]
+    header = os.path.join(ROOT, "include", "b200_kernels.h")
+    src = os.path.join(CSRC, "fastcall.cpp")
+    if force or not _newer(FASTCALL, [src, header]):
+        subprocess.check_call(common + [src, "-o", FASTCALL])
+    src = os.path.join(CSRC, "torch_ops.cpp")
+    if force or not _newer(TORCH_OPS, [src, header]):
+        import torch
+        base = os.path.dirname(torch.__file__)
+        subprocess.check_call(common + ["-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch.compiled_with_cxx11_abi()), "-I" + os.path.join(base, "include"),
+                                        "-I" + os.path.join(base, "include", "torch", "csrc", "api", "include"), "-I/usr/local/cuda/include", src, "-o", TORCH_OPS,
+                                        "-L" + os.path.join(base, "lib"), "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"])
+    return FASTCALL, TORCH_OPS
 
 
 PLUGIN_LIB = os.path.join(HERE, "libb200_backend.so")
@@ -148,6 +151,6 @@ def build_capi(force=False):
 
 if __name__ == "__main__":
     print(build_kernels(force="--force" in sys.argv, verbose="-v" in sys.argv))
-    print(build_torch_ops(force="--force" in sys.argv))
+    print(*build_python(force="--force" in sys.argv))
     print(build_plugin(force="--force" in sys.argv))
     print(build_capi(force="--force" in sys.argv))

@@ -1,15 +1,22 @@
 """ctypes binding of the C ABI declared in include/b200_kernels.h.
 
+The entry points that launch work are native callables (csrc/fastcall.cpp) that take what the ctypes functions take.
 There is no fallback of any kind: if ``libb200_kernels.so`` has not been built, importing this
 module raises; if a call returns a non-zero status, ``check`` raises ``B200Error``.
 """
 import ctypes
 import os
 
+try:
+    from . import _fastcall
+except ImportError as e:
+    raise ImportError("ngraph_b200/_fastcall.so is missing: run `python -m ngraph_b200.build`") from e
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("B200_KERNELS_LIB", os.path.join(HERE, "libb200_kernels.so"))
 
 U8, I8, I32, F32 = 0, 1, 2, 3
+ADDRESS = {}  # entry point -> address in the loaded library
 
 
 class B200Error(RuntimeError):
@@ -103,6 +110,8 @@ def _load():
         fn = getattr(lib, name)
         fn.restype = res
         fn.argtypes = args
+        ADDRESS[name] = ctypes.cast(fn, ctypes.c_void_p).value
+        setattr(lib, name, _fastcall.wrap(name, ADDRESS[name], fn))  # what launches work: without ctypes' conversion per call
     return lib
 
 

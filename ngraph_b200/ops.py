@@ -19,7 +19,7 @@ except ImportError as e:
     raise ImportError("ngraph_b200/_torch_ops.so is missing or does not match this torch: run `python -m ngraph_b200.build`; "
                       "there is no Python fallback") from e
 
-_native.bind(check, {name: ctypes.cast(getattr(LIB, name), ctypes.c_void_p).value for name in (
+_native.bind(check, {name: lib.ADDRESS[name] for name in (
     "b200_quantize", "b200_dequantize", "b200_qgemm", "b200_qconv", "b200_qconv_packed", "b200_qconv_out_shape", "b200_nchw_to_nhwc_u8",
     "b200_nhwc_to_nchw_u8", "b200_transpose_u8", "b200_maxpool_nhwc_u8", "b200_global_avgpool_q_nhwc_u8")})
 

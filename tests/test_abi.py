@@ -82,3 +82,20 @@ def test_argument_validation_of_the_glue_entry_points():
     e.round_half_away, e.out_type = 2, lib.U8                                # raw accumulators exist as int32 only
     assert L.b200_qgemm(None, lib.U8, None, None, 4, 4, 16, ctypes.byref(e), None) == -1
     assert L.b200_requant_zero_points(None, None, None, None, ctypes.byref(e), None, None) == -1
+
+
+def test_native_callables_take_what_ctypes_takes():
+    """integers, None, c_void_p, arrays and floats are converted natively; byref objects, wrong types and wrong counts go through
+    (or raise in) the ctypes function"""
+    import ctypes
+    L = lib.LIB
+    s, e = ctypes.c_void_p(7), lib.Epilogue()
+    assert L.b200_f32_binary(99, 1, 2, 3, 4, None) == -1                                  # no such op: refused before any pointer is used
+    assert L.b200_quantize(1, 2, 3, 4, 1, (ctypes.c_int64 * 2)(3, 4), 2, (ctypes.c_int64 * 1)(), 0, 77, s) == -1
+    assert L.b200_layer_norm_rows_sum_f32(1, 2, 3, 4, 5, -1, 3, ctypes.c_float(1e-5), s) == -1
+    assert L.b200_layer_norm_rows_f32(1, 2, 3, 4, -1, 3, 1e-5, None) == -1
+    assert L.b200_qgemm_packed(1, 9, 2, 3, 4, 5, 16, ctypes.byref(e), s) == -1
+    for call in (lambda: L.b200_f32_binary(1, 2), lambda: L.b200_f32_binary("x", 1, 2, 3, 4, None), lambda: L.b200_f32_binary(0, 1.5, 2, 3, 4, None),
+                 lambda: L.b200_quantize(1, 2, 3, 4, 1, (ctypes.c_int32 * 2)(3, 4), 2, None, 0, 0, s), lambda: L.b200_qgemm(1, 0, 2, 3, 4, 5, 16, 5, s)):
+        with pytest.raises((TypeError, ctypes.ArgumentError)):
+            call()
