@@ -285,6 +285,25 @@ namespace b200
                 : "r"(taddr)
                 : "memory");
         }
+        // 16 lanes x 32 columns (the 16x256b shape four times): registers 4j .. 4j + 3 hold, of columns 8j + 2 (lane % 4) and the next,
+        // row lane / 4 and then row lane / 4 + 8
+        __device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, uint32_t (&r)[16])
+        {
+            asm volatile(
+                "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+                "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                : "r"(taddr)
+                : "memory");
+        }
+        // Waits for this thread's tensor-memory loads; the registers pass through, so that nothing reads them ahead of the wait.
+        __device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[16])
+        {
+            asm volatile("tcgen05.wait::ld.sync.aligned;"
+                         : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]),
+                           "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
+        }
         __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
         // Shared-memory matrix descriptor for a K-major operand tile whose rows are `row_bytes`
