@@ -78,6 +78,22 @@ namespace b200
     }
 #endif
 
+    // n / d for 0 <= n < 2^31 by a multiplication: ceil(2^(31 + l) / d) with l = ceil(log2 d) is exact over that range.
+    struct FastDiv
+    {
+        uint32_t d, mul, shift;
+        FastDiv() = default;
+        explicit FastDiv(uint32_t divisor) : d(divisor), mul(0), shift(0)
+        {
+            while ((uint64_t(1) << shift) < d)
+                ++shift;
+            mul = d > 1 ? uint32_t(((uint64_t(1) << (31 + shift)) + d - 1) / d) : 0;
+        }
+#ifdef __CUDACC__
+        __device__ __forceinline__ uint32_t div(uint32_t n) const { return d > 1 ? __umulhi(n, mul) >> (shift - 1) : n; }
+#endif
+    };
+
     inline size_t dtype_size(int t)
     {
         return (t == B200_U8 || t == B200_I8) ? 1 : 4;

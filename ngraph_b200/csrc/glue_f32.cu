@@ -158,20 +158,6 @@ namespace b200
             out[i] = OP == B200_F32_EXP ? rounded::exp_rounded(x[i], exp_table) : rounded::erf_rounded(x[i], erf_table);
     }
 
-    // n / d for 0 <= n < 2^31 by a multiplication: ceil(2^(31 + l) / d) with l = ceil(log2 d) is exact over that range.
-    struct FastDiv
-    {
-        uint32_t d, mul, shift;
-        FastDiv() = default;
-        explicit FastDiv(uint32_t divisor) : d(divisor), mul(0), shift(0)
-        {
-            while ((uint64_t(1) << shift) < d)
-                ++shift;
-            mul = d > 1 ? uint32_t(((uint64_t(1) << (31 + shift)) + d - 1) / d) : 0;
-        }
-        __device__ __forceinline__ uint32_t div(uint32_t n) const { return d > 1 ? __umulhi(n, mul) >> (shift - 1) : n; }
-    };
-
     // out[idx] = in[mapped(idx)] for 4-byte elements: Broadcast (stride 0 on the new axes) and axis permutations.
     // T: one element (uint32_t) or four neighbours along a last axis that both tensors share (uint4).  The general form
     // divides 64-bit indices; remap_small_kernel serves whatever has fewer than 2^31 elements, RANK axes after merging.

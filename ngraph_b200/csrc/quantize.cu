@@ -12,15 +12,13 @@
 //             block into a small shared-memory table while its loads are under way.
 //   generic - one element per thread with the scale index recomputed from the
 //             coordinates; any axis set, any alignment.
+#include <type_traits>
 #include "common.cuh"
 
 namespace b200
 {
     constexpr int QT = 256;                // threads per block
-    constexpr int QU = 4;                  // independent 4-element vectors per thread (1 for small tensors)
-    constexpr int QBLOCKS = 6;             // blocks an SM should hold (registers are kept below 42 for it)
     constexpr int MIN_INNER = 16;          // shortest row the streaming kernels take
-    constexpr int MAX_ROWS = QT * QU * 4 / MIN_INNER + 2; // rows a block can touch
 
     struct ProjDims
     {
@@ -66,7 +64,8 @@ namespace b200
     struct RowMap
     {
         int64_t total;
-        uint32_t inner, n_scales, rows;
+        uint32_t inner;
+        FastDiv n_scales;
         uint64_t inner_inv64;  // ceil(2^64 / inner): row of a block's first element
         uint32_t inner_inv32;  // ceil(2^32 / inner): rows inside a block, for inner < the block's elements
     };
@@ -79,10 +78,9 @@ namespace b200
     }
 
     // Row (counted from the block's first) of the element `off` = r0 + local, and the elements left in that row.
-    template <int CHUNK>
     __device__ __forceinline__ uint32_t local_row(const RowMap& m, uint32_t off, uint32_t& left)
     {
-        const uint32_t r = m.inner >= CHUNK ? (off >= m.inner ? 1u : 0u) : __umulhi(off, m.inner_inv32);
+        const uint32_t r = __umulhi(off, m.inner_inv32);
         left = (r + 1) * m.inner - off;
         return r;
     }
@@ -91,14 +89,14 @@ namespace b200
     // (correctly rounded reciprocal) and each quotient is  q0 = RN(x*y);  e = x - q0*s (exact in one FMA);
     // q = RN(q0 + e*y), which is the correctly rounded x/s (Markstein's division theorem) whenever s is a normal number
     // whose significand is not all ones and nothing over/underflows.  y == 0 marks a scale that fails that test (or the
-    // switched-off path): its row takes the IEEE division.  Quotients of magnitude >= 2^24, whose 8-bit result saturates
+    // switched-off path): a block that meets one takes the IEEE division instead.  Quotients of magnitude >= 2^24, whose 8-bit result saturates
     // regardless of the last bit, skip the correction (see common.cuh).  Every output byte equals the plain
     // x / s -> rounding -> +zero_point -> clamp sequence of the reference.  An int32 output can be large enough for
     // the last bit of a quotient beyond 2^24 to matter, so it always divides.
     template <typename Q, int MODE, bool FAST>
     __device__ __forceinline__ void quantize4(const float4& v, float s, float y, int zi, Q (&r)[4])
     {
-        if (FAST && y != 0.0f)
+        if (FAST)
         {
             const int lo = int(QLimits<Q>::lo) - zi, hi = int(QLimits<Q>::hi) - zi;
             constexpr bool directed = MODE == B200_ROUND_TOWARD_INFINITY || MODE == B200_ROUND_TOWARD_ZERO || MODE == B200_ROUND_UP ||
@@ -144,30 +142,80 @@ namespace b200
         return e;
     }
 
-    // The scales of the rows a block touches, looked up by as many threads.
-    template <typename Q, bool FAST, int CHUNK>
-    __device__ __forceinline__ void fill_table(RowScale* table, const float* scale, const Q* zp, const RowMap& m, uint32_t row, uint32_t r0, bool fast)
+    // How a block finds the scale of an element, by the rows it can touch.
+    enum Rows
     {
-        const uint32_t n = min((r0 + uint32_t(CHUNK) - 1) / m.inner + 1, m.rows - row);
-        for (uint32_t i = threadIdx.x; i < n; i += QT)
-            table[i] = row_scale<Q, FAST>(scale, zp, (row + i) % m.n_scales, fast);
-    }
+        ONE_ROW,  // per tensor: one scale
+        TWO_ROWS, // rows at least as long as a block's elements: the scales of the block's first row and of the next one, in
+                  // registers, and the place where the second begins
+        MANY_ROWS // shorter ones: a table in shared memory, filled by as many threads as there are rows
+    };
+    template <typename Q, bool FAST, int ROWS, int CHUNK>
+    struct BlockScales
+    {
+        RowScale e0, e1;
+        uint32_t boundary; // TWO_ROWS: first element of the second row, CHUNK if there is none in the block
+        uint32_t r0;
+        RowScale* table;
 
-    // ROWS: more than one row.  U vectors of four elements per thread.  A block that lies inside one row (every block of a
-    // per-tensor call, nearly every block of a call with long rows) keeps its scale in registers; only the others pay for
-    // the table, its barrier and the test for vectors that run into the next row.
-    // Bound by HBM for large tensors (f32 -> u8, round to even, 1 GB per tensor: 6.5 TB/s, a plain copy's rate; the half-way
-    // modes 6.2, the directed ones 6.1-6.3; per channel 6.2) and by load latency below some 100 MB.  Walking the tensor flat
-    // instead of row by row is what keeps odd row lengths on 128-bit accesses: [24, 64, 113, 113] per channel 182 -> 24 us,
-    // [128, 64, 28, 28] 16 us.  Six blocks per SM (40 registers) measured best: at eight the spills of the division's slow
-    // path cost 10 %.
-    template <typename Q, int MODE, bool FAST, bool ROWS, int U>
-    __global__ void __launch_bounds__(QT, QBLOCKS) quantize_stream_kernel(const float* __restrict__ x, const float* __restrict__ scale,
+        // true if every scale of the block admits the fast division
+        __device__ __forceinline__ bool find(const RowMap& m, RowScale* shared, const float* scale, const Q* zp, int64_t base, uint32_t rem, bool fast)
+        {
+            boundary = CHUNK;
+            if (ROWS == ONE_ROW)
+            {
+                e0 = e1 = row_scale<Q, FAST>(scale, zp, 0, fast);
+                return e0.y != 0.0f;
+            }
+            uint32_t row;
+            block_row(m, base, row, r0);
+            const uint32_t first = row - m.n_scales.div(row) * m.n_scales.d;
+            if (ROWS == TWO_ROWS)
+            {
+                e0 = e1 = row_scale<Q, FAST>(scale, zp, first, fast);
+                if (m.inner - r0 < rem)
+                {
+                    boundary = m.inner - r0;
+                    e1 = row_scale<Q, FAST>(scale, zp, first + 1 == m.n_scales.d ? 0 : first + 1, fast);
+                }
+                return e0.y != 0.0f && e1.y != 0.0f;
+            }
+            table = shared;
+            uint32_t left;
+            const uint32_t n = local_row(m, r0 + rem - 1, left) + 1;
+            bool ok = true;
+            for (uint32_t i = threadIdx.x; i < n; i += QT)
+            {
+                const RowScale e = row_scale<Q, FAST>(scale, zp, row + i - m.n_scales.div(row + i) * m.n_scales.d, fast);
+                ok = ok && e.y != 0.0f;
+                shared[i] = e;
+            }
+            return __syncthreads_and(ok);
+        }
+        __device__ __forceinline__ RowScale of(const RowMap& m, uint32_t i) const
+        {
+            if (ROWS == ONE_ROW)
+                return e0;
+            if (ROWS == TWO_ROWS)
+                return i >= boundary ? e1 : e0;
+            uint32_t left;
+            return table[local_row(m, r0 + i, left)];
+        }
+    };
+
+    // U vectors of four elements per thread (see vectors_per_thread); blocks_for: what the registers are kept down for.
+    constexpr int blocks_for(int u) { return u >= 8 ? 4 : 6; }
+    // Bound by HBM for large tensors (f32 -> u8 at 1 GB, per tensor and per channel: round to even 6.7 TB/s, a plain copy's rate,
+    // the half-way modes 6.5-6.7, the directed ones 6.2-6.7) and by load latency below some 100 MB.  Walking the tensor
+    // flat instead of row by row is what keeps odd row lengths on 128-bit accesses: [24, 64, 113, 113] per channel 182 -> 22 us,
+    // [4000, 64, 15, 13] 458 -> 55 us.
+    template <typename Q, int MODE, bool FAST, int ROWS, int U>
+    __global__ void __launch_bounds__(QT, blocks_for(U)) quantize_stream_kernel(const float* __restrict__ x, const float* __restrict__ scale,
                                                                           const Q* __restrict__ zp, Q* __restrict__ out, RowMap m, bool fast)
     {
         after_earlier_kernels(x, scale, zp, out);
         constexpr int CHUNK = QT * U * 4;
-        __shared__ RowScale table[ROWS ? MAX_ROWS : 1];
+        __shared__ RowScale table[ROWS == MANY_ROWS ? CHUNK / MIN_INNER + 2 : 1];
         const int64_t base = int64_t(blockIdx.x) * CHUNK;
         const uint32_t rem = uint32_t(min(m.total - base, int64_t(CHUNK)));
         x += base;
@@ -180,42 +228,26 @@ namespace b200
             if (off + 4 <= rem)
                 v[u] = *reinterpret_cast<const float4*>(x + off);
         }
-        uint32_t row = 0, r0 = 0;
-        if (ROWS)
-            block_row(m, base, row, r0);
-        if (!ROWS || r0 + rem <= m.inner)
+        BlockScales<Q, FAST, ROWS, CHUNK> scales;
+        const bool all_fast = scales.find(m, table, scale, zp, base, rem, fast);
+        auto one = [&](uint32_t i, const RowScale& e) { out[i] = quantize_one<Q, MODE>(x[i], e.s, static_cast<float>(static_cast<Q>(e.zp))); };
+        if (FAST && !all_fast)
         {
-            const RowScale e = row_scale<Q, FAST>(scale, zp, ROWS ? row % m.n_scales : 0, fast);
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-            {
-                const uint32_t off = (u * QT + threadIdx.x) * 4;
-                if (off + 4 <= rem)
-                {
-                    Q r[4];
-                    quantize4<Q, MODE, FAST>(v[u], e.s, e.y, e.zp, r);
-                    store4<Q>(out + off, r[0], r[1], r[2], r[3]);
-                }
-                else // the last, partial vector of the tensor
-                    for (uint32_t i = off; i < rem; ++i)
-                        out[i] = quantize_one<Q, MODE>(x[i], e.s, static_cast<float>(static_cast<Q>(e.zp)));
-            }
+            for (uint32_t i = threadIdx.x; i < rem; i += QT)
+                one(i, scales.of(m, i));
             return;
         }
-        fill_table<Q, FAST, CHUNK>(table, scale, zp, m, row, r0, fast);
-        __syncthreads();
 #pragma unroll
         for (int u = 0; u < U; ++u)
         {
             const uint32_t off = (u * QT + threadIdx.x) * 4;
-            if (off >= rem)
+            if (off + 4 > rem)
                 break;
-            uint32_t left, lr = local_row<CHUNK>(m, r0 + off, left);
-            if (off + 4 <= rem)
+            Q r[4];
+            if (ROWS == MANY_ROWS)
             {
                 // four elements with the vector's row; where it runs into the next row, once more with that row's scale
-                Q r[4];
-                uint32_t done = 0;
+                uint32_t left, lr = local_row(m, scales.r0 + off, left), done = 0;
 #pragma unroll 1
                 do
                 {
@@ -228,15 +260,22 @@ namespace b200
                     done = left;
                     left = 4;
                 } while (done < 4);
-                store4<Q>(out + off, r[0], r[1], r[2], r[3]);
             }
             else
-                for (uint32_t i = off; i < rem; ++i)
-                {
-                    const RowScale e = table[i - off >= left ? lr + 1 : lr];
-                    out[i] = quantize_one<Q, MODE>(x[i], e.s, static_cast<float>(static_cast<Q>(e.zp)));
-                }
+            {
+                const RowScale e = scales.of(m, off);
+                quantize4<Q, MODE, FAST>(v[u], e.s, e.y, e.zp, r);
+            }
+            store4<Q>(out + off, r[0], r[1], r[2], r[3]);
         }
+        // what the whole vectors leave: the elements that a vector of the first row has of the second (the thread that wrote
+        // the vector writes them again), and the last, partial vector of the tensor
+        if (ROWS == TWO_ROWS && (scales.boundary & 3) != 0 && threadIdx.x == (scales.boundary / 4) % QT)
+            for (uint32_t i = scales.boundary; (i & 3) != 0 && i < rem; ++i)
+                one(i, scales.e1);
+        if ((rem & 3) != 0 && threadIdx.x == (rem / 4) % QT)
+            for (uint32_t i = rem & ~3u; i < rem; ++i)
+                one(i, scales.of(m, i));
     }
 
     template <typename Q, int MODE>
@@ -292,13 +331,13 @@ namespace b200
     };
 
     // The same walk as quantize_stream_kernel.
-    template <typename Q, bool ROWS, int U>
-    __global__ void __launch_bounds__(QT, QBLOCKS) dequantize_stream_kernel(const Q* __restrict__ in, const float* __restrict__ scale,
+    template <typename Q, int ROWS, int U>
+    __global__ void __launch_bounds__(QT, blocks_for(U)) dequantize_stream_kernel(const Q* __restrict__ in, const float* __restrict__ scale,
                                                                             const Q* __restrict__ zp, float* __restrict__ out, RowMap m)
     {
         after_earlier_kernels(in, scale, zp, out);
         constexpr int CHUNK = QT * U * 4;
-        __shared__ RowScale table[ROWS ? MAX_ROWS : 1];
+        __shared__ RowScale table[ROWS == MANY_ROWS ? CHUNK / MIN_INNER + 2 : 1];
         const int64_t base = int64_t(blockIdx.x) * CHUNK;
         const uint32_t rem = uint32_t(min(m.total - base, int64_t(CHUNK)));
         in += base;
@@ -311,45 +350,40 @@ namespace b200
             if (off + 4 <= rem)
                 v[u].load(in + off);
         }
-        uint32_t row = 0, r0 = 0;
-        if (ROWS)
-            block_row(m, base, row, r0);
-        const bool one_row = !ROWS || r0 + rem <= m.inner;
-        RowScale e;
-        if (one_row)
-            e = row_scale<Q, false>(scale, zp, ROWS ? row % m.n_scales : 0, false);
-        else
-        {
-            fill_table<Q, false, CHUNK>(table, scale, zp, m, row, r0, false);
-            __syncthreads();
-        }
+        BlockScales<Q, false, ROWS, CHUNK> scales;
+        scales.find(m, table, scale, zp, base, rem, false);
 #pragma unroll
         for (int u = 0; u < U; ++u)
         {
             const uint32_t off = (u * QT + threadIdx.x) * 4;
-            if (off >= rem)
+            if (off + 4 > rem)
                 break;
             uint32_t left = 4;
-            RowScale e2 = e;
-            if (!one_row)
+            RowScale e, e2;
+            if (ROWS == MANY_ROWS)
             {
-                const uint32_t lr = local_row<CHUNK>(m, r0 + off, left);
+                const uint32_t lr = local_row(m, scales.r0 + off, left);
                 e = table[lr];
-                e2 = left < min(4u, rem - off) ? table[lr + 1] : e;
-            }
-            if (off + 4 <= rem)
-            {
-                float4 r;
-                r.x = dequantize_one<Q>(v[u].get(0), e.zp, e.s);
-                r.y = dequantize_one<Q>(v[u].get(1), left > 1 ? e.zp : e2.zp, left > 1 ? e.s : e2.s);
-                r.z = dequantize_one<Q>(v[u].get(2), left > 2 ? e.zp : e2.zp, left > 2 ? e.s : e2.s);
-                r.w = dequantize_one<Q>(v[u].get(3), left > 3 ? e.zp : e2.zp, left > 3 ? e.s : e2.s);
-                *reinterpret_cast<float4*>(out + off) = r;
+                e2 = left < 4 ? table[lr + 1] : e;
             }
             else
-                for (uint32_t i = off; i < rem; ++i)
-                    out[i] = i - off < left ? dequantize_one<Q>(in[i], e.zp, e.s) : dequantize_one<Q>(in[i], e2.zp, e2.s);
+                e = e2 = scales.of(m, off);
+            float4 r;
+            r.x = dequantize_one<Q>(v[u].get(0), e.zp, e.s);
+            r.y = dequantize_one<Q>(v[u].get(1), left > 1 ? e.zp : e2.zp, left > 1 ? e.s : e2.s);
+            r.z = dequantize_one<Q>(v[u].get(2), left > 2 ? e.zp : e2.zp, left > 2 ? e.s : e2.s);
+            r.w = dequantize_one<Q>(v[u].get(3), left > 3 ? e.zp : e2.zp, left > 3 ? e.s : e2.s);
+            *reinterpret_cast<float4*>(out + off) = r;
         }
+        if (ROWS == TWO_ROWS && (scales.boundary & 3) != 0 && threadIdx.x == (scales.boundary / 4) % QT)
+            for (uint32_t i = scales.boundary; (i & 3) != 0 && i < rem; ++i)
+                out[i] = dequantize_one<Q>(in[i], scales.e1.zp, scales.e1.s);
+        if ((rem & 3) != 0 && threadIdx.x == (rem / 4) % QT)
+            for (uint32_t i = rem & ~3u; i < rem; ++i)
+            {
+                const RowScale e = scales.of(m, i);
+                out[i] = dequantize_one<Q>(in[i], e.zp, e.s);
+            }
     }
 
     template <typename Q>
@@ -433,21 +467,28 @@ namespace b200
     {
         if (!p.rows_ok || ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15))
             return false;
-        if (p.rows > 1 && (p.inner < MIN_INNER || p.inner > (int64_t(1) << 30) || p.rows > (int64_t(1) << 31) || p.total > (int64_t(1) << 33)))
+        if (p.rows > 1 && (p.inner < MIN_INNER || p.inner > (int64_t(1) << 30) || p.rows >= (int64_t(1) << 31) || p.total > (int64_t(1) << 33)))
             return false; // beyond these the 64-bit reciprocal below is no longer exact (total * inner < 2^64)
         if (p.total / (QT * 4) >= (int64_t(1) << 31) - 1)
             return false;
         m.total = p.total;
-        m.rows = uint32_t(p.rows);
-        m.n_scales = uint32_t(p.n_scales);
+        m.n_scales = p.rows > 1 ? FastDiv(uint32_t(p.n_scales)) : FastDiv(1);
         m.inner = p.rows > 1 ? uint32_t(p.inner) : 0;
         m.inner_inv64 = p.rows > 1 ? ~uint64_t(0) / uint64_t(p.inner) + 1 : 0;
         m.inner_inv32 = p.rows > 1 ? uint32_t(0xFFFFFFFFull / uint64_t(p.inner) + 1) : 0;
         return true;
     }
 
-    // Vectors per thread: one while that is what it takes to give every SM two blocks, else four.
-    static bool small_tensor(int64_t total) { return total < int64_t(sm_count()) * 2 * QT * QU * 4; }
+    // Vectors per thread.  Few while that is what it takes for the grid to be started early (`launch`: two blocks per SM): 1 MB of
+    // f32 in 1.2 us, 2 MB in 1.4 us.  Eight in large Quantize calls, where the look-up of a block's scales weighs: per channel at
+    // 1 GB 225 us with four, 201 with eight; 16 M elements 16.4 and 18.7 (fewer, longer blocks end less evenly).
+    static int vectors_per_thread(int64_t total, bool quantize)
+    {
+        const int64_t early = int64_t(sm_count()) * 2 * QT * 4; // elements of two blocks per SM, one vector per thread
+        if (quantize)
+            return total <= 2 * early ? 2 : total < (int64_t(1) << 25) ? 4 : 8;
+        return total <= early ? 1 : 4;
+    }
     static unsigned stream_grid(int64_t total, int u) { return unsigned((total + QT * u * 4 - 1) / (QT * u * 4)); }
 
     static unsigned generic_grid(int64_t total)
@@ -469,16 +510,22 @@ namespace b200
         RowMap m;
         if (make_rows(p, x, out, m))
         {
-            const bool fast = g_fast_division.load(std::memory_order_relaxed) != 0, small = small_tensor(p.total);
-            const unsigned grid = stream_grid(p.total, small ? 1 : QU);
-            if (p.rows > 1 && small)
-                launch(quantize_stream_kernel<Q, MODE, FAST, true, 1>, grid, QT, 0, st, x, scale, z, o, m, fast);
-            else if (p.rows > 1)
-                launch(quantize_stream_kernel<Q, MODE, FAST, true, QU>, grid, QT, 0, st, x, scale, z, o, m, fast);
-            else if (small)
-                launch(quantize_stream_kernel<Q, MODE, FAST, false, 1>, grid, QT, 0, st, x, scale, z, o, m, fast);
+            const bool fast = g_fast_division.load(std::memory_order_relaxed) != 0;
+            const int u = vectors_per_thread(p.total, true);
+            const bool two = p.inner >= QT * 4 * u;
+            auto go = [&](auto vectors) {
+                constexpr int U = decltype(vectors)::value;
+                launch(p.rows == 1 ? quantize_stream_kernel<Q, MODE, FAST, ONE_ROW, U>
+                       : two       ? quantize_stream_kernel<Q, MODE, FAST, TWO_ROWS, U>
+                                   : quantize_stream_kernel<Q, MODE, FAST, MANY_ROWS, U>,
+                       stream_grid(p.total, U), QT, 0, st, x, scale, z, o, m, fast);
+            };
+            if (u == 2)
+                go(std::integral_constant<int, 2>());
+            else if (u == 4)
+                go(std::integral_constant<int, 4>());
             else
-                launch(quantize_stream_kernel<Q, MODE, FAST, false, QU>, grid, QT, 0, st, x, scale, z, o, m, fast);
+                go(std::integral_constant<int, 8>());
         }
         else
             quantize_generic_kernel<Q, MODE><<<generic_grid(p.total), QT, 0, st>>>(x, scale, z, o, p.total, p.dims);
@@ -512,16 +559,17 @@ namespace b200
         RowMap m;
         if (make_rows(p, in, out, m))
         {
-            const bool small = small_tensor(p.total);
-            const unsigned grid = stream_grid(p.total, small ? 1 : QU);
-            if (p.rows > 1 && small)
-                launch(dequantize_stream_kernel<Q, true, 1>, grid, QT, 0, st, q, scale, z, out, m);
-            else if (p.rows > 1)
-                launch(dequantize_stream_kernel<Q, true, QU>, grid, QT, 0, st, q, scale, z, out, m);
-            else if (small)
-                launch(dequantize_stream_kernel<Q, false, 1>, grid, QT, 0, st, q, scale, z, out, m);
+            const int u = vectors_per_thread(p.total, false);
+            const bool two = p.inner >= QT * 4 * u;
+            auto go = [&](auto vectors) {
+                constexpr int U = decltype(vectors)::value;
+                launch(p.rows == 1 ? dequantize_stream_kernel<Q, ONE_ROW, U> : two ? dequantize_stream_kernel<Q, TWO_ROWS, U> : dequantize_stream_kernel<Q, MANY_ROWS, U>,
+                       stream_grid(p.total, U), QT, 0, st, q, scale, z, out, m);
+            };
+            if (u == 1)
+                go(std::integral_constant<int, 1>());
             else
-                launch(dequantize_stream_kernel<Q, false, QU>, grid, QT, 0, st, q, scale, z, out, m);
+                go(std::integral_constant<int, 4>());
         }
         else
             dequantize_generic_kernel<Q><<<generic_grid(p.total), QT, 0, st>>>(q, scale, z, out, p.total, p.dims);

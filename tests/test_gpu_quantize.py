@@ -217,12 +217,12 @@ def test_bandwidth_sweep_tool_runs():
     assert any("ROUND_DOWN" in l for l in lines)
 
 
-@pytest.mark.parametrize("rows,inner,axes", [(1200, 1025, (0,)), (83, 17011, (0,)), (700, 4095, (0,)), (700, 4097, (0,)), (90000, 16, (0,)), (90001, 17, (0,)),
+@pytest.mark.parametrize("rows,inner,axes", [(1200, 1025, (0,)), (4200, 8195, (0,)), (200000, 171, (0,)), (83, 17011, (0,)), (700, 4095, (0,)), (700, 4097, (0,)), (90000, 16, (0,)), (90001, 17, (0,)),
                                              (7001, 211, (0,)), (60, 16, (0,)), (61, 1023, (0,)), (1, 1300003, ()), (100000, 15, (0,))])
 def test_rows_that_start_anywhere(ops, rows, inner, axes):
-    """Per-axis rows of any length through the streaming kernels (four vectors per thread for the larger tensors, one for the
-    smaller): row boundaries inside vectors, blocks inside one row, over two and over the most rows a block can touch."""
-    for lead in (1, 2):  # the scales repeat along a leading axis
+    """Per-axis rows of any length through the streaming kernels (one, two, four or eight vectors per thread,
+    by size): row boundaries inside vectors, blocks inside one row, over two and over the most rows a block can touch."""
+    for lead in (1, 2) if rows * inner < 1 << 24 else (1,):  # the scales repeat along a leading axis
         shape = (rows, inner) if lead == 1 else (lead, rows, inner)
         ax = tuple(a + lead - 1 for a in axes)
         rng = np.random.default_rng(rows + inner)
