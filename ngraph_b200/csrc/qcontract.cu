@@ -31,6 +31,7 @@
 #include <algorithm>
 #include <atomic>
 #include <mutex>
+#include <set>
 #include <type_traits>
 #include <unordered_map>
 #include "common.cuh"
@@ -112,7 +113,7 @@ namespace b200
         int cells_w, cells_h;   // its row length and row count per image, in cells
         const int8_t* b_packed; // weights in the block image made by b200_pack_weights_host (null: plain [N,K] matrix through maps.b)
         int b_blocks_n;      // 64-row blocks per k-block in that image: ceil(N / 64)
-        int f32_staged;      // f32 output, regular shape: transposed through the staging blocks for coalesced stores
+        int epilogue;        // which family of epilogue loops (EPI_*) the launch needs
         int tma_sum;         // the residual is fetched by TMA into the staging block its result will be stored from
         int vec_params;      // scale / bias pointers are 16-byte aligned
         int pair;            // 1, or 2: a CTA works on two row tiles (2u, 2u + 1) at a time, which share every B stage
@@ -173,7 +174,14 @@ namespace b200
 
     constexpr int MAX_STAGES = 40;          // small stages (the stem's 2 KB cell runs) need many in flight to cover the load latency
     constexpr int BAR_BYTES = 2048;         // 3*MAX_STAGES + 2*MAX_ACC + 1 + 3*EPI_WARPS mbarriers of 8 bytes
+    // A producer issues every third k-block and waits for its stage by the parity of the stage's uses.  In a ring shorter than the
+    // producers it could be two uses ahead of the consumer, where that parity reads as "free": it would arm a full barrier
+    // twice and overwrite a stage that is being read.  No plan has fewer stages than producers.
+    constexpr int MIN_STAGES = NUM_PRODUCERS;
     constexpr int B_RESIDENT_MAX = 73728;   // a whole filter / weight matrix up to this size stays in shared memory
+
+    // halo mode: a stage is the patch plus the rows the last taps read past it for the junk positions of the last tile row
+    static inline int halo_stage_bytes(int halo_bytes, int junk_positions, int bk) { return (halo_bytes + junk_positions * bk + 1023) / 1024 * 1024; }
 
     template <int BN, int BK>
     struct Cfg
@@ -279,6 +287,12 @@ namespace b200
     {
         float x, y;
     };
+    __device__ __forceinline__ F2 lds_f2(uint32_t addr)
+    {
+        F2 r;
+        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(r.x), "=f"(r.y) : "r"(addr));
+        return r;
+    }
     __device__ __forceinline__ uint64_t pack_f2(float a, float b)
     {
         uint64_t r;
@@ -368,6 +382,29 @@ namespace b200
             // (saturating, NaN -> 0) followed by a saturating pack gives the same byte.
             const int i0 = __float2int_rn(r01.x), i1 = __float2int_rn(r01.y), i2 = __float2int_rn(r23.x), i3 = __float2int_rn(r23.y);
             w[j4] = OUT_U8 ? pack4_u8(i0, i1, i2, i3) : pack4_s8(i0, i1, i2, i3);
+        }
+    }
+
+    // The same 32 columns under the core contract, one-byte output: saturate(half-away(float(acc) * scale) + zero point).
+    // floor(RD(|f| + 0.5)), the sum rounded down, is the magnitude of half-away rounding: the exact sum is never below an
+    // integer that its rounded value reaches.  zp: |out_zp| <= 2^20 (the caller checks), so that the clamp can come first.
+    template <bool OUT_U8>
+    __device__ __forceinline__ void epilogue_chunk_core(const uint32_t (&v)[32], uint32_t (&w)[8], float scale, int zp)
+    {
+        const int lo = (OUT_U8 ? 0 : -128) - zp, hi = (OUT_U8 ? 255 : 127) - zp;
+#pragma unroll
+        for (int j4 = 0; j4 < 8; ++j4)
+        {
+            int q[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+            {
+                const float f = __fmul_rn(__int2float_rn(int32_t(v[4 * j4 + i])), scale);
+                const int a = __float2int_rd(__fadd_rd(fabsf(f), 0.5f));
+                q[i] = min(max(f < 0.0f ? -a : a, lo), hi) + zp;
+                q[i] = f != f ? 0 : q[i];
+            }
+            w[j4] = OUT_U8 ? pack4_u8(q[0], q[1], q[2], q[3]) : pack4_s8(q[0], q[1], q[2], q[3]);
         }
     }
 
@@ -572,7 +609,17 @@ namespace b200
             fail = 3002;
     }
 
-    template <int BN, int BK, bool CTA2 = false, bool SPLITK = false>
+    // The epilogue loops come in families, a kernel each.  Compiled into one kernel they share a register budget and a schedule:
+    // the f32 loop below, added to the one-byte loops, slowed a residual layer from 50 to 84 us.
+    enum
+    {
+        EPI_BYTES,   // one-byte outputs of the fused contract, width a multiple of 16, stored (and the residual fetched) by TMA
+        EPI_SECTORS, // f32 outputs of the fused contract without residual, written from registers in whole sectors
+        EPI_ROWS,    // one-byte outputs without residual of any width and contract, written row by row through shared memory, or
+                     // from registers where the stage ring takes all of it
+        EPI_GENERAL  // everything else: results of any type straight from registers
+    };
+    template <int BN, int BK, bool CTA2 = false, bool SPLITK = false, int EPI = EPI_BYTES>
     __global__ void __launch_bounds__(NUM_THREADS, SPLITK ? 2 : 1)
         qcontract_kernel(const __grid_constant__ TensorMaps maps, const __grid_constant__ ContractParams p)
     {
@@ -1146,17 +1193,10 @@ namespace b200
             const uint32_t stage_blk0 = out_base + uint32_t(ew) * (32 * COLS);
             const uint32_t sw_xor = uint32_t((lane >> 1) & 3);
             // branch-free chunk body for the fused contract with one-byte outputs: 3 * (0: u8, 1: i8, 2: i8 with relu) +
-            // (0: no residual, 1: u8 residual through the fma form, 2: any residual); -1: the general path (core
-            // contract, 4-byte outputs, unaligned residuals)
-            int bytes_variant = -1;
-            if (!p.half_away && esz == 1 && (!has_sum || vec_ok))
-            {
-                const bool fma_form = p.sum_type == B200_U8 && fabsf(__fmul_rn(sum_scale, 8388608.0f)) <= 3.4028234664e38f;
-                bytes_variant = 3 * (p.out_type == B200_U8 ? 0 : (p.relu ? 2 : 1)) + (has_sum ? (fma_form ? 1 : 2) : 0);
-            }
+            // (0: no residual, 1: u8 residual through the fma form, 2: any residual)
+            const bool fma_form = p.sum_type == B200_U8 && fabsf(__fmul_rn(sum_scale, 8388608.0f)) <= 3.4028234664e38f;
+            const int bytes_variant = 3 * (p.out_type == B200_U8 ? 0 : (p.relu ? 2 : 1)) + (has_sum ? (fma_form ? 1 : 2) : 0);
             const uint32_t sc_base = ptx::smem_u32(&epi_scale[ew][0]), bi_base = ptx::smem_u32(&epi_bias[ew][0]);
-            // per-row addresses are only needed for residual loads and for stores that do not go through TMA
-            const bool need_rows = has_sum || !p.tma_store;
             // the tile this CTA handles as its it-th one: tiles blockIdx, blockIdx + grid, ... or, in paired mode, the row
             // tiles 2u and 2u + 1 of the units u = blockIdx, blockIdx + grid, ...
             const int pair = p.pair;
@@ -1170,18 +1210,22 @@ namespace b200
             // chosen by elect.sync at points where the warp is converged: the election is deterministic for a full
             // mask (the bulk groups stay with one thread) and lets the compiler keep the operands in uniform registers.
 
-            // The tile loop, compiled once per MODE.  MODE 0..8 = bytes_variant with TMA stores, a width that is a
-            // multiple of 64 (every chunk full) and, where there is a residual, the residual fetched by TMA into the
-            // staging block its result is stored from: all the per-chunk decisions are made at compile time.
-            // MODE -1 is the general loop (any contract, type and width).
+            // The tile loop, compiled once per MODE so that the per-chunk decisions are made at compile time.
+            //   0 .. 8    EPI_BYTES: bytes_variant with TMA stores and, where there is a residual, the residual fetched by TMA into
+            //             the staging block its result is stored from (what lies beyond the width is clipped or read as zero)
+            //   9, 10     EPI_SECTORS without / with ReLU, rows of whole 16-byte pieces;  16, 17: any rows
+            //   11 .. 13  EPI_ROWS, fused contract: u8, i8, i8 with ReLU;  14, 15: core contract, u8, i8
+            //   18 .. 20  EPI_ROWS without staging (width a multiple of 16), fused contract: u8, i8, i8 with ReLU
+            //   -1        EPI_GENERAL (any contract, type and width)
             auto epilogue_loop = [&](auto mode_tag) {
                 constexpr int MODE = decltype(mode_tag)::value;
-                // MODE 9 / 10: f32 output without / with ReLU, no residual, width a multiple of 64: stored from registers
-                constexpr bool F_F32 = MODE >= 9;
-                constexpr bool FAST = MODE >= 0 && !F_F32; // the one-byte modes, staged and stored by TMA
+                constexpr bool F_F32 = MODE == 9 || MODE == 10 || MODE == 16 || MODE == 17, F_PIECES = MODE < 16;
+                constexpr bool F_ROWS = MODE >= 11 && MODE <= 15, F_CORE = MODE == 14 || MODE == 15, F_DIRECT = MODE >= 18;
+                constexpr bool FAST = MODE >= 0 && MODE <= 8; // the one-byte modes, staged and stored by TMA
                 constexpr int F_SUMK = FAST ? MODE % 3 : 0;
-                constexpr bool F_SUM = F_SUMK != 0, F_RELU = MODE >= 6 && MODE != 9, F_U8 = MODE >= 0 && MODE < 3;
-                constexpr int NBUF = F_SUM ? 3 : 2; // staging blocks per warp
+                constexpr bool F_SUM = F_SUMK != 0, F_RELU = FAST ? MODE >= 6 : MODE == 10 || MODE == 13 || MODE == 17 || MODE == 20;
+                constexpr bool F_U8 = (MODE >= 0 && MODE < 3) || MODE == 11 || MODE == 14 || MODE == 18;
+                constexpr int NBUF = F_SUM ? 3 : F_ROWS ? 1 : 2; // staging blocks per warp
                 int staged_tn = -1;
                 int blk = 0;             // staging block of the current tile: j % NBUF
                 uint32_t sum_ph = 0;     // parity of sum_bar(ew, blk) for the current tile: (j / 3) & 1
@@ -1250,7 +1294,7 @@ namespace b200
                             }
                         }
                     }
-                    else if (j >= 2 && !F_F32)
+                    else if (j >= 2 && FAST)
                     {
                         // the TMA store issued two tiles ago must have finished reading this staging block
                         PROF_MARK(t_w0);
@@ -1281,7 +1325,7 @@ namespace b200
                     er.off = 0;
                     // is the first row of this warp's 32-row block inside the tensor (else the whole block is outside)
                     bool blk_valid;
-                    const bool rows = FAST ? false : (F_F32 ? true : need_rows);
+                    const bool rows = !FAST;
                     if (p.conv)
                     {
                         blk_valid = q0 + blk_w < p.Q && p0 + blk_h < p.P && n0 + blk_n < p.NB;
@@ -1302,22 +1346,7 @@ namespace b200
                             er.off = int64_t(m) * p.N;
                         }
                     }
-                    // General loop: the residual does not depend on the accumulator, so the first chunk's is fetched before
-                    // waiting for the MMAs.  Rows outside the tensor and columns beyond the width compute on a zero
-                    // residual and are never stored.
-                    uint32_t sumw[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-                    const bool sum_regs = !FAST && !F_F32 && has_sum && vec_ok && er.valid;
-                    auto fetch_sum = [&](int c) {
-                        if (sum_regs && colw + 32 * c + 32 <= p.N)
-                        {
-                            const uint4* sp = reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(p.sum_in) + er.off + colw + 32 * c);
-                            const uint4 s0 = sp[0], s1 = sp[1];
-                            sumw[0] = s0.x; sumw[1] = s0.y; sumw[2] = s0.z; sumw[3] = s0.w;
-                            sumw[4] = s1.x; sumw[5] = s1.y; sumw[6] = s1.z; sumw[7] = s1.w;
-                        }
-                    };
-                    if (!FAST && !F_F32)
-                        fetch_sum(0);
+                    uint32_t sumw[8] = {0, 0, 0, 0, 0, 0, 0, 0}; // residual bytes of the columns at hand
                     {
                         PROF_T0();
                         // the verdict is made warp-uniform: the loop body uses full-mask shuffles and warp syncs
@@ -1343,49 +1372,141 @@ namespace b200
                     };
                     if (F_F32)
                     {
-                        // 32 rows x 32 columns of f32 per chunk = 4 KB = this warp's two staging blocks.  Each lane writes its
-                        // row (16-byte pieces XOR-swizzled by the row against bank conflicts), then the warp reads the chunk
-                        // back transposed so that one store instruction covers 4 rows x 128 contiguous bytes.
-                        const uint32_t f32_blk = out_base + uint32_t(ew) * 4096u;
-                        float* const obase = static_cast<float*>(p.out);
-                        const int my_row_ok = er.valid ? 1 : 0;
+                        // Read out of tensor memory in the shape in which four lanes hold eight neighbouring columns of a row, so that
+                        // results go to memory from registers, with no pass through shared memory, which is left to the operand
+                        // stages.  F_PIECES: neighbouring lanes exchange halves of two such groups, after which every lane stores 16
+                        // bytes and an instruction writes 64 contiguous bytes of eight rows; other rows store single elements,
+                        // whose sectors meet in L2.
+                        const int g = lane >> 2, pair_col = 2 * (lane & 3);
+                        const bool odd = (lane & 1) != 0;
+                        // first column a lane stores of a pair of groups 16 columns wide
+                        const int own_col = F_PIECES ? (lane & 2) * 2 + (odd ? 8 : 0) : pair_col;
+                        const int cols = p.N - colw - own_col;
+                        float* dst[4]; // rows g, g + 8, g + 16, g + 24 of the warp's 32
+                        const uint32_t rows_ok = __ballot_sync(0xffffffffu, er.valid) >> g;
 #pragma unroll
-                        for (int c = 0; c < CHUNKS; ++c)
+                        for (int i = 0; i < 4; ++i)
+                            dst[i] = static_cast<float*>(p.out) + __shfl_sync(0xffffffffu, static_cast<long long>(er.off), g + 8 * i) + colw + own_col;
+                        uint32_t v[2][16];
+                        ptx::tmem_ld_16x32(t_addr, v[0]);
+                        ptx::tmem_ld_wait(v[0]);
+#pragma unroll
+                        for (int h = 0; h < 4; ++h) // 16 rows x 32 columns at a time, the next ones on their way meanwhile
                         {
-                            uint32_t v[32];
-                            ptx::tmem_ld_32x32(t_addr + 32 * c, v);
-                            ptx::tmem_ld_wait();
+                            if (h < 3)
+                                ptx::tmem_ld_16x32(t_addr + (uint32_t((h + 1) >> 1) << 20) + 32 * ((h + 1) & 1), v[(h + 1) & 1]);
+                            const uint32_t(&x)[16] = v[h & 1];
+                            const int i = 2 * (h >> 1);
+                            const bool ok0 = ((rows_ok >> (8 * i)) & 1u) != 0, ok1 = ((rows_ok >> (8 * i + 8)) & 1u) != 0;
 #pragma unroll
-                            for (int j4 = 0; j4 < 8; ++j4)
+                            for (int jj = 0; jj < 2; ++jj)
                             {
-                                const float4 s4 = lds_f4(sc_base + 128u * c + 16 * j4);
-                                const int4 b4 = lds_i4(bi_base + 128u * c + 16 * j4);
-                                const float a0 = __int2float_rn(add_fma_pipe(int32_t(v[4 * j4 + 0]), b4.x, p.one));
-                                const float a1 = __int2float_rn(add_fma_pipe(int32_t(v[4 * j4 + 1]), b4.y, p.one));
-                                const float a2 = __int2float_rn(add_fma_pipe(int32_t(v[4 * j4 + 2]), b4.z, p.one));
-                                const float a3 = __int2float_rn(add_fma_pipe(int32_t(v[4 * j4 + 3]), b4.w, p.one));
-                                F2 r01 = unpack_f2(mul2(pack_f2(a0, a1), pack_f2(s4.x, s4.y)));
-                                F2 r23 = unpack_f2(mul2(pack_f2(a2, a3), pack_f2(s4.z, s4.w)));
-                                if (F_RELU)
+                                F2 lo[2], hi[2]; // rows g and g + 8 of two groups of eight columns
+#pragma unroll
+                                for (int u = 0; u < 2; ++u)
                                 {
-                                    r01.x = fmaxf(r01.x, 0.0f);
-                                    r01.y = fmaxf(r01.y, 0.0f);
-                                    r23.x = fmaxf(r23.x, 0.0f);
-                                    r23.y = fmaxf(r23.y, 0.0f);
+                                    const int j4 = 2 * jj + u, col = 32 * (h & 1) + 8 * j4 + pair_col;
+                                    const F2 s2 = lds_f2(sc_base + 4u * col);
+                                    const F2 b2 = lds_f2(bi_base + 4u * col);
+                                    const int32_t b0 = __float_as_int(b2.x), b1 = __float_as_int(b2.y);
+                                    const float a0 = __int2float_rn(add_fma_pipe(int32_t(x[4 * j4 + 0]), b0, p.one));
+                                    const float a1 = __int2float_rn(add_fma_pipe(int32_t(x[4 * j4 + 1]), b1, p.one));
+                                    const float a2 = __int2float_rn(add_fma_pipe(int32_t(x[4 * j4 + 2]), b0, p.one));
+                                    const float a3 = __int2float_rn(add_fma_pipe(int32_t(x[4 * j4 + 3]), b1, p.one));
+                                    const uint64_t scale2 = pack_f2(s2.x, s2.y);
+                                    lo[u] = unpack_f2(mul2(pack_f2(a0, a1), scale2));
+                                    hi[u] = unpack_f2(mul2(pack_f2(a2, a3), scale2));
+                                    if (F_RELU)
+                                    {
+                                        lo[u].x = fmaxf(lo[u].x, 0.0f);
+                                        lo[u].y = fmaxf(lo[u].y, 0.0f);
+                                        hi[u].x = fmaxf(hi[u].x, 0.0f);
+                                        hi[u].y = fmaxf(hi[u].y, 0.0f);
+                                    }
                                 }
-                                asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(f32_blk + uint32_t(lane) * 128u + (uint32_t(j4 ^ (lane & 7)) << 4)),
-                                             "f"(r01.x), "f"(r01.y), "f"(r23.x), "f"(r23.y) : "memory");
+                                const int col = 32 * (h & 1) + 16 * jj; // of the two groups
+                                if (F_PIECES)
+                                {
+                                    // an even lane takes its neighbour's half of the first group and gives its own of the second
+                                    const F2 lo_out = odd ? lo[0] : lo[1], hi_out = odd ? hi[0] : hi[1];
+                                    F2 lo_in, hi_in;
+                                    lo_in.x = __shfl_xor_sync(0xffffffffu, lo_out.x, 1);
+                                    lo_in.y = __shfl_xor_sync(0xffffffffu, lo_out.y, 1);
+                                    hi_in.x = __shfl_xor_sync(0xffffffffu, hi_out.x, 1);
+                                    hi_in.y = __shfl_xor_sync(0xffffffffu, hi_out.y, 1);
+                                    if (ok0 && col < cols)
+                                        *reinterpret_cast<float4*>(dst[i] + col) =
+                                            odd ? make_float4(lo_in.x, lo_in.y, lo[1].x, lo[1].y) : make_float4(lo[0].x, lo[0].y, lo_in.x, lo_in.y);
+                                    if (ok1 && col < cols)
+                                        *reinterpret_cast<float4*>(dst[i + 1] + col) =
+                                            odd ? make_float4(hi_in.x, hi_in.y, hi[1].x, hi[1].y) : make_float4(hi[0].x, hi[0].y, hi_in.x, hi_in.y);
+                                }
+                                else
+                                {
+#pragma unroll
+                                    for (int u = 0; u < 2; ++u)
+                                    {
+                                        const int cu = col + 8 * u;
+                                        if (ok0 && cu < cols)
+                                            dst[i][cu] = lo[u].x;
+                                        if (ok0 && cu + 1 < cols)
+                                            dst[i][cu + 1] = lo[u].y;
+                                        if (ok1 && cu < cols)
+                                            dst[i + 1][cu] = hi[u].x;
+                                        if (ok1 && cu + 1 < cols)
+                                            dst[i + 1][cu + 1] = hi[u].y;
+                                    }
+                                }
+                            }
+                            if (h < 3)
+                                ptx::tmem_ld_wait(v[(h + 1) & 1]);
+                        }
+                    }
+                    else if (F_ROWS)
+                    {
+                        const int cols = min(COLS, p.N - colw);
+                        if (cols > 0) // warp-uniform
+                        {
+#pragma unroll
+                            for (int c = 0; c < CHUNKS; ++c)
+                            {
+                                uint32_t v[32], w[8];
+                                ptx::tmem_ld_32x32(t_addr + 32 * c, v);
+                                ptx::tmem_ld_wait();
+                                if (F_CORE)
+                                    epilogue_chunk_core<F_U8>(v, w, lds_f4(sc_base).x, p.out_zp);
+                                else
+                                    epilogue_chunk_bytes<0, F_RELU, F_U8>(v, w, sc_base + 128u * c, bi_base + 128u * c, sumw, sum_scale, sum_flip, sum_magic, p.one);
+                                stage_bytes_out(c, w);
                             }
                             __syncwarp();
-#pragma unroll
-                            for (int i = 0; i < 8; ++i)
+                            // Two rows at a time, 16 lanes each: the words of a row that are aligned in global memory, put together from
+                            // two staged ones, and the up to six bytes before and behind them.  A lane that stored its own row byte
+                            // by byte touched 32 lines per instruction: 32199 x 801 x 96 took 264 us.
+                            const int k = lane & 15;
+#pragma unroll 4
+                            for (int i = 0; i < 16; ++i)
                             {
-                                const int rr = 4 * i + (lane >> 3), jj = lane & 7;
-                                const long long roff = __shfl_sync(0xffffffffu, static_cast<long long>(er.off), rr);
-                                const int rok = __shfl_sync(0xffffffffu, my_row_ok, rr);
-                                const float4 val = lds_f4(f32_blk + uint32_t(rr) * 128u + (uint32_t(jj ^ (rr & 7)) << 4));
-                                if (rok && colw < p.N)
-                                    *reinterpret_cast<float4*>(obase + roff + colw + 32 * c + 4 * jj) = val;
+                                const int rr = 2 * i + (lane >> 4);
+                                const long long off = __shfl_sync(0xffffffffu, static_cast<long long>(er.off), rr);
+                                const bool ok = __shfl_sync(0xffffffffu, er.valid ? 1 : 0, rr) != 0;
+                                uint8_t* const dst = static_cast<uint8_t*>(p.out) + off + colw;
+                                const int head = min(cols, int((0u - uint32_t(reinterpret_cast<uintptr_t>(dst))) & 3u));
+                                const int full = (cols - head) >> 2, tail = (cols - head) & 3;
+                                const uint32_t staged = stage_blk + uint32_t(rr) * COLS, flip = uint32_t((rr >> 1) & 3) << 4;
+                                const uint32_t w0 = uint32_t(k) * 4u, w1 = min(w0 + 4u, 60u);
+                                uint32_t a, b;
+                                asm volatile("ld.shared.b32 %0, [%1];" : "=r"(a) : "r"(staged + (w0 ^ flip)) : "memory");
+                                asm volatile("ld.shared.b32 %0, [%1];" : "=r"(b) : "r"(staged + (w1 ^ flip)) : "memory");
+                                if (ok && k < full)
+                                    *reinterpret_cast<uint32_t*>(dst + head + 4 * k) = __funnelshift_r(a, b, 8 * head);
+                                if (ok && k < head + tail)
+                                {
+                                    const uint32_t byte = k < head ? uint32_t(k) : uint32_t(cols - tail + k - head);
+                                    uint32_t x;
+                                    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(x) : "r"(staged + (byte ^ flip)) : "memory");
+                                    dst[byte] = uint8_t(x);
+                                }
                             }
                             __syncwarp();
                         }
@@ -1430,14 +1551,30 @@ namespace b200
                             stage_bytes_out(c, w);
                         }
                     }
+                    else if (F_DIRECT)
+                    {
+                        // each lane writes the 64 bytes of its row (a row's pieces of 16 columns are inside or outside as a whole)
+#pragma unroll
+                        for (int c = 0; c < CHUNKS; ++c)
+                        {
+                            uint32_t v[32], w[8];
+                            ptx::tmem_ld_32x32(t_addr + 32 * c, v);
+                            ptx::tmem_ld_wait();
+                            epilogue_chunk_bytes<0, F_RELU, F_U8>(v, w, sc_base + 128u * c, bi_base + 128u * c, sumw, sum_scale, sum_flip, sum_magic, p.one);
+                            uint4* const op = reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.out) + er.off + colw + 32 * c);
+                            if (er.valid && colw + 32 * c < p.N)
+                                op[0] = make_uint4(w[0], w[1], w[2], w[3]);
+                            if (er.valid && colw + 32 * c + 16 < p.N)
+                                op[1] = make_uint4(w[4], w[5], w[6], w[7]);
+                            __syncwarp();
+                        }
+                    }
                     else
                     {
 #pragma unroll 1
                         for (int c = 0; c < CHUNKS; ++c)
                         {
                             uint32_t v[32], w[8];
-                            if (c > 0)
-                                fetch_sum(c);
                             __syncwarp();
                             ptx::tmem_ld_32x32(t_addr + 32 * c, v);
                             ptx::tmem_ld_wait();
@@ -1445,28 +1582,8 @@ namespace b200
                             if (col0 < p.N) // warp-uniform
                             {
                                 const bool full_chunk = col0 + 32 <= p.N;
-                                const uint32_t sc = sc_base + 128u * c, bi = bi_base + 128u * c;
-                                const bool bytes_path = bytes_variant >= 0 && (!has_sum || full_chunk);
-                                if (bytes_path)
-                                {
-                                    switch (bytes_variant)
-                                    {
-                                    case 0: epilogue_chunk_bytes<0, false, true>(v, w, sc, bi, sumw, sum_scale, sum_flip, sum_magic, p.one); break;
-                                    case 1: epilogue_chunk_bytes<1, false, true>(v, w, sc, bi, sumw, sum_scale, sum_flip, sum_magic, p.one); break;
-                                    case 2: epilogue_chunk_bytes<2, false, true>(v, w, sc, bi, sumw, sum_scale, sum_flip, sum_magic, p.one); break;
-                                    case 3: epilogue_chunk_bytes<0, false, false>(v, w, sc, bi, sumw, sum_scale, sum_flip, sum_magic, p.one); break;
-                                    case 4: epilogue_chunk_bytes<1, false, false>(v, w, sc, bi, sumw, sum_scale, sum_flip, sum_magic, p.one); break;
-                                    case 5: epilogue_chunk_bytes<2, false, false>(v, w, sc, bi, sumw, sum_scale, sum_flip, sum_magic, p.one); break;
-                                    case 6: epilogue_chunk_bytes<0, true, false>(v, w, sc, bi, sumw, sum_scale, sum_flip, sum_magic, p.one); break;
-                                    case 7: epilogue_chunk_bytes<1, true, false>(v, w, sc, bi, sumw, sum_scale, sum_flip, sum_magic, p.one); break;
-                                    default: epilogue_chunk_bytes<2, true, false>(v, w, sc, bi, sumw, sum_scale, sum_flip, sum_magic, p.one); break;
-                                    }
-                                }
-                                else
-                                    epilogue_chunk_general(p, v, w, col0, sc, bi, has_sum, sum_scale, er);
-                                if (p.tma_store)
-                                    stage_bytes_out(c, w);
-                                else if (er.valid && esz == 1)
+                                epilogue_chunk_general(p, v, w, col0, sc_base + 128u * c, bi_base + 128u * c, has_sum, sum_scale, er);
+                                if (er.valid && esz == 1)
                                 {
                                     uint8_t* op = static_cast<uint8_t*>(p.out) + er.off + col0;
                                     if (full_chunk && vec_ok)
@@ -1521,7 +1638,7 @@ namespace b200
                         else
                             ptx::mbar_arrive(tempty_bar(acc));
                     }
-                    if (FAST || (!F_F32 && p.tma_store))
+                    if (FAST)
                     {
                         // make the generic-proxy writes visible to the TMA unit, then one lane stores the block;
                         // rows / columns that fall outside the output tensor are clipped by the TMA unit
@@ -1555,23 +1672,43 @@ namespace b200
                     }
                 }
             };
-            const bool fast_ok = bytes_variant >= 0 && p.tma_store && p.N % COLS == 0 && (!has_sum || p.tma_sum);
-            const bool f32_ok = p.f32_staged != 0 && p.smem.out_bufs == 2;
-            switch (fast_ok ? bytes_variant : f32_ok ? (p.relu ? 10 : 9) : -1)
+            if constexpr (EPI == EPI_SECTORS)
             {
-            case 9: epilogue_loop(std::integral_constant<int, 9>{}); break;
-            case 10: epilogue_loop(std::integral_constant<int, 10>{}); break;
-            case 0: epilogue_loop(std::integral_constant<int, 0>{}); break;
-            case 1: epilogue_loop(std::integral_constant<int, 1>{}); break;
-            case 2: epilogue_loop(std::integral_constant<int, 2>{}); break;
-            case 3: epilogue_loop(std::integral_constant<int, 3>{}); break;
-            case 4: epilogue_loop(std::integral_constant<int, 4>{}); break;
-            case 5: epilogue_loop(std::integral_constant<int, 5>{}); break;
-            case 6: epilogue_loop(std::integral_constant<int, 6>{}); break;
-            case 7: epilogue_loop(std::integral_constant<int, 7>{}); break;
-            case 8: epilogue_loop(std::integral_constant<int, 8>{}); break;
-            default: epilogue_loop(std::integral_constant<int, -1>{}); break;
+                if (p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0)
+                    p.relu ? epilogue_loop(std::integral_constant<int, 10>{}) : epilogue_loop(std::integral_constant<int, 9>{});
+                else
+                    p.relu ? epilogue_loop(std::integral_constant<int, 17>{}) : epilogue_loop(std::integral_constant<int, 16>{});
             }
+            else if constexpr (EPI == EPI_ROWS)
+            {
+                const bool u8 = p.out_type == B200_U8;
+                switch (p.half_away ? (u8 ? 14 : 15) : (p.smem.out_bufs ? 11 : 18) + (u8 ? 0 : p.relu ? 2 : 1))
+                {
+                case 11: epilogue_loop(std::integral_constant<int, 11>{}); break;
+                case 12: epilogue_loop(std::integral_constant<int, 12>{}); break;
+                case 13: epilogue_loop(std::integral_constant<int, 13>{}); break;
+                case 14: epilogue_loop(std::integral_constant<int, 14>{}); break;
+                case 18: epilogue_loop(std::integral_constant<int, 18>{}); break;
+                case 19: epilogue_loop(std::integral_constant<int, 19>{}); break;
+                case 20: epilogue_loop(std::integral_constant<int, 20>{}); break;
+                default: epilogue_loop(std::integral_constant<int, 15>{}); break;
+                }
+            }
+            else if constexpr (EPI == EPI_GENERAL)
+                epilogue_loop(std::integral_constant<int, -1>{});
+            else
+                switch (bytes_variant)
+                {
+                case 0: epilogue_loop(std::integral_constant<int, 0>{}); break;
+                case 1: epilogue_loop(std::integral_constant<int, 1>{}); break;
+                case 2: epilogue_loop(std::integral_constant<int, 2>{}); break;
+                case 3: epilogue_loop(std::integral_constant<int, 3>{}); break;
+                case 4: epilogue_loop(std::integral_constant<int, 4>{}); break;
+                case 5: epilogue_loop(std::integral_constant<int, 5>{}); break;
+                case 6: epilogue_loop(std::integral_constant<int, 6>{}); break;
+                case 7: epilogue_loop(std::integral_constant<int, 7>{}); break;
+                default: epilogue_loop(std::integral_constant<int, 8>{}); break;
+                }
             // the staging blocks must have been read before the CTA exits (the end of the grid waits for the writes themselves)
             if (ptx::elect_one())
                 asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -1775,6 +1912,21 @@ namespace b200
         return best;
     }
 
+    // the kernel a launch needs
+    template <int BN, int BK>
+    static auto kernel_of(const ContractParams& p)
+    {
+#ifdef B200_PROFILE_WAITS
+        if (p.cta2)
+            return qcontract_kernel<BN, BK, (BN == 256)>;
+#endif
+        return p.split > 1                 ? qcontract_kernel<BN, BK, false, (BN == 64)>
+               : p.epilogue == EPI_SECTORS ? qcontract_kernel<BN, BK, false, false, EPI_SECTORS>
+               : p.epilogue == EPI_ROWS    ? qcontract_kernel<BN, BK, false, false, EPI_ROWS>
+               : p.epilogue == EPI_GENERAL ? qcontract_kernel<BN, BK, false, false, EPI_GENERAL>
+                                           : qcontract_kernel<BN, BK, false, false, EPI_BYTES>;
+    }
+
     template <int BN, int BK>
     static int fire_contract(const TensorMaps& maps, const ContractParams& p, int grid, cudaStream_t st)
     {
@@ -1810,17 +1962,11 @@ namespace b200
         }
         cfg.attrs = attr;
         cfg.numAttrs = unsigned(nattr);
-#ifdef B200_PROFILE_WAITS
-        // the CTA-pair variant is compiled into instrumented builds only (see ContractParams::cta2)
-        cudaError_t le = p.split > 1 ? cudaLaunchKernelEx(&cfg, qcontract_kernel<BN, BK, false, (BN == 64)>, maps, p)
-                         : p.cta2 ? cudaLaunchKernelEx(&cfg, qcontract_kernel<BN, BK, (BN == 256)>, maps, p)
-                                : cudaLaunchKernelEx(&cfg, qcontract_kernel<BN, BK>, maps, p);
-#else
-        if (p.cta2)
+#ifndef B200_PROFILE_WAITS
+        if (p.cta2) // the CTA-pair variant is compiled into instrumented builds only (see ContractParams::cta2)
             return B200_ERR_UNSUPPORTED;
-        cudaError_t le = p.split > 1 ? cudaLaunchKernelEx(&cfg, qcontract_kernel<BN, BK, false, (BN == 64)>, maps, p)
-                                     : cudaLaunchKernelEx(&cfg, qcontract_kernel<BN, BK>, maps, p);
 #endif
+        cudaError_t le = cudaLaunchKernelEx(&cfg, kernel_of<BN, BK>(p), maps, p);
         if (le != cudaSuccess)
             return cuda_status(le, "cudaLaunchKernelEx(qcontract_kernel)");
         return after_launch("qcontract_kernel");
@@ -1843,24 +1989,6 @@ namespace b200
     static int launch_contract(const TensorMaps& maps, ContractParams& p, cudaStream_t st)
     {
         using C = Cfg<BN, BK>;
-        static bool attr_set[64] = {false};
-        int dev = 0;
-        cudaGetDevice(&dev);
-        dev &= 63;
-        if (!attr_set[dev])
-        {
-            cudaError_t e = cudaFuncSetAttribute(qcontract_kernel<BN, BK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 SMEM_LIMIT);
-#ifdef B200_PROFILE_WAITS
-            if (e == cudaSuccess && BN == 256)
-                e = cudaFuncSetAttribute(qcontract_kernel<BN, BK, (BN == 256)>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
-#endif
-            if (e == cudaSuccess && BN == 64)
-                e = cudaFuncSetAttribute(qcontract_kernel<BN, BK, false, (BN == 64)>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
-            if (e != cudaSuccess)
-                return cuda_status(e, "cudaFuncSetAttribute(qcontract)");
-            attr_set[dev] = true;
-        }
         // shared-memory plan: keep B resident when there is a single column tile and it is small; give the
         // rest to pipeline stages (more bytes in flight hide the HBM latency of the activation stream)
         p.inv_tiles_m = 1.0f / float(p.tiles_m);
@@ -1873,7 +2001,7 @@ namespace b200
         p.split = (BN == 64 && !p.a_cells && !p.halo && p.pair != 2 && !p.cta2) ? pick_split(int64_t(p.tiles_m) * p.tiles_n, nkb) : 1;
         sp.b_resident = (p.tiles_n == 1 && nkb * C::B_BYTES <= B_RESIDENT_MAX && p.split == 1) ? 1 : 0;
         if (p.split > 1) // results are written from registers; the staging area holds the partial sums on their way
-            p.tma_store = p.tma_sum = p.f32_staged = 0;
+            p.tma_store = p.tma_sum = 0;
         if (p.cta2)
         {
             // CTA pairs: the plain tile pipeline with 256-wide column tiles, an even number of row tiles (the caller pads)
@@ -1881,6 +2009,10 @@ namespace b200
                 return B200_ERR_INVALID_ARGUMENT;
             sp.b_resident = 0;
         }
+        // resident weights give way to the result staging: the ring must not get shorter than the producers (see MIN_STAGES)
+        if (sp.b_resident && !p.halo && !p.a_cells &&
+            (SMEM_LIMIT - C::FIXED - nkb * C::B_BYTES - 64 - (p.tma_store ? (p.sum_in ? 3 : 2) * C::OUT_BYTES : 0)) / C::A_BYTES < MIN_STAGES)
+            sp.b_resident = 0;
         sp.b_res_bytes = sp.b_resident ? nkb * C::B_BYTES : 0;
         if (p.pair != 2)
             p.pair = 1;
@@ -1901,8 +2033,7 @@ namespace b200
         {
             if (!sp.b_resident)
                 return B200_ERR_UNSUPPORTED; // the caller only asks for halo mode when the weights stay resident
-            // the patch plus the rows the last taps read past it for the junk positions of the last tile row
-            sp.stage_bytes = ((p.halo_bytes + 64 * BK + 1023) / 1024) * 1024;
+            sp.stage_bytes = halo_stage_bytes(p.halo_bytes, p.RW - p.TW, BK);
         }
         const int room = (p.split > 1 ? SPLIT_SMEM_LIMIT : SMEM_LIMIT) - C::FIXED - sp.b_res_bytes - 64;
         if (p.tma_store && nkb >= 16 && (room - 2 * C::OUT_BYTES) / sp.stage_bytes < (p.cta2 ? 7 : 4))
@@ -1912,14 +2043,33 @@ namespace b200
             p.tma_store = 0;
         }
         // the residual comes in through the staging blocks (three per warp) when everything about it is regular
-        p.tma_sum = p.tma_sum && p.tma_store && p.sum_in && !p.half_away && p.N % COLS == 0;
-        if (p.tma_sum && (room - 3 * C::OUT_BYTES) / sp.stage_bytes < 2)
+        p.tma_sum = p.tma_sum && p.tma_store && p.sum_in && !p.half_away;
+        if (p.tma_sum && (room - 3 * C::OUT_BYTES) / sp.stage_bytes < MIN_STAGES)
             p.tma_sum = 0;
-        sp.out_bufs = p.tma_store ? (p.tma_sum ? 3 : 2) : (p.f32_staged ? 2 : 0);
+        bool rows_staged = false;
+        {
+            const bool one_byte = p.out_type == B200_U8 || p.out_type == B200_I8;
+            const bool aligned = p.N % 16 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+            // long reductions need the ring more than the store needs its staging (as above)
+            const bool staged_fits = (room - C::OUT_BYTES) / sp.stage_bytes >= (nkb >= 16 ? 4 : int(MIN_STAGES));
+            rows_staged = staged_fits || !aligned || p.half_away;
+            if (!p.half_away && p.tma_store && (!p.sum_in || p.tma_sum))
+                p.epilogue = EPI_BYTES;
+            else if (p.out_type == B200_F32 && !p.half_away && !p.sum_in && (reinterpret_cast<uintptr_t>(p.out) & 3) == 0)
+                p.epilogue = EPI_SECTORS;
+            else if (one_byte && p.half_away != 2 && !p.sum_in && (!p.half_away || (p.out_zp >= -(1 << 20) && p.out_zp <= (1 << 20))) &&
+                     (!rows_staged || (room - C::OUT_BYTES) / sp.stage_bytes >= MIN_STAGES))
+                p.epilogue = EPI_ROWS;
+            else
+                p.epilogue = EPI_GENERAL;
+        }
+        if (p.epilogue != EPI_BYTES)
+            p.tma_store = p.tma_sum = 0;
+        sp.out_bufs = p.tma_store ? (p.tma_sum ? 3 : 2) : p.epilogue == EPI_ROWS && rows_staged ? 1 : 0;
         sp.out_bytes = p.split > 1 ? SPLIT_EXCHANGE_BYTES : sp.out_bufs * C::OUT_BYTES;
         int fit = (room - sp.out_bytes) / sp.stage_bytes;
         sp.stages = fit > MAX_STAGES ? MAX_STAGES : fit;
-        if (p.pair == 2 && sp.stages < 3)
+        if (p.pair == 2 && sp.stages < MIN_STAGES)
         {
             // the wider stages of a pair leave too short a ring: the same tiles one at a time (an even, padded tile count is
             // as good as the exact one)
@@ -1928,8 +2078,24 @@ namespace b200
             p.tma_sum = tma_sum_asked;
             goto plan_again;
         }
-        if (sp.stages < 2)
+        if (sp.stages < MIN_STAGES)
             return B200_ERR_UNSUPPORTED;
+        // a kernel is told once per device how much shared memory it may take
+        {
+            static std::mutex mutex;
+            static std::set<std::pair<int, const void*>> told;
+            int dev = 0;
+            cudaGetDevice(&dev);
+            const void* kernel = reinterpret_cast<const void*>(kernel_of<BN, BK>(p));
+            std::lock_guard<std::mutex> lock(mutex);
+            if (told.count({dev, kernel}) == 0)
+            {
+                cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
+                if (e != cudaSuccess)
+                    return cuda_status(e, "cudaFuncSetAttribute(qcontract)");
+                told.insert({dev, kernel});
+            }
+        }
         sp.total_bytes = sp.b_res_bytes + sp.stages * sp.stage_bytes + sp.out_bytes + C::FIXED;
         int tiles = p.tiles_m * p.tiles_n / p.pair; // units of work: tiles, or pairs of row tiles
         int grid = p.split > 1 ? tiles * p.split : tiles < num_sms() ? tiles : num_sms();
@@ -1995,8 +2161,6 @@ namespace b200
         p.vec_params = ((reinterpret_cast<uintptr_t>(p.scale) | reinterpret_cast<uintptr_t>(e->bias)) & 15) == 0;
         const bool one_byte = e->out_type == B200_U8 || e->out_type == B200_I8;
         p.tma_store = one_byte && (p.N % 16 == 0) && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-        p.f32_staged = e->out_type == B200_F32 && !e->round_half_away && !e->sum_in && (p.N % COLS == 0) &&
-                       (reinterpret_cast<uintptr_t>(out) & 15) == 0;
         (void)a_type;
     }
 
@@ -2035,7 +2199,7 @@ namespace b200
         return waves * unit_clk;
     }
 
-    static int pick_pair(int64_t tiles_m, int64_t n_out, int bn, int bk, int64_t nkb, bool residual, bool halo)
+    static int pick_pair(int64_t tiles_m, int64_t n_out, int bn, int bk, int64_t nkb, bool residual, bool halo, bool staged)
     {
 #ifdef B200_PROFILE_WAITS
         if (const char* f = getenv("B200_FORCE_PAIR")) // instrumented build only
@@ -2047,7 +2211,7 @@ namespace b200
         // (which long reductions give up, see launch_contract)
         const bool b_resident = (n_out + bn - 1) / bn == 1 && nkb * int64_t(bn) * bk <= B_RESIDENT_MAX;
         const int64_t stage = 2 * int64_t(BM) * bk + (b_resident ? 0 : int64_t(bn) * bk);
-        const int64_t staging = (residual ? 3 : 2) * int64_t(EPI_WARPS * 32 * COLS);
+        const int64_t staging = staged ? (residual ? 3 : 2) * int64_t(EPI_WARPS * 32 * COLS) : 0;
         const int64_t room = SMEM_LIMIT - 4096 - (b_resident ? nkb * int64_t(bn) * bk : 0);
         const bool keeps_tma_store = !(nkb >= 16 && (room - staging) / stage < 4);
         if ((room - (keeps_tma_store ? staging : 0)) / stage < 3)
@@ -2213,7 +2377,7 @@ static int qgemm_impl(const void* A, int a_type, const int8_t* W, bool packed, v
     p.tiles_m = int((M + BM - 1) / BM);
     const int bn = pick_bn(N, p.tiles_m, bk, epilogue && epilogue->sum_in, K);
     p.tiles_n = int((N + bn - 1) / bn);
-    p.pair = pick_pair(p.tiles_m, N, bn, bk, p.cblocks, epilogue && epilogue->sum_in, false);
+    p.pair = pick_pair(p.tiles_m, N, bn, bk, p.cblocks, epilogue && epilogue->sum_in, false, epilogue->out_type != B200_F32);
 #ifdef B200_PROFILE_WAITS
     if (getenv("B200_FORCE_CTA2") && bn == 256 && N % 256 == 0 && p.tiles_m >= 2 && !(p.tiles_n == 1 && int64_t(p.cblocks) * bn * bk <= B_RESIDENT_MAX))
     {
@@ -2430,8 +2594,13 @@ static int qconv_impl(const void* data, int data_type, const int8_t* filters, bo
         // the weights must stay resident: one column tile, all taps and channel blocks within the resident budget
         const int bn_h = pick_bn(c->K, tiles_h, bk, epilogue && epilogue->sum_in, c->R * c->S * c->C);
         const bool weights_fit = bn_h >= c->K && c->R * c->S * c->C * int64_t(bn_h) <= B_RESIDENT_MAX;
+        // and the ring has to hold its stages beside them and the result staging (3x3 over 128 channels: not with a residual)
+        const bool bytes_out = epilogue->out_type == B200_U8 || epilogue->out_type == B200_I8;
+        const int64_t stage_h = halo_stage_bytes(int(bk * RW * (THh + c->R - 1)), int(c->S - 1), bk);
+        const bool ring_fits = MIN_STAGES * stage_h + (bytes_out ? (epilogue->sum_in ? 3 : 2) * int64_t(EPI_WARPS * 32 * COLS) : 0) +
+                                   c->R * c->S * c->C * int64_t(bn_h) + 1024 + BAR_BYTES + 64 <= SMEM_LIMIT;
         if (!no_halo && sh == 1 && sw == 1 && c->dilation_h == 1 && c->dilation_w == 1 && c->R * c->S > 1 && c->S <= 8 && weights_fit &&
-            c->C <= 128 && tiles_h * 10 <= tiles_n * 13)
+            c->C <= 128 && ring_fits && tiles_h * 10 <= tiles_n * 13)
         {
             p.halo = 1;
             p.RW = int(RW);
@@ -2461,7 +2630,7 @@ static int qconv_impl(const void* data, int data_type, const int8_t* filters, bo
     p.pair = 1;
 #ifdef B200_PROFILE_WAITS
     if (getenv("B200_FORCE_PAIR"))
-        p.pair = pick_pair(p.tiles_m, c->K, bn, bk, int64_t(p.ntaps) * p.cblocks, epilogue && epilogue->sum_in, p.halo != 0);
+        p.pair = pick_pair(p.tiles_m, c->K, bn, bk, int64_t(p.ntaps) * p.cblocks, epilogue && epilogue->sum_in, p.halo != 0, true);
 #endif
 #ifdef B200_PROFILE_WAITS
     if (getenv("B200_FORCE_CTA2") && bn == 256 && c->K % 256 == 0 && p.tiles_m >= 2 && !p.halo && !p.a_cells &&

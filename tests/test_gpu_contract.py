@@ -529,3 +529,70 @@ def test_qconv_split_reductions(ops, cfg):
                                       ref.qconv_fused(data, filt, bias, scale, cs, np.uint8, relu=True))
         np.testing.assert_array_equal(run_conv(ops, data, filt, bias, scale, cs, np.uint8, True, sum_in=sum_u8, sum_scale=0.61, packed=packed),
                                       ref.qconv_fused(data, filt, bias, scale, cs, np.uint8, relu=True, sum_in=sum_u8, sum_scale=np.float32(0.61)))
+
+
+# ---------------------------------------------------------------- widths and contracts off the TMA store path
+@pytest.mark.parametrize("m,n,k", [(20000, 17, 64), (9000, 63, 256), (9001, 65, 96), (4500, 131, 2304), (3300, 258, 160), (20100, 1, 80), (2500, 801, 96), (2500, 1000, 2048)])
+def test_qgemm_ragged_widths(ops, m, n, k):
+    """Every alignment a row can start at, widths that end inside a warp's 64 columns, odd and even f32 rows, both contracts"""
+    rng = np.random.default_rng(m + n + k)
+    a = rng.integers(-128, 128, size=(m, k)).astype(np.int8)
+    w = rng.integers(-127, 128, size=(n, k)).astype(np.int8)
+    bias = rng.integers(-1000, 1001, size=n).astype(np.int32)
+    scale = (np.exp(rng.uniform(np.log(0.5), np.log(2.0), size=n)) * 40.0 / (np.sqrt(k) * 74 * 74)).astype(np.float32)
+    for out_dt, relu in ((np.uint8, True), (np.int8, False), (np.int8, True), (np.float32, False), (np.float32, True), (np.int32, False)):
+        exp = ref.qgemm_fused(a, w, bias, scale, out_dt, relu=relu)
+        got = ops.qgemm(dev(a), dev(w), dev(scale), TDT[np.dtype(out_dt)], bias=dev(bias), relu=relu, packed=relu).cpu().numpy()
+        if out_dt == np.float32:
+            same_f32(got, exp)
+        else:
+            np.testing.assert_array_equal(got, exp, err_msg="%s relu=%d" % (out_dt, relu))
+    tie = np.float32(0.5)  # accumulators times one half: every odd one is a tie
+    for out_dt, zp, s in ((np.int8, 3, scale[0]), (np.uint8, 128, scale[0]), (np.int8, -100, tie), (np.uint8, 1 << 21, scale[0]), (np.int32, -5, scale[0])):
+        got = ops.qgemm(dev(a), dev(w), dev(np.array([s], np.float32)), TDT[np.dtype(out_dt)], core=True, out_zp=zp).cpu().numpy()
+        np.testing.assert_array_equal(got, ref.qgemm_core(a, w, s, zp, out_dt), err_msg="core %s zp %d" % (out_dt, zp))
+
+
+@pytest.mark.parametrize("cfg", [(30, 64, 20, 22, 80, 1, (1, 1)), (12, 128, 30, 29, 176, 3, (1, 1)), (9, 64, 56, 56, 48, 3, (1, 1)), (10, 256, 28, 28, 272, 3, (2, 2)), (6, 64, 30, 31, 75, 3, (1, 1))])
+def test_qconv_widths_that_end_inside_a_block(ops, cfg):
+    """K a multiple of 16 but not of 64 (TMA clips the last block, the residual's is filled with zeros), and K of any size"""
+    n, c, h, w, k, r, stride = cfg
+    rng = np.random.default_rng(sum(cfg[:6]))
+    data = rng.integers(0, 256, size=(n, c, h, w)).astype(np.uint8)
+    filt = rng.integers(-127, 128, size=(k, c, r, r)).astype(np.int8)
+    bias = rng.integers(-1000, 1001, size=k).astype(np.int32)
+    pad = (r // 2, r // 2)
+    cs = ref.conv_shape(data.shape, filt.shape, stride, pad, pad, (1, 1))
+    p, q = ref.conv_out_hw(cs)
+    scale = (np.exp(rng.uniform(np.log(0.5), np.log(2.0), size=k)) * 60.0 / (np.sqrt(c * r * r) * 74 * 147)).astype(np.float32)
+    s_u8 = rng.integers(0, 256, size=(n, k, p, q)).astype(np.uint8)
+    for out_dt, relu, res in ((np.uint8, True, None), (np.uint8, True, s_u8), (np.int8, True, s_u8.view(np.int8)), (np.int8, False, None), (np.float32, False, None)):
+        kw = {} if res is None else {"sum_in": res, "sum_scale": np.float32(0.61)}
+        exp = ref.qconv_fused(data, filt, bias, scale, cs, out_dt, relu=relu, **kw)
+        got = run_conv(ops, data, filt, bias, scale, cs, out_dt, relu, packed=True, **kw)
+        if out_dt == np.float32:
+            same_f32(np.ascontiguousarray(got), np.ascontiguousarray(exp))
+        else:
+            np.testing.assert_array_equal(got, exp, err_msg="%s relu=%d residual=%s" % (out_dt, relu, res is not None))
+
+
+@pytest.mark.parametrize("residual", [False, True])
+@pytest.mark.parametrize("cfg", [(40, 128, 28, 30, 64, 3), (64, 128, 14, 64, 32, 3), (40, 64, 33, 30, 48, 5), (30, 128, 20, 64, 48, 2)])
+def test_qconv_resident_weights_over_many_tiles(ops, cfg, residual):
+    """The largest resident weights leave the shortest stage rings: many tiles per CTA through them, patch and tap forms"""
+    n, c, h, w, k, r = cfg
+    rng = np.random.default_rng(sum(cfg))
+    data = rng.integers(0, 256, size=(n, c, h, w)).astype(np.uint8)
+    filt = rng.integers(-127, 128, size=(k, c, r, r)).astype(np.int8)
+    bias = rng.integers(-1000, 1001, size=k).astype(np.int32)
+    scale = np.full(k, 60.0 / (np.sqrt(c * r * r) * 74 * 147), np.float32)
+    pad = (r // 2, r // 2)
+    cs = ref.conv_shape(data.shape, filt.shape, (1, 1), pad, pad, (1, 1))
+    p, q = ref.conv_out_hw(cs)
+    s_u8 = rng.integers(0, 256, size=(n, k, p, q)).astype(np.uint8)
+    kw = {"sum_in": s_u8, "sum_scale": np.float32(0.61)} if residual else {}
+    got = run_conv(ops, data, filt, bias, scale, cs, np.uint8, True, packed=True, **kw)
+    sl = [0, 1, n // 2, n - 1]
+    cs_s = ref.conv_shape((len(sl),) + data.shape[1:], filt.shape, (1, 1), pad, pad, (1, 1))
+    kw = {"sum_in": s_u8[sl], "sum_scale": np.float32(0.61)} if residual else {}
+    np.testing.assert_array_equal(got[sl], ref.qconv_fused(data[sl], filt, bias, scale, cs_s, np.uint8, relu=True, **kw))
