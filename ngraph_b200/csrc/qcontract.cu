@@ -614,6 +614,7 @@ namespace b200
     enum
     {
         EPI_BYTES,   // one-byte outputs of the fused contract, width a multiple of 16, stored (and the residual fetched) by TMA
+        EPI_BYTES_2, // the same with a residual, two staging blocks per warp instead of three, and widths that leave whole blocks empty
         EPI_SECTORS, // f32 outputs of the fused contract without residual, written from registers in whole sectors
         EPI_ROWS,    // one-byte outputs without residual of any width and contract, written row by row through shared memory, or
                      // from registers where the stage ring takes all of it
@@ -1225,10 +1226,10 @@ namespace b200
                 constexpr int F_SUMK = FAST ? MODE % 3 : 0;
                 constexpr bool F_SUM = F_SUMK != 0, F_RELU = FAST ? MODE >= 6 : MODE == 10 || MODE == 13 || MODE == 17 || MODE == 20;
                 constexpr bool F_U8 = (MODE >= 0 && MODE < 3) || MODE == 11 || MODE == 14 || MODE == 18;
-                constexpr int NBUF = F_SUM ? 3 : F_ROWS ? 1 : 2; // staging blocks per warp
+                constexpr int NBUF = F_SUM && EPI != EPI_BYTES_2 ? 3 : F_ROWS ? 1 : 2; // staging blocks per warp
                 int staged_tn = -1;
                 int blk = 0;             // staging block of the current tile: j % NBUF
-                uint32_t sum_ph = 0;     // parity of sum_bar(ew, blk) for the current tile: (j / 3) & 1
+                uint32_t sum_ph = 0;     // parity of sum_bar(ew, blk) for the current tile: (j / NBUF) & 1
                 // Tile coordinates: each lane decodes one of the warp's next tiles (the divisions are done once per tile
                 // instead of once per tile and lane) and the loop broadcasts them with shuffles.  The window is
                 // refreshed every 31 tiles so that the next tile's coordinates are always in it.
@@ -1278,8 +1279,9 @@ namespace b200
                     const uint32_t stage_row = stage_blk + uint32_t(lane) * COLS;
                     if (F_SUM)
                     {
-                        // Residual of this warp's NEXT tile -> the block that tile's result will be stored from.  That block
-                        // was last used two tiles ago: all but the most recent store must have finished reading.
+                        // Residual of this warp's NEXT tile -> the block that tile's result will be stored from.  Of three blocks it
+                        // was last used two tiles ago, and all but the most recent store must have finished reading; of two,
+                        // all stores.
                         const bool has_next = tile_of(tile_it + GROUPS) < num_tiles;
                         int na, np0, nn0, ntn;
                         coords_of(idx + 1, na, np0, nn0, ntn);
@@ -1289,8 +1291,11 @@ namespace b200
                                 fetch_residual(0, ia, p0, n0, tn);
                             if (has_next)
                             {
-                                asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                                fetch_residual(blk == 2 ? 0 : blk + 1, na, np0, nn0, ntn);
+                                if (NBUF == 3)
+                                    asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                                else
+                                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                                fetch_residual(blk + 1 == NBUF ? 0 : blk + 1, na, np0, nn0, ntn);
                             }
                         }
                     }
@@ -1511,6 +1516,10 @@ namespace b200
                             __syncwarp();
                         }
                     }
+                    else if (F_SUM && EPI == EPI_BYTES_2 && colw >= p.N)
+                    {
+                        // the whole block lies beyond the width (only widths that have such blocks pay for the test)
+                    }
                     else if (F_SUM)
                     {
                         // with a residual: 16 columns at a time, the next 16 on their way out of tensor memory meanwhile (64 -> 256
@@ -1699,13 +1708,13 @@ namespace b200
             else
                 switch (bytes_variant)
                 {
-                case 0: epilogue_loop(std::integral_constant<int, 0>{}); break;
+                case 0: epilogue_loop(std::integral_constant<int, EPI == EPI_BYTES ? 0 : 1>{}); break; // (without residual: EPI_BYTES only)
                 case 1: epilogue_loop(std::integral_constant<int, 1>{}); break;
                 case 2: epilogue_loop(std::integral_constant<int, 2>{}); break;
-                case 3: epilogue_loop(std::integral_constant<int, 3>{}); break;
+                case 3: epilogue_loop(std::integral_constant<int, EPI == EPI_BYTES ? 3 : 4>{}); break;
                 case 4: epilogue_loop(std::integral_constant<int, 4>{}); break;
                 case 5: epilogue_loop(std::integral_constant<int, 5>{}); break;
-                case 6: epilogue_loop(std::integral_constant<int, 6>{}); break;
+                case 6: epilogue_loop(std::integral_constant<int, EPI == EPI_BYTES ? 6 : 7>{}); break;
                 case 7: epilogue_loop(std::integral_constant<int, 7>{}); break;
                 default: epilogue_loop(std::integral_constant<int, 8>{}); break;
                 }
@@ -1922,6 +1931,7 @@ namespace b200
 #endif
         return p.split > 1                 ? qcontract_kernel<BN, BK, false, (BN == 64)>
                : p.epilogue == EPI_SECTORS ? qcontract_kernel<BN, BK, false, false, EPI_SECTORS>
+               : p.epilogue == EPI_BYTES_2 ? qcontract_kernel<BN, BK, false, false, EPI_BYTES_2>
                : p.epilogue == EPI_ROWS    ? qcontract_kernel<BN, BK, false, false, EPI_ROWS>
                : p.epilogue == EPI_GENERAL ? qcontract_kernel<BN, BK, false, false, EPI_GENERAL>
                                            : qcontract_kernel<BN, BK, false, false, EPI_BYTES>;
@@ -2011,7 +2021,7 @@ namespace b200
         }
         // resident weights give way to the result staging: the ring must not get shorter than the producers (see MIN_STAGES)
         if (sp.b_resident && !p.halo && !p.a_cells &&
-            (SMEM_LIMIT - C::FIXED - nkb * C::B_BYTES - 64 - (p.tma_store ? (p.sum_in ? 3 : 2) * C::OUT_BYTES : 0)) / C::A_BYTES < MIN_STAGES)
+            (SMEM_LIMIT - C::FIXED - nkb * C::B_BYTES - 64 - (p.tma_store ? 2 * C::OUT_BYTES : 0)) / C::A_BYTES < MIN_STAGES)
             sp.b_resident = 0;
         sp.b_res_bytes = sp.b_resident ? nkb * C::B_BYTES : 0;
         if (p.pair != 2)
@@ -2044,7 +2054,11 @@ namespace b200
         }
         // the residual comes in through the staging blocks (three per warp) when everything about it is regular
         p.tma_sum = p.tma_sum && p.tma_store && p.sum_in && !p.half_away;
-        if (p.tma_sum && (room - 3 * C::OUT_BYTES) / sp.stage_bytes < MIN_STAGES)
+        // Two blocks where the third costs a stage of a ring that is short for the reduction: a tile then lasts longer than
+        // the store it waits for (3x3 128 -> 672 with a residual 26.4 -> 23.4 us, 512 -> 512 on 14x14 38 -> 32).
+        const int deep = (room - 2 * C::OUT_BYTES) / sp.stage_bytes, shallow = (room - 3 * C::OUT_BYTES) / sp.stage_bytes;
+        const int sum_bufs = shallow >= MIN_STAGES && (nkb < 8 || shallow >= 6 || shallow == deep) && p.tiles_n * BN - p.N < COLS ? 3 : 2;
+        if (p.tma_sum && deep < MIN_STAGES)
             p.tma_sum = 0;
         bool rows_staged = false;
         {
@@ -2054,7 +2068,7 @@ namespace b200
             const bool staged_fits = (room - C::OUT_BYTES) / sp.stage_bytes >= (nkb >= 16 ? 4 : int(MIN_STAGES));
             rows_staged = staged_fits || !aligned || p.half_away;
             if (!p.half_away && p.tma_store && (!p.sum_in || p.tma_sum))
-                p.epilogue = EPI_BYTES;
+                p.epilogue = p.tma_sum && sum_bufs == 2 ? EPI_BYTES_2 : EPI_BYTES;
             else if (p.out_type == B200_F32 && !p.half_away && !p.sum_in && (reinterpret_cast<uintptr_t>(p.out) & 3) == 0)
                 p.epilogue = EPI_SECTORS;
             else if (one_byte && p.half_away != 2 && !p.sum_in && (!p.half_away || (p.out_zp >= -(1 << 20) && p.out_zp <= (1 << 20))) &&
@@ -2063,9 +2077,9 @@ namespace b200
             else
                 p.epilogue = EPI_GENERAL;
         }
-        if (p.epilogue != EPI_BYTES)
+        if (p.epilogue != EPI_BYTES && p.epilogue != EPI_BYTES_2)
             p.tma_store = p.tma_sum = 0;
-        sp.out_bufs = p.tma_store ? (p.tma_sum ? 3 : 2) : p.epilogue == EPI_ROWS && rows_staged ? 1 : 0;
+        sp.out_bufs = p.tma_store ? (p.tma_sum ? sum_bufs : 2) : p.epilogue == EPI_ROWS && rows_staged ? 1 : 0;
         sp.out_bytes = p.split > 1 ? SPLIT_EXCHANGE_BYTES : sp.out_bufs * C::OUT_BYTES;
         int fit = (room - sp.out_bytes) / sp.stage_bytes;
         sp.stages = fit > MAX_STAGES ? MAX_STAGES : fit;
@@ -2594,10 +2608,10 @@ static int qconv_impl(const void* data, int data_type, const int8_t* filters, bo
         // the weights must stay resident: one column tile, all taps and channel blocks within the resident budget
         const int bn_h = pick_bn(c->K, tiles_h, bk, epilogue && epilogue->sum_in, c->R * c->S * c->C);
         const bool weights_fit = bn_h >= c->K && c->R * c->S * c->C * int64_t(bn_h) <= B_RESIDENT_MAX;
-        // and the ring has to hold its stages beside them and the result staging (3x3 over 128 channels: not with a residual)
+        // and the ring has to hold its stages beside them and the result staging
         const bool bytes_out = epilogue->out_type == B200_U8 || epilogue->out_type == B200_I8;
         const int64_t stage_h = halo_stage_bytes(int(bk * RW * (THh + c->R - 1)), int(c->S - 1), bk);
-        const bool ring_fits = MIN_STAGES * stage_h + (bytes_out ? (epilogue->sum_in ? 3 : 2) * int64_t(EPI_WARPS * 32 * COLS) : 0) +
+        const bool ring_fits = MIN_STAGES * stage_h + (bytes_out ? 2 * int64_t(EPI_WARPS * 32 * COLS) : 0) +
                                    c->R * c->S * c->C * int64_t(bn_h) + 1024 + BAR_BYTES + 64 <= SMEM_LIMIT;
         if (!no_halo && sh == 1 && sw == 1 && c->dilation_h == 1 && c->dilation_w == 1 && c->R * c->S > 1 && c->S <= 8 && weights_fit &&
             c->C <= 128 && ring_fits && tiles_h * 10 <= tiles_n * 13)
