@@ -2,9 +2,9 @@
 //
 // A program that issues its launches through ctypes spends about 1 us per call on converting arguments, half of what the
 // launch itself takes on the host (an encoder layer on 128 tokens: 40 calls around 130 us of kernels).  The callables here
-// take the same arguments - integers, None, c_void_p, ctypes arrays, floats - and convert them by the types of the
-// declaration in b200_kernels.h.  Whatever they do not recognise (byref objects, wrong counts or types) goes to the ctypes
-// function they stand for, which accepts it or raises.
+// take the same arguments - integers, None, c_void_p, ctypes arrays, floats, byref of the ABI's structures - and convert them
+// by the types of the declaration in b200_kernels.h.  Whatever they do not recognise (wrong counts or types) goes to the
+// ctypes function they stand for, which accepts it or raises.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <stdint.h>
@@ -17,6 +17,33 @@
 namespace
 {
     PyTypeObject *void_pointer_type, *float_type, *array_type; // ctypes.c_void_p, c_float, Array
+
+    // What byref() makes is opaque; where its pointer, its tag and the object it refers to lie is found out at import, against
+    // known objects (find_byref_layout).  Where that does not hold, byref arguments go to ctypes.
+    struct ByRef
+    {
+        PyObject_HEAD void* ffi_type;
+        char tag;
+        alignas(16) void* pointer; // of a union as wide as a long double
+        alignas(16) PyObject* object;
+    };
+    PyTypeObject* byref_type; // null: layout not recognised
+
+    // the ctypes structures of lib.py, by the ABI's
+    template <typename T>
+    PyTypeObject* structure_type = nullptr;
+
+    template <typename T>
+    bool by_reference(PyObject* o, T*& out)
+    {
+        if (!byref_type || Py_TYPE(o) != byref_type || !structure_type<std::remove_cv_t<T>>)
+            return false;
+        const ByRef* r = reinterpret_cast<const ByRef*>(o);
+        if (r->tag != 'P' || !r->object || Py_TYPE(r->object) != structure_type<std::remove_cv_t<T>>)
+            return false;
+        out = static_cast<T*>(r->pointer);
+        return true;
+    }
 
     bool bytes_of(PyObject* o, void* to, Py_ssize_t n)
     {
@@ -54,6 +81,8 @@ namespace
         }
         if (Py_TYPE(o) == void_pointer_type)
             return bytes_of(o, &out, sizeof(out));
+        if constexpr (std::is_class<T>::value)
+            return by_reference(o, out);
         if (PyObject_TypeCheck(o, array_type))
         {
             Py_buffer v;
@@ -152,7 +181,44 @@ namespace
         return fallback;
     }
 
-    PyMethodDef methods[] = {{"wrap", wrap, METH_VARARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
+    // structures(epilogue type, convolution parameter type)
+    PyObject* structures(PyObject*, PyObject* args)
+    {
+        PyObject *epilogue, *conv;
+        if (!PyArg_ParseTuple(args, "O!O!", &PyType_Type, &epilogue, &PyType_Type, &conv))
+            return nullptr;
+        Py_INCREF(epilogue);
+        Py_INCREF(conv);
+        structure_type<b200_epilogue> = reinterpret_cast<PyTypeObject*>(epilogue);
+        structure_type<b200_conv_params> = reinterpret_cast<PyTypeObject*>(conv);
+        Py_RETURN_NONE;
+    }
+
+    // byref objects of a known buffer, one with an offset
+    void find_byref_layout(PyObject* ctypes)
+    {
+        PyObject* buffer = PyObject_CallMethod(ctypes, "create_string_buffer", "i", 16);
+        PyObject* address = buffer ? PyObject_CallMethod(ctypes, "addressof", "O", buffer) : nullptr;
+        PyObject* plain = address ? PyObject_CallMethod(ctypes, "byref", "O", buffer) : nullptr;
+        PyObject* shifted = plain ? PyObject_CallMethod(ctypes, "byref", "Oi", buffer, 8) : nullptr;
+        if (shifted && Py_TYPE(plain)->tp_basicsize >= Py_ssize_t(sizeof(ByRef)) && Py_TYPE(plain) == Py_TYPE(shifted))
+        {
+            const ByRef *p = reinterpret_cast<const ByRef*>(plain), *q = reinterpret_cast<const ByRef*>(shifted);
+            char* at = static_cast<char*>(PyLong_AsVoidPtr(address));
+            if (p->tag == 'P' && q->tag == 'P' && p->object == buffer && q->object == buffer && p->pointer == at && q->pointer == at + 8)
+            {
+                byref_type = Py_TYPE(plain);
+                Py_INCREF(byref_type);
+            }
+        }
+        PyErr_Clear();
+        Py_XDECREF(shifted);
+        Py_XDECREF(plain);
+        Py_XDECREF(address);
+        Py_XDECREF(buffer);
+    }
+
+    PyMethodDef methods[] = {{"structures", structures, METH_VARARGS, nullptr}, {"wrap", wrap, METH_VARARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
     PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fastcall", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 }
 
@@ -163,6 +229,7 @@ PyMODINIT_FUNC PyInit__fastcall(void)
         return nullptr;
     auto type = [&](const char* name) { return reinterpret_cast<PyTypeObject*>(PyObject_GetAttrString(ctypes, name)); };
     void_pointer_type = type("c_void_p"), float_type = type("c_float"), array_type = type("Array");
+    find_byref_layout(ctypes);
     Py_DECREF(ctypes);
     return void_pointer_type && float_type && array_type ? PyModule_Create(&module) : nullptr;
 }

@@ -47,6 +47,7 @@ def _load():
         raise ImportError("%s is missing: run `python -m ngraph_b200.build` (needs nvcc); "
                           "there is no CPU or PyTorch fallback" % LIB_PATH)
     lib = ctypes.CDLL(LIB_PATH)
+    _fastcall.structures(Epilogue, ConvParams)
     vp, i64, ci = ctypes.c_void_p, ctypes.c_int64, ctypes.c_int
     p64 = ctypes.POINTER(ctypes.c_int64)
     sigs = {

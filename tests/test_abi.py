@@ -85,7 +85,7 @@ def test_argument_validation_of_the_glue_entry_points():
 
 
 def test_native_callables_take_what_ctypes_takes():
-    """integers, None, c_void_p, arrays and floats are converted natively; byref objects, wrong types and wrong counts go through
+    """integers, None, c_void_p, arrays and floats are converted natively; byref of the wrong structure, wrong types and wrong counts go through
     (or raise in) the ctypes function"""
     import ctypes
     L = lib.LIB
@@ -96,6 +96,7 @@ def test_native_callables_take_what_ctypes_takes():
     assert L.b200_layer_norm_rows_f32(1, 2, 3, 4, -1, 3, 1e-5, None) == -1
     assert L.b200_qgemm_packed(1, 9, 2, 3, 4, 5, 16, ctypes.byref(e), s) == -1
     for call in (lambda: L.b200_f32_binary(1, 2), lambda: L.b200_f32_binary("x", 1, 2, 3, 4, None), lambda: L.b200_f32_binary(0, 1.5, 2, 3, 4, None),
-                 lambda: L.b200_quantize(1, 2, 3, 4, 1, (ctypes.c_int32 * 2)(3, 4), 2, None, 0, 0, s), lambda: L.b200_qgemm(1, 0, 2, 3, 4, 5, 16, 5, s)):
+                 lambda: L.b200_quantize(1, 2, 3, 4, 1, (ctypes.c_int32 * 2)(3, 4), 2, None, 0, 0, s), lambda: L.b200_qgemm(1, 0, 2, 3, 4, 5, 16, 5, s),
+                 lambda: L.b200_qgemm(1, 0, 2, 3, 4, 5, 16, ctypes.byref(lib.ConvParams()), s)):
         with pytest.raises((TypeError, ctypes.ArgumentError)):
             call()
