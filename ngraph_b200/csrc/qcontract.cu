@@ -21,7 +21,7 @@
 //   half of the tile's columns: tcgen05.ld -> bias/scale/sum/ReLU/round/saturate in registers ->
 //   (one-byte outputs) a swizzled shared-memory staging block of its own -> one TMA store, so
 //   global writes are whole lines and rows/columns outside the tensor are clipped by the TMA
-//   unit.  Four-byte outputs and ragged widths are written straight from registers.
+//   unit.  Ragged widths leave the staging block by plain stores, four-byte outputs go straight from registers.
 // * Every wait is bounded (ptx::mbar_wait); a timeout sets g_contract_status, the CTA
 //   drains and frees its TMEM, and the host reports B200_ERR_DEVICE_STATUS.
 #include <cuda.h>
@@ -30,6 +30,7 @@
 #include <cstring>
 #include <algorithm>
 #include <atomic>
+#include <memory>
 #include <mutex>
 #include <set>
 #include <type_traits>
@@ -794,11 +795,6 @@ namespace b200
             int use_p = pw; // running index of this producer's k-block over the whole launch (instrumentation)
             (void)use_p;
             uint32_t ph = 0;
-            while (s >= STAGES)
-            {
-                s -= STAGES;
-                ph ^= 1;
-            }
             // a unit of work: one tile, or in paired mode the two row tiles 2u and 2u + 1 (the host makes tiles_m even)
             const int pair = p.pair;
             const int num_units = CTA2 ? num_tiles / 2 : num_tiles / pair;
@@ -916,7 +912,7 @@ namespace b200
                             ++tap;
                         }
                         s += NUM_PRODUCERS;
-                        while (s >= STAGES) // a ring shorter than the number of producers wraps more than once
+                        if (s >= STAGES) // once: the ring is no shorter than the number of producers
                         {
                             s -= STAGES;
                             ph ^= 1;
@@ -1833,55 +1829,57 @@ namespace b200
     // A compiled graph calls the same entry point with the same arguments (pointers included) at every step.  Everything
     // between the arguments and the launch - tile choice, tap table, five or six cuTensorMapEncodeTiled calls, the
     // shared-memory plan - depends on those arguments alone, so it is kept: the second and every later call with an
-    // identical argument list copies the finished TensorMaps / ContractParams and launches (host time per launch drops
+    // identical argument list launches straight from the finished TensorMaps / ContractParams (host time per launch drops
     // from ~20 us to a few, which matters once two streams have to be kept fed).  The key is the raw argument list.
     struct Plan
     {
         TensorMaps maps;
         ContractParams p;
-        int bn = 0, bk = 0, grid = 0;
+        const void* kernel = nullptr;
+        int grid = 0;
     };
     struct PlanKey
     {
-        uint64_t w[48];
+        uint64_t w[28];
         bool operator==(const PlanKey& o) const { return memcmp(w, o.w, sizeof(w)) == 0; }
     };
     struct PlanKeyHash
     {
         size_t operator()(const PlanKey& k) const
         {
-            uint64_t h = 1469598103934665603ull;
-            for (uint64_t v : k.w)
-                h = (h ^ v) * 1099511628211ull;
-            return size_t(h);
+            // four chains side by side: one chain of 28 dependent multiplications is a tenth of a microsecond
+            uint64_t h[4] = {1469598103934665603ull, 0x9E3779B97F4A7C15ull, 0xC2B2AE3D27D4EB4Full, 0x165667B19E3779F9ull};
+            for (int i = 0; i < 28; i += 4)
+                for (int j = 0; j < 4; ++j)
+                    h[j] = (h[j] ^ k.w[i + j]) * 1099511628211ull;
+            const uint64_t all = (h[0] ^ (h[1] >> 17)) + (h[2] ^ (h[3] << 23));
+            return size_t(all ^ (all >> 32));
         }
     };
     static std::mutex g_plan_mutex;
-    static std::unordered_map<PlanKey, Plan, PlanKeyHash>& plan_cache()
+    // plans are shared, not copied: a launch may still read one that the bound below has dropped
+    static std::unordered_map<PlanKey, std::shared_ptr<const Plan>, PlanKeyHash>& plan_cache()
     {
-        static std::unordered_map<PlanKey, Plan, PlanKeyHash> cache;
+        static std::unordered_map<PlanKey, std::shared_ptr<const Plan>, PlanKeyHash> cache;
         return cache;
     }
     static thread_local Plan* t_capture = nullptr; // set while an entry point builds a plan it wants to keep
 
-    static bool plan_lookup(const PlanKey& key, Plan& out)
+    static std::shared_ptr<const Plan> plan_lookup(const PlanKey& key)
     {
 #ifdef B200_PROFILE_WAITS
-        return false; // the instrumented build changes tile choices between calls through its environment switches
+        return nullptr; // the instrumented build changes tile choices between calls through its environment switches
 #endif
         std::lock_guard<std::mutex> lock(g_plan_mutex);
         auto it = plan_cache().find(key);
-        if (it == plan_cache().end())
-            return false;
-        out = it->second;
-        return true;
+        return it == plan_cache().end() ? nullptr : it->second;
     }
-    static void plan_store(const PlanKey& key, const Plan& plan)
+    static void plan_store(const PlanKey& key, std::shared_ptr<const Plan> plan)
     {
         std::lock_guard<std::mutex> lock(g_plan_mutex);
         if (plan_cache().size() >= 8192) // bounded: a client that never repeats an argument list gains nothing anyway
             plan_cache().clear();
-        plan_cache()[key] = plan;
+        plan_cache()[key] = std::move(plan);
     }
     static void key_epilogue(PlanKey& k, int at, const b200_epilogue* e)
     {
@@ -1937,8 +1935,7 @@ namespace b200
                                            : qcontract_kernel<BN, BK, false, false, EPI_BYTES>;
     }
 
-    template <int BN, int BK>
-    static int fire_contract(const TensorMaps& maps, const ContractParams& p, int grid, cudaStream_t st)
+    static int fire_contract(const void* kernel, const TensorMaps& maps, const ContractParams& p, int grid, cudaStream_t st)
     {
         // Programmatic dependent launch: the CTAs of this launch may become resident while the previous kernel of the
         // stream drains (SM by SM), set up their barriers, tensor memory and descriptors, and then wait in
@@ -1976,24 +1973,15 @@ namespace b200
         if (p.cta2) // the CTA-pair variant is compiled into instrumented builds only (see ContractParams::cta2)
             return B200_ERR_UNSUPPORTED;
 #endif
-        cudaError_t le = cudaLaunchKernelEx(&cfg, kernel_of<BN, BK>(p), maps, p);
+        // by address: the two structures (1.6 KB) go from the plan to the driver without a copy in between
+        void* args[2] = {const_cast<TensorMaps*>(&maps), const_cast<ContractParams*>(&p)};
+        cudaError_t le = cudaLaunchKernelExC(&cfg, kernel, args);
         if (le != cudaSuccess)
             return cuda_status(le, "cudaLaunchKernelEx(qcontract_kernel)");
         return after_launch("qcontract_kernel");
     }
 
-    static int fire_plan(const Plan& plan, cudaStream_t st)
-    {
-        if (plan.bk == 128)
-        {
-            if (plan.bn == 64) return fire_contract<64, 128>(plan.maps, plan.p, plan.grid, st);
-            if (plan.bn == 128) return fire_contract<128, 128>(plan.maps, plan.p, plan.grid, st);
-            return fire_contract<256, 128>(plan.maps, plan.p, plan.grid, st);
-        }
-        if (plan.bn == 64) return fire_contract<64, 64>(plan.maps, plan.p, plan.grid, st);
-        if (plan.bn == 128) return fire_contract<128, 64>(plan.maps, plan.p, plan.grid, st);
-        return fire_contract<256, 64>(plan.maps, plan.p, plan.grid, st);
-    }
+    static int fire_plan(const Plan& plan, cudaStream_t st) { return fire_contract(plan.kernel, plan.maps, plan.p, plan.grid, st); }
 
     template <int BN, int BK>
     static int launch_contract(const TensorMaps& maps, ContractParams& p, cudaStream_t st)
@@ -2095,12 +2083,12 @@ namespace b200
         if (sp.stages < MIN_STAGES)
             return B200_ERR_UNSUPPORTED;
         // a kernel is told once per device how much shared memory it may take
+        const void* kernel = reinterpret_cast<const void*>(kernel_of<BN, BK>(p));
         {
             static std::mutex mutex;
             static std::set<std::pair<int, const void*>> told;
             int dev = 0;
             cudaGetDevice(&dev);
-            const void* kernel = reinterpret_cast<const void*>(kernel_of<BN, BK>(p));
             std::lock_guard<std::mutex> lock(mutex);
             if (told.count({dev, kernel}) == 0)
             {
@@ -2119,11 +2107,10 @@ namespace b200
         {
             t_capture->maps = maps;
             t_capture->p = p;
-            t_capture->bn = BN;
-            t_capture->bk = BK;
+            t_capture->kernel = kernel;
             t_capture->grid = grid;
         }
-        return fire_contract<BN, BK>(maps, p, grid, st);
+        return fire_contract(kernel, maps, p, grid, st);
     }
 
     static int dispatch_contract(int bn, int bk, const TensorMaps& maps, ContractParams& p, cudaStream_t st)
@@ -2378,9 +2365,9 @@ static int qgemm_impl(const void* A, int a_type, const int8_t* W, bool packed, v
     key.w[5] = uint64_t(N);
     key.w[6] = uint64_t(K);
     key_epilogue(key, 8, epilogue);
-    Plan plan;
-    if (plan_lookup(key, plan))
-        return fire_plan(plan, static_cast<cudaStream_t>(stream));
+    if (const auto kept = plan_lookup(key))
+        return fire_plan(*kept, static_cast<cudaStream_t>(stream));
+    const auto plan = std::make_shared<Plan>();
 
     const int bk = 128;
     ContractParams p = {};
@@ -2431,7 +2418,7 @@ static int qgemm_impl(const void* A, int a_type, const int8_t* W, bool packed, v
         p.blk_bytes = 32 * COLS;
         make_out_maps(maps, p, 2, dims_o, str_o, box_o);
     }
-    t_capture = &plan;
+    t_capture = plan.get();
     rc = dispatch_contract(bn, bk, maps, p, static_cast<cudaStream_t>(stream));
     t_capture = nullptr;
     if (rc == B200_OK)
@@ -2563,9 +2550,9 @@ static int qconv_impl(const void* data, int data_type, const int8_t* filters, bo
     static_assert(sizeof(b200_conv_params) == 15 * 8, "key layout");
     memcpy(&key.w[4], c, sizeof(b200_conv_params));
     key_epilogue(key, 20, epilogue);
-    Plan plan;
-    if (plan_lookup(key, plan))
-        return fire_plan(plan, static_cast<cudaStream_t>(stream));
+    if (const auto kept = plan_lookup(key))
+        return fire_plan(*kept, static_cast<cudaStream_t>(stream));
+    const auto plan = std::make_shared<Plan>();
 
     const int bk = (c->C % 128 == 0) ? 128 : 64;
     ContractParams p = {};
@@ -2703,7 +2690,7 @@ static int qconv_impl(const void* data, int data_type, const int8_t* filters, bo
         p.blk_bytes = int(box_o[1] * box_o[2] * box_o[3]) * COLS;
         make_out_maps(maps, p, 4, dims_o, str_o, box_o);
     }
-    t_capture = &plan;
+    t_capture = plan.get();
     rc = dispatch_contract(bn, bk, maps, p, static_cast<cudaStream_t>(stream));
     t_capture = nullptr;
     if (rc == B200_OK)
@@ -2768,9 +2755,9 @@ extern "C" int b200_qconv_stem(const void* cells, int data_type, const int8_t* p
     const int64_t key_dims[10] = {N, H, W, K, R, S, pad_h, pad_w, pad_h_above, pad_w_above};
     memcpy(&key.w[4], key_dims, sizeof(key_dims));
     key_epilogue(key, 16, epilogue);
-    Plan plan;
-    if (plan_lookup(key, plan))
-        return fire_plan(plan, static_cast<cudaStream_t>(stream));
+    if (const auto kept = plan_lookup(key))
+        return fire_plan(*kept, static_cast<cudaStream_t>(stream));
+    const auto plan = std::make_shared<Plan>();
 
     const int bk = 64;
     ContractParams p = {};
@@ -2841,7 +2828,7 @@ extern "C" int b200_qconv_stem(const void* cells, int data_type, const int8_t* p
         p.RW = p.TW;
         make_out_maps(maps, p, 4, dims_o, str_o, box_o);
     }
-    t_capture = &plan;
+    t_capture = plan.get();
     rc = dispatch_contract(bn, bk, maps, p, static_cast<cudaStream_t>(stream));
     t_capture = nullptr;
     if (rc == B200_OK)

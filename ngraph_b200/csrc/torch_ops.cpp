@@ -7,7 +7,10 @@
 // that ngraph_b200/lib.py loaded is the one that runs.
 #include <Python.h>
 #include <ATen/ATen.h>
+#include <ATen/EmptyTensor.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
@@ -51,18 +54,19 @@ namespace
         }
         return THPVariable_Unpack(o);
     }
-    // a CUDA tensor, contiguous (a copy where it is not)
-    inline at::Tensor dev(PyObject* o)
+    // a CUDA tensor, contiguous: the caller's own (which the caller holds during the call), a copy where it is not
+    using Dev = c10::MaybeOwned<at::Tensor>;
+    inline Dev dev(PyObject* o)
     {
         const at::Tensor& t = tensor(o);
         require(t.is_cuda(), "b200 ops take CUDA tensors");
-        return t.is_contiguous() ? t : t.contiguous();
+        return t.expect_contiguous();
     }
-    inline at::Tensor dev(PyObject* o, at::ScalarType type)
+    inline Dev dev(PyObject* o, at::ScalarType type)
     {
-        at::Tensor t = dev(o);
-        if (t.scalar_type() != type)
-            fail_assert((std::string("tensor of ") + c10::toString(t.scalar_type()) + " where " + c10::toString(type) + " is wanted").c_str());
+        Dev t = dev(o);
+        if (t->scalar_type() != type)
+            fail_assert((std::string("tensor of ") + c10::toString(t->scalar_type()) + " where " + c10::toString(type) + " is wanted").c_str());
         return t;
     }
     inline int code(at::ScalarType t)
@@ -131,8 +135,12 @@ namespace
         Py_DECREF(f);
         return int(n);
     }
+    // torch.empty on the device of `like`; on the current device (where `like` shows that CUDA is initialised) without the
+    // device guard and the initialisation checks, a fifth of the allocation
     inline at::Tensor empty(at::IntArrayRef shape, at::ScalarType type, const at::Tensor& like)
     {
+        if (like.get_device() == c10::cuda::current_device())
+            return at::Tensor(at::detail::empty_generic(shape, c10::cuda::CUDACachingAllocator::get(), c10::DispatchKeySet(c10::DispatchKey::CUDA), type, c10::nullopt));
         return at::Tensor(at::detail::empty_cuda(shape, type, like.device(), c10::nullopt));
     }
     inline void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
@@ -180,16 +188,16 @@ namespace
     PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t n)
     {
         return guarded(n, 6, [&]() -> PyObject* {
-            const at::Tensor x = dev(a[0], at::kFloat), scale = dev(a[1], at::kFloat), zp = dev(a[2]);
+            const Dev x = dev(a[0], at::kFloat), scale = dev(a[1], at::kFloat), zp = dev(a[2]);
             int64_t axes[B200_MAX_RANK];
             const int n_axes = integers(a[3], axes);
             std::sort(axes, axes + n_axes);
-            const int mode = int(integer(a[4])), type = code(zp.scalar_type());
-            const at::Tensor out = a[5] == Py_None ? empty(x.sizes(), zp.scalar_type(), x) : tensor(a[5]);
+            const int mode = int(integer(a[4])), type = code(zp->scalar_type());
+            const at::Tensor out = a[5] == Py_None ? empty(x->sizes(), zp->scalar_type(), *x) : tensor(a[5]);
             void* st = stream();
             check(unlocked([&] {
-                      return p_quantize(static_cast<const float*>(x.data_ptr()), static_cast<const float*>(scale.data_ptr()), zp.data_ptr(), out.data_ptr(),
-                                        type, x.sizes().data(), int(x.dim()), axes, n_axes, mode, st);
+                      return p_quantize(static_cast<const float*>(x->data_ptr()), static_cast<const float*>(scale->data_ptr()), zp->data_ptr(), out.data_ptr(),
+                                        type, x->sizes().data(), int(x->dim()), axes, n_axes, mode, st);
                   }),
                   "b200_quantize");
             return THPVariable_Wrap(out);
@@ -198,17 +206,17 @@ namespace
     PyObject* dequantize(PyObject*, PyObject* const* a, Py_ssize_t n)
     {
         return guarded(n, 5, [&]() -> PyObject* {
-            const at::Tensor x = dev(a[0]), scale = dev(a[1], at::kFloat), zp = dev(a[2]);
-            require(zp.scalar_type() == x.scalar_type(), "zero_point has the type of x");
+            const Dev x = dev(a[0]), scale = dev(a[1], at::kFloat), zp = dev(a[2]);
+            require(zp->scalar_type() == x->scalar_type(), "zero_point has the type of x");
             int64_t axes[B200_MAX_RANK];
             const int n_axes = integers(a[3], axes);
             std::sort(axes, axes + n_axes);
-            const int type = code(x.scalar_type());
-            const at::Tensor out = a[4] == Py_None ? empty(x.sizes(), at::kFloat, x) : tensor(a[4]);
+            const int type = code(x->scalar_type());
+            const at::Tensor out = a[4] == Py_None ? empty(x->sizes(), at::kFloat, *x) : tensor(a[4]);
             void* st = stream();
             check(unlocked([&] {
-                      return p_dequantize(x.data_ptr(), static_cast<const float*>(scale.data_ptr()), zp.data_ptr(), static_cast<float*>(out.data_ptr()), type,
-                                          x.sizes().data(), int(x.dim()), axes, n_axes, st);
+                      return p_dequantize(x->data_ptr(), static_cast<const float*>(scale->data_ptr()), zp->data_ptr(), static_cast<float*>(out.data_ptr()), type,
+                                          x->sizes().data(), int(x->dim()), axes, n_axes, st);
                   }),
                   "b200_dequantize");
             return THPVariable_Wrap(out);
@@ -219,25 +227,25 @@ namespace
     struct EpilogueArgs
     {
         b200_epilogue e{};
-        at::Tensor scale, bias, sum_in, sum_scale;
+        Dev scale, bias, sum_in, sum_scale;
         // a: scale, out_dtype, bias, relu, sum_in, sum_scale, core, out_zp
         explicit EpilogueArgs(PyObject* const* a)
         {
             scale = dev(a[0], at::kFloat);
-            e.scale = static_cast<const float*>(scale.data_ptr());
-            e.scale_count = scale.numel();
+            e.scale = static_cast<const float*>(scale->data_ptr());
+            e.scale_count = scale->numel();
             if (a[2] != Py_None)
             {
                 bias = dev(a[2], at::kInt);
-                e.bias = static_cast<const int32_t*>(bias.data_ptr());
+                e.bias = static_cast<const int32_t*>(bias->data_ptr());
             }
             if (a[4] != Py_None)
             {
                 sum_in = dev(a[4]);
                 sum_scale = dev(a[5], at::kFloat);
-                e.sum_in = sum_in.data_ptr();
-                e.sum_type = code(sum_in.scalar_type());
-                e.sum_scale = static_cast<const float*>(sum_scale.data_ptr());
+                e.sum_in = sum_in->data_ptr();
+                e.sum_type = code(sum_in->scalar_type());
+                e.sum_scale = static_cast<const float*>(sum_scale->data_ptr());
             }
             e.relu = truth(a[3]);
             e.round_half_away = truth(a[6]);
@@ -255,14 +263,14 @@ namespace
     PyObject* qgemm(PyObject*, PyObject* const* a, Py_ssize_t n)
     {
         return guarded(n, 11, [&]() -> PyObject* {
-            const at::Tensor x = dev(a[0]), w = dev(a[1]);
-            const int types = operands(x, w);
-            require(x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1), "a is [M,K] and w is [N,K]");
+            const Dev x = dev(a[0]), w = dev(a[1]);
+            const int types = operands(*x, *w);
+            require(x->dim() == 2 && w->dim() == 2 && x->size(1) == w->size(1), "a is [M,K] and w is [N,K]");
             const EpilogueArgs e(a + 3);
-            const int64_t m = x.size(0), k = x.size(1), cols = w.size(0);
-            const at::Tensor out = a[2] == Py_None ? empty({m, cols}, dtype(a[4]), x) : tensor(a[2]);
+            const int64_t m = x->size(0), k = x->size(1), cols = w->size(0);
+            const at::Tensor out = a[2] == Py_None ? empty({m, cols}, dtype(a[4]), *x) : tensor(a[2]);
             void* st = stream();
-            check(unlocked([&] { return p_qgemm(x.data_ptr(), types, static_cast<const int8_t*>(w.data_ptr()), out.data_ptr(), m, cols, k, &e.e, st); }),
+            check(unlocked([&] { return p_qgemm(x->data_ptr(), types, static_cast<const int8_t*>(w->data_ptr()), out.data_ptr(), m, cols, k, &e.e, st); }),
                   "b200_qgemm");
             return THPVariable_Wrap(out);
         });
@@ -291,17 +299,17 @@ namespace
     PyObject* qconv(PyObject*, PyObject* const* a, Py_ssize_t n)
     {
         return guarded(n, 13, [&]() -> PyObject* {
-            const at::Tensor x = dev(a[0]), f = dev(a[1]);
-            const int types = operands(x, f);
+            const Dev x = dev(a[0]), f = dev(a[1]);
+            const int types = operands(*x, *f);
             const Params cp(a[2]);
             const bool packed = truth(a[3]);
             const EpilogueArgs e(a + 5);
             int64_t p, q;
             check(p_qconv_out_shape(cp.get(), &p, &q), "b200_qconv_out_shape");
-            const at::Tensor out = a[4] == Py_None ? empty({cp.get()->N, p, q, cp.get()->K}, dtype(a[6]), x) : tensor(a[4]);
+            const at::Tensor out = a[4] == Py_None ? empty({cp.get()->N, p, q, cp.get()->K}, dtype(a[6]), *x) : tensor(a[4]);
             void* st = stream();
             check(unlocked([&] {
-                      return (packed ? p_qconv_packed : p_qconv)(x.data_ptr(), types, static_cast<const int8_t*>(f.data_ptr()), out.data_ptr(), cp.get(), &e.e,
+                      return (packed ? p_qconv_packed : p_qconv)(x->data_ptr(), types, static_cast<const int8_t*>(f->data_ptr()), out.data_ptr(), cp.get(), &e.e,
                                                                  st);
                   }),
                   packed ? "b200_qconv_packed" : "b200_qconv");
@@ -313,35 +321,35 @@ namespace
     PyObject* nchw_to_nhwc(PyObject*, PyObject* const* a, Py_ssize_t n)
     {
         return guarded(n, 2, [&]() -> PyObject* {
-            const at::Tensor x = dev(a[0]);
-            require(x.element_size() == 1 && x.dim() == 4, "one-byte elements, four dimensions");
-            const int64_t N = x.size(0), c = x.size(1), h = x.size(2), w = x.size(3), c_pad = a[1] == Py_None ? c : integer(a[1]);
-            const at::Tensor out = empty({N, h, w, c_pad}, x.scalar_type(), x);
+            const Dev x = dev(a[0]);
+            require(x->element_size() == 1 && x->dim() == 4, "one-byte elements, four dimensions");
+            const int64_t N = x->size(0), c = x->size(1), h = x->size(2), w = x->size(3), c_pad = a[1] == Py_None ? c : integer(a[1]);
+            const at::Tensor out = empty({N, h, w, c_pad}, x->scalar_type(), *x);
             void* st = stream();
-            check(unlocked([&] { return p_nchw_to_nhwc(x.data_ptr(), out.data_ptr(), N, c, h, w, c_pad, st); }), "b200_nchw_to_nhwc_u8");
+            check(unlocked([&] { return p_nchw_to_nhwc(x->data_ptr(), out.data_ptr(), N, c, h, w, c_pad, st); }), "b200_nchw_to_nhwc_u8");
             return THPVariable_Wrap(out);
         });
     }
     PyObject* nhwc_to_nchw(PyObject*, PyObject* const* a, Py_ssize_t n)
     {
         return guarded(n, 2, [&]() -> PyObject* {
-            const at::Tensor x = dev(a[0]);
-            require(x.element_size() == 1 && x.dim() == 4, "one-byte elements, four dimensions");
-            const int64_t N = x.size(0), h = x.size(1), w = x.size(2), c_pad = x.size(3), c = a[1] == Py_None ? c_pad : integer(a[1]);
-            const at::Tensor out = empty({N, c, h, w}, x.scalar_type(), x);
+            const Dev x = dev(a[0]);
+            require(x->element_size() == 1 && x->dim() == 4, "one-byte elements, four dimensions");
+            const int64_t N = x->size(0), h = x->size(1), w = x->size(2), c_pad = x->size(3), c = a[1] == Py_None ? c_pad : integer(a[1]);
+            const at::Tensor out = empty({N, c, h, w}, x->scalar_type(), *x);
             void* st = stream();
-            check(unlocked([&] { return p_nhwc_to_nchw(x.data_ptr(), out.data_ptr(), N, c, h, w, c_pad, st); }), "b200_nhwc_to_nchw_u8");
+            check(unlocked([&] { return p_nhwc_to_nchw(x->data_ptr(), out.data_ptr(), N, c, h, w, c_pad, st); }), "b200_nhwc_to_nchw_u8");
             return THPVariable_Wrap(out);
         });
     }
     PyObject* transpose(PyObject*, PyObject* const* a, Py_ssize_t n)
     {
         return guarded(n, 1, [&]() -> PyObject* {
-            const at::Tensor x = dev(a[0]);
-            require(x.element_size() == 1 && x.dim() == 2, "one-byte elements, two dimensions");
-            const at::Tensor out = empty({x.size(1), x.size(0)}, x.scalar_type(), x);
+            const Dev x = dev(a[0]);
+            require(x->element_size() == 1 && x->dim() == 2, "one-byte elements, two dimensions");
+            const at::Tensor out = empty({x->size(1), x->size(0)}, x->scalar_type(), *x);
             void* st = stream();
-            check(unlocked([&] { return p_transpose(x.data_ptr(), out.data_ptr(), x.size(0), x.size(1), st); }), "b200_transpose_u8");
+            check(unlocked([&] { return p_transpose(x->data_ptr(), out.data_ptr(), x->size(0), x->size(1), st); }), "b200_transpose_u8");
             return THPVariable_Wrap(out);
         });
     }
@@ -350,8 +358,8 @@ namespace
     PyObject* maxpool(PyObject*, PyObject* const* a, Py_ssize_t n)
     {
         return guarded(n, 5, [&]() -> PyObject* {
-            const at::Tensor x = dev(a[0], at::kByte);
-            require(x.dim() == 4, "x is [N,H,W,C]");
+            const Dev x = dev(a[0], at::kByte);
+            require(x->dim() == 4, "x is [N,H,W,C]");
             int64_t v[4][2];
             for (int i = 0; i < 4; ++i)
                 if (integers(a[1 + i], v[i]) != 2)
@@ -359,7 +367,7 @@ namespace
                     PyErr_SetString(PyExc_ValueError, "window, stride and paddings are pairs");
                     throw PyError();
                 }
-            const int64_t N = x.size(0), h = x.size(1), w = x.size(2), c = x.size(3);
+            const int64_t N = x->size(0), h = x->size(1), w = x->size(2), c = x->size(3);
             int64_t d[2];
             for (int i = 0; i < 2; ++i)
             {
@@ -371,10 +379,10 @@ namespace
                 const int64_t room = (i == 0 ? h : w) + v[2][i] + v[3][i] - v[0][i];
                 d[i] = (room >= 0 ? room / v[1][i] : -((-room + v[1][i] - 1) / v[1][i])) + 1;
             }
-            const at::Tensor out = empty({N, d[0], d[1], c}, at::kByte, x);
+            const at::Tensor out = empty({N, d[0], d[1], c}, at::kByte, *x);
             void* st = stream();
             check(unlocked([&] {
-                      return p_maxpool(x.data_ptr(), out.data_ptr(), N, h, w, c, v[0][0], v[0][1], v[1][0], v[1][1], v[2][0], v[2][1], v[3][0], v[3][1], st);
+                      return p_maxpool(x->data_ptr(), out.data_ptr(), N, h, w, c, v[0][0], v[0][1], v[1][0], v[1][1], v[2][0], v[2][1], v[3][0], v[3][1], st);
                   }),
                   "b200_maxpool_nhwc_u8");
             return THPVariable_Wrap(out);
@@ -384,13 +392,13 @@ namespace
     PyObject* global_avgpool(PyObject*, PyObject* const* a, Py_ssize_t n)
     {
         return guarded(n, 3, [&]() -> PyObject* {
-            const at::Tensor x = dev(a[0], at::kByte), in = dev(a[1], at::kFloat), o = dev(a[2], at::kFloat);
-            require(x.dim() == 4, "x is [N,H,W,C]");
-            const at::Tensor out = empty({x.size(0), x.size(3)}, at::kByte, x);
+            const Dev x = dev(a[0], at::kByte), in = dev(a[1], at::kFloat), o = dev(a[2], at::kFloat);
+            require(x->dim() == 4, "x is [N,H,W,C]");
+            const at::Tensor out = empty({x->size(0), x->size(3)}, at::kByte, *x);
             void* st = stream();
             check(unlocked([&] {
-                      return p_avgpool(x.data_ptr(), out.data_ptr(), static_cast<const float*>(in.data_ptr()), static_cast<const float*>(o.data_ptr()), x.size(0),
-                                       x.size(1), x.size(2), x.size(3), st);
+                      return p_avgpool(x->data_ptr(), out.data_ptr(), static_cast<const float*>(in->data_ptr()), static_cast<const float*>(o->data_ptr()), x->size(0),
+                                       x->size(1), x->size(2), x->size(3), st);
                   }),
                   "b200_global_avgpool_q_nhwc_u8");
             return THPVariable_Wrap(out);
