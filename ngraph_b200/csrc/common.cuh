@@ -39,14 +39,14 @@ namespace b200
         return n;
     }
 
-    // Programmatic dependent launch of small kernels: in a chain of kernels of 2-5 us each, about 0.5 us per launch is the way
-    // from one kernel's end to the next one's first instruction.  A kernel launched with `launch` may become resident while
-    // its predecessor drains, and must call after_earlier_kernels before it touches global memory.
-    // Only grids of at most two blocks per SM are launched this way: early blocks crowd onto the SMs that the predecessor leaves
-    // free, which costs a larger kernel more than it gains (measured: ResNet-50 at batch 128 +29 us with pooling and packing
-    // launched early, the 24576-token encoder layer +38 us).  Nor do these kernels let their successors in before their
-    // end, as the contractions do: successors of theirs gained nothing from it (small encoder layer 148 us of kernels with it, 131
-    // without, 147 with plain launches).
+    // Programmatic dependent launch: in a stream a plain launch costs about 2.2 us between one kernel's end and the next one's
+    // first instruction, such a launch 0.3-0.5 (chains of kernels of 3 us, 148 blocks: 6.1 against 3.6 us each).  A kernel
+    // launched with `launch` may become resident while its predecessor drains, and must call after_earlier_kernels before it
+    // touches global memory.  Kernels of this kind do not let their successors in before their end (small encoder layer 148 us of
+    // kernels if they do, 131 without); a contraction that fills the GPU does when its last results are left to write, so
+    // that the blocks of a large successor do not crowd onto the SMs that are free first (ResNet-50 at batch 128: 1243 us
+    // with contractions that let it in at once, 1225 so, 1230 with plain launches of large kernels; Quantize of 98 MB
+    // 20.5 -> 19.1, Dequantize of 256 MB 53.7 -> 51.8).
     template <typename... P, typename... A>
     inline void launch(void (*kernel)(P...), unsigned grid, unsigned block, size_t shared, cudaStream_t st, A... args)
     {
@@ -59,7 +59,7 @@ namespace b200
         cfg.dynamicSmemBytes = shared;
         cfg.stream = st;
         cfg.attrs = &attr;
-        cfg.numAttrs = grid <= 2u * unsigned(sm_count()) ? 1 : 0;
+        cfg.numAttrs = 1;
         cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...); // an error is picked up by after_launch
     }
 #ifdef __CUDACC__

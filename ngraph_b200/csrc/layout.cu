@@ -82,6 +82,7 @@ namespace b200
                                                                   int win_w, int stride_h, int stride_w, int pad_h,
                                                                   int pad_w)
     {
+        after_earlier_kernels(in, out);
         int64_t total = int64_t(N) * P * Q * C16;
         for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x)
         {
@@ -121,6 +122,7 @@ namespace b200
                                                                         int N, int H, int W, int C16, int P, int Q, int stride_h,
                                                                         int stride_w, int pad_h, int pad_w)
     {
+        after_earlier_kernels(in, out);
         const uint32_t total = uint32_t(N) * P * Q * C16;
         for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
         {
@@ -158,6 +160,7 @@ namespace b200
     __global__ void __launch_bounds__(256) maxpool_nhwc_u8_3x3s2_pair_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, int N, int H,
                                                                              int W, int C16, int P, int Q, int pad_h, int pad_w)
     {
+        after_earlier_kernels(in, out);
         const uint32_t Q2 = uint32_t(Q + 1) / 2;
         const uint32_t total = uint32_t(N) * P * Q2 * C16;
         for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
@@ -216,6 +219,7 @@ namespace b200
                                                                    const float* __restrict__ s_in,
                                                                    const float* __restrict__ s_out, int N, int HW, int C)
     {
+        after_earlier_kernels(in, out, s_in, s_out);
         int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
         if (i >= int64_t(N) * C)
             return;
@@ -619,25 +623,23 @@ static int maxpool_nhwc_bytes(bool is_signed, const void* in, void* out, int64_t
     const uint4* in4 = static_cast<const uint4*>(in);
     uint4* out4 = static_cast<uint4*>(out);
     if (is_signed)
-        maxpool_nhwc_u8_kernel<true><<<grid, 256, 0, st>>>(static_cast<const uint8_t*>(in), static_cast<uint8_t*>(out), int(N), int(H),
-                                                           int(W), int(C / 16), int(P), int(Q), int(win_h), int(win_w),
-                                                           int(stride_h), int(stride_w), int(pad_h), int(pad_w));
+        launch(maxpool_nhwc_u8_kernel<true>, grid, 256, 0, st, static_cast<const uint8_t*>(in), static_cast<uint8_t*>(out), int(N), int(H),
+               int(W), int(C / 16), int(P), int(Q), int(win_h), int(win_w), int(stride_h), int(stride_w), int(pad_h), int(pad_w));
     else if (small && win_h == 3 && win_w == 3 && stride_h == 2 && stride_w == 2)
     {
         const int64_t threads = N * P * ((Q + 1) / 2) * (C / 16), pair_blocks = (threads + 255) / 256;
-        maxpool_nhwc_u8_3x3s2_pair_kernel<<<unsigned(pair_blocks < b200::sm_count() * 32 ? pair_blocks : b200::sm_count() * 32), 256, 0, st>>>(
-            in4, out4, int(N), int(H), int(W), int(C / 16), int(P), int(Q), int(pad_h), int(pad_w));
+        launch(maxpool_nhwc_u8_3x3s2_pair_kernel, unsigned(pair_blocks < b200::sm_count() * 32 ? pair_blocks : b200::sm_count() * 32), 256, 0, st,
+               in4, out4, int(N), int(H), int(W), int(C / 16), int(P), int(Q), int(pad_h), int(pad_w));
     }
     else if (small && win_h == 3 && win_w == 3)
-        maxpool_nhwc_u8_fixed_kernel<3, 3><<<grid, 256, 0, st>>>(in4, out4, int(N), int(H), int(W), int(C / 16), int(P), int(Q),
-                                                                 int(stride_h), int(stride_w), int(pad_h), int(pad_w));
+        launch(maxpool_nhwc_u8_fixed_kernel<3, 3>, grid, 256, 0, st, in4, out4, int(N), int(H), int(W), int(C / 16), int(P), int(Q),
+               int(stride_h), int(stride_w), int(pad_h), int(pad_w));
     else if (small && win_h == 2 && win_w == 2)
-        maxpool_nhwc_u8_fixed_kernel<2, 2><<<grid, 256, 0, st>>>(in4, out4, int(N), int(H), int(W), int(C / 16), int(P), int(Q),
-                                                                 int(stride_h), int(stride_w), int(pad_h), int(pad_w));
+        launch(maxpool_nhwc_u8_fixed_kernel<2, 2>, grid, 256, 0, st, in4, out4, int(N), int(H), int(W), int(C / 16), int(P), int(Q),
+               int(stride_h), int(stride_w), int(pad_h), int(pad_w));
     else
-        maxpool_nhwc_u8_kernel<false><<<grid, 256, 0, st>>>(static_cast<const uint8_t*>(in), static_cast<uint8_t*>(out), int(N), int(H),
-                                                     int(W), int(C / 16), int(P), int(Q), int(win_h), int(win_w),
-                                                     int(stride_h), int(stride_w), int(pad_h), int(pad_w));
+        launch(maxpool_nhwc_u8_kernel<false>, grid, 256, 0, st, static_cast<const uint8_t*>(in), static_cast<uint8_t*>(out), int(N), int(H),
+               int(W), int(C / 16), int(P), int(Q), int(win_h), int(win_w), int(stride_h), int(stride_w), int(pad_h), int(pad_w));
     return after_launch(what);
 }
 
@@ -668,8 +670,8 @@ extern "C" int b200_global_avgpool_q_nhwc_u8(const void* in, void* out, const fl
     if (!in || !out || !scale_in || !scale_out)
         return B200_ERR_INVALID_ARGUMENT;
     int64_t total = N * C;
-    global_avgpool_q_kernel<<<unsigned((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint8_t*>(in), static_cast<uint8_t*>(out), scale_in, scale_out, int(N), int(H * W), int(C));
+    launch(global_avgpool_q_kernel, unsigned((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(in),
+           static_cast<uint8_t*>(out), scale_in, scale_out, int(N), int(H * W), int(C));
     return after_launch("b200_global_avgpool_q_nhwc_u8");
 }
 
@@ -805,6 +807,7 @@ namespace b200
     __global__ void __launch_bounds__(256) s2d_pack_kernel(const uint8_t* __restrict__ in, uint4* __restrict__ out, int N, int C,
                                                            int H, int W, int Hc, int Wc, int eh, int ew)
     {
+        after_earlier_kernels(in, out);
         // eh / ew: even shift of image rows / columns inside the cell grid
         int64_t total = int64_t(N) * Hc * Wc;
         for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x)
@@ -864,6 +867,7 @@ namespace b200
                                                                const Q* __restrict__ zero_point, int mode, uint4* __restrict__ out,
                                                                int N, int C, int H, int W, int Hc, int Wc, int eh, int ew)
     {
+        after_earlier_kernels(in, scale, zero_point, out);
         const float s = __ldg(scale);
         const int zi = int(__ldg(zero_point));
         const float zp = float(zi), y = __frcp_rn(s);
@@ -944,6 +948,7 @@ namespace b200
                                                                     const Q* __restrict__ zero_point, int mode, uint4* __restrict__ out,
                                                                     int N, int C, int H, int W, int Hc, int Wc, int eh, int ew)
     {
+        after_earlier_kernels(in, scale, zero_point, out);
         const float s = __ldg(scale);
         const int zi = int(__ldg(zero_point));
         const float zp = float(zi), y = __frcp_rn(s);
@@ -1065,9 +1070,8 @@ extern "C" int b200_stem_pack_input(const void* in_nchw, void* cells, int64_t N,
     int64_t total = N * Hc * Wc;
     int64_t blocks = (total + 255) / 256;
     unsigned grid = unsigned(blocks < b200::sm_count() * 32 ? blocks : b200::sm_count() * 32);
-    s2d_pack_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const uint8_t*>(in_nchw),
-                                                                       static_cast<uint4*>(cells), int(N), int(C), int(H), int(W),
-                                                                       int(Hc), int(Wc), int(eh), int(ew));
+    b200::launch(s2d_pack_kernel, grid, 256, 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(in_nchw), static_cast<uint4*>(cells),
+                 int(N), int(C), int(H), int(W), int(Hc), int(Wc), int(eh), int(ew));
     return after_launch("b200_stem_pack_input");
 }
 
@@ -1098,20 +1102,18 @@ extern "C" int b200_stem_pack_input_f32(const float* in_nchw, const float* scale
     const bool pairs = (W % 2 == 0) && (reinterpret_cast<uintptr_t>(in_nchw) & 7) == 0;
     // round-to-nearest-even may take the division-free quotient; the kernel checks the scale (it lives on the device)
     const bool rne = round_mode == B200_ROUND_NEAREST_TOWARD_EVEN && (g_fast_division.load(std::memory_order_relaxed) != 0);
-#define B200_S2D_LAUNCH(Q, FAST, PAIRS)                                                                                         \
-    s2d_pack_f32_kernel<Q, FAST, PAIRS><<<grid, 256, 0, st>>>(in_nchw, scale, static_cast<const Q*>(zero_point), round_mode,     \
-                                                              static_cast<uint4*>(cells), int(N), int(C), int(H), int(W), int(Hc), \
-                                                              int(Wc), int(eh), int(ew))
+#define B200_S2D_LAUNCH(Q, FAST, PAIRS)                                                                                          \
+    launch(s2d_pack_f32_kernel<Q, FAST, PAIRS>, grid, 256, 0, st, in_nchw, scale, static_cast<const Q*>(zero_point), round_mode, \
+           static_cast<uint4*>(cells), int(N), int(C), int(H), int(W), int(Hc), int(Wc), int(eh), int(ew))
     // rows that can be read four floats at a time: two cells per thread
     const bool quads = (W % 4 == 0) && (ew % 4 == 0) && (reinterpret_cast<uintptr_t>(in_nchw) & 15) == 0;
     if (quads)
     {
         const int64_t threads = N * Hc * ((Wc + 1) / 2);
         const unsigned qgrid = unsigned((threads + 255) / 256);
-#define B200_S2D_QUAD(Q, FAST)                                                                                                  \
-    s2d_pack_f32_quad_kernel<Q, FAST><<<qgrid, 256, 0, st>>>(in_nchw, scale, static_cast<const Q*>(zero_point), round_mode,      \
-                                                             static_cast<uint4*>(cells), int(N), int(C), int(H), int(W), int(Hc), \
-                                                             int(Wc), int(eh), int(ew))
+#define B200_S2D_QUAD(Q, FAST)                                                                                                   \
+    launch(s2d_pack_f32_quad_kernel<Q, FAST>, qgrid, 256, 0, st, in_nchw, scale, static_cast<const Q*>(zero_point), round_mode,  \
+           static_cast<uint4*>(cells), int(N), int(C), int(H), int(W), int(Hc), int(Wc), int(eh), int(ew))
         if (q_type == B200_U8)
         {
             if (rne) B200_S2D_QUAD(uint8_t, true);

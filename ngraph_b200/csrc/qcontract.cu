@@ -126,6 +126,7 @@ namespace b200
                              // (8192^3: 1.5 against 3.0 POP/s): with the same bytes in flight per SM the stage loop is twice
                              // as long (free -> landed takes 3 us per 32 KB stage, six stages per 4 us).  Never chosen; the
                              // variant is compiled into instrumented builds only, which can force it.
+        int late_successor;  // the stream's next kernel is let in when this one is about done (otherwise: at once)
         int split;           // CTAs that share one tile's reduction (a thread-block cluster), 1: none
         void* out;
         uint32_t idesc;
@@ -737,7 +738,8 @@ namespace b200
         // here left 0.8-1.1 us of tile decoding and cold parameter reads between its return and the first load of every
         // launch.  (No-ops when the launch is not a programmatic dependent one.)
         auto wait_for_earlier_kernels = []() { asm volatile("griddepcontrol.wait;" ::: "memory"); };
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        if (!p.late_successor)
+            asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
         const int num_tiles = p.tiles_m * p.tiles_n;
         // naps between polls spare the epilogue's issue slots in a steady state; a CTA with one unit of work has none, and every
@@ -1146,6 +1148,8 @@ namespace b200
                     if (pair == 2)
                         ptx::mma_commit(tfull_bar(acc + 1));
                 }
+                if (p.late_successor) // this CTA has only its last results left to write
+                    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
             }
         }
         else
@@ -2103,6 +2107,10 @@ namespace b200
         int grid = p.split > 1 ? tiles * p.split : tiles < num_sms() ? tiles : num_sms();
         if (p.cta2) // two CTAs per unit of two row tiles
             grid = 2 * std::min(tiles / 2, num_sms() / 2);
+        // A launch that fills the GPU lets the next kernel in when its last accumulators are done: there is no room for it earlier,
+        // and blocks let in at once gather on the SMs that finish first (see `launch`).  A smaller one lets it in at once:
+        // the next kernel sets up on the SMs that this one leaves idle.
+        p.late_successor = p.split == 1 && grid >= num_sms();
         if (t_capture)
         {
             t_capture->maps = maps;

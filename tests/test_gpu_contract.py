@@ -596,3 +596,34 @@ def test_qconv_resident_weights_over_many_tiles(ops, cfg, residual):
     cs_s = ref.conv_shape((len(sl),) + data.shape[1:], filt.shape, (1, 1), pad, pad, (1, 1))
     kw = {"sum_in": s_u8[sl], "sum_scale": np.float32(0.61)} if residual else {}
     np.testing.assert_array_equal(got[sl], ref.qconv_fused(data[sl], filt, bias, scale, cs_s, np.uint8, relu=True, **kw))
+
+
+@pytest.mark.parametrize("m,n", [(1, 16), (300, 128), (148 * 128, 128), (30001, 272)])
+def test_chained_launches_share_their_buffers(ops, m, n):
+    """Kernels become resident while their predecessors drain: shared intermediates are read and overwritten in stream order,
+    whether the predecessor fills the GPU or not"""
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    xs = [torch.randn((m, 256), generator=gen, device="cuda") for _ in range(6)]
+    w = torch.randint(-127, 128, (n, 256), generator=gen, device="cuda", dtype=torch.int8)
+    s_x, s_y, zp = torch.full((), 0.03, device="cuda"), torch.full((), 4.0, device="cuda"), torch.zeros((), dtype=torch.int8, device="cuda")
+    scale = torch.full((n,), 0.01, device="cuda")
+
+    def passes(wait):
+        q = torch.empty((m, 256), dtype=torch.int8, device="cuda")
+        y, z = torch.empty((m, n), device="cuda"), torch.empty((m, n), dtype=torch.int8, device="cuda")
+        outs = [torch.empty((m, n), device="cuda") for _ in xs]
+        torch.cuda.synchronize()
+        for x, out in zip(xs, outs):
+            for step in (lambda: ops.quantize(x, s_x, zp, out=q), lambda: ops.qgemm(q, w, scale, torch.float32, out=y),
+                         lambda: ops.quantize(y, s_y, zp, out=z), lambda: ops.dequantize(z, s_y, zp, out=out)):
+                step()
+                if wait:
+                    torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return outs
+
+    one_by_one = passes(True)
+    assert one_by_one[0].abs().max() > 0
+    for _ in range(5):
+        for a, b in zip(passes(False), one_by_one):
+            assert torch.equal(a, b)
