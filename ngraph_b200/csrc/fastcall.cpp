@@ -17,6 +17,7 @@
 namespace
 {
     PyTypeObject *void_pointer_type, *float_type, *array_type; // ctypes.c_void_p, c_float, Array
+    char int64_format[8]; // how the buffer of a c_int64 array names its elements
 
     // What byref() makes is opaque; where its pointer, its tag and the object it refers to lie is found out at import, against
     // known objects (find_byref_layout).  Where that does not hold, byref arguments go to ctypes.
@@ -79,10 +80,13 @@ namespace
             out = nullptr;
             return true;
         }
-        if (Py_TYPE(o) == void_pointer_type)
-            return bytes_of(o, &out, sizeof(out));
+        // lib.py declares int64_t* and the structures as POINTER: of those ctypes takes arrays of the very type (or byref), no
+        // c_void_p and no array of another type of the same size
+        constexpr bool typed = std::is_same<std::remove_cv_t<T>, int64_t>::value;
         if constexpr (std::is_class<T>::value)
             return by_reference(o, out);
+        if (Py_TYPE(o) == void_pointer_type)
+            return !typed && bytes_of(o, &out, sizeof(out));
         if (PyObject_TypeCheck(o, array_type))
         {
             Py_buffer v;
@@ -92,7 +96,7 @@ namespace
                 return false;
             }
             out = static_cast<T*>(v.buf);
-            const bool ok = v.itemsize == Py_ssize_t(sizeof(std::conditional_t<std::is_void<T>::value, int64_t, T>));
+            const bool ok = !typed || (v.ndim == 1 && v.format && strcmp(v.format, int64_format) == 0);
             PyBuffer_Release(&v); // the caller holds the array
             return ok;
         }
@@ -218,6 +222,25 @@ namespace
         Py_XDECREF(buffer);
     }
 
+    bool find_int64_format(PyObject* ctypes)
+    {
+        PyObject* type = PyObject_GetAttrString(ctypes, "c_int64");
+        PyObject* value = type ? PyObject_CallNoArgs(type) : nullptr;
+        Py_buffer v;
+        bool ok = value && PyObject_GetBuffer(value, &v, PyBUF_FORMAT) == 0;
+        if (ok)
+        {
+            ok = v.format && v.itemsize == 8 && strlen(v.format) < sizeof(int64_format);
+            if (ok)
+                strcpy(int64_format, v.format);
+            PyBuffer_Release(&v);
+        }
+        PyErr_Clear();
+        Py_XDECREF(value);
+        Py_XDECREF(type);
+        return ok;
+    }
+
     PyMethodDef methods[] = {{"structures", structures, METH_VARARGS, nullptr}, {"wrap", wrap, METH_VARARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
     PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fastcall", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 }
@@ -230,6 +253,8 @@ PyMODINIT_FUNC PyInit__fastcall(void)
     auto type = [&](const char* name) { return reinterpret_cast<PyTypeObject*>(PyObject_GetAttrString(ctypes, name)); };
     void_pointer_type = type("c_void_p"), float_type = type("c_float"), array_type = type("Array");
     find_byref_layout(ctypes);
+    if (!find_int64_format(ctypes))
+        PyErr_SetString(PyExc_ImportError, "the buffer of a ctypes c_int64 does not name its type");
     Py_DECREF(ctypes);
-    return void_pointer_type && float_type && array_type ? PyModule_Create(&module) : nullptr;
+    return void_pointer_type && float_type && array_type && !PyErr_Occurred() ? PyModule_Create(&module) : nullptr;
 }

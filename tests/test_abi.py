@@ -100,3 +100,21 @@ def test_native_callables_take_what_ctypes_takes():
                  lambda: L.b200_qgemm(1, 0, 2, 3, 4, 5, 16, ctypes.byref(lib.ConvParams()), s)):
         with pytest.raises((TypeError, ctypes.ArgumentError)):
             call()
+
+
+def test_native_callables_refuse_what_ctypes_refuses():
+    """a POINTER(c_int64) argument takes arrays of c_int64 only: neither another type of eight bytes, nor rows of them, nor a bare address"""
+    L = lib.LIB
+    e = lib.Epilogue()
+    for shape in ((ctypes.c_double * 2)(3, 4), (ctypes.c_uint64 * 2)(3, 4), ((ctypes.c_int64 * 1) * 2)(), (ctypes.c_void_p * 2)(3, 4), ctypes.c_void_p(0), 0):
+        with pytest.raises((TypeError, ctypes.ArgumentError)):
+            L.b200_quantize(None, None, None, None, lib.U8, shape, 2, None, 0, 11, None)  # (round mode 11: nothing is launched)
+        with pytest.raises((TypeError, ctypes.ArgumentError)):
+            L.b200_permute_b32(None, None, shape, -1, None, None)  # (rank -1)
+    for epilogue in (ctypes.c_void_p(0), 0):
+        with pytest.raises((TypeError, ctypes.ArgumentError)):
+            L.b200_qgemm(None, 9, None, None, 4, 4, 16, epilogue, None)
+    # what ctypes takes for a pointer: the object itself, an array of it, None
+    for epilogue in (e, (lib.Epilogue * 1)(), None):
+        assert L.b200_qgemm(None, 9, None, None, 4, 4, 16, epilogue, None) == -1
+    assert L.b200_quantize(None, None, None, None, lib.U8, None, 2, None, 0, 4, None) == -1
