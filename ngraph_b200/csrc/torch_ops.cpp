@@ -29,6 +29,7 @@ namespace
     decltype(&b200_maxpool_nhwc_u8) p_maxpool;
     decltype(&b200_global_avgpool_q_nhwc_u8) p_avgpool;
     PyObject* p_check; // lib.check(status, what): raises B200Error
+    PyObject* p_conv_params; // the type lib.ConvParams
 
     // raised as a Python exception that is already set
     struct PyError
@@ -91,9 +92,10 @@ namespace
         }
         return reinterpret_cast<THPDtype*>(o)->scalar_type;
     }
-    inline long long integer(PyObject* o)
+    // int(o), where `exact` is not asked for; with it what is an integer already (sizes: 3.7 is none)
+    inline long long integer(PyObject* o, bool exact = false)
     {
-        PyObject* i = PyNumber_Long(o);
+        PyObject* i = exact ? PyNumber_Index(o) : PyNumber_Long(o);
         if (!i)
             throw PyError();
         const long long v = PyLong_AsLongLong(i);
@@ -134,6 +136,26 @@ namespace
         }
         Py_DECREF(f);
         return int(n);
+    }
+    // the first two items of a sequence of sizes
+    inline void pair(PyObject* o, int64_t (&v)[2])
+    {
+        for (Py_ssize_t i = 0; i < 2; ++i)
+        {
+            PyObject* item = PySequence_GetItem(o, i);
+            if (!item)
+                throw PyError();
+            try
+            {
+                v[i] = integer(item, true);
+            }
+            catch (...)
+            {
+                Py_DECREF(item);
+                throw;
+            }
+            Py_DECREF(item);
+        }
     }
     // torch.empty on the device of `like`; on the current device (where `like` shows that CUDA is initialised) without the
     // device guard and the initialisation checks, a fifth of the allocation
@@ -282,6 +304,11 @@ namespace
         Py_buffer view{};
         explicit Params(PyObject* o)
         {
+            const int is = PyObject_IsInstance(o, p_conv_params);
+            if (is == 0)
+                PyErr_SetString(PyExc_TypeError, "a ConvParams is wanted");
+            if (is != 1)
+                throw PyError();
             if (PyObject_GetBuffer(o, &view, PyBUF_SIMPLE) != 0)
                 throw PyError();
             if (view.len != Py_ssize_t(sizeof(b200_conv_params)))
@@ -323,7 +350,7 @@ namespace
         return guarded(n, 2, [&]() -> PyObject* {
             const Dev x = dev(a[0]);
             require(x->element_size() == 1 && x->dim() == 4, "one-byte elements, four dimensions");
-            const int64_t N = x->size(0), c = x->size(1), h = x->size(2), w = x->size(3), c_pad = a[1] == Py_None ? c : integer(a[1]);
+            const int64_t N = x->size(0), c = x->size(1), h = x->size(2), w = x->size(3), c_pad = a[1] == Py_None ? c : integer(a[1], true);
             const at::Tensor out = empty({N, h, w, c_pad}, x->scalar_type(), *x);
             void* st = stream();
             check(unlocked([&] { return p_nchw_to_nhwc(x->data_ptr(), out.data_ptr(), N, c, h, w, c_pad, st); }), "b200_nchw_to_nhwc_u8");
@@ -335,7 +362,7 @@ namespace
         return guarded(n, 2, [&]() -> PyObject* {
             const Dev x = dev(a[0]);
             require(x->element_size() == 1 && x->dim() == 4, "one-byte elements, four dimensions");
-            const int64_t N = x->size(0), h = x->size(1), w = x->size(2), c_pad = x->size(3), c = a[1] == Py_None ? c_pad : integer(a[1]);
+            const int64_t N = x->size(0), h = x->size(1), w = x->size(2), c_pad = x->size(3), c = a[1] == Py_None ? c_pad : integer(a[1], true);
             const at::Tensor out = empty({N, c, h, w}, x->scalar_type(), *x);
             void* st = stream();
             check(unlocked([&] { return p_nhwc_to_nchw(x->data_ptr(), out.data_ptr(), N, c, h, w, c_pad, st); }), "b200_nhwc_to_nchw_u8");
@@ -362,11 +389,7 @@ namespace
             require(x->dim() == 4, "x is [N,H,W,C]");
             int64_t v[4][2];
             for (int i = 0; i < 4; ++i)
-                if (integers(a[1 + i], v[i]) != 2)
-                {
-                    PyErr_SetString(PyExc_ValueError, "window, stride and paddings are pairs");
-                    throw PyError();
-                }
+                pair(a[1 + i], v[i]);
             const int64_t N = x->size(0), h = x->size(1), w = x->size(2), c = x->size(3);
             int64_t d[2];
             for (int i = 0; i < 2; ++i)
@@ -405,10 +428,10 @@ namespace
         });
     }
 
-    // bind(check, {name: address})
+    // bind(check, {name: address}, type of the convolution parameters)
     PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n)
     {
-        return guarded(n, 2, [&]() -> PyObject* {
+        return guarded(n, 3, [&]() -> PyObject* {
             auto take = [&](auto& fn, const char* name) {
                 PyObject* v = PyDict_GetItemString(a[1], name);
                 if (!v)
@@ -434,6 +457,9 @@ namespace
             Py_INCREF(a[0]);
             Py_XDECREF(p_check);
             p_check = a[0];
+            Py_INCREF(a[2]);
+            Py_XDECREF(p_conv_params);
+            p_conv_params = a[2];
             Py_RETURN_NONE;
         });
     }

@@ -21,7 +21,7 @@ except ImportError as e:
 
 _native.bind(check, {name: lib.ADDRESS[name] for name in (
     "b200_quantize", "b200_dequantize", "b200_qgemm", "b200_qconv", "b200_qconv_packed", "b200_qconv_out_shape", "b200_nchw_to_nhwc_u8",
-    "b200_nhwc_to_nchw_u8", "b200_transpose_u8", "b200_maxpool_nhwc_u8", "b200_global_avgpool_q_nhwc_u8")})
+    "b200_nhwc_to_nchw_u8", "b200_transpose_u8", "b200_maxpool_nhwc_u8", "b200_global_avgpool_q_nhwc_u8")}, ConvParams)
 
 _DT = {torch.uint8: U8, torch.int8: I8, torch.int32: I32, torch.float32: F32}
 _TORCH = {U8: torch.uint8, I8: torch.int8, I32: torch.int32, F32: torch.float32}

@@ -256,3 +256,20 @@ def test_wrapper_arguments(ops):
         ops.quantize(x, s, z.double(), (1,))
     with pytest.raises(TypeError):
         ops.quantize(x.cpu().numpy(), s, z, (1,))
+
+
+def test_wrapper_sizes(ops):
+    """sizes are integers, windows and paddings sequences whose first two items count, convolution parameters a ConvParams"""
+    import ctypes
+    x = torch.randint(0, 256, (2, 8, 9, 16), device="cuda", dtype=torch.uint8)
+    want = ops.maxpool_nhwc(x, (3, 3), (2, 2), (1, 1))
+    assert torch.equal(ops.maxpool_nhwc(x, [3, 3, 1], (2, 2, 9), torch.Size([1, 1, 5]), (1, 1, 7)), want)
+    f, s = torch.zeros((16, 1, 1, 64), dtype=torch.int8, device="cuda"), torch.ones(1, device="cuda")
+    data, cp = torch.zeros((1, 4, 4, 64), dtype=torch.uint8, device="cuda"), ops.conv_params((1, 4, 4, 64), (16, 1, 1, 64))
+    assert ops.qconv(data, f, s, torch.int8, cp).shape == (1, 4, 4, 16)
+    for call in (lambda: ops.maxpool_nhwc(x, (3.7, 3), (2, 2)), lambda: ops.maxpool_nhwc(x, (3, 3), (2, 2), (1.0, 1)), lambda: ops.nchw_to_nhwc(x, 16.5),
+                 lambda: ops.nhwc_to_nchw(x, 3.0), lambda: ops.qconv(data, f, s, torch.int8, bytes(cp)), lambda: ops.qconv(data, f, s, torch.int8, (ctypes.c_int64 * 15)())):
+        with pytest.raises(TypeError):
+            call()
+    with pytest.raises(IndexError):
+        ops.maxpool_nhwc(x, (3,), (2, 2))
