@@ -431,6 +431,52 @@ namespace b200
         return m;
     }
 
+    // The reference's loops replace on a strict comparison, so a result of zero is the FIRST zero of the input, and its sign shows.
+    // The forms above take elements in other orders: for Max and Min they look for that zero in a second pass, which only a
+    // result of zero pays for.  The lowest index of a zero among elements t, t + threads, ... (n: none); `at` reads an element.
+    template <typename At>
+    __device__ __forceinline__ uint32_t first_zero(At at, uint32_t n, uint32_t t, uint32_t threads)
+    {
+        for (uint32_t i = t; i < n; i += 8 * threads)
+        {
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                v[j] = at(min(i + j * threads, n - 1)); // past the end: the last element again
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (v[j] == 0.0f)
+                    return min(i + j * threads, n - 1);
+        }
+        return n;
+    }
+    // the lowest of all threads of the block, in all of them
+    __device__ __forceinline__ uint32_t lowest_of_block(uint32_t i, uint32_t* lowest)
+    {
+        __syncthreads(); // an earlier result has been read
+        if (threadIdx.x == 0)
+            *lowest = 0xFFFFFFFFu;
+        i = __reduce_min_sync(0xffffffffu, i);
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0)
+            atomicMin(lowest, i);
+        __syncthreads();
+        return *lowest;
+    }
+    // the first zero of a run, by one block of THREADS, stopping where it is found (n: there is none)
+    template <int THREADS, typename At>
+    __device__ __forceinline__ int64_t first_zero_of_run(At at, int64_t n, uint32_t* lowest)
+    {
+        for (int64_t i = 0; i < n; i += 8 * THREADS)
+        {
+            const uint32_t part = uint32_t(min(n - i, int64_t(8 * THREADS)));
+            const uint32_t k = lowest_of_block(first_zero([&](uint32_t e) { return at(i + e); }, part, threadIdx.x, THREADS), lowest);
+            if (k < part)
+                return i + k;
+        }
+        return n;
+    }
+
     // few outputs, long reductions: one block per output
     template <int OP>
     __global__ void __launch_bounds__(256) reduce_extreme_block_kernel(const float* __restrict__ in, float* __restrict__ out, Dims keep,
@@ -442,6 +488,12 @@ namespace b200
         for (int64_t r = threadIdx.x; r < n_red; r += blockDim.x)
             m = extreme_of<OP>(m, base[mapped_offset(red, r)]);
         m = extreme_of_block<OP>(m, partial);
+        if (OP != B200_REDUCE_MAX_ABS && __syncthreads_or(threadIdx.x == 0 && m == 0.0f))
+        {
+            __shared__ uint32_t lowest;
+            auto at = [&](int64_t r) { return base[mapped_offset(red, r)]; };
+            m = at(first_zero_of_run<256>(at, n_red, &lowest));
+        }
         if (threadIdx.x == 0)
             out[blockIdx.x] = m;
     }
@@ -460,27 +512,53 @@ namespace b200
         asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); // this block runs: its shared memory may be written
         const float m = extreme_of_block<OP>(extreme_of_run<OP>(in, n, int64_t(blockIdx.x) * 1024 + threadIdx.x, EXTREME_CLUSTER * 1024), partial);
         asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
-        if (threadIdx.x == 0)
-        {
+        auto to_every_block = [](auto* slot, uint32_t value) {
+            // thread b < EXTREME_CLUSTER stores this block's value in block b
             uint32_t dst;
-            asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(dst) : "r"(uint32_t(__cvta_generic_to_shared(&of_block[blockIdx.x]))));
-            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(m) : "memory");
-        }
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(uint32_t(__cvta_generic_to_shared(slot))), "r"(threadIdx.x));
+            asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(dst), "r"(value) : "memory");
+        };
+        __shared__ float block_result;
+        if (threadIdx.x == 0)
+            block_result = m;
+        __syncwarp(); // the first warp's lanes hand it on
+        if (threadIdx.x < EXTREME_CLUSTER)
+            to_every_block(&of_block[blockIdx.x], __float_as_uint(block_result));
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-        if (blockIdx.x == 0 && threadIdx.x == 0)
-        {
-            float r = of_block[0];
+        float r = of_block[0]; // in every thread of the cluster
 #pragma unroll
-            for (int b = 1; b < EXTREME_CLUSTER; ++b)
-                r = extreme_of<OP == B200_REDUCE_MAX_ABS ? int(B200_REDUCE_MAX) : OP>(r, of_block[b]);
-            out[0] = r;
+        for (int b = 1; b < EXTREME_CLUSTER; ++b)
+            r = extreme_of<OP == B200_REDUCE_MAX_ABS ? int(B200_REDUCE_MAX) : OP>(r, of_block[b]);
+        if (OP != B200_REDUCE_MAX_ABS && r == 0.0f)
+        {
+            __shared__ uint32_t lowest, lowest_of[EXTREME_CLUSTER];
+            auto at = [&](uint32_t k) { return in[k]; };
+            // every block looks at the start of the tensor, where a zero usually is (Min of rectified values), then at its share
+            const uint32_t count = uint32_t(n), start = min(count, 8u * 1024);
+            uint32_t first = lowest_of_block(first_zero(at, start, threadIdx.x, 1024), &lowest);
+            if (first >= start)
+            {
+                const uint32_t i = lowest_of_block(first_zero(at, count, blockIdx.x * 1024 + threadIdx.x, EXTREME_CLUSTER * 1024), &lowest);
+                if (threadIdx.x < EXTREME_CLUSTER)
+                    to_every_block(&lowest_of[blockIdx.x], i);
+                asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+                asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+                first = lowest_of[0];
+#pragma unroll
+                for (int b = 1; b < EXTREME_CLUSTER; ++b)
+                    first = min(first, lowest_of[b]);
+            }
+            r = at(first);
         }
+        if (blockIdx.x == 0 && threadIdx.x == 0)
+            out[0] = r;
     }
 
     // Larger tensors: many blocks, each over a slice, combined with an atomic on the ordered integer image of the float
     // (non-negative floats order like signed ints, negative ones like reversed unsigned ints); the output must hold the
-    // starting value on entry.  Bound by HBM.
+    // starting value on entry.  Bound by HBM.  Of two zeros the image prefers +0 for Max (as this form always did) and -0 for Min,
+    // whose sign the next kernel then makes the first zero's.
     template <int OP>
     __global__ void __launch_bounds__(256) reduce_extreme_all_kernel(const float* __restrict__ in, float* __restrict__ out, int64_t n)
     {
@@ -496,6 +574,18 @@ namespace b200
             else
                 OP == B200_REDUCE_MIN ? atomicMin(as_int, __float_as_int(m)) : atomicMax(as_int, __float_as_int(m));
         }
+    }
+
+    // One block: if the result is zero, the first zero of the input takes its place (see first_zero).
+    __global__ void __launch_bounds__(1024) first_zero_kernel(const float* __restrict__ in, float* __restrict__ out, int64_t n)
+    {
+        after_earlier_kernels(in, out);
+        __shared__ uint32_t lowest;
+        if (*out != 0.0f)
+            return;
+        const int64_t first = first_zero_of_run<1024>([&](int64_t k) { return in[k]; }, n, &lowest);
+        if (threadIdx.x == 0 && first < n)
+            *out = in[first];
     }
 
     __global__ void fill_f32_kernel(float* out, float value, int64_t n)
@@ -1323,6 +1413,11 @@ extern "C" int b200_reduce_f32(int op, const float* in, float* out, const int64_
         case B200_REDUCE_MIN:
             small ? launch(reduce_extreme_cluster_kernel<B200_REDUCE_MIN>, grid, 1024, 0, st, in, out, n_red)
                   : launch(reduce_extreme_all_kernel<B200_REDUCE_MIN>, grid, 256, 0, st, in, out, n_red);
+            if (!small)
+            {
+                launch(first_zero_kernel, 1, 1024, 0, st, in, out, n_red);
+                g_launches.fetch_add(1, std::memory_order_relaxed);
+            }
             break;
         default:
             small ? launch(reduce_extreme_cluster_kernel<B200_REDUCE_MAX_ABS>, grid, 1024, 0, st, in, out, n_red)

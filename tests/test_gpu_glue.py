@@ -365,3 +365,26 @@ def test_permutes_that_move_the_last_axis(L, shape):
     for order in itertools.islice(itertools.permutations(range(len(shape))), 0, None, 1 if len(shape) < 5 else 7):
         L.check(L.LIB.b200_permute_b32(xd.data_ptr(), o.data_ptr(), i64(shape), len(shape), i64(order), stream()), "permute")
         np.testing.assert_array_equal(o.cpu().numpy(), np.transpose(x, order).ravel(), err_msg=str(order))
+
+
+@pytest.mark.parametrize("shape,axes", [((1,), (0,)), ((2,), (0,)), ((1000,), (0,)), ((1025,), (0,)), ((65535,), (0,)), ((1 << 20,), (0,)), (((1 << 20) + 1,), (0,)), ((3000001,), (0,)),
+                                        ((10, 5000), (1,)), ((5000, 10), (0,)), ((3, 40, 3, 50), (1, 3)), ((70, 40), (1,))])
+def test_a_zero_extreme_is_the_first_zero(L, shape, axes):
+    """Max and Min replace on a strict comparison: of zeros of both signs the first one in row-major order is the result, wherever it lies"""
+    rng = np.random.default_rng(int(np.prod(shape)))
+    kept = [i for i in range(len(shape)) if i not in axes]
+    for op, sign in ((1, -1.0), (2, 1.0)):
+        if op == 1 and len(kept) == 0 and shape[0] > 1 << 20:
+            continue  # Max of more elements: the sign of a zero is not fixed
+        for share in (1.0, 0.3, 2.0 / shape[-1], 0.0):
+            x = (np.float32(sign) * (np.abs(rng.standard_normal(shape)) + 0.1)).astype(np.float32)
+            zero = rng.random(shape) < share
+            zero.reshape(-1)[-1] = True
+            x[zero] = np.where(rng.random(shape) < 0.5, np.float32(-0.0), np.float32(0.0))[zero]
+            rows = np.ascontiguousarray(np.transpose(x, kept + list(axes))).reshape(-1, int(np.prod([shape[a] for a in axes])))
+            want = rows.max(axis=1) if op == 1 else rows.min(axis=1)
+            first = rows[np.arange(len(rows)), (rows == 0).argmax(axis=1)]
+            want = np.where(want == 0, first, want)
+            xd, out = dev(x), torch.full((len(rows),), 7.0, device="cuda")
+            L.check(L.LIB.b200_reduce_f32(op, xd.data_ptr(), out.data_ptr(), i64(shape), len(shape), i64(axes), len(axes), stream()), "reduce")
+            np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(want), err_msg="op %d share %g" % (op, share))
