@@ -64,11 +64,14 @@ namespace b200
     }
 #ifdef __CUDACC__
     // Waits until the earlier kernels of the stream are complete and their writes visible.  The pointers whose memory earlier
-    // kernels may write pass through, so that no load (a read-only one included) is scheduled ahead of the wait.
+    // kernels may write pass through, so that no load (a read-only one included) is scheduled ahead of the wait.  What comes out
+    // is an address of unknown space to the compiler, which is told again that it is a global one (so none of them may be null):
+    // with generic accesses Softmax of 30000 rows of 1535 took 568 us, with global ones 285, LayerNorm 647 and 448.
     template <typename P>
     __device__ __forceinline__ void not_before_here(P& p)
     {
         asm volatile("" : "+l"(p)::"memory");
+        __builtin_assume(__isGlobal(p));
     }
     template <typename... P>
     __device__ __forceinline__ void after_earlier_kernels(P&... pointers)

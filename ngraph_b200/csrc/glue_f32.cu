@@ -685,7 +685,10 @@ namespace b200
         __shared__ double exp_table[rounded::EXP_STEPS];
         __shared__ float row_sum[R];
         rounded::load_exp_table(exp_table);
-        after_earlier_kernels(in, factor, out);
+        if constexpr (FACTOR)
+            after_earlier_kernels(in, factor, out);
+        else
+            after_earlier_kernels(in, out);
         const int stride = staged_row_stride(L, VEC), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
         const int64_t row0 = int64_t(blockIdx.x) * R;
         const int n_rows = int(min(rows - row0, int64_t(R)));
@@ -815,7 +818,10 @@ namespace b200
                                                                           float* __restrict__ out, int64_t rows, int L, float count, float eps,
                                                                           int64_t ahead)
     {
-        after_earlier_kernels(in, addend, gamma, beta, out);
+        if constexpr (ADDEND)
+            after_earlier_kernels(in, addend, gamma, beta, out);
+        else
+            after_earlier_kernels(in, gamma, beta, out);
         constexpr int R = NORM_ROWS, WARPS = ROW_THREADS / 32;
         extern __shared__ __align__(16) float tile[];
         __shared__ float row_mean[R], row_sd[R];
@@ -1571,6 +1577,8 @@ extern "C" int b200_bmm_f32(const float* a, const float* b, float* out, int64_t 
         return B200_OK;
     if (!out || (K > 0 && (!a || !b)))
         return B200_ERR_INVALID_ARGUMENT;
+    if (K == 0) // the operands, which may be null, are not read
+        a = b = out;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // the largest tile that spreads over the scheduler partitions: smaller ones load their operands more often, larger ones
     // leave partitions idle on small products (12 x [128, 128] x [128, 128] is 24 tiles of 128 x 64 for 148 SMs)

@@ -1,0 +1,44 @@
+"""Calls off the sizes that the kernels were tuned at, timed on the device beside a comparable call: a form chosen where another
+one is several times faster shows as a ratio, whatever the clock."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def L():
+    from ngraph_b200 import lib
+    return lib
+
+
+def stream():
+    return torch.cuda.current_stream().cuda_stream
+
+
+def us(call):
+    """shortest time per call of a run of launches"""
+    best = float("inf")
+    for _ in range(8):
+        first, last = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        first.record()
+        for _ in range(20):
+            assert call() == 0
+        last.record()
+        last.synchronize()
+        best = min(best, first.elapsed_time(last) * 1000 / 20)
+    return best
+
+
+def rows_kernel(L, kind, rows, n):
+    x, o = torch.rand(rows * n, device="cuda"), torch.empty(rows * n, device="cuda")
+    g, b = torch.rand(n, device="cuda"), torch.rand(n, device="cuda")
+    if kind == "softmax":
+        return lambda: L.LIB.b200_softmax_rows_f32(x.data_ptr(), o.data_ptr(), rows, n, stream())
+    return lambda: L.LIB.b200_layer_norm_rows_f32(x.data_ptr(), g.data_ptr(), b.data_ptr(), o.data_ptr(), rows, n, 1e-5, stream())
+
+
+@pytest.mark.parametrize("kind,times", [("softmax", 1.8), ("norm", 2.05)])
+def test_rows_of_odd_length(L, kind, times):
+    """beside rows that move in whole vectors; with generic instead of global accesses 2.4 times as long, otherwise 1.2 and 1.7"""
+    assert us(rows_kernel(L, kind, 30000, 1535)) < times * us(rows_kernel(L, kind, 30000, 1532))
