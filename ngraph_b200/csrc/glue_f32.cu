@@ -1141,6 +1141,70 @@ namespace b200
             }
     }
 
+    // Small matrices: a panel would mostly hold padding (32 x 32 x 32 is the least a block works on).  A thread owns 4 x 4
+    // outputs and reads its operands straight from memory; the same sums in the same order.
+    __global__ void __launch_bounds__(128) bmm_small_kernel(const float* __restrict__ a, const float* __restrict__ bm, float* __restrict__ out, int64_t batch,
+                                                            int M, int K, int N)
+    {
+        after_earlier_kernels(a, bm, out);
+        const int tiles_n = (N + 3) / 4, tiles_m = (M + 3) / 4;
+        const int64_t total = batch * tiles_m * tiles_n;
+        for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x)
+        {
+            const int tn = int(i % tiles_n);
+            const int64_t t = i / tiles_n;
+            const int tm = int(t % tiles_m);
+            const int64_t b = t / tiles_m;
+            const int m0 = tm * 4, n0 = tn * 4;
+            const float* ap = a + (b * M + m0) * K;
+            const float* bp = bm + b * K * N + n0;
+            // rows / columns beyond the matrix read the last valid one (their results are not stored)
+            const int r1 = m0 + 1 < M ? 1 : 0, r2 = m0 + 2 < M ? 2 : r1, r3 = m0 + 3 < M ? 3 : r2;
+            const int c1 = n0 + 1 < N ? 1 : 0, c2 = n0 + 2 < N ? 2 : c1, c3 = n0 + 3 < N ? 3 : c2;
+            double acc[4][4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    acc[r][c] = 0.0;
+            for (int k = 0; k < K; ++k)
+            {
+                const double x0 = ap[k], x1 = ap[int64_t(r1) * K + k], x2 = ap[int64_t(r2) * K + k], x3 = ap[int64_t(r3) * K + k];
+                const float* brow = bp + int64_t(k) * N;
+                const double y0 = brow[0], y1 = brow[c1], y2 = brow[c2], y3 = brow[c3];
+                const double xs[4] = {x0, x1, x2, x3}, ys[4] = {y0, y1, y2, y3};
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        acc[r][c] = fma(xs[r], ys[c], acc[r][c]); // a product of two floats is exact in double: one rounding, like mul + add
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if (m0 + r < M && n0 + c < N)
+                        out[(b * M + m0 + r) * N + n0 + c] = static_cast<float>(acc[r][c]);
+        }
+    }
+
+    // Estimated times in us, fitted to both forms at 1500 shapes (up to 20000 products, sides of 1 to 500): the choice by them is within
+    // 0.6 % of the better form on average, 1.7 times in the worst case.  Small form: operand loads, which the lanes of a warp
+    // share the better the more tiles a product has, the chain over K, or memory.  Panels: a block's turn per 32 of K, or the chain.
+    // 10000 x [4, 4] x [4, 4]: 3.7 us in the small form against 23, 10000 x [33, 1] x [1, 1] 3.5 against 59,
+    // 10000 x [33, 64] x [64, 24] 151 against 87.
+    static double bmm_small_us(int64_t batch, int64_t M, int64_t K, int64_t N)
+    {
+        const double m = double((M + 3) / 4), n = double((N + 3) / 4), steps = double(batch) * m * n * double(K);
+        const double bytes = 4.0 * double(batch) * (double(M) * double(K) + double(K) * double(N) + double(M) * double(N));
+        return 3.08 + std::max({steps * std::max(4.0e-6, 11.8e-6 / n + 26.0e-6 / (m * n)), double(K) * (N <= 4 ? 0.2 : 0.145), bytes * 3.4e-7});
+    }
+    static double bmm_panels_us(int64_t blocks, int64_t K, bool vec, bool smallest_tile, bool half_size)
+    {
+        const double panels = double((K + BMM_KC - 1) / BMM_KC), turn = smallest_tile ? (vec ? 2.06e-3 : 2.74e-3) : (vec ? 8.9e-3 : 9.9e-3);
+        return 2.51 + std::max(double(blocks) * panels * turn * (half_size ? 1.0 : 2.0), panels * 1.05);
+    }
+
     // One tile shape of the product: what it would cost, and its launch.
     template <int WM, int WN, int MT, int NT>
     struct BmmShape
@@ -1586,9 +1650,17 @@ extern "C" int b200_bmm_f32(const float* a, const float* b, float* out, int64_t 
     using Mid = BmmShape<2, 2, 4, 4>;
     using Small = BmmShape<2, 2, 2, 2>;
     const double big = Big::cost(batch, M, N), mid = Mid::cost(batch, M, N), small = Small::cost(batch, M, N);
-    const bool ok = big <= mid && big <= small ? Big::launch(a, b, out, batch, int(M), int(K), int(N), st)
-                    : mid <= small             ? Mid::launch(a, b, out, batch, int(M), int(K), int(N), st)
-                                               : Small::launch(a, b, out, batch, int(M), int(K), int(N), st);
+    const bool is_big = big <= mid && big <= small, is_mid = !is_big && mid <= small, vec = K % 4 == 0 && N % 4 == 0 && all_aligned16({a, b, out});
+    const int64_t blocks = is_big ? Big::tiles(batch, M, N) : is_mid ? Mid::tiles(batch, M, N) : Small::tiles(batch, M, N);
+    if (K > 0x7FFFFF00 /* where the panels' counters end */ || bmm_small_us(batch, M, K, N) < bmm_panels_us(blocks, K, vec, !is_big && !is_mid, !is_big))
+    {
+        const int64_t tiles = batch * ((M + 3) / 4) * ((N + 3) / 4);
+        launch(bmm_small_kernel, grid_for(tiles, 128), 128, 0, st, a, b, out, batch, int(M), int(K), int(N));
+        return after_launch("b200_bmm_f32");
+    }
+    const bool ok = is_big   ? Big::launch(a, b, out, batch, int(M), int(K), int(N), st)
+                    : is_mid ? Mid::launch(a, b, out, batch, int(M), int(K), int(N), st)
+                             : Small::launch(a, b, out, batch, int(M), int(K), int(N), st);
     if (!ok)
         return B200_ERR_TOO_LARGE;
     return after_launch("b200_bmm_f32");

@@ -388,3 +388,18 @@ def test_a_zero_extreme_is_the_first_zero(L, shape, axes):
             xd, out = dev(x), torch.full((len(rows),), 7.0, device="cuda")
             L.check(L.LIB.b200_reduce_f32(op, xd.data_ptr(), out.data_ptr(), i64(shape), len(shape), i64(axes), len(axes), stream()), "reduce")
             np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(want), err_msg="op %d share %g" % (op, share))
+
+
+@pytest.mark.parametrize("batch,m,k,n", [(3000, 33, 1, 1), (2000, 1, 9, 287), (700, 140, 2, 3), (5000, 4, 4, 4), (900, 5, 7, 6), (40, 8, 64, 9), (1, 1, 1, 1)])
+def test_bmm_of_small_matrices(L, batch, m, k, n):
+    """shapes of the form without panels: tiles of 4 x 4 that end early on either side, rows of one element"""
+    rng = np.random.default_rng(batch + m)
+    a = (rng.standard_normal((batch, m, k)) * 50).astype(np.float32)
+    b = (rng.standard_normal((batch, k, n)) * 50).astype(np.float32)
+    acc = np.zeros((batch, m, n), np.float64)
+    for kk in range(k):
+        acc += a[:, :, kk, None].astype(np.float64) * b[:, kk, None, :].astype(np.float64)
+    out = torch.full((batch, m, n), 7.0, device="cuda")
+    ad, bd = dev(a), dev(b)
+    L.check(L.LIB.b200_bmm_f32(ad.data_ptr(), bd.data_ptr(), out.data_ptr(), batch, m, k, n, stream()), "bmm")
+    np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(acc.astype(np.float32)))

@@ -42,3 +42,16 @@ def rows_kernel(L, kind, rows, n):
 def test_rows_of_odd_length(L, kind, times):
     """beside rows that move in whole vectors; with generic instead of global accesses 2.4 times as long, otherwise 1.2 and 1.7"""
     assert us(rows_kernel(L, kind, 30000, 1535)) < times * us(rows_kernel(L, kind, 30000, 1532))
+
+
+def binary(L, n, op=0):
+    a, b, o = (torch.rand(n, device="cuda") for _ in range(3))
+    return lambda: L.LIB.b200_f32_binary(op, a.data_ptr(), b.data_ptr(), o.data_ptr(), n, stream())
+
+
+@pytest.mark.parametrize("batch,m,k,n", [(10000, 4, 4, 4), (10000, 33, 1, 1), (2000, 140, 2, 1)])
+def test_many_small_products(L, batch, m, k, n):
+    """about the elements of an elementwise call; a 32 x 32 x 32 block per product takes seven to fourteen times as long"""
+    a, b, o = torch.rand(batch * m * k, device="cuda"), torch.rand(batch * k * n, device="cuda"), torch.empty(batch * m * n, device="cuda")
+    t = us(lambda: L.LIB.b200_bmm_f32(a.data_ptr(), b.data_ptr(), o.data_ptr(), batch, m, k, n, stream()))
+    assert t < 3.0 * us(binary(L, batch * m * n))
