@@ -65,7 +65,21 @@ namespace b200
                                                          float* __restrict__ out, int64_t n)
     {
         after_earlier_kernels(a, b, out);
-        for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
+        // Bound by HBM.  Four loads of each operand under way, issued here: behind the dependency wait the compiler does not know
+        // that stores leave the operands alone (12.6 M elements: 34.5 us one element at a time, 24.3 so).
+        const int64_t threads = int64_t(gridDim.x) * blockDim.x;
+        int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+        for (; i + 3 * threads < n; i += 4 * threads)
+        {
+            float x[4], y[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                x[j] = a[i + j * threads], y[j] = b[i + j * threads];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                out[i + j * threads] = binary_op<OP>(x[j], y[j]);
+        }
+        for (; i < n; i += threads)
             out[i] = binary_op<OP>(a[i], b[i]);
     }
 
@@ -95,11 +109,25 @@ namespace b200
             }
         }
         else
-            for (IDX i = IDX(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += IDX(gridDim.x) * blockDim.x)
+        {
+            const IDX threads = IDX(gridDim.x) * blockDim.x;
+            IDX i = IDX(blockIdx.x) * blockDim.x + threadIdx.x;
+            for (; n - i > 3 * threads && i < n; i += 4 * threads) // four loads under way (see binary_kernel)
+            {
+                float x[4], y[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    x[j] = a[i + j * threads], y[j] = __ldg(v + (i + j * threads) % period);
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    out[i + j * threads] = V_LEFT ? binary_op<OP>(y[j], x[j]) : binary_op<OP>(x[j], y[j]);
+            }
+            for (; i < n; i += threads)
             {
                 const float x = a[i], y = __ldg(v + i % period);
                 out[i] = V_LEFT ? binary_op<OP>(y, x) : binary_op<OP>(x, y);
             }
+        }
     }
 
     template <int OP, typename IDX>

@@ -403,3 +403,22 @@ def test_bmm_of_small_matrices(L, batch, m, k, n):
     ad, bd = dev(a), dev(b)
     L.check(L.LIB.b200_bmm_f32(ad.data_ptr(), bd.data_ptr(), out.data_ptr(), batch, m, k, n, stream()), "bmm")
     np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(acc.astype(np.float32)))
+
+
+@pytest.mark.parametrize("extra", [0, 1, 2 * 606208 + 5, 3 * 606208 - 1, 3 * 606208, 3 * 606208 + 1, 7 * 606208 + 11])
+def test_elementwise_beyond_one_element_per_thread(L, extra):
+    """the loops that take four elements at a time and what they leave (16 blocks of 256 threads per SM: 606208 threads on 148)"""
+    n = 606208 + extra
+    a, b = torch.randn(n, device="cuda"), torch.randn(n, device="cuda")
+    out = torch.full((n,), 7.0, device="cuda")
+    L.check(L.LIB.b200_f32_binary(1, a.data_ptr(), b.data_ptr(), out.data_ptr(), n, stream()), "sub")
+    assert torch.equal(out, a - b)
+    for period in (7, 1):
+        m = n // period * period
+        v = torch.randn(period, device="cuda")
+        for left in (0, 1):
+            # an unaligned result takes single elements where the operand has one
+            out = torch.full((m + 1,), 7.0, device="cuda")[1:]
+            L.check(L.LIB.b200_f32_binary_periodic(1, a.data_ptr(), v.data_ptr(), out.data_ptr(), m, period, left, stream()), "sub")
+            x = a[:m].view(-1, period)
+            assert torch.equal(out.view(-1, period), v - x if left else x - v)

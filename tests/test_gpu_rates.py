@@ -55,3 +55,11 @@ def test_many_small_products(L, batch, m, k, n):
     a, b, o = torch.rand(batch * m * k, device="cuda"), torch.rand(batch * k * n, device="cuda"), torch.empty(batch * m * n, device="cuda")
     t = us(lambda: L.LIB.b200_bmm_f32(a.data_ptr(), b.data_ptr(), o.data_ptr(), batch, m, k, n, stream()))
     assert t < 3.0 * us(binary(L, batch * m * n))
+
+
+def test_large_elementwise(L):
+    """three tensors beside the two that an operand of one element leaves: half as much again, and not twice as long"""
+    n = 12 << 20
+    a, v, o = torch.rand(n, device="cuda"), torch.rand(1, device="cuda"), torch.empty(n, device="cuda")
+    two = us(lambda: L.LIB.b200_f32_binary_periodic(0, a.data_ptr(), v.data_ptr(), o.data_ptr(), n, 1, 0, stream()))
+    assert us(binary(L, n)) < 1.9 * two
