@@ -2,12 +2,11 @@
 //
 // The general double routines cost some 40-100 instructions each; that, not memory, bounded Softmax and Gelu.  A float
 // argument needs less: the value is a table entry at an equidistant point and a short Taylor step, about a dozen
-// double-precision multiply-adds, with an error below 2^-47 of the result (2^-47 absolute for erf), which the rounding to
-// float sees in fewer than one result of a million.  All ends of the range (denormal and overflowing results, infinities,
+// double-precision multiply-adds, with an error below 2^-47 of the result (2^-51 for erf).  All ends of the range (denormal and overflowing results, infinities,
 // NaN) come out of the same instructions.
 //
 //   exp(x) = 2^(k >> 4) * 2^((k & 15) / 16) * e^r      k = rint(16 x / ln 2), |r| <= ln2 / 32, degree 6
-//   erf(x) = E(g) + D(g) (d - g d^2 + ...)              g = rint(256 |x|) / 256, |d| <= 1 / 512, D = erf', degree 4
+//   erf(x) = E(g) + D(g) (d - g d^2 + ...)              g = rint(256 |x|) / 256, |d| <= 1 / 512, D = erf', degree 5
 //
 // The tables are constant-evaluated from the defining series (all terms positive: nothing cancels) and copied to shared memory
 // by the kernels that use them.  Against the general routines, over all 2^32 arguments: exp never
@@ -124,9 +123,11 @@ namespace b200
             constexpr float magic = 12582912.0f; // 1.5 * 2^23
             const float jm = __fmaf_rn(a, float(ERF_STEPS), magic), gf = __fmul_rn(__fsub_rn(jm, magic), 1.0f / ERF_STEPS);
             const ErfPoint t = table[__float_as_int(jm) & 2047];
-            const double g = gf, d = __fsub_rn(a, gf), g2 = g * g; // both exact
-            const double c3 = fma(g2, 2.0 / 3.0, -1.0 / 3.0), c4 = g * fma(g2, -1.0 / 3.0, 0.5);
-            const double u = fma(d, fma(d, c4, c3), -g);
+            // the terms of d^4 and d^5 weigh less than 2^-27 of the result: single precision is enough for them
+            const float df = __fsub_rn(a, gf), gf2 = gf * gf; // df is exact
+            const float c4 = gf * fmaf(gf2, -1.0f / 3.0f, 0.5f), c5 = fmaf(gf2, fmaf(gf2, 2.0f / 15.0f, -0.4f), 0.1f);
+            const double g = gf, d = df, c3 = fma(g * g, 2.0 / 3.0, -1.0 / 3.0);
+            const double u = fma(d, fma(d, double(fmaf(df, c5, c4)), c3), -g);
             return static_cast<float>(fma(t.d, fma(d * d, u, d), t.e));
         }
         __device__ __forceinline__ float erf_rounded(float x, const ErfPoint* table)
