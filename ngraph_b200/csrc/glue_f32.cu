@@ -171,19 +171,46 @@ namespace b200
             out[i] = unary_op<OP>(x[i]);
     }
 
-    // Exp and Erf.  A block copies the function's table once and then strides over the tensor.
-    template <int OP>
+    // Exp and Erf.  A block copies the function's table to shared memory once and then strides over the tensor; few elements
+    // look it up where it is, without the copy and its barrier: erf of 10000 elements 4.3 us with a copy, 2.7 without, 400000 4.2 and
+    // 3.6, 600000 4.3 and 4.4, a million 5.0 and 6.1 (exp 3.7 and 2.7, 3.4 and 2.8, 3.5 and 3.5, 3.8 and 5.0).
+    constexpr int64_t TABLE_COPY_FROM = int64_t(1) << 19;
+    template <int OP, bool COPY>
     __global__ void __launch_bounds__(256) unary_table_kernel(const float* __restrict__ x, float* __restrict__ out, int64_t n)
     {
-        __shared__ double exp_table[OP == B200_F32_EXP ? rounded::EXP_STEPS : 1];
-        __shared__ __align__(16) rounded::ErfPoint erf_table[OP == B200_F32_ERF ? rounded::ERF_ENTRIES : 1];
-        if (OP == B200_F32_EXP)
-            rounded::load_exp_table(exp_table);
-        else
-            rounded::load_erf_table(erf_table);
-        __syncthreads();
-        for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-            out[i] = OP == B200_F32_EXP ? rounded::exp_rounded(x[i], exp_table) : rounded::erf_rounded(x[i], erf_table);
+        __shared__ double exp_copy[COPY && OP == B200_F32_EXP ? rounded::EXP_STEPS : 1];
+        __shared__ __align__(16) rounded::ErfPoint erf_copy[COPY && OP == B200_F32_ERF ? rounded::ERF_ENTRIES : 1];
+        if (COPY && OP == B200_F32_EXP)
+            rounded::load_exp_table(exp_copy);
+        else if (COPY)
+            rounded::load_erf_table(erf_copy);
+        const double* exp_table = COPY ? exp_copy : rounded::g_exp_table.v;
+        const rounded::ErfPoint* erf_table = COPY ? erf_copy : rounded::g_erf_table.v;
+        after_earlier_kernels(x, out);
+        if (COPY)
+            __syncthreads();
+        auto f = [&](float v) { return OP == B200_F32_EXP ? rounded::exp_rounded(v, exp_table) : rounded::erf_rounded(v, erf_table); };
+        const int64_t threads = int64_t(gridDim.x) * blockDim.x;
+        int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+        for (; COPY && i + 3 * threads < n; i += 4 * threads) // four loads under way (see binary_kernel)
+        {
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                v[j] = x[i + j * threads];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                out[i + j * threads] = f(v[j]);
+        }
+        for (; i < n; i += threads)
+            out[i] = f(x[i]);
+    }
+    template <int OP>
+    static void launch_unary_table(const float* x, float* out, int64_t n, cudaStream_t st)
+    {
+        // blocks that copy get at least eight elements per thread
+        const int64_t blocks = n < TABLE_COPY_FROM ? (n + 255) / 256 : std::min<int64_t>((n + 2047) / 2048, int64_t(sm_count()) * 8);
+        launch(n < TABLE_COPY_FROM ? unary_table_kernel<OP, false> : unary_table_kernel<OP, true>, unsigned(blocks), 256, 0, st, x, out, n);
     }
 
     // out[idx] = in[mapped(idx)] for 4-byte elements: Broadcast (stride 0 on the new axes) and axis permutations.
@@ -942,13 +969,16 @@ namespace b200
         const float e = copysignf(rounded::erf_abs(fabsf(q), table), v);
         return __fmul_rn(__fmul_rn(0.5f, v), __fadd_rn(1.0f, e));
     }
-    template <bool VEC>
+    template <bool VEC, bool COPY>
     __global__ void __launch_bounds__(256, 6) gelu_kernel(const float* __restrict__ x, float* __restrict__ out, int64_t n)
     {
-        __shared__ __align__(16) rounded::ErfPoint table[rounded::ERF_ENTRIES];
-        rounded::load_erf_table(table);
+        __shared__ __align__(16) rounded::ErfPoint copy[COPY ? rounded::ERF_ENTRIES : 1];
+        const rounded::ErfPoint* table = COPY ? copy : rounded::g_erf_table.v;
+        if (COPY)
+            rounded::load_erf_table(copy);
         after_earlier_kernels(x, out);
-        __syncthreads();
+        if (COPY)
+            __syncthreads();
         const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, threads = int64_t(gridDim.x) * blockDim.x;
         if (VEC)
         {
@@ -1358,8 +1388,8 @@ extern "C" int b200_f32_unary(int op, const float* x, float* out, int64_t n, voi
     case B200_F32_ABS: unary_kernel<B200_F32_ABS><<<g, 256, 0, st>>>(x, out, n); break;
     case B200_F32_NEG: unary_kernel<B200_F32_NEG><<<g, 256, 0, st>>>(x, out, n); break;
     case B200_F32_SQRT: unary_kernel<B200_F32_SQRT><<<g, 256, 0, st>>>(x, out, n); break;
-    case B200_F32_EXP: unary_table_kernel<B200_F32_EXP><<<g, 256, 0, st>>>(x, out, n); break;
-    case B200_F32_ERF: unary_table_kernel<B200_F32_ERF><<<g, 256, 0, st>>>(x, out, n); break;
+    case B200_F32_EXP: launch_unary_table<B200_F32_EXP>(x, out, n, st); break;
+    case B200_F32_ERF: launch_unary_table<B200_F32_ERF>(x, out, n, st); break;
     default: unary_kernel<B200_F32_RELU><<<g, 256, 0, st>>>(x, out, n); break;
     }
     return after_launch("b200_f32_unary");
@@ -1651,12 +1681,15 @@ extern "C" int b200_gelu_f32(const float* x, float* out, int64_t n, void* stream
         return B200_ERR_INVALID_ARGUMENT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool vec = all_aligned16({x, out});
-    // blocks that stay (each copies the table first); short tensors get about two vectors per thread
+    // blocks that stay (each copies the table first); short tensors get about two vectors per thread.  Few elements that cannot
+    // move as vectors get a thread each and no copy (12000: 4.2 us with one, 2.7 without)
     const unsigned grid = unsigned(std::min<int64_t>((n + 2047) / 2048, int64_t(sm_count()) * 6));
     if (vec)
-        launch(gelu_kernel<true>, grid, 256, 0, st, x, out, n);
+        launch(gelu_kernel<true, true>, grid, 256, 0, st, x, out, n);
+    else if (n >= TABLE_COPY_FROM)
+        launch(gelu_kernel<false, true>, grid, 256, 0, st, x, out, n);
     else
-        launch(gelu_kernel<false>, grid, 256, 0, st, x, out, n);
+        launch(gelu_kernel<false, false>, unsigned((n + 255) / 256), 256, 0, st, x, out, n);
     return after_launch("b200_gelu_f32");
 }
 

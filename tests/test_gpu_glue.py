@@ -437,3 +437,17 @@ def test_exp_and_erf_over_every_float(L, op, fn, differ):
         want = fn(x.double()).float()
         bad += int(((out.view(torch.int32) != want.view(torch.int32)) & ~(out.isnan() & want.isnan())).sum())
     assert bad <= differ, bad
+
+
+@pytest.mark.parametrize("n", [1, 257, (1 << 19) - 1, 1 << 19, (1 << 19) + 3])
+def test_table_lookups_with_and_without_a_copy(L, n):
+    """either side of the size from which blocks copy the table, results that start on 16 bytes and that do not"""
+    x = torch.randn(n + 1, device="cuda") * 2
+    for off in (0, 1):
+        v, out = x[off:off + n], torch.full((n + 1,), 7.0, device="cuda")[off:off + n]
+        for op, fn in ((9, torch.exp), (10, torch.erf)):
+            L.check(L.LIB.b200_f32_unary(op, v.data_ptr(), out.data_ptr(), n, stream()), "unary")
+            assert int((out != fn(v.double()).float()).sum()) <= 1
+        L.check(L.LIB.b200_gelu_f32(v.data_ptr(), out.data_ptr(), n, stream()), "gelu")
+        want = (0.5 * v) * (1.0 + torch.erf((v / torch.tensor(2.0 ** 0.5, device="cuda")).double()).float())
+        assert int((out != want).sum()) <= 1
