@@ -100,6 +100,13 @@ B200_API int b200_device_status(int* status_out);
 B200_API int b200_selftest_bounded_wait(int64_t limit_ns, void* stream);
 
 /*
+ * The same for the contractions whose reduction is shared by a cluster of CTAs (diagnostic): one of two CTAs hands on its part
+ * after four times limit_ns (1 .. 100 000 000), the other gives up after limit_ns and then has to stay until the part has
+ * landed in its shared memory.  The status word holds 9002 if it did, 9003 if not.
+ */
+B200_API int b200_selftest_split_give_up(int64_t limit_ns, void* stream);
+
+/*
  * Quantize: f32 -> u8 / i8 / i32.
  *
  * Replaces runtime::reference::quantize<float,QUANT>

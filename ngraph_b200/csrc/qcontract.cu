@@ -489,6 +489,20 @@ namespace b200
     constexpr int SPLIT_EXCHANGE_BYTES = BM * 64 * 4;  // the parts a CTA receives: split x (64 / split) columns x 128 rows
     constexpr int SPLIT_SMEM_LIMIT = 112 * 1024;       // two CTAs per SM
 
+    // The way out for a CTA whose waits gave up, by all its threads.  Otherwise a CTA leaves when every part has landed and nothing
+    // writes to it any more; here parts may still be on their way.  The barrier counts the cluster's threads that have not left:
+    // past it every other CTA has issued its stores, and what they wrote lands within the (bounded) wait.
+    __device__ __forceinline__ void split_leave(uint32_t landed)
+    {
+        ptx::cluster_sync();
+        if (threadIdx.x == 0)
+        {
+            volatile int go_on = 0; // the CTA's own flag says that it has given up
+            ptx::mbar_wait(landed, 0, &go_on);
+        }
+        __syncthreads();
+    }
+
     __device__ __forceinline__ void split_epilogue(const ContractParams& p, int tile, int rank, int warp, int lane, uint32_t tmem_base, uint32_t exchange,
                                                    uint32_t tfull, uint32_t landed, volatile int* abortp, int& fail)
     {
@@ -1744,6 +1758,8 @@ namespace b200
             for (int i = 0; i < 50; ++i)
                 __nanosleep(1000);
             __syncthreads();
+            if (SPLITK)
+                split_leave(sum_bar(0, 0));
         }
         if (CTA2)
             ptx::cluster_sync(); // neither CTA leaves while the other may still read its shared memory or arrive on its barriers
@@ -2346,6 +2362,58 @@ extern "C" int b200_selftest_bounded_wait(int64_t limit_ns, void* stream)
         return B200_ERR_INVALID_ARGUMENT;
     bounded_wait_selftest_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<unsigned long long>(limit_ns));
     return after_launch("bounded_wait_selftest_kernel");
+}
+
+// ---- self-test of the way out of a split reduction whose waits gave up ---------------------------------------
+// A cluster of two CTAs: rank 1 sends its part four times limit_ns late, rank 0 gives up after limit_ns and leaves by
+// split_leave.  The status word is 9002 if rank 0 had the part when it left, 9003 if it would have left before it came.
+namespace b200
+{
+    __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64) split_leave_selftest_kernel(unsigned long long limit_ns)
+    {
+        __shared__ __align__(16) uint4 part;
+        __shared__ __align__(8) unsigned long long bar;
+        __shared__ int abort_flag;
+        const uint32_t rank = ptx::cluster_ctarank(), landed = ptx::smem_u32(&bar);
+        if (threadIdx.x == 0)
+        {
+            abort_flag = 0;
+            part = make_uint4(0, 0, 0, 0);
+            ptx::mbar_init(landed, 1);
+            ptx::mbar_expect_tx(landed, 16);
+            ptx::fence_barrier_init();
+        }
+        __syncthreads();
+        ptx::cluster_sync();
+        if (rank == 1)
+        {
+            const uint64_t t0 = ptx::globaltimer();
+            while (ptx::globaltimer() - t0 < 4 * limit_ns)
+                __nanosleep(10000);
+            if (threadIdx.x == 0)
+            {
+                const uint32_t dst = ptx::mapa(ptx::smem_u32(&part), 0);
+                ptx::store_async(dst, 1, 2, 3, 4, ptx::mapa(landed, 0));
+            }
+            return;
+        }
+        if (threadIdx.x == 0)
+            ptx::mbar_wait(landed, 0, &abort_flag, 64, limit_ns);
+        __syncthreads();
+        if (abort_flag)
+            split_leave(landed);
+        if (threadIdx.x == 0)
+            atomicCAS(&g_contract_status, 0, abort_flag && part.x == 1 && part.w == 4 ? 9002 : 9003);
+    }
+}
+
+extern "C" int b200_selftest_split_give_up(int64_t limit_ns, void* stream)
+{
+    using namespace b200;
+    if (limit_ns <= 0 || limit_ns > 100000000)
+        return B200_ERR_INVALID_ARGUMENT;
+    split_leave_selftest_kernel<<<2, 64, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<unsigned long long>(limit_ns));
+    return after_launch("split_leave_selftest_kernel");
 }
 
 static int qgemm_impl(const void* A, int a_type, const int8_t* W, bool packed, void* out, int64_t M, int64_t N, int64_t K,

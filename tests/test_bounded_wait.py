@@ -42,11 +42,25 @@ def test_wait_runs_out_status_is_latched_once_and_the_context_stays_usable():
     lib.device_status()
 
 
+def test_a_cta_that_gave_up_stays_until_its_cluster_has_sent():
+    """a part that arrives after the wait ran out still finds the CTA there: the exit waits for the cluster, and ends"""
+    from ngraph_b200 import lib
+    lib.device_status()
+    t0 = time.time()
+    assert lib.LIB.b200_selftest_split_give_up(2_000_000, _stream()) == 0
+    torch.cuda.synchronize()
+    assert time.time() - t0 < 5.0
+    code = ctypes.c_int(0)
+    assert lib.LIB.b200_device_status(ctypes.byref(code)) == -4 and code.value == 9002
+    assert lib.LIB.b200_device_status(ctypes.byref(code)) == 0
+
+
 def test_bad_limits_are_refused_on_the_host():
     from ngraph_b200 import lib
     before = lib.launch_count()
     assert lib.LIB.b200_selftest_bounded_wait(0, None) == -1
     assert lib.LIB.b200_selftest_bounded_wait(10_000_000_000, None) == -1  # seconds-long waits are not offered
+    assert lib.LIB.b200_selftest_split_give_up(0, None) == -1 and lib.LIB.b200_selftest_split_give_up(10_000_000_000, None) == -1
     assert lib.launch_count() == before
 
 
