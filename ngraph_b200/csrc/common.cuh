@@ -73,6 +73,13 @@ namespace b200
         asm volatile("" : "+l"(p)::"memory");
         __builtin_assume(__isGlobal(p));
     }
+    // The same for one use of a pointer that may be null, in code whose wait is elsewhere (the assembly keeps its order behind it).
+    template <typename P>
+    __device__ __forceinline__ P* ordered(P* p)
+    {
+        asm volatile("" : "+l"(p)::"memory");
+        return p;
+    }
     template <typename... P>
     __device__ __forceinline__ void after_earlier_kernels(P&... pointers)
     {

@@ -423,13 +423,14 @@ namespace b200
         }
         else if (p.half_away)
         {
-            const float scale = __ldg(p.scale);
+            const float scale = __ldg(ordered(p.scale));
 #pragma unroll
             for (int j = 0; j < 32; ++j)
                 v[j] = epilogue_core(p, int32_t(v[j]), scale);
         }
         else
         {
+            const void* const sum_in = ordered(p.sum_in);
 #pragma unroll
             for (int j4 = 0; j4 < 8; ++j4)
             {
@@ -443,7 +444,7 @@ namespace b200
                     const int j = 4 * j4 + i;
                     float f = __fmul_rn(__int2float_rn(int32_t(v[j]) + bb[i]), ss[i]);
                     if (has_sum && er.valid && col0 + j < p.N)
-                        f = __fadd_rn(f, __fmul_rn(sum_scale, load_sum(p.sum_in, p.sum_type, er.off + col0 + j)));
+                        f = __fadd_rn(f, __fmul_rn(sum_scale, load_sum(sum_in, p.sum_type, er.off + col0 + j)));
                     if (p.relu)
                         f = fmaxf(f, 0.0f);
                     if (p.out_type == B200_F32)
@@ -546,7 +547,10 @@ namespace b200
         const int first = tn * 64 + rank * quads * 4; // first column finished here
         const bool one_byte = p.out_type == B200_U8 || p.out_type == B200_I8;
         const bool aligned = p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out) & (one_byte ? 3 : 15)) == 0;
-        const float sum_scale = p.sum_in ? __ldg(p.sum_scale) : 0.0f;
+        const float sum_scale = p.sum_in ? __ldg(ordered(p.sum_scale)) : 0.0f;
+        const float* const scales = ordered(p.scale);
+        const int32_t* const biases = ordered(p.bias);
+        const uint8_t* const residual = ordered(static_cast<const uint8_t*>(p.sum_in));
         bool waited = false;
 #pragma unroll 1
         for (int quad = group; quad < quads; quad += 4)
@@ -558,9 +562,9 @@ namespace b200
 #pragma unroll
             for (int i = 0; i < 4; ++i)
             {
-                scale[i] = i < cols && p.scale ? __ldg(p.scale + (p.scale_per_channel ? col + i : 0)) : 0.0f;
-                bias[i] = i < cols && p.bias ? __ldg(p.bias + col + i) : 0;
-                sum[i] = i < cols && valid && p.sum_in ? static_cast<const uint8_t*>(p.sum_in)[off + col + i] : 0;
+                scale[i] = i < cols && p.scale ? __ldg(scales + (p.scale_per_channel ? col + i : 0)) : 0.0f;
+                bias[i] = i < cols && p.bias ? __ldg(biases + col + i) : 0;
+                sum[i] = i < cols && valid && p.sum_in ? residual[off + col + i] : 0;
             }
             if (!waited && !__all_sync(0xffffffffu, ptx::mbar_wait(landed, 0, abortp, 0)))
                 fail = 3002;
@@ -750,7 +754,8 @@ namespace b200
         // the stream itself, right before it first reads or overwrites their memory (a producer before its first load, an
         // epilogue warp before its first scale or residual; the MMA issuer touches no global memory).  One wait for all roles
         // here left 0.8-1.1 us of tile decoding and cold parameter reads between its return and the first load of every
-        // launch.  (No-ops when the launch is not a programmatic dependent one.)
+        // launch.  (No-ops when the launch is not a programmatic dependent one.)  Every load of what earlier kernels may have written
+        // goes through `ordered`, so that none is scheduled ahead of its role's wait.
         auto wait_for_earlier_kernels = []() { asm volatile("griddepcontrol.wait;" ::: "memory"); };
         if (!p.late_successor)
             asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -1198,7 +1203,7 @@ namespace b200
             }
             const bool has_sum = p.sum_in != nullptr;
             wait_for_earlier_kernels();
-            const float sum_scale = has_sum ? __ldg(p.sum_scale) : 0.0f;
+            const float sum_scale = has_sum ? __ldg(ordered(p.sum_scale)) : 0.0f;
             const uint32_t sum_flip = p.sum_type == B200_U8 ? 0u : 0x80808080u;
             const float sum_magic = p.sum_type == B200_U8 ? 8388608.0f : 8388736.0f;
             const int esz = (p.out_type == B200_U8 || p.out_type == B200_I8) ? 1 : 4;
@@ -1329,12 +1334,14 @@ namespace b200
                     {
                         // (re)stage this warp's scales and biases; the column tile changes at most tiles_n times per CTA
                         __syncwarp();
+                        const float* const scales = ordered(p.scale);
+                        const int32_t* const biases = ordered(p.bias);
                         for (int jj = lane; jj < COLS; jj += 32)
                         {
                             const int col = colw + jj;
                             const bool in_n = col < p.N;
-                            epi_scale[ew][jj] = (in_n && p.scale) ? __ldg(p.scale + (p.scale_per_channel ? col : 0)) : 0.0f;
-                            epi_bias[ew][jj] = (in_n && p.bias) ? __ldg(p.bias + col) : 0;
+                            epi_scale[ew][jj] = (in_n && p.scale) ? __ldg(scales + (p.scale_per_channel ? col : 0)) : 0.0f;
+                            epi_bias[ew][jj] = (in_n && p.bias) ? __ldg(biases + col) : 0;
                         }
                         staged_tn = tn;
                     }

@@ -627,3 +627,38 @@ def test_chained_launches_share_their_buffers(ops, m, n):
     for _ in range(5):
         for a, b in zip(passes(False), one_by_one):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("m,n,k,out,residual", [(20000, 128, 128, torch.uint8, False), (20000, 128, 128, torch.uint8, True), (20000, 128, 128, torch.float32, False),
+                                                (20000, 100, 128, torch.int8, False), (20000, 100, 128, torch.float32, True), (20000, 128, 128, torch.int32, False),
+                                                (4096, 256, 2304, torch.int8, True), (128, 1000, 2048, torch.int8, True), (64, 64, 128, torch.uint8, True)])
+def test_parameters_written_by_the_kernel_before(ops, m, n, k, out, residual):
+    """Scales, residual and its scale made on the device right before every product, other ones each time: no epilogue reads the last ones"""
+    from ngraph_b200 import lib
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = torch.randint(-128, 128, (m, k), generator=gen, device="cuda", dtype=torch.int8)
+    w = torch.randint(-127, 128, (n, k), generator=gen, device="cuda", dtype=torch.int8)
+    base, zp = torch.rand(n, generator=gen, device="cuda") * 0.01 / k ** 0.5 + 0.005 / k ** 0.5, torch.zeros((), dtype=torch.uint8, device="cuda")
+    steps = [torch.full((1,), 0.5 + 0.25 * i, device="cuda") for i in range(8)]
+    x, q_scale = torch.rand((m, n), generator=gen, device="cuda") * 4, torch.full((), 0.02, device="cuda")
+    scale, sum_scale, s = torch.empty(n, device="cuda"), torch.empty(1, device="cuda"), torch.empty((m, n), dtype=torch.uint8, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+
+    def passes(wait):
+        outs = []
+        for step in steps:
+            for call in (lambda: ops.quantize(x, q_scale if step is not steps[3] else q_scale * 2, zp, out=s),
+                         lambda: lib.LIB.b200_f32_binary(2, step.data_ptr(), step.data_ptr(), sum_scale.data_ptr(), 1, st),
+                         lambda: lib.LIB.b200_f32_binary_periodic(2, base.data_ptr(), step.data_ptr(), scale.data_ptr(), n, 1, 0, st),
+                         lambda: outs.append(ops.qgemm(a, w, scale, out, sum_in=s if residual else None, sum_scale=sum_scale if residual else None))):
+                call()
+                if wait:
+                    torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return outs
+
+    one_by_one = passes(True)
+    assert not torch.equal(one_by_one[0], one_by_one[1])
+    for _ in range(3):
+        for got, want in zip(passes(False), one_by_one):
+            assert torch.equal(got, want)
