@@ -482,8 +482,8 @@ namespace b200
     // Split reductions (SPLITK, 64-wide tiles): a product with few tiles and a long reduction leaves most SMs idle and pays for
     // every k-block in turn (0.2 us each).  A cluster of p.split CTAs then shares a tile: each multiplies its range of
     // k-blocks, hands its int32 partial sums to the CTAs that finish them - CTA r the columns 64 / split * r and up - by
-    // asynchronous stores into distributed shared memory that complete on one barrier of the receiving CTA (a cluster barrier
-    // with its release fence took 1.1 us), and that CTA adds the parts - exact integers, any order - and runs the epilogue, four
+    // asynchronous stores into distributed shared memory that complete on one barrier of the receiving CTA, awaited with acquire at
+    // cluster scope (a cluster barrier with its release fence took 1.1 us), and that CTA adds the parts - exact integers, any order - and runs the epilogue, four
     // columns of a row per thread.  This code runs once per launch: it is kept short, unrolled over 16 columns of a warp it
     // spent 2.6 us, mostly on fetching instructions.
     constexpr int MAX_SPLIT = 8;
@@ -499,7 +499,7 @@ namespace b200
         if (threadIdx.x == 0)
         {
             volatile int go_on = 0; // the CTA's own flag says that it has given up
-            ptx::mbar_wait(landed, 0, &go_on);
+            ptx::mbar_wait<true>(landed, 0, &go_on);
         }
         __syncthreads();
     }
@@ -566,7 +566,7 @@ namespace b200
                 bias[i] = i < cols && p.bias ? __ldg(biases + col + i) : 0;
                 sum[i] = i < cols && valid && p.sum_in ? residual[off + col + i] : 0;
             }
-            if (!waited && !__all_sync(0xffffffffu, ptx::mbar_wait(landed, 0, abortp, 0)))
+            if (!waited && !__all_sync(0xffffffffu, ptx::mbar_wait<true>(landed, 0, abortp, 0)))
                 fail = 3002;
             waited = true;
             const uint32_t part = exchange + uint32_t(quad * BM + row) * 16;
@@ -625,7 +625,7 @@ namespace b200
             }
         }
         // a warp without a quad of its own leaves only when every part has landed: the senders' stores need this CTA's memory
-        if (!waited && !__all_sync(0xffffffffu, ptx::mbar_wait(landed, 0, abortp, 0)))
+        if (!waited && !__all_sync(0xffffffffu, ptx::mbar_wait<true>(landed, 0, abortp, 0)))
             fail = 3002;
     }
 
@@ -2405,7 +2405,7 @@ namespace b200
             return;
         }
         if (threadIdx.x == 0)
-            ptx::mbar_wait(landed, 0, &abort_flag, 64, limit_ns);
+            ptx::mbar_wait<true>(landed, 0, &abort_flag, 64, limit_ns);
         __syncthreads();
         if (abort_flag)
             split_leave(landed);
