@@ -1926,21 +1926,21 @@ namespace b200
         return uint64_t(uint32_t(dev));
     }
 
-    // CTAs that share a tile's reduction.  Measured here (launches in a row): 3.5 us + 0.19 us per k-block of a 64-wide tile
-    // whole, 1.9 us more and the k-blocks divided when split; clusters of eight fit 128 of the 148 SMs at a time.
-    // [1, 512, 7, 7] 3x3 -> 512: 10.5 -> 6.3 us, 128 x 1000 x 2048: 17.4 -> 6.4 us, [1, 256, 14, 14] 3x3 -> 256: 7.0 -> 5.8 us.
+    // CTAs that share a tile's reduction: an estimate fitted to 1450 products measured whole and split in 2, 4 and 8 (1 to 640 rows,
+    // 16 to 3456 columns, 2 to 48 k-blocks; launches in a row).  Whole, a k-block of a 64-wide tile takes 0.19 us.  Split, the
+    // exchange takes 1.4-2.1 us and a k-block 0.27 us, because half the shared memory holds a ring of three stages, or 0.45 us
+    // where two CTAs run on an SM at a time; a third waits for them to end.  Clusters of eight fit 128 of the 148 SMs at a time.
+    // [1, 512, 7, 7] 3x3 -> 512: 10.5 us whole, 6.5 in eight; 128 x 1000 x 2048: 17.4 and 6.4; 20 x 2432 x 3072: 8.1 whole, 11.7 in two.
     static int pick_split(int64_t tiles, int64_t nkb)
     {
         int best = 1;
-        double best_us = 1e30;
-        for (int s = 1; s <= MAX_SPLIT && s <= nkb; s *= 2)
+        double best_us = 0.19 * double(nkb) * double((tiles + num_sms() - 1) / num_sms());
+        for (int s = 2; s <= MAX_SPLIT && s <= nkb; s *= 2)
         {
-            const int64_t room = s == 1 ? num_sms() : s == MAX_SPLIT ? num_sms() * 7 / 8 : num_sms() * 15 / 16;
-            // two split CTAs run on an SM at a time and share its loads; a third waits for them to end (three per SM instead
-            // of a smaller split: 300 x 720 x 3072 11.6 against 9.0 us, 128 x 2432 x 3072 11.9 against 8.6)
+            const int64_t room = s == MAX_SPLIT ? num_sms() * 7 / 8 : num_sms() * 15 / 16;
             const int64_t per_sm = (tiles * s + room - 1) / room, rounds = (per_sm + 1) / 2;
-            const double us = double(per_sm) * double((nkb + s - 1) / s) * 0.19 + (s > 1 ? 1.9 * double(rounds) + 3.0 * double(rounds - 1) : 0.0);
-            if (us < best_us - 0.15)
+            const double us = (s == MAX_SPLIT ? 1.4 : 2.1) + double((nkb + s - 1) / s) * (per_sm == 1 ? 0.27 : 0.45) * double(rounds) + 3.9 * double(rounds - 1);
+            if (us < best_us)
             {
                 best = s;
                 best_us = us;

@@ -71,3 +71,21 @@ def test_erf_of_few_elements(L, n):
     x, o = torch.randn(n, device="cuda").abs(), torch.empty(n, device="cuda")
     t = [us(lambda: L.LIB.b200_f32_unary(op, x.data_ptr(), o.data_ptr(), n, stream())) for op in (10, 8)]
     assert t[0] < 1.25 * t[1]
+
+
+@pytest.mark.parametrize("m,n,k,wide", [(20, 2432, 3072, 9600), (5760, 30, 4096, 30)])
+def test_a_reduction_is_not_split_where_that_is_slower(L, m, n, k, wide):
+    """beside a product with the same k-blocks per SM and tiles for all SMs, which is not split: half as much again if this one is"""
+    from ngraph_b200 import ops
+    a, s = torch.randint(-100, 100, (148 * 128 if wide == n else m, k), device="cuda", dtype=torch.int32).to(torch.int8), torch.ones(1, device="cuda")
+    w, o = torch.ones((wide, k), device="cuda", dtype=torch.int8), torch.empty((148 * 128 if wide == n else m) * wide, dtype=torch.uint8, device="cuda")
+    t = []
+    for rows, cols in ((m, n), (148 * 128, n) if wide == n else (m, wide)):
+        x, f, out = a[:rows], w[:cols], o[:rows * cols].view(rows, cols)
+        ops.qgemm(x, f, s, torch.uint8, out=out)
+
+        def call():
+            ops.qgemm(x, f, s, torch.uint8, out=out)
+            return 0
+        t.append(us(call))
+    assert t[0] < 1.12 * t[1]
