@@ -55,21 +55,38 @@ TORCH_OPS = os.path.join(HERE, "_torch_ops.so")
 FASTCALL = os.path.join(HERE, "_fastcall.so")
 
 
+def _made_by(stamp, made_by):
+    """whether the file `stamp` names this Python, this torch and this command"""
+    try:
+        return open(stamp).read() == made_by
+    except OSError:
+        return False
+
+
+def _build_extension(target, src, cmd, with_what, force, run=subprocess.check_call):
+    """Compile one CPython extension where its sources are newer or what it was built with (an ABI without promises) has changed."""
+    stamp = os.path.join(HERE, "build", os.path.basename(target) + ".made_by")
+    made_by = "\n".join([with_what] + cmd)
+    if force or not _newer(target, [src, os.path.join(ROOT, "include", "b200_kernels.h")]) or not _made_by(stamp, made_by):
+        run(cmd)
+        os.makedirs(os.path.dirname(stamp), exist_ok=True)
+        with open(stamp, "w") as f:
+            f.write(made_by)
+
+
 def build_python(force=False):
     """g++ the two CPython extensions: the native callables of lib.py, and the native half of ops.py over torch's C++ tensors."""
     import sysconfig
     common = ["g++", "-std=c++17", "-O2", "-fPIC", "-w", "-shared", "-fvisibility=hidden", "-I" + os.path.join(ROOT, "include"), "-I" + sysconfig.get_paths()["include"]]
-    header = os.path.join(ROOT, "include", "b200_kernels.h")
     src = os.path.join(CSRC, "fastcall.cpp")
-    if force or not _newer(FASTCALL, [src, header]):
-        subprocess.check_call(common + [src, "-o", FASTCALL])
+    _build_extension(FASTCALL, src, common + [src, "-o", FASTCALL], sys.version, force)
     src = os.path.join(CSRC, "torch_ops.cpp")
-    if force or not _newer(TORCH_OPS, [src, header]):
-        import torch
-        base = os.path.dirname(torch.__file__)
-        subprocess.check_call(common + ["-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch.compiled_with_cxx11_abi()), "-I" + os.path.join(base, "include"),
-                                        "-I" + os.path.join(base, "include", "torch", "csrc", "api", "include"), "-I/usr/local/cuda/include", src, "-o", TORCH_OPS,
-                                        "-L" + os.path.join(base, "lib"), "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"])
+    import torch
+    base = os.path.dirname(torch.__file__)
+    cmd = common + ["-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch.compiled_with_cxx11_abi()), "-I" + os.path.join(base, "include"),
+                    "-I" + os.path.join(base, "include", "torch", "csrc", "api", "include"), "-I/usr/local/cuda/include", src, "-o", TORCH_OPS,
+                    "-L" + os.path.join(base, "lib"), "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+    _build_extension(TORCH_OPS, src, cmd, sys.version + "\ntorch " + torch.__version__, force)
     return FASTCALL, TORCH_OPS
 
 

@@ -118,3 +118,26 @@ def test_native_callables_refuse_what_ctypes_refuses():
     for epilogue in (e, (lib.Epilogue * 1)(), None):
         assert L.b200_qgemm(None, 9, None, None, 4, 4, 16, epilogue, None) == -1
     assert L.b200_quantize(None, None, None, None, lib.U8, None, 2, None, 0, 4, None) == -1
+
+
+def test_extensions_are_rebuilt_for_another_torch(tmp_path, monkeypatch):
+    """the extensions link ABIs without promises: other versions or flags make them stale, whatever the timestamps say"""
+    from ngraph_b200 import build
+    monkeypatch.setattr(build, "HERE", str(tmp_path))
+    src, target, ran = tmp_path / "x.cpp", tmp_path / "x.so", []
+    src.write_text("")
+    target.write_text("")
+    os.utime(target, (2e9, 2e9))
+
+    def once(cmd, with_what, force=False):
+        ran.clear()
+        build._build_extension(str(target), str(src), cmd, with_what, force, ran.append)
+        return len(ran)
+
+    assert once(["g++", "-O2"], "torch 1") == 1  # nothing says what the file was made with
+    assert once(["g++", "-O2"], "torch 1") == 0
+    assert once(["g++", "-O2"], "torch 2") == 1 and once(["g++", "-O2"], "torch 2") == 0
+    assert once(["g++", "-O3"], "torch 2") == 1
+    assert once(["g++", "-O3"], "torch 2", force=True) == 1
+    os.utime(src, (2.1e9, 2.1e9))
+    assert once(["g++", "-O3"], "torch 2") == 1
