@@ -410,6 +410,19 @@ namespace b200
         }
     }
 
+    // A four-byte result of any contract but the raw one: f32 bits or int32.
+    __device__ __forceinline__ uint32_t epilogue_word(const ContractParams& p, uint32_t acc, float scale, int32_t bias, float sum_scale, float residual)
+    {
+        if (p.half_away)
+            return epilogue_core(p, int32_t(acc), scale);
+        float f = __fmul_rn(__int2float_rn(int32_t(acc) + bias), scale);
+        if (p.sum_in)
+            f = __fadd_rn(f, __fmul_rn(sum_scale, residual));
+        if (p.relu)
+            f = fmaxf(f, 0.0f);
+        return p.out_type == B200_F32 ? __float_as_uint(f) : uint32_t(clamp_cast<int32_t>(round_quant<B200_ROUND_NEAREST_TOWARD_EVEN>(f)));
+    }
+
     // Every other case (core contract, 4-byte outputs, ragged / unaligned residuals): v[] holds the int32
     // accumulators on entry and the output values on return (f32 bit patterns / int32), w[] the packed bytes
     // for one-byte outputs.
@@ -638,6 +651,9 @@ namespace b200
         EPI_SECTORS, // f32 outputs of the fused contract without residual, written from registers in whole sectors
         EPI_ROWS,    // one-byte outputs without residual of any width and contract, written row by row through shared memory, or
                      // from registers where the stage ring takes all of it
+        EPI_WORDS,   // four-byte results otherwise: i32 of every contract, f32 with a residual; the stores of EPI_SECTORS
+        EPI_SUM,     // one-byte results with a residual that TMA does not bring (or a ring that leaves it no room): the residual into
+                     // registers ahead of the accumulator, the stores of EPI_ROWS
         EPI_GENERAL  // everything else: results of any type straight from registers
     };
     template <int BN, int BK, bool CTA2 = false, bool SPLITK = false, int EPI = EPI_BYTES>
@@ -1207,6 +1223,7 @@ namespace b200
             const uint32_t sum_flip = p.sum_type == B200_U8 ? 0u : 0x80808080u;
             const float sum_magic = p.sum_type == B200_U8 ? 8388608.0f : 8388736.0f;
             const int esz = (p.out_type == B200_U8 || p.out_type == B200_I8) ? 1 : 4;
+            const bool residual_pieces = (p.N & 15) == 0 && (reinterpret_cast<uintptr_t>(p.sum_in) & 15) == 0;
             const bool vec_ok = ((esz == 1) ? ((p.N & 15) == 0) : ((p.N & 3) == 0)) &&
                                 ((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.sum_in)) & 15) == 0;
             // this warp's staging blocks (one per tile in flight): 32 rows x 64 bytes, swizzled like the TMA unit expects
@@ -1236,15 +1253,19 @@ namespace b200
             //   9, 10     EPI_SECTORS without / with ReLU, rows of whole 16-byte pieces;  16, 17: any rows
             //   11 .. 13  EPI_ROWS, fused contract: u8, i8, i8 with ReLU;  14, 15: core contract, u8, i8
             //   18 .. 20  EPI_ROWS without staging (width a multiple of 16), fused contract: u8, i8, i8 with ReLU
+            //   21, 22    EPI_WORDS, rows of whole 16-byte pieces and any rows;  23, 24: the same for raw accumulators
+            //   25 .. 27  EPI_SUM: u8, i8, i8 with ReLU;  28 .. 30: the same without staging
             //   -1        EPI_GENERAL (any contract, type and width)
             auto epilogue_loop = [&](auto mode_tag) {
                 constexpr int MODE = decltype(mode_tag)::value;
-                constexpr bool F_F32 = MODE == 9 || MODE == 10 || MODE == 16 || MODE == 17, F_PIECES = MODE < 16;
-                constexpr bool F_ROWS = MODE >= 11 && MODE <= 15, F_CORE = MODE == 14 || MODE == 15, F_DIRECT = MODE >= 18;
+                constexpr bool F_RAW = MODE == 23 || MODE == 24, F_WORD = MODE == 21 || MODE == 22;
+                constexpr bool F_F32 = MODE == 9 || MODE == 10 || MODE == 16 || MODE == 17 || F_WORD || F_RAW, F_PIECES = MODE < 16 || MODE == 21 || MODE == 23;
+                constexpr bool F_RES = MODE >= 25, F_ROWS = (MODE >= 11 && MODE <= 15) || (MODE >= 25 && MODE <= 27), F_CORE = MODE == 14 || MODE == 15;
+                constexpr bool F_DIRECT = (MODE >= 18 && MODE <= 20) || MODE >= 28;
                 constexpr bool FAST = MODE >= 0 && MODE <= 8; // the one-byte modes, staged and stored by TMA
                 constexpr int F_SUMK = FAST ? MODE % 3 : 0;
-                constexpr bool F_SUM = F_SUMK != 0, F_RELU = FAST ? MODE >= 6 : MODE == 10 || MODE == 13 || MODE == 17 || MODE == 20;
-                constexpr bool F_U8 = (MODE >= 0 && MODE < 3) || MODE == 11 || MODE == 14 || MODE == 18;
+                constexpr bool F_SUM = F_SUMK != 0, F_RELU = FAST ? MODE >= 6 : MODE == 10 || MODE == 13 || MODE == 17 || MODE == 20 || MODE == 27 || MODE == 30;
+                constexpr bool F_U8 = (MODE >= 0 && MODE < 3) || MODE == 11 || MODE == 14 || MODE == 18 || MODE == 25 || MODE == 28;
                 constexpr int NBUF = F_SUM && EPI != EPI_BYTES_2 ? 3 : F_ROWS ? 1 : 2; // staging blocks per warp
                 int staged_tn = -1;
                 int blk = 0;             // staging block of the current tile: j % NBUF
@@ -1373,6 +1394,35 @@ namespace b200
                         }
                     }
                     uint32_t sumw[8] = {0, 0, 0, 0, 0, 0, 0, 0}; // residual bytes of the columns at hand
+                    // EPI_SUM: this row's residual, which does not depend on the accumulator.  Rows and columns outside the tensor
+                    // compute on zeros and are not stored.
+                    uint32_t residual[F_RES ? CHUNKS : 1][8] = {};
+                    if (F_RES && er.valid)
+                    {
+                        const uint8_t* const sp = ordered(static_cast<const uint8_t*>(p.sum_in)) + er.off + colw;
+                        const int n = p.N - colw;
+#pragma unroll
+                        for (int c = 0; c < (F_RES ? CHUNKS : 0); ++c)
+                        {
+                            if (residual_pieces)
+                            {
+#pragma unroll
+                                for (int half = 0; half < 2; ++half)
+                                    if (32 * c + 16 * half < n)
+                                    {
+                                        const uint4 r = *reinterpret_cast<const uint4*>(sp + 32 * c + 16 * half);
+                                        residual[c][4 * half] = r.x, residual[c][4 * half + 1] = r.y, residual[c][4 * half + 2] = r.z, residual[c][4 * half + 3] = r.w;
+                                    }
+                            }
+                            else
+                            {
+#pragma unroll
+                                for (int b = 0; b < 32; ++b)
+                                    if (32 * c + b < n)
+                                        residual[c][b >> 2] |= uint32_t(sp[32 * c + b]) << (8 * (b & 3));
+                            }
+                        }
+                    }
                     {
                         PROF_T0();
                         // the verdict is made warp-uniform: the loop body uses full-mask shuffles and warp syncs
@@ -1414,15 +1464,26 @@ namespace b200
                         for (int i = 0; i < 4; ++i)
                             dst[i] = static_cast<float*>(p.out) + __shfl_sync(0xffffffffu, static_cast<long long>(er.off), g + 8 * i) + colw + own_col;
                         uint32_t v[2][16];
-                        ptx::tmem_ld_16x32(t_addr, v[0]);
-                        ptx::tmem_ld_wait(v[0]);
-#pragma unroll
-                        for (int h = 0; h < 4; ++h) // 16 rows x 32 columns at a time, the next ones on their way meanwhile
+                        if (!F_WORD)
                         {
-                            if (h < 3)
+                            ptx::tmem_ld_16x32(t_addr, v[0]);
+                            ptx::tmem_ld_wait(v[0]);
+                        }
+                        // 16 rows x 32 columns at a time, the next ones on their way meanwhile.  The general words take one step after
+                        // the other in one body: unrolled, a small product spent twice its time on fetching instructions.
+#pragma unroll(F_WORD ? 1 : 4)
+                        for (int h = 0; h < 4; ++h)
+                        {
+                            if (F_WORD)
+                            {
+                                ptx::tmem_ld_16x32(t_addr + (uint32_t(h >> 1) << 20) + 32 * (h & 1), v[0]);
+                                ptx::tmem_ld_wait(v[0]);
+                            }
+                            else if (h < 3)
                                 ptx::tmem_ld_16x32(t_addr + (uint32_t((h + 1) >> 1) << 20) + 32 * ((h + 1) & 1), v[(h + 1) & 1]);
-                            const uint32_t(&x)[16] = v[h & 1];
+                            const uint32_t(&x)[16] = v[F_WORD ? 0 : h & 1];
                             const int i = 2 * (h >> 1);
+                            float *const d0 = h < 2 ? dst[0] : dst[2], *const d1 = h < 2 ? dst[1] : dst[3];
                             const bool ok0 = ((rows_ok >> (8 * i)) & 1u) != 0, ok1 = ((rows_ok >> (8 * i + 8)) & 1u) != 0;
 #pragma unroll
                             for (int jj = 0; jj < 2; ++jj)
@@ -1432,9 +1493,32 @@ namespace b200
                                 for (int u = 0; u < 2; ++u)
                                 {
                                     const int j4 = 2 * jj + u, col = 32 * (h & 1) + 8 * j4 + pair_col;
+                                    if (F_RAW)
+                                    {
+                                        lo[u].x = __uint_as_float(x[4 * j4 + 0]), lo[u].y = __uint_as_float(x[4 * j4 + 1]);
+                                        hi[u].x = __uint_as_float(x[4 * j4 + 2]), hi[u].y = __uint_as_float(x[4 * j4 + 3]);
+                                        continue;
+                                    }
                                     const F2 s2 = lds_f2(sc_base + 4u * col);
                                     const F2 b2 = lds_f2(bi_base + 4u * col);
                                     const int32_t b0 = __float_as_int(b2.x), b1 = __float_as_int(b2.y);
+                                    if (F_WORD)
+                                    {
+                                        float r[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                                        if (has_sum)
+                                        {
+                                            const uint8_t* const sum_in = ordered(static_cast<const uint8_t*>(p.sum_in)) + (col - own_col);
+#pragma unroll
+                                            for (int e = 0; e < 4; ++e)
+                                                if ((e < 2 ? ok0 : ok1) && col + (e & 1) < p.N - colw)
+                                                    r[e] = load_sum(sum_in, p.sum_type, (e < 2 ? d0 : d1) - static_cast<const float*>(p.out) + (e & 1));
+                                        }
+                                        lo[u].x = __uint_as_float(epilogue_word(p, x[4 * j4 + 0], s2.x, b0, sum_scale, r[0]));
+                                        lo[u].y = __uint_as_float(epilogue_word(p, x[4 * j4 + 1], s2.y, b1, sum_scale, r[1]));
+                                        hi[u].x = __uint_as_float(epilogue_word(p, x[4 * j4 + 2], s2.x, b0, sum_scale, r[2]));
+                                        hi[u].y = __uint_as_float(epilogue_word(p, x[4 * j4 + 3], s2.y, b1, sum_scale, r[3]));
+                                        continue;
+                                    }
                                     const float a0 = __int2float_rn(add_fma_pipe(int32_t(x[4 * j4 + 0]), b0, p.one));
                                     const float a1 = __int2float_rn(add_fma_pipe(int32_t(x[4 * j4 + 1]), b1, p.one));
                                     const float a2 = __int2float_rn(add_fma_pipe(int32_t(x[4 * j4 + 2]), b0, p.one));
@@ -1461,10 +1545,10 @@ namespace b200
                                     hi_in.x = __shfl_xor_sync(0xffffffffu, hi_out.x, 1);
                                     hi_in.y = __shfl_xor_sync(0xffffffffu, hi_out.y, 1);
                                     if (ok0 && col < cols)
-                                        *reinterpret_cast<float4*>(dst[i] + col) =
+                                        *reinterpret_cast<float4*>(d0 + col) =
                                             odd ? make_float4(lo_in.x, lo_in.y, lo[1].x, lo[1].y) : make_float4(lo[0].x, lo[0].y, lo_in.x, lo_in.y);
                                     if (ok1 && col < cols)
-                                        *reinterpret_cast<float4*>(dst[i + 1] + col) =
+                                        *reinterpret_cast<float4*>(d1 + col) =
                                             odd ? make_float4(hi_in.x, hi_in.y, hi[1].x, hi[1].y) : make_float4(hi[0].x, hi[0].y, hi_in.x, hi_in.y);
                                 }
                                 else
@@ -1474,17 +1558,17 @@ namespace b200
                                     {
                                         const int cu = col + 8 * u;
                                         if (ok0 && cu < cols)
-                                            dst[i][cu] = lo[u].x;
+                                            d0[cu] = lo[u].x;
                                         if (ok0 && cu + 1 < cols)
-                                            dst[i][cu + 1] = lo[u].y;
+                                            d0[cu + 1] = lo[u].y;
                                         if (ok1 && cu < cols)
-                                            dst[i + 1][cu] = hi[u].x;
+                                            d1[cu] = hi[u].x;
                                         if (ok1 && cu + 1 < cols)
-                                            dst[i + 1][cu + 1] = hi[u].y;
+                                            d1[cu + 1] = hi[u].y;
                                     }
                                 }
                             }
-                            if (h < 3)
+                            if (!F_WORD && h < 3)
                                 ptx::tmem_ld_wait(v[(h + 1) & 1]);
                         }
                     }
@@ -1502,7 +1586,8 @@ namespace b200
                                 if (F_CORE)
                                     epilogue_chunk_core<F_U8>(v, w, lds_f4(sc_base).x, p.out_zp);
                                 else
-                                    epilogue_chunk_bytes<0, F_RELU, F_U8>(v, w, sc_base + 128u * c, bi_base + 128u * c, sumw, sum_scale, sum_flip, sum_magic, p.one);
+                                    epilogue_chunk_bytes<F_RES ? 2 : 0, F_RELU, F_U8>(v, w, sc_base + 128u * c, bi_base + 128u * c, residual[F_RES ? c : 0], sum_scale,
+                                                                                      sum_flip, sum_magic, p.one);
                                 stage_bytes_out(c, w);
                             }
                             __syncwarp();
@@ -1590,7 +1675,8 @@ namespace b200
                             uint32_t v[32], w[8];
                             ptx::tmem_ld_32x32(t_addr + 32 * c, v);
                             ptx::tmem_ld_wait();
-                            epilogue_chunk_bytes<0, F_RELU, F_U8>(v, w, sc_base + 128u * c, bi_base + 128u * c, sumw, sum_scale, sum_flip, sum_magic, p.one);
+                            epilogue_chunk_bytes<F_RES ? 2 : 0, F_RELU, F_U8>(v, w, sc_base + 128u * c, bi_base + 128u * c, residual[F_RES ? c : 0], sum_scale, sum_flip,
+                                                                              sum_magic, p.one);
                             uint4* const op = reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.out) + er.off + colw + 32 * c);
                             if (er.valid && colw + 32 * c < p.N)
                                 op[0] = make_uint4(w[0], w[1], w[2], w[3]);
@@ -1724,6 +1810,24 @@ namespace b200
                 default: epilogue_loop(std::integral_constant<int, 15>{}); break;
                 }
             }
+            else if constexpr (EPI == EPI_WORDS)
+            {
+                const bool pieces = p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+                if (p.half_away == 2)
+                    pieces ? epilogue_loop(std::integral_constant<int, 23>{}) : epilogue_loop(std::integral_constant<int, 24>{});
+                else
+                    pieces ? epilogue_loop(std::integral_constant<int, 21>{}) : epilogue_loop(std::integral_constant<int, 22>{});
+            }
+            else if constexpr (EPI == EPI_SUM)
+                switch ((p.smem.out_bufs ? 25 : 28) + (p.out_type == B200_U8 ? 0 : p.relu ? 2 : 1))
+                {
+                case 25: epilogue_loop(std::integral_constant<int, 25>{}); break;
+                case 26: epilogue_loop(std::integral_constant<int, 26>{}); break;
+                case 27: epilogue_loop(std::integral_constant<int, 27>{}); break;
+                case 28: epilogue_loop(std::integral_constant<int, 28>{}); break;
+                case 29: epilogue_loop(std::integral_constant<int, 29>{}); break;
+                default: epilogue_loop(std::integral_constant<int, 30>{}); break;
+                }
             else if constexpr (EPI == EPI_GENERAL)
                 epilogue_loop(std::integral_constant<int, -1>{});
             else
@@ -1961,6 +2065,8 @@ namespace b200
                : p.epilogue == EPI_SECTORS ? qcontract_kernel<BN, BK, false, false, EPI_SECTORS>
                : p.epilogue == EPI_BYTES_2 ? qcontract_kernel<BN, BK, false, false, EPI_BYTES_2>
                : p.epilogue == EPI_ROWS    ? qcontract_kernel<BN, BK, false, false, EPI_ROWS>
+               : p.epilogue == EPI_WORDS   ? qcontract_kernel<BN, BK, false, false, EPI_WORDS>
+               : p.epilogue == EPI_SUM     ? qcontract_kernel<BN, BK, false, false, EPI_SUM>
                : p.epilogue == EPI_GENERAL ? qcontract_kernel<BN, BK, false, false, EPI_GENERAL>
                                            : qcontract_kernel<BN, BK, false, false, EPI_BYTES>;
     }
@@ -2089,6 +2195,10 @@ namespace b200
                 p.epilogue = p.tma_sum && sum_bufs == 2 ? EPI_BYTES_2 : EPI_BYTES;
             else if (p.out_type == B200_F32 && !p.half_away && !p.sum_in && (reinterpret_cast<uintptr_t>(p.out) & 3) == 0)
                 p.epilogue = EPI_SECTORS;
+            else if (!one_byte && (reinterpret_cast<uintptr_t>(p.out) & 3) == 0)
+                p.epilogue = EPI_WORDS;
+            else if (one_byte && !p.half_away && p.sum_in && (!rows_staged || (room - C::OUT_BYTES) / sp.stage_bytes >= MIN_STAGES))
+                p.epilogue = EPI_SUM;
             else if (one_byte && p.half_away != 2 && !p.sum_in && (!p.half_away || (p.out_zp >= -(1 << 20) && p.out_zp <= (1 << 20))) &&
                      (!rows_staged || (room - C::OUT_BYTES) / sp.stage_bytes >= MIN_STAGES))
                 p.epilogue = EPI_ROWS;
@@ -2097,7 +2207,7 @@ namespace b200
         }
         if (p.epilogue != EPI_BYTES && p.epilogue != EPI_BYTES_2)
             p.tma_store = p.tma_sum = 0;
-        sp.out_bufs = p.tma_store ? (p.tma_sum ? sum_bufs : 2) : p.epilogue == EPI_ROWS && rows_staged ? 1 : 0;
+        sp.out_bufs = p.tma_store ? (p.tma_sum ? sum_bufs : 2) : (p.epilogue == EPI_ROWS || p.epilogue == EPI_SUM) && rows_staged ? 1 : 0;
         sp.out_bytes = p.split > 1 ? SPLIT_EXCHANGE_BYTES : sp.out_bufs * C::OUT_BYTES;
         int fit = (room - sp.out_bytes) / sp.stage_bytes;
         sp.stages = fit > MAX_STAGES ? MAX_STAGES : fit;

@@ -662,3 +662,54 @@ def test_parameters_written_by_the_kernel_before(ops, m, n, k, out, residual):
     for _ in range(3):
         for got, want in zip(passes(False), one_by_one):
             assert torch.equal(got, want)
+
+
+def _at(t, offset):
+    """the same data `offset` elements into a larger buffer"""
+    buf = torch.empty(t.numel() + 64, dtype=t.dtype, device="cuda")
+    view = buf[offset:offset + t.numel()].view(t.shape)
+    view.copy_(t)
+    return view
+
+
+@pytest.mark.parametrize("m,n,k", [(4096, 768, 3072), (640, 4096, 2304), (1000, 256, 512), (20000, 100, 128), (3000, 33, 64), (2500, 801, 96), (47, 16, 16), (130, 31, 48), (60, 8, 1040), (20001, 7, 64), (5000, 258, 272)])
+def test_qgemm_residuals_and_words_off_the_tma_paths(ops, m, n, k):
+    """one-byte results with a residual of any width, start and reduction length, four-byte results of every contract with and without
+    a residual, raw accumulators: against the products in double and the contract's single-precision steps"""
+    import ctypes
+    from ngraph_b200 import lib
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = torch.randint(-128, 128, (m, k), generator=gen, device="cuda", dtype=torch.int32).to(torch.int8)
+    w = torch.randint(-127, 128, (n, k), generator=gen, device="cuda", dtype=torch.int32).to(torch.int8)
+    bias = torch.randint(-1000, 1001, (n,), generator=gen, device="cuda", dtype=torch.int32)
+    scale = torch.rand(n, generator=gen, device="cuda") * 0.01 / k ** 0.5 + 0.005 / k ** 0.5
+    ss = torch.full((1,), 0.37, device="cuda")
+    acc = (a.double() @ w.double().t()).to(torch.int32)
+    base = (acc + bias).float() * scale
+    res = {torch.uint8: torch.randint(0, 256, (m, n), generator=gen, device="cuda", dtype=torch.int32).to(torch.uint8),
+           torch.int8: torch.randint(-128, 128, (m, n), generator=gen, device="cuda", dtype=torch.int32).to(torch.int8)}
+
+    def finish(f, out, relu):
+        f = f.clamp(min=0) if relu else f
+        if out == torch.float32:
+            return f
+        lo, hi = {torch.uint8: (0, 255), torch.int8: (-128, 127), torch.int32: (-2 ** 31, 2 ** 31 - 1)}[out]
+        return f.round().double().clamp(lo, hi).to(out)
+
+    for out, relu, r, r_at, out_at in ((torch.uint8, True, torch.uint8, 0, 0), (torch.int8, False, torch.int8, 1, 0), (torch.int8, True, torch.uint8, 16, 0), (torch.uint8, False, torch.int8, 0, 1),
+                                       (torch.int8, True, torch.int8, 3, 5), (torch.uint8, True, None, 0, 3), (torch.int8, False, None, 0, 1), (torch.float32, True, torch.uint8, 0, 0),
+                                       (torch.float32, False, torch.int8, 1, 1), (torch.int32, False, torch.int8, 0, 0), (torch.int32, True, None, 0, 1), (torch.int32, False, None, 0, 0)):
+        want = finish(base if r is None else base + ss * res[r].float(), out, relu)
+        o = _at(torch.zeros((m, n), dtype=out, device="cuda"), out_at)
+        ops.qgemm(a, w, scale, out, bias=bias, relu=relu, sum_in=None if r is None else _at(res[r], r_at), sum_scale=None if r is None else ss, out=o)
+        assert torch.equal(o, want), (out, relu, r, r_at, out_at)
+    o = _at(torch.zeros((m, n), dtype=torch.int32, device="cuda"), 1)
+    ops.qgemm(a, w, scale[:1], torch.int32, core=True, out_zp=-5, out=o)
+    f = acc.float() * scale[0]
+    assert torch.equal(o, (torch.sign(f) * (f.abs().double() + 0.5).floor()).to(torch.int32) - 5)
+    e = lib.Epilogue()
+    e.round_half_away, e.out_type = 2, lib.I32
+    for at in (0, 1):
+        o = _at(torch.zeros((m, n), dtype=torch.int32, device="cuda"), at)
+        lib.check(lib.LIB.b200_qgemm(a.data_ptr(), lib.I8, w.data_ptr(), o.data_ptr(), m, n, k, ctypes.byref(e), torch.cuda.current_stream().cuda_stream), "raw")
+        assert torch.equal(o, acc)

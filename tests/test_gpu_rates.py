@@ -89,3 +89,19 @@ def test_a_reduction_is_not_split_where_that_is_slower(L, m, n, k, wide):
             return 0
         t.append(us(call))
     assert t[0] < 1.12 * t[1]
+
+
+@pytest.mark.parametrize("m,n,k,out,at,times", [(4096, 768, 3072, torch.uint8, 0, 1.5), (2048, 2048, 4096, torch.int8, 0, 1.4), (1000, 256, 512, torch.int8, 1, 3.0), (19000, 128, 512, torch.float32, 0, 2.8)])
+def test_products_with_a_residual(L, m, n, k, out, at, times):
+    """beside the same product without one; residual bytes fetched one by one behind the accumulator: 2.2, 2.1, 4.4 and 3.4 times"""
+    from ngraph_b200 import ops
+    a = torch.randint(-100, 100, (m, k), device="cuda", dtype=torch.int32).to(torch.int8)
+    w, s, o = torch.ones((n, k), device="cuda", dtype=torch.int8), torch.full((1,), 0.01, device="cuda"), torch.empty((m, n), device="cuda", dtype=out)
+    r = torch.zeros(m * n + 16, device="cuda", dtype=torch.uint8)[at:at + m * n].view(m, n)
+    t = []
+    for residual in (r, None):
+        def call():
+            ops.qgemm(a, w, s, out, sum_in=residual, sum_scale=None if residual is None else s, out=o)
+            return 0
+        t.append(us(call))
+    assert t[0] < times * t[1], t
