@@ -285,7 +285,7 @@ def test_bmm_tile_edges(L, batch, m, k, n):
     np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(acc.astype(np.float32)))
 
 
-@pytest.mark.parametrize("n", [1, 3, 1023, 65535, 65536, (1 << 20) - 1, 1 << 20, (1 << 20) + 1, 3000001])
+@pytest.mark.parametrize("n", [1, 3, 1023, 65535, 65536, (1 << 19) - 1, 1 << 19, (1 << 19) + 1, (1 << 20) - 1, 1 << 20, (1 << 20) + 1, 3000001])
 def test_extremes_of_a_whole_tensor(L, n):
     """Max, Min and Max over Abs of every element: the cluster form and the atomic form, runs that do not start on 16 bytes,
     negative results, NaNs that never win"""
@@ -367,14 +367,14 @@ def test_permutes_that_move_the_last_axis(L, shape):
         np.testing.assert_array_equal(o.cpu().numpy(), np.transpose(x, order).ravel(), err_msg=str(order))
 
 
-@pytest.mark.parametrize("shape,axes", [((1,), (0,)), ((2,), (0,)), ((1000,), (0,)), ((1025,), (0,)), ((65535,), (0,)), ((1 << 20,), (0,)), (((1 << 20) + 1,), (0,)), ((3000001,), (0,)),
+@pytest.mark.parametrize("shape,axes", [((1,), (0,)), ((2,), (0,)), ((1000,), (0,)), ((1025,), (0,)), ((65535,), (0,)), ((1 << 19,), (0,)), (((1 << 19) + 1,), (0,)), (((1 << 20) + 1,), (0,)), ((3000001,), (0,)),
                                         ((10, 5000), (1,)), ((5000, 10), (0,)), ((3, 40, 3, 50), (1, 3)), ((70, 40), (1,))])
 def test_a_zero_extreme_is_the_first_zero(L, shape, axes):
     """Max and Min replace on a strict comparison: of zeros of both signs the first one in row-major order is the result, wherever it lies"""
     rng = np.random.default_rng(int(np.prod(shape)))
     kept = [i for i in range(len(shape)) if i not in axes]
     for op, sign in ((1, -1.0), (2, 1.0)):
-        if op == 1 and len(kept) == 0 and shape[0] > 1 << 20:
+        if op == 1 and len(kept) == 0 and shape[0] > 1 << 19:
             continue  # Max of more elements: the sign of a zero is not fixed
         for share in (1.0, 0.3, 2.0 / shape[-1], 0.0):
             x = (np.float32(sign) * (np.abs(rng.standard_normal(shape)) + 0.1)).astype(np.float32)

@@ -105,3 +105,13 @@ def test_products_with_a_residual(L, m, n, k, out, at, times):
             return 0
         t.append(us(call))
     assert t[0] < times * t[1], t
+
+
+def test_largest_value_around_the_forms(L):
+    """the size up to which one cluster does it costs no more than a little beyond it"""
+    import ctypes
+    t = {}
+    for n in (3 << 18, 1 << 20, (1 << 20) + (1 << 17)):
+        x, o = torch.rand(n, device="cuda"), torch.empty(1, device="cuda")
+        t[n] = us(lambda: L.LIB.b200_reduce_f32(1, x.data_ptr(), o.data_ptr(), (ctypes.c_int64 * 1)(n), 1, (ctypes.c_int64 * 1)(0), 1, stream()))
+    assert t[1 << 20] < 1.15 * t[(1 << 20) + (1 << 17)], t
