@@ -63,25 +63,28 @@ namespace b200
     // The [rows, inner] view of a tensor, with what replaces divisions by `inner` (see make_rows).
     struct RowMap
     {
-        int64_t total;
-        uint32_t inner;
+        int64_t total, inner;
         FastDiv n_scales;
         uint64_t inner_inv64;  // ceil(2^64 / inner): row of a block's first element
         uint32_t inner_inv32;  // ceil(2^32 / inner): rows inside a block, for inner < the block's elements
     };
 
-    // Where a block's first element lies: its row, and its offset inside that row.
-    __device__ __forceinline__ void block_row(const RowMap& m, int64_t base, uint32_t& row, uint32_t& r0)
+    // Where a block's first element lies: its row, and its offset inside that row.  The product with the rounded-up reciprocal is
+    // the quotient or one more, whatever the sizes.
+    __device__ __forceinline__ void block_row(const RowMap& m, int64_t base, uint32_t& row, int64_t& r0)
     {
-        row = uint32_t(__umul64hi(uint64_t(base), m.inner_inv64));
-        r0 = uint32_t(base - int64_t(row) * m.inner);
+        int64_t q = int64_t(__umul64hi(uint64_t(base), m.inner_inv64));
+        if (q * m.inner > base)
+            --q;
+        row = uint32_t(q);
+        r0 = base - q * m.inner;
     }
 
     // Row (counted from the block's first) of the element `off` = r0 + local, and the elements left in that row.
     __device__ __forceinline__ uint32_t local_row(const RowMap& m, uint32_t off, uint32_t& left)
     {
         const uint32_t r = __umulhi(off, m.inner_inv32);
-        left = (r + 1) * m.inner - off;
+        left = (r + 1) * uint32_t(m.inner) - off; // (rows shorter than a block)
         return r;
     }
 
@@ -168,14 +171,16 @@ namespace b200
                 return e0.y != 0.0f;
             }
             uint32_t row;
-            block_row(m, base, row, r0);
+            int64_t in_row;
+            block_row(m, base, row, in_row);
+            r0 = uint32_t(in_row); // (of rows shorter than a block)
             const uint32_t first = row - m.n_scales.div(row) * m.n_scales.d;
             if (ROWS == TWO_ROWS)
             {
                 e0 = e1 = row_scale<Q, FAST>(scale, zp, first, fast);
-                if (m.inner - r0 < rem)
+                if (m.inner - in_row < int64_t(rem))
                 {
-                    boundary = m.inner - r0;
+                    boundary = uint32_t(m.inner - in_row);
                     e1 = row_scale<Q, FAST>(scale, zp, first + 1 == m.n_scales.d ? 0 : first + 1, fast);
                 }
                 return e0.y != 0.0f && e1.y != 0.0f;
@@ -467,13 +472,13 @@ namespace b200
     {
         if (!p.rows_ok || ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15))
             return false;
-        if (p.rows > 1 && (p.inner < MIN_INNER || p.inner > (int64_t(1) << 30) || p.rows >= (int64_t(1) << 31) || p.total > (int64_t(1) << 33)))
-            return false; // beyond these the 64-bit reciprocal below is no longer exact (total * inner < 2^64)
+        if (p.rows > 1 && (p.inner < MIN_INNER || p.rows >= (int64_t(1) << 31)))
+            return false;
         if (p.total / (QT * 4) >= (int64_t(1) << 31) - 1)
             return false;
         m.total = p.total;
         m.n_scales = p.rows > 1 ? FastDiv(uint32_t(p.n_scales)) : FastDiv(1);
-        m.inner = p.rows > 1 ? uint32_t(p.inner) : 0;
+        m.inner = p.rows > 1 ? p.inner : 0;
         m.inner_inv64 = p.rows > 1 ? ~uint64_t(0) / uint64_t(p.inner) + 1 : 0;
         m.inner_inv32 = p.rows > 1 ? uint32_t(0xFFFFFFFFull / uint64_t(p.inner) + 1) : 0;
         return true;

@@ -16,17 +16,17 @@ def stream():
     return torch.cuda.current_stream().cuda_stream
 
 
-def us(call):
+def us(call, run=20):
     """shortest time per call of a run of launches"""
     best = float("inf")
     for _ in range(8):
         first, last = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         first.record()
-        for _ in range(20):
+        for _ in range(run):
             assert call() == 0
         last.record()
         last.synchronize()
-        best = min(best, first.elapsed_time(last) * 1000 / 20)
+        best = min(best, first.elapsed_time(last) * 1000 / run)
     return best
 
 
@@ -115,3 +115,32 @@ def test_largest_value_around_the_forms(L):
         x, o = torch.rand(n, device="cuda"), torch.empty(1, device="cuda")
         t[n] = us(lambda: L.LIB.b200_reduce_f32(1, x.data_ptr(), o.data_ptr(), (ctypes.c_int64 * 1)(n), 1, (ctypes.c_int64 * 1)(0), 1, stream()))
     assert t[1 << 20] < 1.15 * t[(1 << 20) + (1 << 17)], t
+
+
+@pytest.mark.parametrize("rows,inner", [(2, (1 << 30) + 16), (257, 1 << 25)])
+def test_the_longest_rows(L, rows, inner):
+    """Per-axis Quantize and Dequantize of rows beyond 2^30 elements and of more than 2^33: the rate of one scale per tensor, and its values.
+    Element by element, with a division per axis, three times as long."""
+    import ctypes
+    n = rows * inner
+    x, q = torch.empty(n, device="cuda").uniform_(-4, 4), torch.empty(n, dtype=torch.int8, device="cuda")
+    s, z = torch.rand(rows, device="cuda") * 0.05 + 0.02, torch.arange(rows, device="cuda").to(torch.int8)
+
+    def quantize(shape, axes, scale, zp):
+        return lambda: L.LIB.b200_quantize(x.data_ptr(), scale.data_ptr(), zp.data_ptr(), q.data_ptr(), L.I8, (ctypes.c_int64 * len(shape))(*shape), len(shape),
+                                           (ctypes.c_int64 * 1)(*axes), len(axes), 4, stream())
+
+    def dequantize(shape, axes, scale, zp):
+        return lambda: L.LIB.b200_dequantize(q.data_ptr(), scale.data_ptr(), zp.data_ptr(), x.data_ptr(), L.I8, (ctypes.c_int64 * len(shape))(*shape), len(shape),
+                                             (ctypes.c_int64 * 1)(*axes), len(axes), stream())
+
+    ends = [0, inner - 3, (rows // 2) * inner - 3, (rows - 1) * inner - 3, n - 7]  # the elements around row boundaries and at the ends
+    rows_of = torch.cat([torch.arange(e, e + 7, device="cuda") for e in ends])
+    idx = rows_of // inner
+    assert quantize((rows, inner), (0,), s, z)() == 0
+    want = (x[rows_of] / s[idx]).round() + z[idx].float()
+    assert torch.equal(q[rows_of], want.clamp(-128, 127).to(torch.int8))
+    assert us(quantize((rows, inner), (0,), s, z), 3) < 1.5 * us(quantize((n,), (), s[:1], z[:1]), 3)
+    assert dequantize((rows, inner), (0,), s, z)() == 0
+    assert torch.equal(x[rows_of], (q[rows_of].int() - z[idx].int()).float() * s[idx])
+    assert us(dequantize((rows, inner), (0,), s, z), 3) < 1.5 * us(dequantize((n,), (), s[:1], z[:1]), 3)
