@@ -2,10 +2,10 @@
 // GELU, residual adds, dynamic activation scales) with the arithmetic of nGraph's reference kernels:
 //
 //   elementwise +, -, *, /, max, min, abs, neg, sqrt, relu   IEEE single, one rounding each, nothing contracted
-//   exp, erf                                                   reference: std::exp / std::erf on float; here the double
-//                                                              routine rounded to float (differs from a given libm in
-//                                                              the last bit on a small share of inputs), computed in
-//                                                              single precision with a rounding test (rounded_math.cuh)
+//   exp, erf                                                   reference: std::exp / std::erf on float; here the value
+//                                                              rounded to float once (differs from a given libm in the
+//                                                              last bit on a small share of inputs), from a table and a
+//                                                              Taylor step in double (rounded_math.cuh)
 //   Sum          runtime/reference/sum.hpp:56-90     Kahan-compensated, inputs taken in row-major order
 //   Max          runtime/reference/max.hpp:32-58     start at -inf, replace when x > max
 //   Broadcast    runtime/reference/broadcast.hpp     output coordinate with the broadcast axes dropped
@@ -392,8 +392,6 @@ namespace b200
         return true;
     }
 
-    // One thread per output element; the reduced coordinates are walked in row-major order, as the reference does.
-    // keep: the kept axes (thread index -> input offset); red: the reduced axes.
     // One step of the reference's compensated sum (runtime/reference/sum.hpp:56-90).
     __device__ __forceinline__ void kahan_step(float& z, float& c, float x)
     {
@@ -422,6 +420,8 @@ namespace b200
     {
         return OP == B200_REDUCE_MIN ? INFINITY : -INFINITY;
     }
+    // One thread per output element; the reduced coordinates are walked in row-major order, as the reference does.
+    // keep: the kept axes (thread index -> input offset); red: the reduced axes.
     template <int OP> // b200_reduce_op
     __global__ void __launch_bounds__(128) reduce_kernel(const float* __restrict__ in, float* __restrict__ out, Dims keep, Dims red,
                                                          int64_t n_out, int64_t n_red)

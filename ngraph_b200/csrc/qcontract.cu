@@ -116,7 +116,6 @@ namespace b200
         int b_blocks_n;      // 64-row blocks per k-block in that image: ceil(N / 64)
         int epilogue;        // which family of epilogue loops (EPI_*) the launch needs
         int tma_sum;         // the residual is fetched by TMA into the staging block its result will be stored from
-        int vec_params;      // scale / bias pointers are 16-byte aligned
         int pair;            // 1, or 2: a CTA works on two row tiles (2u, 2u + 1) at a time, which share every B stage
         int cta2;            // CTA pairs (thread-block clusters of two, tcgen05 cta_group::2): the pair works on row tiles 2u and
                              // 2u + 1 of a 256-wide column tile with ONE 256 x 256 instruction stream; each CTA loads its own
@@ -2320,7 +2319,6 @@ namespace b200
         p.out_zp = e->out_zero_point;
         p.out_type = e->out_type;
         p.out = out;
-        p.vec_params = ((reinterpret_cast<uintptr_t>(p.scale) | reinterpret_cast<uintptr_t>(e->bias)) & 15) == 0;
         const bool one_byte = e->out_type == B200_U8 || e->out_type == B200_I8;
         p.tma_store = one_byte && (p.N % 16 == 0) && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
         (void)a_type;

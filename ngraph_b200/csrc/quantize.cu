@@ -8,7 +8,7 @@
 //   stream  - the tensor is viewed as [rows, inner] where every row has ONE scale / zero point (per-tensor: a single
 //             row; per-axis on axis a: rows = prod(shape[0..a]), inner = prod(shape[a+1..])) but is walked as one flat
 //             run of 16-byte vectors, wherever the rows start and end: 128-bit loads, packed 32-bit (or 128-bit) stores,
-//             4 independent loads in flight per thread.  The scales of the rows a block touches are looked up once per
+//             one to eight independent loads in flight per thread, by size.  The scales of the rows a block touches are looked up once per
 //             block into a small shared-memory table while its loads are under way.
 //   generic - one element per thread with the scale index recomputed from the
 //             coordinates; any axis set, any alignment.
@@ -210,9 +210,8 @@ namespace b200
 
     // U vectors of four elements per thread (see vectors_per_thread); blocks_for: what the registers are kept down for.
     constexpr int blocks_for(int u) { return u >= 8 ? 4 : 6; }
-    // Bound by HBM for large tensors (f32 -> u8 at 1 GB, per tensor and per channel: round to even 6.7 TB/s, a plain copy's rate,
-    // the half-way modes 6.5-6.7, the directed ones 6.2-6.7) and by load latency below some 100 MB.  Walking the tensor
-    // flat instead of row by row is what keeps odd row lengths on 128-bit accesses: [24, 64, 113, 113] per channel 182 -> 22 us,
+    // Bound by HBM for large tensors (f32 -> u8 at 1 GB: 6.3 TB/s in a half-way mode, a plain copy's rate) and by load latency below some 100 MB.  Walking the tensor
+    // flat instead of row by row is what keeps odd row lengths on 128-bit accesses: [24, 64, 113, 113] per channel 182 -> 20 us,
     // [4000, 64, 15, 13] 458 -> 55 us.
     template <typename Q, int MODE, bool FAST, int ROWS, int U>
     __global__ void __launch_bounds__(QT, blocks_for(U)) quantize_stream_kernel(const float* __restrict__ x, const float* __restrict__ scale,

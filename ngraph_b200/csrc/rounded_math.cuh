@@ -9,8 +9,8 @@
 //   erf(x) = E(g) + D(g) (d - g d^2 + ...)              g = rint(256 |x|) / 256, |d| <= 1 / 512, D = erf', degree 5
 //
 // The tables are constant-evaluated from the defining series (all terms positive: nothing cancels) and copied to shared memory
-// by the kernels that use them.  Against the general routines, over all 2^32 arguments: exp never
-// differs, erf for 208 of them (in the last bit).
+// by the kernels that use them.  Against the general double routines rounded to float, over all 2^32 arguments: exp never
+// differs, erf for two of them (in the last bit).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
