@@ -483,9 +483,10 @@ namespace b200
         return true;
     }
 
-    // Vectors per thread.  Few while that is what it takes for the grid to be started early (`launch`: two blocks per SM): 1 MB of
-    // f32 in 1.2 us, 2 MB in 1.4 us.  Eight in large Quantize calls, where the look-up of a block's scales weighs: per channel at
-    // 1 GB 225 us with four, 201 with eight; 16 M elements 16.4 and 18.7 (fewer, longer blocks end less evenly).
+    // Vectors per thread.  Few in small calls, which spread over the SMs that way: 1 MB of f32 in 1.2 us, 2 MB in 1.4 us (up to two
+    // blocks of one or two vectors per SM; the line was drawn when only such grids were launched early, and has not moved since).
+    // Eight in large Quantize calls, where the look-up of a block's scales weighs: per channel at 1 GB 225 us with four, 201 with
+    // eight; 16 M elements 16.4 and 18.7 (fewer, longer blocks end less evenly).
     static int vectors_per_thread(int64_t total, bool quantize)
     {
         const int64_t early = int64_t(sm_count()) * 2 * QT * 4; // elements of two blocks per SM, one vector per thread
