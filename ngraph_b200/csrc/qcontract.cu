@@ -1458,7 +1458,7 @@ namespace b200
                         const int own_col = F_PIECES ? (lane & 2) * 2 + (odd ? 8 : 0) : pair_col;
                         const int cols = p.N - colw - own_col;
                         float* dst[4]; // rows g, g + 8, g + 16, g + 24 of the warp's 32
-                        const uint32_t rows_ok = __ballot_sync(0xffffffffu, er.valid) >> g;
+                        const uint32_t all_rows_ok = __ballot_sync(0xffffffffu, er.valid), rows_ok = all_rows_ok >> g;
 #pragma unroll
                         for (int i = 0; i < 4; ++i)
                             dst[i] = static_cast<float*>(p.out) + __shfl_sync(0xffffffffu, static_cast<long long>(er.off), g + 8 * i) + colw + own_col;
@@ -1473,6 +1473,8 @@ namespace b200
 #pragma unroll(F_WORD ? 1 : 4)
                         for (int h = 0; h < 4; ++h)
                         {
+                            if (F_WORD && (32 * (h & 1) >= p.N - colw || ((all_rows_ok >> (16 * (h >> 1))) & 0xFFFFu) == 0))
+                                continue; // nothing of these rows and columns is inside (warp-uniform)
                             if (F_WORD)
                             {
                                 ptx::tmem_ld_16x32(t_addr + (uint32_t(h >> 1) << 20) + 32 * (h & 1), v[0]);
@@ -2051,10 +2053,11 @@ namespace b200
     // exchange takes 1.4-2.1 us and a k-block 0.27 us, because half the shared memory holds a ring of three stages, or 0.45 us
     // where two CTAs run on an SM at a time; a third waits for them to end.  Clusters of eight fit 128 of the 148 SMs at a time.
     // [1, 512, 7, 7] 3x3 -> 512: 10.5 us whole, 6.5 in eight; 128 x 1000 x 2048: 17.4 and 6.4; 20 x 2432 x 3072: 8.1 whole, 11.7 in two.
-    static int pick_split(int64_t tiles, int64_t nkb)
+    // `words`: the results are what EPI_WORDS computes, which four of a whole tile's warps take 3 us for.
+    static int pick_split(int64_t tiles, int64_t nkb, bool words)
     {
         int best = 1;
-        double best_us = 0.19 * double(nkb) * double((tiles + num_sms() - 1) / num_sms());
+        double best_us = 0.19 * double(nkb) * double((tiles + num_sms() - 1) / num_sms()) + (words ? 3.0 : 0.0);
         for (int s = 2; s <= MAX_SPLIT && s <= nkb; s *= 2)
         {
             const int64_t room = s == MAX_SPLIT ? num_sms() * 7 / 8 : num_sms() * 15 / 16;
@@ -2148,7 +2151,7 @@ namespace b200
             return B200_ERR_TOO_LARGE;
         const int nkb = p.ntaps * p.cblocks;
         SmemPlan& sp = p.smem;
-        p.split = (BN == 64 && !p.a_cells && !p.halo && p.pair != 2 && !p.cta2) ? pick_split(int64_t(p.tiles_m) * p.tiles_n, nkb) : 1;
+        p.split = (BN == 64 && !p.a_cells && !p.halo && p.pair != 2 && !p.cta2) ? pick_split(int64_t(p.tiles_m) * p.tiles_n, nkb, p.half_away != 2 && (p.out_type == B200_I32 || (p.out_type == B200_F32 && p.sum_in))) : 1;
         sp.b_resident = (p.tiles_n == 1 && nkb * C::B_BYTES <= B_RESIDENT_MAX && p.split == 1) ? 1 : 0;
         if (p.split > 1) // results are written from registers; the staging area holds the partial sums on their way
             p.tma_store = p.tma_sum = 0;
