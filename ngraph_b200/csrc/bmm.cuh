@@ -1,0 +1,21 @@
+// BatchMatMul's two kernels for larger matrices: panels on the double-precision matrix instruction (glue_f32.cu) and digit planes
+// on the integer tensor cores (bmm_digits.cu).
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace b200
+{
+    // Digit form: what it takes (`vec`: K and N are multiples of 4, the pointers 16-byte aligned), its estimated time in us, and its launch.
+    bool bmm_digits_accepts(int64_t batch, int64_t M, int64_t K, int64_t N, bool vec);
+    double bmm_digits_us(int64_t batch, int64_t M, int64_t K, int64_t N);
+    int launch_bmm_digits(const float* a, const float* b, float* out, int64_t batch, int M, int K, int N, cudaStream_t st);
+    // the word in which kernels record a wait that gave up (qcontract.cu); null if it cannot be had
+    int* contract_status_address();
+
+    // (m8n8k4: each output receives its four exact products in ascending k, one rounding each)
+    __device__ __forceinline__ void dmma(double (&c)[2], double a, double b)
+    {
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
+    }
+}

@@ -1,0 +1,927 @@
+// BatchMatMul on the integer tensor cores, with the bits of the double-precision sum.
+//
+// reference::dot sums double(a) * double(b) over k and rounds to float once.  The double-precision pipe gives 64 multiply-adds per
+// clock and SM; the int8 tensor cores 4096 and more.  So a row of A and a column of B are written as 55-bit fixed-point numbers
+// relative to their largest magnitude, in seven signed digits of 8 bits, X = sum_i d_i 2^(8 (6 - i)); the products of digits i of A and
+// j of B with i + j = s <= 6 are summed exactly in one int32 accumulator per s (28 int8 products for one of doubles), and
+//   V = sum_s D_s 2^(8 (5 - s))
+// is the wanted sum in fixed point but for what was left out, which is less than 2 K + 2 units of V:
+//   the products of i + j = 7 (six of at most 2^14, 2^-16 units each: 1.5 K) and beyond,
+//   the half unit that X may be off, on either side (0.25 K), and the fraction of the last accumulator.
+// Where V - 2 K - 2 and V + 2 K + 2 round to the same float, that is the float of the exact sum.  Otherwise, for results that are
+// not normal numbers and for rows or columns with an infinity or a NaN, the output is computed again in double, in k order.  That
+// happens to two outputs in a million for normally distributed values, half of them sums that all but cancel (with six digits
+// 50 times as often).
+#include <cuda_runtime.h>
+#include <algorithm>
+#include <atomic>
+#include "common.cuh"
+#include "ptx.cuh"
+#include "bmm.cuh"
+
+namespace b200
+{
+    namespace digits
+    {
+        constexpr int PLANES = 7, TM = 128, TN = 64, SUB = 32 /* columns of one accumulator: while one is read the other is computed */, KC = 64 /* of K per pipeline stage */, MAX_K = 4096 /* V is a 64-bit number */;
+        constexpr int A_PLANE = TM * KC, A_BYTES = PLANES * A_PLANE, B_BYTES = PLANES * TN * KC;
+        constexpr int A_SLOTS = 2, B_SLOTS = 3, S_SLOTS = 4;
+        constexpr int WORK_WARPS = 24, MMA_WARP = WORK_WARPS, THREADS = (MMA_WARP + 4) * 32;
+        // registers of a thread at launch (what 896 threads leave each), and after the warps that only issue have given theirs up
+        constexpr int LAUNCH_REGS = 72, WORK_REGS = 80, MMA_REGS = 24;
+        static_assert(WORK_WARPS * WORK_REGS + 4 * MMA_REGS <= (WORK_WARPS + 4) * LAUNCH_REGS, "more registers than the block was launched with");
+        constexpr int QUEUE = 768; // pairs of outputs left to the end
+        constexpr int SHARED = A_SLOTS * A_BYTES + B_SLOTS * B_BYTES + QUEUE * 16 + 128;
+        constexpr int TMEM_COLS = 512, ACC_COLS = PLANES * SUB; // two times seven accumulators of 32 columns
+        static_assert(WORK_WARPS * 4096 <= A_SLOTS * A_BYTES, "room for the products of pair_in_order");
+
+        struct Params
+        {
+            const float *a, *b;
+            float* out;
+            int* status;
+            int M, K, N, tiles_m, tiles_n;
+            int group;            // column tiles of a unit of work (they share the digits of its row tile when K <= KC)
+            int groups;           // units per row tile
+            int64_t units;        // batch * tiles_m * groups
+            int eps;
+            // powers of two as multipliers that the compiler does not know: a wide multiply-add each on a pipe with room to spare,
+            // where shifts and adds of register pairs would be four on the one that bounds the kernel
+            int one, up8, up16, up24;
+        };
+
+        // Exponent e of a row whose largest magnitude has these bits: |x| < 2^e, and the upper digit of no element leaves [-128, 127].
+        // Not below -78: the factors made of it are normal numbers.
+        __device__ __forceinline__ int row_exponent(uint32_t max_bits) { return max(int((max_bits + 0x18000u) >> 23) - 126, -78); }
+        __device__ __forceinline__ float power_of_two(int e) { return __int_as_float((e + 127) << 23); }
+        __device__ __forceinline__ float digit_scale(uint32_t max_bits) { return power_of_two(22 - row_exponent(max_bits)); }
+        // what an output of this row is multiplied by (V counts 2^(e_a + e_b - 52)); 0 for an empty row, NaN for one that is not finite
+        __device__ __forceinline__ float result_scale(uint32_t max_bits)
+        {
+            const float f = power_of_two(row_exponent(max_bits) - 26);
+            return max_bits == 0 ? 0.0f : max_bits >= 0x7F800000u ? __int_as_float(0x7FFFFFFF) : f;
+        }
+
+        __device__ __forceinline__ long long mad_wide(int a, int b, long long c)
+        {
+            long long d;
+            asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+            return d;
+        }
+        __device__ __forceinline__ uint64_t mad_wide_u(uint32_t a, uint32_t b, uint64_t c)
+        {
+            uint64_t d;
+            asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+            return d;
+        }
+        // Loads that stay where they are written, ahead of the waits behind which their values are used (the compiler moves plain ones
+        // down to there); 0 if not `in`.
+        __device__ __forceinline__ float load_now(const float* p)
+        {
+            float x;
+            asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(x) : "l"(p));
+            return x;
+        }
+        __device__ __forceinline__ float load_now(const float* p, bool in)
+        {
+            float x;
+            asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@p ld.global.nc.f32 %0, [%1];\n\t}" : "=&f"(x) : "l"(p), "r"(int(in)));
+            return x;
+        }
+        __device__ __forceinline__ void load_now4(float* x, const float* p, bool in)
+        {
+            asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\tmov.f32 %2, 0f00000000;\n\t"
+                         "mov.f32 %3, 0f00000000;\n\t@p ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+                         : "=&f"(x[0]), "=&f"(x[1]), "=&f"(x[2]), "=&f"(x[3])
+                         : "l"(p), "r"(int(in)));
+        }
+        // max(m, |x|), NaN if either is
+        __device__ __forceinline__ float max_magnitude(float m, float x)
+        {
+            float d;
+            asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(m), "f"(fabsf(x)));
+            return d;
+        }
+        __device__ __forceinline__ uint64_t pack2(float x, float y)
+        {
+            uint64_t r;
+            asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+            return r;
+        }
+        __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
+        {
+            uint64_t d;
+            asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+            return d;
+        }
+        __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
+        {
+            uint64_t d;
+            asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+            return d;
+        }
+        __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
+        {
+            uint64_t d;
+            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+            return d;
+        }
+
+        // The seven digits of four elements (consecutive k), word p = digit p of each.  Limbs of 22, 16 and 16 bits come off by adding
+        // 1.5 * 2^23 (every step but the last rounding is exact), the low words of the sums are put together by one multiply-add; the
+        // constants in them make balanced digits: 0x8080... added, 0x80 taken off every byte but the top one, which has an excess of
+        // 0x40.  Per element 4 packed float operations, one wide multiply-add, 3.75 byte permutes and two xors or adds.
+        __device__ __forceinline__ void four_digits(const float (&x)[4], float scale, uint32_t up16, uint32_t (&d)[PLANES])
+        {
+            constexpr float M0 = 12582912.0f - float(0x4B40) + float(0x8080), M1 = 12582912.0f + float(0x8080) - float(0x4B40), M2 = 12582912.0f + float(0x8080);
+            const uint64_t s = pack2(scale, scale), neg = pack2(-1.0f, -1.0f), up = pack2(65536.0f, 65536.0f);
+            const uint64_t m0 = pack2(M0, M0), m1 = pack2(M1, M1), m2 = pack2(M2, M2);
+            uint32_t lo[4], hi[4];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+            {
+                const uint64_t f = mul2(pack2(x[2 * h], x[2 * h + 1]), s);
+                const uint64_t t0 = add2(f, m0), r0 = add2(f, fma2(t0, neg, m0));
+                const uint64_t t1 = fma2(r0, up, m1), r1 = fma2(r0, up, fma2(t1, neg, m1));
+                const uint64_t t2 = fma2(r1, up, m2);
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                {
+                    const uint32_t w0 = uint32_t(j ? t0 >> 32 : t0), w1 = uint32_t(j ? t1 >> 32 : t1), w2 = uint32_t(j ? t2 >> 32 : t2);
+                    const uint64_t y = mad_wide_u(w1, up16, uint64_t(w0) << 32 | w2);
+                    lo[2 * h + j] = uint32_t(y);
+                    hi[2 * h + j] = uint32_t(y >> 32);
+                }
+            }
+            const uint32_t x01 = __byte_perm(lo[0], lo[1], 0x5140), x23 = __byte_perm(lo[2], lo[3], 0x5140);
+            const uint32_t y01 = __byte_perm(lo[0], lo[1], 0x7362), y23 = __byte_perm(lo[2], lo[3], 0x7362);
+            const uint32_t h01 = __byte_perm(hi[0], hi[1], 0x5140), h23 = __byte_perm(hi[2], hi[3], 0x5140);
+            const uint32_t g01 = __byte_perm(hi[0], hi[1], 0x0062), g23 = __byte_perm(hi[2], hi[3], 0x0062);
+            d[0] = (__byte_perm(g01, g23, 0x5410) + 0x40404040u) ^ 0x80808080u;
+            d[1] = __byte_perm(h01, h23, 0x7632) ^ 0x80808080u;
+            d[2] = __byte_perm(h01, h23, 0x5410) ^ 0x80808080u;
+            d[3] = __byte_perm(y01, y23, 0x7632) ^ 0x80808080u;
+            d[4] = __byte_perm(y01, y23, 0x5410) ^ 0x80808080u;
+            d[5] = __byte_perm(x01, x23, 0x7632) ^ 0x80808080u;
+            d[6] = __byte_perm(x01, x23, 0x5410) ^ 0x80808080u;
+        }
+
+        __device__ __forceinline__ void sts(uint32_t addr, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+
+        // K-major operand without swizzle: 16-byte pieces of 8 rows lie together (128 bytes), groups of 8 rows follow each other, and
+        // `piece` bytes further on comes the next 16 bytes of K.
+        __device__ __forceinline__ uint64_t descriptor(uint32_t addr, uint32_t piece)
+        {
+            return uint64_t((addr & 0x3FFFF) >> 4) | uint64_t(piece >> 4) << 16 | uint64_t(128 >> 4) << 32 | uint64_t(1) << 46;
+        }
+        __device__ __forceinline__ void tmem_ld_16x16(uint32_t taddr, int (&r)[8])
+        {
+            asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                         : "r"(taddr)
+                         : "memory");
+        }
+        __device__ __forceinline__ void tmem_wait(int (&r)[8])
+        {
+            asm volatile("tcgen05.wait::ld.sync.aligned;"
+                         : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])::"memory");
+        }
+
+        // The outputs of a warp (32 x 16 at (m0, n0); lane (g, t) holds row 8 i + g, columns 8 j + 2 t and the next in bit 2 i + j of `marked`)
+        // that the digits do not settle, where they are many: blocks of 8 x 8 on the double-precision matrix instruction, k ascending.
+        // The lane that stored an output before is the one that stores it again.
+        __device__ __noinline__ void settle_blocks(const float* a, const float* b, float* out, int M, int K, int N, int m0, int n0, uint32_t marked)
+        {
+            const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll 1
+            for (int block = 0; block < 8; ++block)
+            {
+                if (!__any_sync(0xFFFFFFFFu, (marked >> block) & 1))
+                    continue;
+                const int m8 = m0 + 8 * (block >> 1), n8 = n0 + 8 * (block & 1);
+                const bool m_in = m8 + g < M, n_in = n8 + g < N;
+                const float* ap = a + int64_t(m8 + g) * K + t;
+                const float* bp = b + int64_t(t) * N + n8 + g;
+                double acc[2] = {0.0, 0.0};
+                for (int k0 = 0; k0 < K; k0 += 32)
+                {
+                    float x[8], y[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                    {
+                        const bool in = k0 + 4 * i + t < K;
+                        x[i] = in && m_in ? __ldg(ap + k0 + 4 * i) : 0.0f;
+                        y[i] = in && n_in ? __ldg(bp + int64_t(k0 + 4 * i) * N) : 0.0f;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        dmma(acc, double(x[i]), double(y[i])); // beyond K: fma(0, 0, acc) = acc
+                }
+                if (m_in)
+#pragma unroll
+                    for (int c = 0; c < 2; ++c)
+                        if (n8 + 2 * t + c < N)
+                            out[int64_t(m8 + g) * N + n8 + 2 * t + c] = static_cast<float>(acc[c]);
+            }
+        }
+
+        // Few of them are left to the end, where all warps of the block share them; many, or too many, are settled here.
+        __device__ __noinline__ void leave_or_settle(int4* queue, int* queued, const float* a, const float* b, float* out, int M, int K, int N, int batch,
+                                                     int m0, int n0, uint32_t marked)
+        {
+            const int lane = threadIdx.x & 31, count = __reduce_add_sync(0xFFFFFFFFu, __popc(marked));
+            int first = QUEUE;
+            if (count <= 8 && lane == 0)
+                first = atomicAdd(queued, count);
+            first = __shfl_sync(0xFFFFFFFFu, first, 0);
+            const bool room = first + count <= QUEUE;
+            for (int i = 0; i < 8; ++i) // (the places are filled whether there is room for all or not)
+            {
+                const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, (marked >> i) & 1);
+                const int at = first + __popc(lanes & ((1u << lane) - 1));
+                if (((marked >> i) & 1) && at < QUEUE)
+                    queue[at] = make_int4(room ? batch : -1, m0 + 8 * (i >> 1) + (lane >> 2), n0 + 8 * (i & 1) + 2 * (lane & 3), 0);
+                first += __popc(lanes);
+            }
+            if (!room)
+                settle_blocks(a + int64_t(batch) * M * K, b + int64_t(batch) * K * N, out + int64_t(batch) * M * N, M, K, N, m0, n0, marked);
+        }
+
+        // Outputs (m, n) and (m, n + 1) by one warp: the lanes make the products (exact in double) and leave them in `room` (4 KB), two of
+        // them add these up in k order.
+        __device__ __noinline__ void pair_in_order(const float* a, const float* b, float* out, int K, int N, int m, int n, double2* room)
+        {
+            const int lane = threadIdx.x & 31, n1 = min(n + 1, N - 1);
+            double sum = 0.0;
+            for (int k0 = 0; k0 < K; k0 += 256)
+            {
+                const int n_k = min(256, K - k0);
+                __syncwarp();
+#pragma unroll 4
+                for (int k = lane; k < n_k; k += 32)
+                {
+                    const double x = __ldg(a + int64_t(m) * K + k0 + k);
+                    const float* y = b + int64_t(k0 + k) * N;
+                    room[k] = make_double2(x * double(__ldg(y + n)), x * double(__ldg(y + n1)));
+                }
+                __syncwarp();
+                if (lane < 2)
+#pragma unroll 8
+                    for (int k = 0; k < n_k; ++k)
+                        sum += reinterpret_cast<const double*>(room)[2 * k + lane];
+            }
+            if (lane < 2 && n + lane < N)
+                out[int64_t(m) * N + n + lane] = static_cast<float>(sum);
+        }
+
+        // Roles.  The first warps are the epilogue, each 16 (LONG: twice 16) columns of a TMEM lane quarter; the others of warps 0-23 turn
+        // f32 into digits (plain loads, stores into the MMA's layout); warp 24 issues the MMAs.  LONG (K > KC): the largest magnitudes of a
+        // tile's rows and columns need a pass over all of K of their own, ahead of its digits; the epilogue warps, which have little else to
+        // do then, make it and bring into L2 what the one after it will read.
+        // K and N are multiples of 4 and the pointers 16-byte aligned.
+        template <bool LONG>
+        __global__ void __launch_bounds__(THREADS, 1) bmm_digits_kernel(const Params p)
+        {
+            constexpr int EPI_WARPS = LONG ? 8 : 16, CONV_WARPS = WORK_WARPS - EPI_WARPS;
+            extern __shared__ uint8_t raw[];
+            __shared__ int abort_flag;
+            __shared__ uint32_t tmem_slot;
+            __shared__ __align__(8) uint64_t bars[2 * A_SLOTS + 2 * B_SLOTS + 2 * S_SLOTS + 5];
+            __shared__ uint32_t a_max[LONG ? S_SLOTS : 1][TM], b_max[LONG ? S_SLOTS : 1][TN]; // the bits of the largest magnitudes
+            __shared__ float a_scale[S_SLOTS][TM], b_scale[S_SLOTS][TN];                      // result_scale of them
+            __shared__ int queued;
+            const uint32_t base = (ptx::smem_u32(raw) + 127u) & ~127u;
+            auto a_slot = [&](int s) { return base + uint32_t(s) * A_BYTES; };
+            auto b_slot = [&](int s) { return base + A_SLOTS * A_BYTES + uint32_t(s) * B_BYTES; };
+            const uint32_t bar0 = ptx::smem_u32(bars);
+            auto a_full = [&](int s) { return bar0 + 8u * s; };
+            auto a_empty = [&](int s) { return bar0 + 8u * (A_SLOTS + s); };
+            auto b_full = [&](int s) { return bar0 + 8u * (2 * A_SLOTS + s); };
+            auto b_empty = [&](int s) { return bar0 + 8u * (2 * A_SLOTS + B_SLOTS + s); };
+            auto s_full = [&](int s) { return bar0 + 8u * (2 * A_SLOTS + 2 * B_SLOTS + s); };
+            auto s_empty = [&](int s) { return bar0 + 8u * (2 * A_SLOTS + 2 * B_SLOTS + S_SLOTS + s); };
+            const uint32_t t_full = bar0 + 8u * (2 * A_SLOTS + 2 * B_SLOTS + 2 * S_SLOTS), t_empty = t_full + 16, drained = t_full + 32; // one of either per accumulator
+            int4* queue = reinterpret_cast<int4*>(raw + (base - ptx::smem_u32(raw)) + A_SLOTS * A_BYTES + B_SLOTS * B_BYTES); // batch, m, n
+            const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+            volatile int* abortp = &abort_flag;
+            if (threadIdx.x == 0)
+            {
+                abort_flag = 0;
+                queued = 0;
+                for (int s = 0; s < A_SLOTS; ++s)
+                    ptx::mbar_init(a_full(s), CONV_WARPS), ptx::mbar_init(a_empty(s), 1);
+                for (int s = 0; s < B_SLOTS; ++s)
+                    ptx::mbar_init(b_full(s), CONV_WARPS), ptx::mbar_init(b_empty(s), 1);
+                for (int s = 0; s < S_SLOTS; ++s)
+                    ptx::mbar_init(s_full(s), LONG ? EPI_WARPS : CONV_WARPS), ptx::mbar_init(s_empty(s), EPI_WARPS);
+                for (int s = 0; s < 2; ++s)
+                    ptx::mbar_init(t_full + 8 * s, 1), ptx::mbar_init(t_empty + 8 * s, 8 /* warps */);
+                ptx::mbar_init(drained, 1);
+                ptx::fence_barrier_init();
+            }
+            if (warp == MMA_WARP)
+            {
+                ptx::tmem_alloc(ptx::smem_u32(&tmem_slot), TMEM_COLS);
+                ptx::tmem_relinquish();
+            }
+            ptx::tc_fence_before_sync();
+            __syncthreads();
+            ptx::tc_fence_after_sync();
+            const uint32_t tmem = tmem_slot;
+            const float *a_all = p.a, *b_all = p.b;
+            float* out_all = p.out;
+            after_earlier_kernels(a_all, b_all, out_all);
+
+            const int64_t unit_begin = p.units * blockIdx.x / gridDim.x, unit_end = p.units * (blockIdx.x + 1) / gridDim.x;
+            const int M = p.M, K = p.K, N = p.N, chunks = (K + KC - 1) / KC;
+            struct Unit
+            {
+                int64_t batch;
+                int m0, first, last; // row of the tile, its column tiles
+            };
+            auto unit_at = [&](int64_t u) {
+                Unit r;
+                const int64_t row_tile = u / p.groups;
+                r.batch = row_tile / p.tiles_m;
+                r.m0 = int(row_tile - r.batch * p.tiles_m) * TM;
+                r.first = int(u - row_tile * p.groups) * p.group;
+                r.last = min(r.first + p.group, p.tiles_n);
+                return r;
+            };
+            int fail = 0;
+
+            if (warp >= EPI_WARPS && warp < MMA_WARP)
+            {
+                asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(WORK_REGS));
+                // ---------------------------------------------------------------- digits
+                // Lane (g, q) takes row / column g of a group of eight and four of every 16 elements of K, so that a warp's store of one plane
+                // is one run of 128 bytes.
+                const int w = warp - EPI_WARPS, g = lane >> 2, q = lane & 3;
+                const uint32_t lane_at = uint32_t(lane) * 4, up16 = uint32_t(p.up16);
+                int a_it = 0, b_it = 0, tile_it = 0;
+                auto load_a = [&](const float* a, int m, int k0, float (&v)[16]) {
+                    const float* at = a + (int64_t(m) * K + k0 + 4 * q);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        load_now4(v + 4 * i, at + 16 * i, m < M && k0 + 16 * i + 4 * q < K);
+                };
+                // (four elements of each of several pieces of 16 of K)
+                auto load_b = [&](const float* b, int n, int k0, auto& v) {
+                    constexpr int PIECES = sizeof(v) / 16;
+                    const float* at = b + (int64_t(k0 + 4 * q) * N + n);
+                    const int64_t step = N;
+                    if (k0 + 16 * PIECES <= K && (n | 7) < N) // (the warp's eight columns)
+                    {
+#pragma unroll
+                        for (int i = 0; i < PIECES; ++i, at += 16 * step)
+                        {
+                            v[4 * i] = load_now(at);
+                            v[4 * i + 1] = load_now(at + step);
+                            v[4 * i + 2] = load_now(at + 2 * step);
+                            v[4 * i + 3] = load_now(at + 3 * step);
+                        }
+                        return;
+                    }
+#pragma unroll
+                    for (int i = 0; i < PIECES; ++i, at += 16 * step)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            v[4 * i + j] = load_now(at + j * step, n < N && k0 + 16 * i + 4 * q + j < K);
+                };
+                auto store = [&](const auto& v, float scale, uint32_t at, uint32_t plane, uint32_t piece) {
+#pragma unroll
+                    for (int i = 0; i < int(sizeof(v)) / 16; ++i)
+                    {
+                        const float x[4] = {v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]};
+                        uint32_t d[PLANES];
+                        four_digits(x, scale, up16, d);
+#pragma unroll
+                        for (int l = 0; l < PLANES; ++l)
+                            sts(at + l * plane + i * piece, d[l]);
+                    }
+                };
+                auto largest = [&](const float (&v)[16]) { // of a row or column: the four lanes of a group together have all of it
+                    float f = 0.0f;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        f = max_magnitude(f, v[i]);
+                    uint32_t m = __float_as_uint(f);
+                    m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, 1));
+                    return max(m, __shfl_xor_sync(0xFFFFFFFFu, m, 2));
+                };
+                auto wait = [&](uint32_t bar, int it, int slots, int code) { // for the slot's use number it / slots to be over
+                    if (!ptx::mbar_wait(bar, ((it / slots) & 1) ^ 1, abortp))
+                        fail = code;
+                    fail = __any_sync(0xFFFFFFFFu, fail != 0) ? code : 0;
+                };
+                auto publish = [&](uint32_t bar) {
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0)
+                        ptx::mbar_arrive(bar);
+                };
+                constexpr uint32_t B_PLANE = SUB * 16, B_PIECE = PLANES * TN * 16, A_PIECE = TM * 16;
+                // column 8 c of B: its accumulator's planes lie together, 32 rows each
+                auto column_at = [](int c) { return uint32_t((c >> 2) * (PLANES * SUB) + 8 * (c & 3)) * 16; };
+                if (!LONG)
+                {
+                    // Warp w makes rows 16 w .. 16 w + 15 of A and columns 8 w .. 8 w + 7 of B.  One group of loads is always under way while the one before it is turned into digits: a column tile of B, and for
+                    // the first of a unit the two groups of rows of A behind it.
+                    const uint32_t a_at = uint32_t(16 * w) * 16 + lane_at, b_at = column_at(w) + lane_at;
+                    float v[16], next[16];
+                    if (unit_begin < unit_end)
+                    {
+                        const Unit r = unit_at(unit_begin);
+                        load_b(b_all + r.batch * K * N, r.first * TN + 8 * w + g, 0, next);
+                    }
+                    auto take_next = [&]() {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i)
+                            v[i] = next[i];
+                    };
+                    for (int64_t u = unit_begin; u < unit_end && !fail; ++u, ++a_it)
+                    {
+                        const Unit r = unit_at(u);
+                        const float* a = a_all + r.batch * M * K;
+                        for (int tn = r.first; tn < r.last && !fail; ++tn, ++b_it, ++tile_it)
+                        {
+                            const int ss = tile_it % S_SLOTS;
+                            auto load_next_b = [&]() {
+                                if (tn + 1 < r.last)
+                                    load_b(b_all + r.batch * K * N, (tn + 1) * TN + 8 * w + g, 0, next);
+                                else if (u + 1 < unit_end)
+                                {
+                                    const Unit f = unit_at(u + 1);
+                                    load_b(b_all + f.batch * K * N, f.first * TN + 8 * w + g, 0, next);
+                                }
+                            };
+                            wait(s_empty(ss), tile_it, S_SLOTS, 5001);
+                            take_next();
+                            if (tn == r.first)
+                                load_a(a, r.m0 + 16 * w + g, 0, next);
+                            else
+                                load_next_b();
+                            {
+                                const uint32_t m = largest(v);
+                                wait(b_empty(b_it % B_SLOTS), b_it, B_SLOTS, 5003);
+                                if (fail)
+                                    break;
+                                if (q == 0)
+                                    b_scale[ss][8 * w + g] = result_scale(m);
+                                store(v, digit_scale(m), b_slot(b_it % B_SLOTS) + b_at, B_PLANE, B_PIECE);
+                                publish(b_full(b_it % B_SLOTS));
+                            }
+                            if (tn == r.first)
+                            {
+                                wait(a_empty(a_it % A_SLOTS), a_it, A_SLOTS, 5002);
+                                if (fail)
+                                    break;
+#pragma unroll
+                                for (int h = 0; h < 2; ++h)
+                                {
+                                    take_next();
+                                    if (h == 0)
+                                        load_a(a, r.m0 + 16 * w + 8 + g, 0, next);
+                                    else
+                                        load_next_b();
+                                    const uint32_t m = largest(v);
+                                    if (q == 0)
+                                        a_scale[a_it % S_SLOTS][16 * w + 8 * h + g] = result_scale(m);
+                                    store(v, digit_scale(m), a_slot(a_it % A_SLOTS) + a_at + 128 * h, A_PLANE, A_PIECE);
+                                }
+                                publish(a_full(a_it % A_SLOTS));
+                            }
+                            __syncwarp();
+                            if (lane == 0)
+                                ptx::mbar_arrive(s_full(ss));
+                        }
+                    }
+                }
+                else
+                {
+                    // Warp w makes rows 8 w .. 8 w + 7 of A and, of columns 8 (w % 8) .. 8 (w % 8) + 7 of B, half of the stage's K
+                    const int half = w >> 3;
+                    const uint32_t a_at = uint32_t(8 * w) * 16 + lane_at, b_at = column_at(w & 7) + uint32_t(2 * half) * B_PIECE + lane_at;
+                    for (int64_t u = unit_begin; u < unit_end && !fail; ++u)
+                    {
+                        const Unit r = unit_at(u);
+                        const float *a = a_all + r.batch * M * K, *b = b_all + r.batch * K * N;
+                        for (int tn = r.first; tn < r.last && !fail; ++tn, ++tile_it)
+                        {
+                            const int m = r.m0 + 8 * w + g, n = tn * TN + 8 * (w & 7) + g, ss = tile_it % S_SLOTS;
+                            float v[16], x[8];
+                            load_a(a, m, 0, v);
+                            load_b(b, n, 32 * half, x);
+                            wait(s_full(ss), tile_it + S_SLOTS /* its use number tile_it / S_SLOTS */, S_SLOTS, 5004);
+                            if (fail)
+                                break;
+                            const float sa = digit_scale(a_max[ss][8 * w + g]), sb = digit_scale(b_max[ss][8 * (w & 7) + g]);
+                            for (int c = 0; c < chunks; ++c, ++a_it, ++b_it)
+                            {
+                                // the next stage's elements are under way while these are turned into digits
+                                float v_next[16], x_next[8];
+                                if (c + 1 < chunks)
+                                {
+                                    load_a(a, m, (c + 1) * KC, v_next);
+                                    load_b(b, n, (c + 1) * KC + 32 * half, x_next);
+                                }
+                                wait(a_empty(a_it % A_SLOTS), a_it, A_SLOTS, 5002);
+                                if (fail)
+                                    break;
+                                store(v, sa, a_slot(a_it % A_SLOTS) + a_at, A_PLANE, A_PIECE);
+                                wait(b_empty(b_it % B_SLOTS), b_it, B_SLOTS, 5003);
+                                if (fail)
+                                    break;
+                                store(x, sb, b_slot(b_it % B_SLOTS) + b_at, B_PLANE, B_PIECE);
+                                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                                __syncwarp();
+                                if (lane == 0)
+                                    ptx::mbar_arrive(a_full(a_it % A_SLOTS)), ptx::mbar_arrive(b_full(b_it % B_SLOTS));
+#pragma unroll
+                                for (int i = 0; i < 16; ++i)
+                                    v[i] = v_next[i];
+#pragma unroll
+                                for (int i = 0; i < 8; ++i)
+                                    x[i] = x_next[i];
+                            }
+                        }
+                    }
+                }
+            }
+            else if (warp >= MMA_WARP)
+            {
+                asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(MMA_REGS));
+                // ---------------------------------------------------------------- MMA issue
+                if (warp == MMA_WARP && ptx::elect_one())
+                {
+                    // kind::i8, signed operands, int32 sums, M = 128
+                    constexpr uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | (uint32_t(TM >> 4) << 24);
+                    auto width = [](int n) { return idesc | uint32_t(n >> 3) << 17; };
+                    int a_it = 0, b_it = 0, tile_it = 0;
+                    for (int64_t u = unit_begin; u < unit_end && !fail; ++u)
+                    {
+                        const Unit r = unit_at(u);
+                        for (int tn = r.first; tn < r.last && !fail; ++tn, ++tile_it)
+                        {
+                            for (int c = 0; c < chunks; ++c, ++b_it)
+                            {
+                                const int as = a_it % A_SLOTS, bs = b_it % B_SLOTS;
+                                if (!ptx::mbar_wait(a_full(as), (a_it / A_SLOTS) & 1, abortp) || !ptx::mbar_wait(b_full(bs), (b_it / B_SLOTS) & 1, abortp))
+                                {
+                                    fail = 5102;
+                                    break;
+                                }
+                                ptx::tc_fence_after_sync();
+                                const int steps = min(KC, K - c * KC) > 32 ? 2 : 1;
+                                const uint64_t a_desc = descriptor(a_slot(as), TM * 16), b_desc = descriptor(b_slot(bs), PLANES * TN * 16);
+#pragma unroll
+                                for (int sub = 0; sub < 2; ++sub)
+                                {
+                                    if (c == 0)
+                                    {
+                                        if (!ptx::mbar_wait(t_empty + 8 * sub, (tile_it & 1) ^ 1, abortp))
+                                        {
+                                            fail = 5101;
+                                            break;
+                                        }
+                                        ptx::tc_fence_after_sync();
+                                    }
+                                    for (int k = 0; k < steps; ++k)
+                                        // digit i of A against digits 0 .. 6 - i of B, which lie side by side as one operand of 32 (7 - i) rows: column
+                                        // block j of the result is sum i + j, 32 columns apart in tensor memory (descriptors count 16 bytes)
+#pragma unroll
+                                        for (int i = 0; i < PLANES; ++i)
+                                            ptx::mma_i8(tmem + ACC_COLS * sub + SUB * i, a_desc + uint64_t(i * (A_PLANE / 16) + k * (2 * TM)),
+                                                        b_desc + uint64_t(sub * (PLANES * SUB) + k * (2 * PLANES * TN)), width(SUB * (PLANES - i)),
+                                                        c > 0 || k > 0 || i > 0 ? 1u : 0u);
+                                    if (c == chunks - 1)
+                                        ptx::mma_commit(t_full + 8 * sub);
+                                }
+                                if (fail)
+                                    break;
+                                ptx::mma_commit(b_empty(bs));
+                                if (LONG || tn + 1 == r.last)
+                                {
+                                    ptx::mma_commit(a_empty(as));
+                                    ++a_it;
+                                }
+                            }
+                        }
+                    }
+                    ptx::mma_commit(drained);
+                    if (!ptx::mbar_wait(drained, 0, abortp) && !fail)
+                        fail = 5103;
+                }
+            }
+            else
+            {
+                asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(WORK_REGS));
+                // ---------------------------------------------------------------- epilogue
+                // A warp reads 16 columns of a TMEM lane quarter: of one of the two accumulators, or (LONG) of both in turn
+                constexpr int PASSES = LONG ? 2 : 1;
+                const int quarter = warp & 3, g = lane >> 2, t = lane & 3;
+                const int eps = p.eps, one = p.one, up8 = p.up8, up16 = p.up16, up24 = p.up24;
+                int tile_it = 0;
+                int64_t scanned_batch = -1;
+                int scanned_tn = -1, scanned_slot = 0;
+                // LONG: the largest magnitudes of tile `it`, of 16 rows and 8 columns per warp (indexes beyond the matrix are pulled back into it:
+                // they repeat an element of the same row or column, or fill rows and columns that are not stored)
+                auto scan = [&](const Unit& r, int tn, int it, int64_t unit) {
+                    const float *a = a_all + r.batch * M * K, *b = b_all + r.batch * K * N;
+                    const int ss = it % S_SLOTS;
+                    constexpr int W = 4, STEP = 32 * W;
+#pragma unroll 1
+                    for (int part = 0; part < 4; ++part)
+                    {
+                        float m[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                        const int row = r.m0 + 16 * warp + 4 * part;
+                        for (int k0 = W * lane; k0 < K + W * lane; k0 += 3 * STEP)
+                        {
+                            float x[4][3][W];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                                for (int j = 0; j < 3; ++j)
+                                {
+                                    const float* at = a + int64_t(min(row + i, M - 1)) * K + (k0 + j * STEP < K ? k0 + j * STEP : 0);
+                                    load_now4(x[i][j], at, true);
+                                }
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                                for (int j = 0; j < 3; ++j)
+#pragma unroll
+                                    for (int e = 0; e < W; ++e)
+                                        m[i] = max_magnitude(m[i], x[i][j][e]);
+                        }
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                        {
+                            const uint32_t bits = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(m[i]));
+                            if (lane == 0)
+                                a_max[ss][16 * warp + 4 * part + i] = bits, a_scale[ss][16 * warp + 4 * part + i] = result_scale(bits);
+                        }
+                    }
+                    // columns: lane takes W of the eight, every (4 W)th row of K; the row tiles of one matrix share them
+                    const int col = 8 * warp;
+                    if (r.batch == scanned_batch && tn == scanned_tn)
+                    {
+                        if (lane < 8)
+                            b_max[ss][col + lane] = b_max[scanned_slot][col + lane], b_scale[ss][col + lane] = b_scale[scanned_slot][col + lane];
+                    }
+                    else
+                    {
+                        const int n = min(tn * TN + col + 4 * (lane & 1), N - 4);
+                        float m[W];
+#pragma unroll
+                        for (int e = 0; e < W; ++e)
+                            m[e] = 0.0f;
+                        for (int k0 = lane / (8 / W); k0 < K + lane / (8 / W); k0 += 12 * 4 * W)
+                        {
+                            float x[12][W];
+#pragma unroll
+                            for (int j = 0; j < 12; ++j)
+                            {
+                                const float* at = b + int64_t(min(k0 + j * 4 * W, K - 1)) * N + n;
+                                load_now4(x[j], at, true);
+                            }
+#pragma unroll
+                            for (int j = 0; j < 12; ++j)
+#pragma unroll
+                                for (int e = 0; e < W; ++e)
+                                    m[e] = max_magnitude(m[e], x[j][e]);
+                        }
+#pragma unroll
+                        for (int e = 0; e < W; ++e)
+                        {
+                            uint32_t bits = __float_as_uint(m[e]);
+#pragma unroll
+                            for (int d = 8 / W; d < 32; d *= 2)
+                                bits = max(bits, __shfl_xor_sync(0xFFFFFFFFu, bits, d));
+                            if (lane < 8 / W)
+                                b_max[ss][col + W * lane + e] = bits, b_scale[ss][col + W * lane + e] = result_scale(bits);
+                        }
+                    }
+                    scanned_batch = r.batch, scanned_tn = tn, scanned_slot = ss;
+                    if (tn + 1 == r.last && unit + 1 < unit_end)
+                    {
+                        const Unit f = unit_at(unit + 1);
+                        const char* rows = reinterpret_cast<const char*>(a_all + (f.batch * M + f.m0) * K);
+                        const int64_t bytes = int64_t(min(TM, M - f.m0)) * K * 4;
+                        for (int64_t i = int64_t(threadIdx.x) * 128; i < bytes; i += EPI_WARPS * 32 * 128)
+                            asm volatile("prefetch.global.L2 [%0];" ::"l"(rows + i));
+                    }
+                    __syncwarp();
+                    if (lane == 0)
+                        ptx::mbar_arrive(s_full(ss));
+                };
+                if (LONG && unit_begin < unit_end)
+                {
+                    const Unit r = unit_at(unit_begin);
+                    scan(r, r.first, 0, unit_begin);
+                }
+                int unit_it = 0;
+                for (int64_t u = unit_begin; u < unit_end && !fail; ++u, ++unit_it)
+                {
+                    const Unit r = unit_at(u);
+                    float* out = out_all + r.batch * M * N;
+                    for (int tn = r.first; tn < r.last && !fail; ++tn, ++tile_it)
+                    {
+                        const int ss = tile_it % S_SLOTS;
+                        if (LONG)
+                        {
+                            // four slots: whoever is here has seen tile tile_it - 1 complete, for which all had finished with tile tile_it - 3, whose
+                            // magnitudes are overwritten
+                            if (tn + 1 < r.last)
+                                scan(r, tn + 1, tile_it + 1, u);
+                            else if (u + 1 < unit_end)
+                            {
+                                const Unit f = unit_at(u + 1);
+                                scan(f, f.first, tile_it + 1, u + 1);
+                            }
+                        }
+                        if (!ptx::mbar_wait(s_full(ss), (tile_it / S_SLOTS) & 1, abortp))
+                            fail = 5202;
+                        const int m_w = r.m0 + quarter * 32;
+#pragma unroll 1
+                        for (int pass = 0; pass < PASSES; ++pass)
+                        {
+                            const int acc = LONG ? pass : warp >> 3, col_acc = 16 * ((warp >> 2) & 1), col = acc * SUB + col_acc, n_w = tn * TN + col;
+                            if (!ptx::mbar_wait(t_full + 8 * acc, tile_it & 1, abortp))
+                                fail = 5201;
+                            fail = __any_sync(0xFFFFFFFFu, fail != 0) ? 5201 : 0;
+                            if (fail)
+                                break;
+                            ptx::tc_fence_after_sync();
+                            long long v[2][8]; // V - eps, of rows 0 .. 15 and 16 .. 31
+#pragma unroll
+                            for (int h = 0; h < 2; ++h)
+                            {
+                                const uint32_t at = tmem + (uint32_t(quarter * 32 + 16 * h) << 16) + uint32_t(ACC_COLS * acc + col_acc);
+                                int d[3][8], e[2][8];
+#pragma unroll
+                                for (int s = 0; s < 3; ++s)
+                                    tmem_ld_16x16(at + SUB * (4 + s), d[s]);
+#pragma unroll
+                                for (int s = 0; s < 3; ++s)
+                                    tmem_wait(d[s]);
+#pragma unroll
+                                for (int i = 0; i < 8; ++i)
+                                    v[h][i] = mad_wide(d[0][i], up8, mad_wide(d[1][i] + (d[2][i] >> 8) - eps, one, 0));
+#pragma unroll
+                                for (int s = 0; s < 4; s += 2)
+                                {
+                                    tmem_ld_16x16(at + SUB * s, e[0]);
+                                    tmem_ld_16x16(at + SUB * (s + 1), e[1]);
+                                    tmem_wait(e[0]);
+                                    tmem_wait(e[1]);
+#pragma unroll
+                                    for (int i = 0; i < 8; ++i)
+                                        if (s == 0)
+                                            v[h][i] += static_cast<long long>(static_cast<unsigned long long>(uint32_t(e[0][i] * up8 + e[1][i])) << 32);
+                                        else
+                                            v[h][i] = mad_wide(e[0][i], up24, mad_wide(e[1][i], up16, v[h][i]));
+                                }
+                            }
+                            ptx::tc_fence_before_sync();
+                            __syncwarp();
+                            if (lane == 0)
+                                ptx::mbar_arrive(t_empty + 8 * acc);
+                            float fa[4], fb[4];
+                            const int sa = LONG ? ss : unit_it % S_SLOTS;
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                            {
+                                fa[i] = a_scale[sa][quarter * 32 + 8 * i + g];
+                                fb[i] = b_scale[ss][col + 8 * (i >> 1) + 2 * t + (i & 1)];
+                            }
+                            if (!LONG)
+                            {
+                                __syncwarp();
+                                if (lane == 0)
+                                    ptx::mbar_arrive(s_empty(ss));
+                            }
+                            float doubt[4][2]; // not 0 where one of a pair is not settled
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) // rows 8 i .. 8 i + 7 of the warp's 32
+                            {
+                                const int m = m_w + 8 * i + g;
+                                float* row = out + (int64_t(m) * N + n_w + 2 * t);
+#pragma unroll
+                                for (int j = 0; j < 2; ++j)
+                                {
+                                    const int n = n_w + 8 * j + 2 * t;
+                                    float o[2], apart[2];
+#pragma unroll
+                                    for (int c = 0; c < 2; ++c)
+                                    {
+                                        const long long x = v[i >> 1][4 * j + 2 * (i & 1) + c];
+                                        const float lo = __ll2float_rn(x), hi = __ll2float_rn(mad_wide(eps, 2 * one, x));
+                                        o[c] = hi * (fa[i] * fb[2 * j + c]);
+                                        apart[c] = hi - lo;
+                                    }
+                                    doubt[i][j] = apart[0] + apart[1]; // (neither is negative)
+                                    if (m < M && n < N)
+                                        *reinterpret_cast<float2*>(row + 8 * j) = make_float2(o[0], o[1]);
+                                }
+                            }
+                            // where every product of the scales lies between these, a V that is settled (so not 0) gives a normal number
+                            // (an empty row's 0 and a NaN fail)
+                            constexpr float LEAST = 1.17549435e-38f, MOST = 1.8446744e19f;
+                            const float least = fminf(fminf(fa[0], fa[1]), fminf(fa[2], fa[3])) * fminf(fminf(fb[0], fb[1]), fminf(fb[2], fb[3]));
+                            const float most = fmaxf(fmaxf(fa[0], fa[1]), fmaxf(fa[2], fa[3])) * fmaxf(fmaxf(fb[0], fb[1]), fmaxf(fb[2], fb[3]));
+                            const float all = fa[0] + fa[1] + fa[2] + fa[3] + fb[0] + fb[1] + fb[2] + fb[3];
+                            const float doubts = ((doubt[0][0] + doubt[0][1]) + (doubt[1][0] + doubt[1][1])) + ((doubt[2][0] + doubt[2][1]) + (doubt[3][0] + doubt[3][1]));
+                            if (!__all_sync(0xFFFFFFFFu, doubts == 0.0f && least >= LEAST && most <= MOST && all <= 3.40282347e38f))
+                            {
+                                uint32_t marked = 0;
+#pragma unroll
+                                for (int i = 0; i < 8; ++i)
+                                {
+                                    const float f = fa[i >> 1], h0 = fb[2 * (i & 1)], h1 = fb[2 * (i & 1) + 1];
+                                    const bool plain = f * fminf(h0, h1) >= LEAST && f * fmaxf(h0, h1) <= MOST && f + h0 + h1 <= 3.40282347e38f;
+                                    // an empty row or two empty columns: 0 (or the NaN that it is)
+                                    if (!(plain && doubt[i >> 1][i & 1] == 0.0f) && f != 0.0f && (h0 != 0.0f || h1 != 0.0f) && m_w + 8 * (i >> 1) + g < M &&
+                                        n_w + 8 * (i & 1) + 2 * t < N)
+                                        marked |= 1u << i;
+                                }
+                                if (__any_sync(0xFFFFFFFFu, marked != 0))
+                                    leave_or_settle(queue, &queued, a_all, b_all, out_all, M, K, N, int(r.batch), m_w, n_w, marked);
+                            }
+                        }
+                    }
+                }
+            }
+            if (fail)
+                *abortp = 1;
+            if (fail && p.status)
+                atomicCAS(p.status, 0, fail);
+            ptx::tc_fence_before_sync();
+            __syncthreads();
+            if (warp == MMA_WARP)
+                ptx::tmem_dealloc(tmem, TMEM_COLS);
+            // nothing reads the digits any more: their memory takes the products
+            if (warp < WORK_WARPS && !abort_flag)
+                for (int i = warp; i < min(queued, QUEUE); i += WORK_WARPS)
+                {
+                    const int4 at = queue[i];
+                    if (at.x >= 0)
+                        pair_in_order(a_all + int64_t(at.x) * M * K, b_all + int64_t(at.x) * K * N, out_all + int64_t(at.x) * M * N, K, N, at.y, at.z,
+                                      reinterpret_cast<double2*>(raw + (base - ptx::smem_u32(raw)) + warp * 4096));
+                }
+        }
+    }
+
+    // What the form takes: matrices that 16-byte loads may walk (it is no faster otherwise), sums that fit 64 bits.
+    bool bmm_digits_accepts(int64_t batch, int64_t M, int64_t K, int64_t N, bool vec)
+    {
+        using namespace digits;
+        return vec && K >= 1 && K <= MAX_K && batch <= 0x7FFFFFFF && batch * ((M + TM - 1) / TM) * ((N + TN - 1) / TN) < 0x7FFFFFFF;
+    }
+
+    // Column tiles of a unit of work: they share the digits of its row tile when K <= KC, as long as the units still go around.
+    static int64_t bmm_digits_group(int64_t row_tiles, int64_t tiles_n, int64_t K)
+    {
+        return K <= digits::KC ? std::max<int64_t>(1, std::min<int64_t>(tiles_n, row_tiles * tiles_n / (4 * sm_count()))) : 1;
+    }
+
+    // Estimated time in us, from whole rounds of units over the SMs: 3.3 us per column tile and 2.3 per row tile, or (K > KC) 11 per tile and
+    // 2 per stage of K (the epilogue's warps make a pass over the operands there).  Within 10 % at 25 shapes; measured against the panels
+    // form, us: 768 x [384, 64] x [64, 384] 363 (478), 768 x [384, 384] x [384, 64] 368 (456; probabilities 394), 120 x [384, 64] x [64, 384]
+    // 69 (80), 384 x [256, 64] x [64, 256] 101 (108), 768 x [200, 64] x [64, 200] 170 (163), 768 x [128, 128] x [128, 64] 92 (63).
+    double bmm_digits_us(int64_t batch, int64_t M, int64_t K, int64_t N)
+    {
+        using namespace digits;
+        const int64_t row_tiles = batch * ((M + TM - 1) / TM), tiles_n = (N + TN - 1) / TN, group = bmm_digits_group(row_tiles, tiles_n, K);
+        const int64_t units = row_tiles * ((tiles_n + group - 1) / group), rounds = (units + sm_count() - 1) / sm_count();
+        return 8.0 + double(rounds) * (K <= KC ? 2.3 + 3.3 * double(group) : 11.0 + 2.05 * double((K + KC - 1) / KC));
+    }
+
+    int launch_bmm_digits(const float* a, const float* b, float* out, int64_t batch, int M, int K, int N, cudaStream_t st)
+    {
+        using namespace digits;
+        Params p;
+        p.a = a, p.b = b, p.out = out, p.status = contract_status_address();
+        p.M = M, p.K = K, p.N = N;
+        p.tiles_m = (M + TM - 1) / TM, p.tiles_n = (N + TN - 1) / TN;
+        p.eps = 2 * K + 2;
+        p.one = 1, p.up8 = 1 << 8, p.up16 = 1 << 16, p.up24 = 1 << 24;
+        const int64_t row_tiles = batch * p.tiles_m;
+        p.group = int(bmm_digits_group(row_tiles, p.tiles_n, K));
+        p.groups = (p.tiles_n + p.group - 1) / p.group;
+        p.units = row_tiles * p.groups;
+        const unsigned grid = unsigned(std::min<int64_t>(p.units, sm_count()));
+        static std::atomic<uint64_t> told{0};
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (!((told.load(std::memory_order_relaxed) >> (dev & 63)) & 1))
+        {
+            for (auto kernel : {bmm_digits_kernel<false>, bmm_digits_kernel<true>})
+                if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SHARED); e != cudaSuccess)
+                    return cuda_status(e, "b200_bmm_f32");
+            told.fetch_or(uint64_t(1) << (dev & 63), std::memory_order_relaxed);
+        }
+        launch(K <= KC ? bmm_digits_kernel<false> : bmm_digits_kernel<true>, grid, THREADS, SHARED, st, p);
+        return after_launch("b200_bmm_f32");
+    }
+}

@@ -20,6 +20,7 @@
 #include <math.h>
 #include <algorithm>
 #include <initializer_list>
+#include "bmm.cuh"
 #include "common.cuh"
 #include "rounded_math.cuh"
 
@@ -1082,11 +1083,6 @@ namespace b200
     {
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
     }
-    __device__ __forceinline__ void dmma(double (&c)[2], double a, double b)
-    {
-        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
-    }
-
     template <int WM, int WN, int MT, int NT, bool VEC>
     __global__ void __launch_bounds__(WM* WN * 32) bmm_f32_kernel(const float* __restrict__ a, const float* __restrict__ bm, float* __restrict__ out,
                                                                   int M, int K, int N, uint32_t tiles_m, uint32_t tiles_n)
@@ -1713,7 +1709,11 @@ extern "C" int b200_bmm_f32(const float* a, const float* b, float* out, int64_t 
     const double big = Big::cost(batch, M, N), mid = Mid::cost(batch, M, N), small = Small::cost(batch, M, N);
     const bool is_big = big <= mid && big <= small, is_mid = !is_big && mid <= small, vec = K % 4 == 0 && N % 4 == 0 && all_aligned16({a, b, out});
     const int64_t blocks = is_big ? Big::tiles(batch, M, N) : is_mid ? Mid::tiles(batch, M, N) : Small::tiles(batch, M, N);
-    if (K > 0x7FFFFF00 /* where the panels' counters end */ || bmm_small_us(batch, M, K, N) < bmm_panels_us(blocks, K, vec, !is_big && !is_mid, !is_big))
+    const double small_us = bmm_small_us(batch, M, K, N), panels_us = bmm_panels_us(blocks, K, vec, !is_big && !is_mid, !is_big);
+    // the digit form where it gains more than the estimates are off
+    if (bmm_digits_accepts(batch, M, K, N, vec) && bmm_digits_us(batch, M, K, N) < 0.95 * std::min(small_us, panels_us))
+        return launch_bmm_digits(a, b, out, batch, int(M), int(K), int(N), st);
+    if (K > 0x7FFFFF00 /* where the panels' counters end */ || small_us < panels_us)
     {
         const int64_t tiles = batch * ((M + 3) / 4) * ((N + 3) / 4);
         launch(bmm_small_kernel, grid_for(tiles, 128), 128, 0, st, a, b, out, batch, int(M), int(K), int(N));

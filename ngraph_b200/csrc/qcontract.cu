@@ -35,6 +35,7 @@
 #include <set>
 #include <type_traits>
 #include <unordered_map>
+#include "bmm.cuh"
 #include "common.cuh"
 #include "ptx.cuh"
 
@@ -2449,6 +2450,23 @@ extern "C" __attribute__((visibility("default"))) int b200_debug_wait_cycles(lon
     return 0;
 }
 #endif
+
+int* b200::contract_status_address()
+{
+    static std::atomic<int*> of_device[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64)
+        return nullptr;
+    int* p = of_device[dev].load(std::memory_order_relaxed);
+    if (!p)
+    {
+        void* q = nullptr;
+        if (cudaGetSymbolAddress(&q, g_contract_status) != cudaSuccess)
+            return nullptr;
+        of_device[dev].store(p = static_cast<int*>(q), std::memory_order_relaxed);
+    }
+    return p;
+}
 
 extern "C" int b200_device_status(int* status_out)
 {

@@ -285,6 +285,40 @@ def test_bmm_tile_edges(L, batch, m, k, n):
     np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(acc.astype(np.float32)))
 
 
+@pytest.mark.parametrize("batch,m,k,n", [(200, 384, 64, 384), (230, 380, 64, 388), (160, 384, 384, 64), (170, 381, 324, 64), (14, 512, 516, 520)])
+def test_bmm_of_large_matrices(L, batch, m, k, n):
+    """shapes of the digit form, tiles and stages of K that end early among them: the bits of the sum in double, in k order, for values of
+    one size and for those that the digits do not settle (sizes far apart, sums that cancel, empty rows and columns, denormal and
+    overflowing results, infinities and NaN)"""
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+
+    def rand(*shape):
+        return torch.randn(shape, generator=g, device="cuda")
+
+    a, b = rand(batch, m, k), rand(batch, k, n)
+    a[1] = torch.softmax(4 * a[1], dim=-1)
+    a[2], b[2] = a[2] * torch.exp(12 * rand(m, k)), b[2] * torch.exp(12 * rand(k, n))
+    a[3], b[3] = (10 * a[3]).round(), (10 * b[3]).round()
+    a[4] *= (torch.rand((m, k), generator=g, device="cuda") < 0.05)
+    b[4] *= (torch.rand((k, n), generator=g, device="cuda") < 0.05)
+    a[5, ::3], b[5, :, ::5] = 0.0, 0.0
+    a[6, :, 1::2] = -a[6, :, 0::2][:, : k // 2]
+    b[6, 1::2] = b[6, 0::2][: k // 2] * (1 + 1e-6 * rand(k // 2, n))
+    a[7] *= 1e-40
+    a[8], b[8] = a[8] * 1e-30, b[8] * 1e-12
+    a[9], b[9] = a[9] * 1e30, b[9] * 1e8
+    a[10, 5, 7], a[10, 200, 3], b[10, 9, 60], b[10, 11, 3] = float("nan"), float("inf"), -float("inf"), float("nan")
+    acc = torch.zeros((batch, m, n), dtype=torch.float64, device="cuda")
+    for kk in range(k):
+        acc += a[:, :, kk, None].double() * b[:, kk, None, :].double()  # the product of two floats is exact
+    out = torch.full((batch, m, n), 7.0, device="cuda")
+    L.check(L.LIB.b200_bmm_f32(a.data_ptr(), b.data_ptr(), out.data_ptr(), batch, m, k, n, stream()), "bmm")
+    want, nan = acc.float(), torch.isnan(acc)
+    assert torch.equal(torch.isnan(out), nan)
+    assert torch.equal(out.view(torch.int32)[~nan], want.view(torch.int32)[~nan])
+    L.device_status()  # no wait gave up
+
+
 @pytest.mark.parametrize("n", [1, 3, 1023, 65535, 65536, (1 << 19) - 1, 1 << 19, (1 << 19) + 1, (1 << 20) - 1, 1 << 20, (1 << 20) + 1, 3000001])
 def test_extremes_of_a_whole_tensor(L, n):
     """Max, Min and Max over Abs of every element: the cluster form and the atomic form, runs that do not start on 16 bytes,
