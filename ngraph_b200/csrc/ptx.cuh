@@ -304,6 +304,14 @@ namespace b200
                          : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]),
                            "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
         }
+        // 16 lanes x 16 columns (the 16x256b shape twice) into registers `at` .. `at` + 7: 4j .. 4j + 3 as in tmem_ld_16x32
+        __device__ __forceinline__ void tmem_ld_16x16(uint32_t taddr, uint32_t (&r)[16], const int at)
+        {
+            asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                         : "=r"(r[at]), "=r"(r[at + 1]), "=r"(r[at + 2]), "=r"(r[at + 3]), "=r"(r[at + 4]), "=r"(r[at + 5]), "=r"(r[at + 6]), "=r"(r[at + 7])
+                         : "r"(taddr)
+                         : "memory");
+        }
         __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
         // Shared-memory matrix descriptor for a K-major operand tile whose rows are `row_bytes`

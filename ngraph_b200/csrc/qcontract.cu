@@ -127,6 +127,8 @@ namespace b200
                              // as long (free -> landed takes 3 us per 32 KB stage, six stages per 4 us).  Never chosen; the
                              // variant is compiled into instrumented builds only, which can force it.
         int late_successor;  // the stream's next kernel is let in when this one is about done (otherwise: at once)
+        int one_shot;        // one tile of 64 columns, or a part of its reduction, per CTA (see below)
+        int rows;            // rows of a tile: BM, or 64 in one-shot launches (the MMA's other 64 rows compute on what lies there)
         int split;           // CTAs that share one tile's reduction (a thread-block cluster), 1: none
         void* out;
         uint32_t idesc;
@@ -502,6 +504,7 @@ namespace b200
     constexpr int MAX_SPLIT = 8;
     constexpr int SPLIT_EXCHANGE_BYTES = BM * 64 * 4;  // the parts a CTA receives: split x (64 / split) columns x 128 rows
     constexpr int SPLIT_SMEM_LIMIT = 112 * 1024;       // two CTAs per SM
+    constexpr int ONE_SHOT_STAGED_BYTES = EPI_WARPS * 128; // scales and biases of each warp's 16 columns
 
     // The way out for a CTA whose waits gave up, by all its threads.  Otherwise a CTA leaves when every part has landed and nothing
     // writes to it any more; here parts may still be on their way.  The barrier counts the cluster's threads that have not left:
@@ -517,6 +520,81 @@ namespace b200
         __syncthreads();
     }
 
+    // Row `row` of a one-shot tile: its offset in the result, whether it is inside; returns the column tile.
+    __device__ __forceinline__ int row_of_tile(const ContractParams& p, int tile, int row, bool& valid, int64_t& off)
+    {
+        int tm, tn, q0, p0, n0;
+        decode_tile(p, tile, tm, tn, q0, p0, n0);
+        if (p.conv) // the patch's extents are powers of two
+        {
+            const int w = __ffs(p.RW) - 1, h = __ffs(p.TH) - 1;
+            const int q = q0 + (row & (p.RW - 1)), pp = p0 + ((row >> w) & (p.TH - 1)), n = n0 + (row >> (w + h));
+            valid = row < p.rows && q < p.Q && pp < p.P && n < p.NB;
+            off = ((int64_t(n) * p.P + pp) * p.Q + q) * p.N;
+        }
+        else
+        {
+            const int m = tm * p.rows + row;
+            valid = row < p.rows && m < p.M;
+            off = int64_t(m) * p.N;
+        }
+        return tn;
+    }
+
+    // Four columns of a row, of any contract and type, from their accumulators to memory (element offset `at`, `cols` columns inside;
+    // `aligned`: four results may be stored at once).
+    __device__ __forceinline__ void finish_quad(const ContractParams& p, int (&v)[4], const float (&scale)[4], const int (&bias)[4], const uint32_t (&sum)[4],
+                                                float sum_scale, int64_t at, int cols, bool aligned, bool valid)
+    {
+        const bool one_byte = p.out_type == B200_U8 || p.out_type == B200_I8;
+        uint32_t bytes = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+        {
+            if (p.half_away == 1)
+                v[i] = int(epilogue_core(p, v[i], scale[i]));
+            else if (p.half_away == 0)
+            {
+                float f = __fmul_rn(__int2float_rn(v[i] + bias[i]), scale[i]);
+                if (p.sum_in)
+                    f = __fadd_rn(f, __fmul_rn(sum_scale, p.sum_type == B200_U8 ? float(sum[i]) : float(int8_t(sum[i]))));
+                if (p.relu)
+                    f = fmaxf(f, 0.0f);
+                if (p.out_type == B200_F32)
+                    v[i] = __float_as_int(f);
+                else if (p.out_type == B200_I32)
+                    v[i] = clamp_cast<int32_t>(round_quant<B200_ROUND_NEAREST_TOWARD_EVEN>(f));
+                else
+                    v[i] = min(max(__float2int_rn(f), p.out_type == B200_U8 ? 0 : -128), p.out_type == B200_U8 ? 255 : 127);
+            }
+            bytes |= (uint32_t(v[i]) & 0xFFu) << (8 * i);
+        }
+        if (!valid)
+            return;
+        if (one_byte)
+        {
+            uint8_t* o = static_cast<uint8_t*>(p.out) + at;
+            if (aligned && cols >= 4)
+                *reinterpret_cast<uint32_t*>(o) = bytes;
+            else
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (i < cols)
+                        o[i] = uint8_t(bytes >> (8 * i));
+        }
+        else
+        {
+            int* o = static_cast<int*>(p.out) + at;
+            if (aligned && cols >= 4)
+                *reinterpret_cast<int4*>(o) = make_int4(v[0], v[1], v[2], v[3]);
+            else
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (i < cols)
+                        o[i] = v[i];
+        }
+    }
+
     __device__ __forceinline__ void split_epilogue(const ContractParams& p, int tile, int rank, int warp, int lane, uint32_t tmem_base, uint32_t exchange,
                                                    uint32_t tfull, uint32_t landed, volatile int* abortp, int& fail)
     {
@@ -524,6 +602,7 @@ namespace b200
         const int row = quarter * 32 + lane, split_log2 = __ffs(p.split) - 1;
         const int quads = 16 >> split_log2; // groups of four columns this CTA finishes; thread: quads group, group + 4, ...
         const uint32_t remote0 = exchange + uint32_t(rank) * uint32_t(quads) * (BM * 16) + uint32_t(row) * 16;
+        const bool rows_here = quarter * 32 < p.rows; // warp-uniform
         if (!__all_sync(0xffffffffu, ptx::mbar_wait(tfull, 0, abortp, 0)))
             fail = 3001;
         ptx::tc_fence_after_sync();
@@ -533,7 +612,7 @@ namespace b200
             ptx::tmem_ld_wait();
             ptx::cluster_wait(); // every CTA of the cluster runs, its barrier is initialised
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
+            for (int j = 0; rows_here && j < 4; ++j)
             {
                 // [part's rank][quad][row], 16 bytes each: a warp's store is 512 contiguous bytes
                 const int quad = group * 4 + j, owner = quad / quads;
@@ -541,22 +620,9 @@ namespace b200
                 ptx::store_async(ptx::mapa(dst, uint32_t(owner)), v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3], ptx::mapa(landed, uint32_t(owner)));
             }
         }
-        int tm, tn, q0, p0, n0;
-        decode_tile(p, tile, tm, tn, q0, p0, n0);
         bool valid;
         int64_t off;
-        if (p.conv) // the patch's extents are powers of two
-        {
-            const int w = __ffs(p.RW) - 1, h = __ffs(p.TH) - 1;
-            const int q = q0 + (row & (p.RW - 1)), pp = p0 + ((row >> w) & (p.TH - 1)), n = n0 + (row >> (w + h));
-            valid = q < p.Q && pp < p.P && n < p.NB;
-            off = ((int64_t(n) * p.P + pp) * p.Q + q) * p.N;
-        }
-        else
-        {
-            valid = tm * BM + row < p.M;
-            off = int64_t(tm * BM + row) * p.N;
-        }
+        const int tn = row_of_tile(p, tile, row, valid, off);
         const int first = tn * 64 + rank * quads * 4; // first column finished here
         const bool one_byte = p.out_type == B200_U8 || p.out_type == B200_I8;
         const bool aligned = p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out) & (one_byte ? 3 : 15)) == 0;
@@ -564,9 +630,10 @@ namespace b200
         const float* const scales = ordered(p.scale);
         const int32_t* const biases = ordered(p.bias);
         const uint8_t* const residual = ordered(static_cast<const uint8_t*>(p.sum_in));
+        const bool sum_words = p.sum_in && p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(p.sum_in) & 3) == 0;
         bool waited = false;
 #pragma unroll 1
-        for (int quad = group; quad < quads; quad += 4)
+        for (int quad = group; rows_here && quad < quads; quad += 4)
         {
             const int col = first + 4 * quad, cols = p.N - col; // may be <= 0
             float scale[4];
@@ -577,7 +644,14 @@ namespace b200
             {
                 scale[i] = i < cols && p.scale ? __ldg(scales + (p.scale_per_channel ? col + i : 0)) : 0.0f;
                 bias[i] = i < cols && p.bias ? __ldg(biases + col + i) : 0;
-                sum[i] = i < cols && valid && p.sum_in ? residual[off + col + i] : 0;
+                sum[i] = !sum_words && i < cols && valid && p.sum_in ? residual[off + col + i] : 0;
+            }
+            if (sum_words && valid && cols > 0) // (the width is a multiple of 4)
+            {
+                const uint32_t four = *reinterpret_cast<const uint32_t*>(residual + off + col);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    sum[i] = (four >> (8 * i)) & 0xFFu;
             }
             if (!waited && !__all_sync(0xffffffffu, ptx::mbar_wait<true>(landed, 0, abortp, 0)))
                 fail = 3002;
@@ -590,56 +664,97 @@ namespace b200
                 const int4 w = lds_i4(part + uint32_t(r) * uint32_t(quads) * (BM * 16));
                 v[0] += w.x, v[1] += w.y, v[2] += w.z, v[3] += w.w;
             }
-            uint32_t bytes = 0;
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-            {
-                if (p.half_away == 1)
-                    v[i] = int(epilogue_core(p, v[i], scale[i]));
-                else if (p.half_away == 0)
-                {
-                    float f = __fmul_rn(__int2float_rn(v[i] + bias[i]), scale[i]);
-                    if (p.sum_in)
-                        f = __fadd_rn(f, __fmul_rn(sum_scale, p.sum_type == B200_U8 ? float(sum[i]) : float(int8_t(sum[i]))));
-                    if (p.relu)
-                        f = fmaxf(f, 0.0f);
-                    if (p.out_type == B200_F32)
-                        v[i] = __float_as_int(f);
-                    else if (p.out_type == B200_I32)
-                        v[i] = clamp_cast<int32_t>(round_quant<B200_ROUND_NEAREST_TOWARD_EVEN>(f));
-                    else
-                        v[i] = min(max(__float2int_rn(f), p.out_type == B200_U8 ? 0 : -128), p.out_type == B200_U8 ? 255 : 127);
-                }
-                bytes |= (uint32_t(v[i]) & 0xFFu) << (8 * i);
-            }
-            if (!valid)
-                continue;
-            if (one_byte)
-            {
-                uint8_t* o = static_cast<uint8_t*>(p.out) + off + col;
-                if (aligned && cols >= 4)
-                    *reinterpret_cast<uint32_t*>(o) = bytes;
-                else
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (i < cols)
-                            o[i] = uint8_t(bytes >> (8 * i));
-            }
-            else
-            {
-                int* o = static_cast<int*>(p.out) + off + col;
-                if (aligned && cols >= 4)
-                    *reinterpret_cast<int4*>(o) = make_int4(v[0], v[1], v[2], v[3]);
-                else
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (i < cols)
-                            o[i] = v[i];
-            }
+            finish_quad(p, v, scale, bias, sum, sum_scale, off + col, cols, aligned, valid);
         }
         // a warp without a quad of its own leaves only when every part has landed: the senders' stores need this CTA's memory
         if (!waited && !__all_sync(0xffffffffu, ptx::mbar_wait<true>(landed, 0, abortp, 0)))
             fail = 3002;
+    }
+
+    // One-shot launches (few tiles of 64 columns, one per CTA): the whole reduction in one CTA.  Such a launch waits for everything in
+    // turn, so all 16 warps share the tile (16 columns of 32 rows each; the persistent kernels leave it to four) and write their
+    // results straight from registers.  (Two accumulators in turn for the k-steps made no difference to their rate.)
+    template <int SUM>
+    __device__ __forceinline__ void one_shot_bytes(const ContractParams& p, const uint32_t (&v)[16], uint32_t (&w)[4], uint32_t sc, uint32_t bi,
+                                                   const uint32_t (&sumw)[4], float sum_scale)
+    {
+        const uint32_t sum_flip = p.sum_type == B200_U8 ? 0u : 0x80808080u;
+        const float sum_magic = p.sum_type == B200_U8 ? 8388608.0f : 8388736.0f;
+        if (p.out_type == B200_U8)
+            epilogue_chunk_bytes<SUM, false, true>(v, w, sc, bi, sumw, sum_scale, sum_flip, sum_magic, p.one);
+        else if (p.relu)
+            epilogue_chunk_bytes<SUM, true, false>(v, w, sc, bi, sumw, sum_scale, sum_flip, sum_magic, p.one);
+        else
+            epilogue_chunk_bytes<SUM, false, false>(v, w, sc, bi, sumw, sum_scale, sum_flip, sum_magic, p.one);
+    }
+    __device__ __forceinline__ void one_shot_epilogue(const ContractParams& p, int tile, int warp, int lane, uint32_t tmem_base, uint32_t staged, uint32_t tfull, volatile int* abortp,
+                                                      int& fail)
+    {
+        const int quarter = warp & 3, group = (warp - 4) >> 2; // accumulator rows 32 * quarter .. + 31, columns 16 * group .. + 15
+        bool valid;
+        int64_t off;
+        const int col = row_of_tile(p, tile, quarter * 32 + lane, valid, off) * 64 + group * 16, cols = p.N - col;
+        if (quarter * 32 >= p.rows || cols <= 0)
+            return; // warp-uniform; the first warp of the first group always has work, so the CTA stays until its products are complete
+        const bool one_byte = p.out_type == B200_U8 || p.out_type == B200_I8;
+        const float sum_scale = p.sum_in ? __ldg(ordered(p.sum_scale)) : 0.0f;
+        const uint32_t sc = staged + uint32_t(warp - 4) * 128, bi = sc + 64;
+        if (lane < 16)
+        {
+            const float scale = lane < cols ? __ldg(ordered(p.scale) + (p.scale_per_channel ? col + lane : 0)) : 0.0f;
+            const int32_t bias = lane < cols && p.bias ? __ldg(ordered(p.bias) + col + lane) : 0;
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(sc + 4 * lane), "f"(scale) : "memory");
+            asm volatile("st.shared.b32 [%0], %1;" ::"r"(bi + 4 * lane), "r"(bias) : "memory");
+        }
+        uint4 sum = make_uint4(0, 0, 0, 0);
+        if (valid && p.sum_in)
+            sum = *reinterpret_cast<const uint4*>(ordered(static_cast<const uint8_t*>(p.sum_in)) + off + col);
+        if (!__all_sync(0xffffffffu, ptx::mbar_wait(tfull, 0, abortp, 0)))
+        {
+            fail = 3001;
+            return;
+        }
+        ptx::tc_fence_after_sync();
+        __syncwarp(); // the staged scales and biases
+        const uint32_t t_addr = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(group) * 16;
+        uint32_t v[16];
+        if (one_byte)
+        {
+            ptx::tmem_ld_32x16(t_addr, v);
+            ptx::tmem_ld_wait(v);
+            uint32_t w[4];
+            const uint32_t sumw[4] = {sum.x, sum.y, sum.z, sum.w};
+            if (p.sum_in)
+                one_shot_bytes<2>(p, v, w, sc, bi, sumw, sum_scale);
+            else
+                one_shot_bytes<0>(p, v, w, sc, bi, sumw, sum_scale);
+            if (valid)
+                *reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.out) + off + col) = make_uint4(w[0], w[1], w[2], w[3]);
+            return;
+        }
+        // f32: four lanes hold eight neighbouring columns of a row, a store writes whole sectors of eight rows
+        const int g = lane >> 2, pair_col = 2 * (lane & 3);
+        const uint32_t rows_ok = __ballot_sync(0xffffffffu, valid) >> g;
+        ptx::tmem_ld_16x16(t_addr, v, 0);
+        ptx::tmem_ld_16x16(t_addr + (16u << 16), v, 8);
+        ptx::tmem_ld_wait(v);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) // rows g + 8 i
+        {
+            float* const o = static_cast<float*>(p.out) + __shfl_sync(0xffffffffu, static_cast<long long>(off), g + 8 * i) + col + pair_col;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) // columns 8 j + pair_col and the next
+            {
+                const F2 s2 = lds_f2(sc + 4u * (8 * j + pair_col)), b2 = lds_f2(bi + 4u * (8 * j + pair_col));
+                const uint32_t* x = v + 8 * (i >> 1) + 4 * j + 2 * (i & 1);
+                float2 r = make_float2(__fmul_rn(__int2float_rn(int32_t(x[0]) + __float_as_int(b2.x)), s2.x),
+                                       __fmul_rn(__int2float_rn(int32_t(x[1]) + __float_as_int(b2.y)), s2.y));
+                if (p.relu)
+                    r = make_float2(fmaxf(r.x, 0.0f), fmaxf(r.y, 0.0f));
+                if (((rows_ok >> (8 * i)) & 1u) != 0 && 8 * j + pair_col < cols)
+                    *reinterpret_cast<float2*>(o + 8 * j) = r;
+            }
+        }
     }
 
     // The epilogue loops come in families, a kernel each.  Compiled into one kernel they share a register budget and a schedule:
@@ -654,7 +769,8 @@ namespace b200
         EPI_WORDS,   // four-byte results otherwise: i32 of every contract, f32 with a residual; the stores of EPI_SECTORS
         EPI_SUM,     // one-byte results with a residual that TMA does not bring (or a ring that leaves it no room): the residual into
                      // registers ahead of the accumulator, the stores of EPI_ROWS
-        EPI_GENERAL  // everything else: results of any type straight from registers
+        EPI_GENERAL, // everything else: results of any type straight from registers
+        EPI_ONE_SHOT // a kernel of its own: one tile per CTA (one_shot_epilogue)
     };
     template <int BN, int BK, bool CTA2 = false, bool SPLITK = false, int EPI = EPI_BYTES>
     __global__ void __launch_bounds__(NUM_THREADS, SPLITK ? 2 : 1)
@@ -662,16 +778,17 @@ namespace b200
     {
         using C = Cfg<BN, BK>;
         constexpr int SPLIT = C::SPLIT, GROUPS = C::GROUPS, NACC = C::NACC;
+        constexpr bool EXCHANGE = SPLITK && EPI != EPI_ONE_SHOT; // the tile's CTAs are a cluster
         // a split tile has one accumulator: two of these CTAs, of one launch or of consecutive ones, share an SM
         constexpr uint32_t TMEM_COLS = SPLITK ? BN : C::TMEM_COLS;
         // CTA pairs: rank 0 issues the pair's MMAs; a "worker" is what takes units of work in turn (a CTA, or a pair)
         const uint32_t cta_rank = CTA2 ? ptx::cluster_ctarank() : 0u;
-        const int worker = CTA2 ? int(blockIdx.x >> 1) : SPLITK ? int(blockIdx.x) / p.split : int(blockIdx.x);
-        const int nworkers = CTA2 ? int(gridDim.x >> 1) : SPLITK ? int(gridDim.x) / p.split : int(gridDim.x);
+        const int worker = CTA2 ? int(blockIdx.x >> 1) : EXCHANGE ? int(blockIdx.x) / p.split : int(blockIdx.x);
+        const int nworkers = CTA2 ? int(gridDim.x >> 1) : EXCHANGE ? int(gridDim.x) / p.split : int(gridDim.x);
         // this CTA's share of the tile's k-blocks
-        const int split_rank = SPLITK ? int(ptx::cluster_ctarank()) : 0;
+        const int split_rank = EXCHANGE ? int(ptx::cluster_ctarank()) : 0;
         const int kb_total = p.ntaps * p.cblocks;
-        const int kb_begin = SPLITK ? kb_total * split_rank / p.split : 0, kb_end = SPLITK ? kb_total * (split_rank + 1) / p.split : kb_total;
+        const int kb_begin = EXCHANGE ? kb_total * split_rank / p.split : 0, kb_end = EXCHANGE ? kb_total * (split_rank + 1) / p.split : kb_total;
         // bytes of B one CTA stages per k-block: the whole column tile, or this CTA's half of it
         constexpr uint32_t B_STAGE_BYTES = CTA2 ? uint32_t(C::B_BYTES) / 2 : uint32_t(C::B_BYTES);
 #ifdef B200_PROFILE_WAITS
@@ -728,8 +845,8 @@ namespace b200
                 ptx::mbar_init(sum_bar((t - 96) / 3, (t - 96) % 3), 1);
             else if (CTA2 && t >= 160 && t < 160 + STAGES)
                 ptx::mbar_init(peer_full_bar(t - 160), 1);
-            if (SPLITK && t == 96)
-                ptx::mbar_expect_tx(sum_bar(0, 0), SPLIT_EXCHANGE_BYTES); // the partial sums of the columns finished here
+            if (EXCHANGE && t == 96)
+                ptx::mbar_expect_tx(sum_bar(0, 0), uint32_t(p.rows) * (64 * 4)); // the partial sums of the columns finished here
             if (t >= 0 && t < 224)
                 ptx::fence_barrier_init();
         }
@@ -750,7 +867,7 @@ namespace b200
         __syncthreads();
         if (CTA2)
             ptx::cluster_sync(); // the peer's barriers exist before anything arrives on them from here
-        if (SPLITK)
+        if (EXCHANGE)
             ptx::cluster_arrive_relaxed(); // this CTA runs: its shared memory may be written from now on
         ptx::tc_fence_after_sync();
         const uint32_t tmem_base = tmem_base_slot;
@@ -877,7 +994,7 @@ namespace b200
                     // packed weights: this column tile's 64-row blocks of a k-block are one contiguous piece
                     const int b_blocks = CTA2 ? BN / 128 : min(BN / 64, p.b_blocks_n - tn * (BN / 64));
                     const uint32_t b_bytes = p.smem.b_resident ? 0u : (p.b_packed ? uint32_t(b_blocks) * (64 * BK) : B_STAGE_BYTES);
-                    const uint32_t tx_bytes = (p.a_cells ? LINEAR_A_BYTES * uint32_t(p.ntaps) : p.halo ? uint32_t(p.halo_bytes) : uint32_t(C::A_BYTES) * uint32_t(pair)) + b_bytes;
+                    const uint32_t tx_bytes = (p.a_cells ? LINEAR_A_BYTES * uint32_t(p.ntaps) : p.halo ? uint32_t(p.halo_bytes) : uint32_t(p.rows * BK) * uint32_t(pair)) + b_bytes;
                     int tap = 0, cb = j; // k-block j of the tile = (tap, channel block)
                     while (cb >= p.cblocks)
                     {
@@ -899,7 +1016,7 @@ namespace b200
                         const Tap tp = p.taps[tap];
                         const int kcol = j * BK; // byte column of the k-block in the B matrix
                         const uint32_t a_dst = smem_base + s * stage_bytes;
-                        const uint32_t b_dst = a_dst + uint32_t(pair) * C::A_BYTES; // [A of tile 2u][A of tile 2u + 1][B]
+                        const uint32_t b_dst = a_dst + uint32_t(pair * p.rows * BK); // [A of tile 2u][A of tile 2u + 1][B]
                         if (!waited)
                             wait_for_earlier_kernels();
                         waited = true;
@@ -927,7 +1044,7 @@ namespace b200
                         }
                         else
                         {
-                            ptx::tma_load_2d(a_dst, &maps.a[0], full_bar(s), kcol, tm * BM);
+                            ptx::tma_load_2d(a_dst, &maps.a[0], full_bar(s), kcol, tm * p.rows);
                             if (pair == 2)
                                 ptx::tma_load_2d(a_dst + C::A_BYTES, &maps.a[0], full_bar(s), kcol, ia2 * BM);
                         }
@@ -1016,7 +1133,7 @@ namespace b200
                 // 16-byte K pieces 16 bytes apart, rows 16 bytes apart, 8-row groups 128 bytes apart, no swizzle
                 const uint64_t a_desc0 = p.a_cells ? ptx::smem_desc_overlapping_rows(smem_base) : ptx::smem_desc_kmajor(smem_base, BK);
                 const int pair = p.pair;
-                const uint64_t b_desc0 = ptx::smem_desc_kmajor(p.smem.b_resident ? bres_base : smem_base + uint32_t(pair) * C::A_BYTES, BK);
+                const uint64_t b_desc0 = ptx::smem_desc_kmajor(p.smem.b_resident ? bres_base : smem_base + uint32_t(pair * p.rows * BK), BK);
                 // CTA pairs: the hardware reads the other 128 rows of A and the other half of B at the same offsets of the odd CTA
                 // descriptor address fields count 16-byte units
                 const uint32_t b_step = p.smem.b_resident ? (C::B_BYTES >> 4) : (stage_bytes >> 4);
@@ -1193,7 +1310,10 @@ namespace b200
             if constexpr (SPLITK)
             {
                 wait_for_earlier_kernels();
-                split_epilogue(p, worker, split_rank, warp, lane, tmem_base, out_base, tfull_bar(0), sum_bar(0, 0), abortp, fail);
+                if constexpr (!EXCHANGE)
+                    one_shot_epilogue(p, worker, warp, lane, tmem_base, out_base, tfull_bar(0), abortp, fail);
+                else
+                    split_epilogue(p, worker, split_rank, warp, lane, tmem_base, out_base, tfull_bar(0), sum_bar(0, 0), abortp, fail);
             }
             else
             {
@@ -1876,7 +1996,7 @@ namespace b200
         if (fail)
             atomicCAS(&g_contract_status, 0, fail);
         __syncwarp();
-        if (SPLITK && warp < 4)
+        if (EXCHANGE && warp < 4)
         {
             ptx::cluster_wait(); // the barrier that the epilogue warps waited on counts every thread of the cluster
         }
@@ -1888,7 +2008,7 @@ namespace b200
             for (int i = 0; i < 50; ++i)
                 __nanosleep(1000);
             __syncthreads();
-            if (SPLITK)
+            if (EXCHANGE)
                 split_leave(sum_bar(0, 0));
         }
         if (CTA2)
@@ -2055,19 +2175,48 @@ namespace b200
     // where two CTAs run on an SM at a time; a third waits for them to end.  Clusters of eight fit 128 of the 148 SMs at a time.
     // [1, 512, 7, 7] 3x3 -> 512: 10.5 us whole, 6.5 in eight; 128 x 1000 x 2048: 17.4 and 6.4; 20 x 2432 x 3072: 8.1 whole, 11.7 in two.
     // `words`: the results are what EPI_WORDS computes, which four of a whole tile's warps take 3 us for.
-    static int pick_split(int64_t tiles, int64_t nkb, bool words)
+    //
+    // One-shot launches with whole reductions (`pieces`: the results allow it): tiles of 64 rows while they leave half the SMs to the next
+    // launch, which sets up there meanwhile (a k-block takes 0.2 us either way, the tensor pipe's rate at 64 columns; the shorter
+    // boxes land 0.15 us earlier), otherwise whole tiles where the reduction is short or the weights are one column tile.  More
+    // k-blocks and tiles run as fast in the persistent kernel (400 x 768 x 768: 3.74 us there, 3.94 one-shot).  Reductions are also shared
+    // by tiles of 64 rows, which exchange half as much.  Chains of launches, before and after, us: 128 x 128 x 128 2.69, 2.10;
+    // 256 x 1024 x 1024 4.09, 3.91; 128 x 768 x 3072 6.40, 5.12; 64 -> 64 on 56x56 3.16, 2.22; 512 -> 512 3x3 on 7x7 5.64, 4.81;
+    // 512 -> 2048 on 7x7 with a residual 3.69, 3.11.  tiles64: 0 where such tiles cannot be had.
+    struct Shape
     {
-        int best = 1;
-        double best_us = 0.19 * double(nkb) * double((tiles + num_sms() - 1) / num_sms()) + (words ? 3.0 : 0.0);
-        for (int s = 2; s <= MAX_SPLIT && s <= nkb; s *= 2)
+        int rows, split, one_shot;
+    };
+    static Shape pick_shape(int64_t tiles128, int64_t tiles64, int64_t tiles_n, int64_t nkb, bool words, bool pieces, bool f32)
+    {
+        Shape best{BM, 1, pieces && tiles128 <= (f32 ? num_sms() * 7 / 16 : num_sms()) && (nkb <= 2 || tiles_n == 1)};
+        double best_us = 0.19 * double(nkb) * double((tiles128 + num_sms() - 1) / num_sms()) + (words && !best.one_shot ? 3.0 : 0.0);
+        for (int r = BM; r >= 64; r -= 64)
         {
-            const int64_t room = s == MAX_SPLIT ? num_sms() * 7 / 8 : num_sms() * 15 / 16;
-            const int64_t per_sm = (tiles * s + room - 1) / room, rounds = (per_sm + 1) / 2;
-            const double us = (s == MAX_SPLIT ? 1.4 : 2.1) + double((nkb + s - 1) / s) * (per_sm == 1 ? 0.27 : 0.45) * double(rounds) + 3.9 * double(rounds - 1);
-            if (us < best_us)
+            const int64_t tiles = r == BM ? tiles128 : tiles64;
+            const double kb = r == BM ? 1.0 : 0.68;
+            if (tiles == 0)
+                continue;
+            if (r == 64 && pieces && tiles <= num_sms() / 2 && 0.19 * double(nkb) - 0.15 < best_us)
             {
-                best = s;
-                best_us = us;
+                best_us = 0.19 * double(nkb) - 0.15;
+                best = {r, 1, 1};
+            }
+            for (int s = 2; s <= MAX_SPLIT && s <= nkb; s *= 2)
+            {
+                const int64_t room = s == MAX_SPLIT ? num_sms() * 7 / 8 : num_sms() * 15 / 16;
+                const int64_t per_sm = (tiles * s + room - 1) / room, rounds = (per_sm + 1) / 2;
+                if (r == 64 && (per_sm > 1 || (s == MAX_SPLIT && tiles != tiles128 && tiles * s > 64)))
+                    break;
+                const double exchange = s == MAX_SPLIT ? (r == BM ? 1.75 : 1.4) + (tiles * s > 64 ? 0.5 : 0.0)
+                                        : r == BM      ? 2.1
+                                                       : (s == 2 ? 3.0 : 1.6);
+                const double us = exchange + (pieces && per_sm > 1 ? 0.5 : 0.0) + double((nkb + s - 1) / s) * kb * (per_sm == 1 ? 0.27 : 0.45) * double(rounds) + 3.9 * double(rounds - 1);
+                if (us < best_us)
+                {
+                    best_us = us;
+                    best = {r, s, 1};
+                }
             }
         }
         return best;
@@ -2082,6 +2231,7 @@ namespace b200
             return qcontract_kernel<BN, BK, (BN == 256)>;
 #endif
         return p.split > 1                 ? qcontract_kernel<BN, BK, false, (BN == 64)>
+               : p.one_shot                ? qcontract_kernel<BN, BK, false, (BN == 64), (BN == 64 ? EPI_ONE_SHOT : EPI_BYTES)>
                : p.epilogue == EPI_SECTORS ? qcontract_kernel<BN, BK, false, false, EPI_SECTORS>
                : p.epilogue == EPI_BYTES_2 ? qcontract_kernel<BN, BK, false, false, EPI_BYTES_2>
                : p.epilogue == EPI_ROWS    ? qcontract_kernel<BN, BK, false, false, EPI_ROWS>
@@ -2152,9 +2302,12 @@ namespace b200
             return B200_ERR_TOO_LARGE;
         const int nkb = p.ntaps * p.cblocks;
         SmemPlan& sp = p.smem;
-        p.split = (BN == 64 && !p.a_cells && !p.halo && p.pair != 2 && !p.cta2) ? pick_split(int64_t(p.tiles_m) * p.tiles_n, nkb, p.half_away != 2 && (p.out_type == B200_I32 || (p.out_type == B200_F32 && p.sum_in))) : 1;
-        sp.b_resident = (p.tiles_n == 1 && nkb * C::B_BYTES <= B_RESIDENT_MAX && p.split == 1) ? 1 : 0;
-        if (p.split > 1) // results are written from registers; the staging area holds the partial sums on their way
+        if (BN != 64 || p.a_cells || p.halo || p.pair == 2 || p.cta2) // (the caller has chosen: pick_shape)
+            p.one_shot = 0;
+        if (!p.one_shot)
+            p.split = 1, p.rows = BM;
+        sp.b_resident = (p.tiles_n == 1 && nkb * C::B_BYTES <= B_RESIDENT_MAX && !p.one_shot) ? 1 : 0;
+        if (p.one_shot) // results are written from registers; the staging area holds the partial sums on their way
             p.tma_store = p.tma_sum = 0;
         if (p.cta2)
         {
@@ -2176,7 +2329,7 @@ namespace b200
             return B200_ERR_INVALID_ARGUMENT; // the caller pads the row tiles to an even count
         const int tma_store_asked = p.tma_store, tma_sum_asked = p.tma_sum;
     plan_again:
-        sp.stage_bytes = p.pair * C::A_BYTES + (sp.b_resident ? 0 : p.cta2 ? C::B_BYTES / 2 : C::B_BYTES);
+        sp.stage_bytes = p.pair * p.rows * BK + (sp.b_resident ? 0 : p.cta2 ? C::B_BYTES / 2 : C::B_BYTES);
         if (p.a_cells)
         {
             if (!sp.b_resident)
@@ -2189,6 +2342,8 @@ namespace b200
                 return B200_ERR_UNSUPPORTED; // the caller only asks for halo mode when the weights stay resident
             sp.stage_bytes = halo_stage_bytes(p.halo_bytes, p.RW - p.TW, BK);
         }
+        // (whole reductions: one CTA per SM.  Two of one launch on an SM share its operand rate while others idle: 256 -> 128 on 56x56 3.2 us
+        // against 2.7)
         const int room = (p.split > 1 ? SPLIT_SMEM_LIMIT : SMEM_LIMIT) - C::FIXED - sp.b_res_bytes - 64;
         if (p.tma_store && nkb >= 16 && (room - 2 * C::OUT_BYTES) / sp.stage_bytes < (p.cta2 ? 7 : 4))
         {
@@ -2228,7 +2383,7 @@ namespace b200
         if (p.epilogue != EPI_BYTES && p.epilogue != EPI_BYTES_2)
             p.tma_store = p.tma_sum = 0;
         sp.out_bufs = p.tma_store ? (p.tma_sum ? sum_bufs : 2) : (p.epilogue == EPI_ROWS || p.epilogue == EPI_SUM) && rows_staged ? 1 : 0;
-        sp.out_bytes = p.split > 1 ? SPLIT_EXCHANGE_BYTES : sp.out_bufs * C::OUT_BYTES;
+        sp.out_bytes = p.one_shot ? (p.split > 1 ? SPLIT_EXCHANGE_BYTES : ONE_SHOT_STAGED_BYTES) : sp.out_bufs * C::OUT_BYTES;
         int fit = (room - sp.out_bytes) / sp.stage_bytes;
         sp.stages = fit > MAX_STAGES ? MAX_STAGES : fit;
         if (p.pair == 2 && sp.stages < MIN_STAGES)
@@ -2260,13 +2415,13 @@ namespace b200
         }
         sp.total_bytes = sp.b_res_bytes + sp.stages * sp.stage_bytes + sp.out_bytes + C::FIXED;
         int tiles = p.tiles_m * p.tiles_n / p.pair; // units of work: tiles, or pairs of row tiles
-        int grid = p.split > 1 ? tiles * p.split : tiles < num_sms() ? tiles : num_sms();
+        int grid = p.one_shot ? tiles * p.split : tiles < num_sms() ? tiles : num_sms();
         if (p.cta2) // two CTAs per unit of two row tiles
             grid = 2 * std::min(tiles / 2, num_sms() / 2);
         // A launch that fills the GPU lets the next kernel in when its last accumulators are done: there is no room for it earlier,
         // and blocks let in at once gather on the SMs that finish first (see `launch`).  A smaller one lets it in at once:
         // the next kernel sets up on the SMs that this one leaves idle.
-        p.late_successor = p.split == 1 && grid >= num_sms();
+        p.late_successor = !p.one_shot && grid >= num_sms();
         if (t_capture)
         {
             t_capture->maps = maps;
@@ -2308,6 +2463,27 @@ namespace b200
             return B200_ERR_INVALID_ARGUMENT;
         return B200_OK;
     }
+
+    // results that EPI_WORDS computes
+    static bool four_byte_words(const b200_epilogue* e)
+    {
+        return e->round_half_away != 2 && (e->out_type == B200_I32 || (e->out_type == B200_F32 && e->sum_in));
+    }
+
+    // what a one-shot launch with a whole reduction writes: a fused contract, results in whole pieces
+    static bool one_shot_pieces(const b200_epilogue* e, const void* out, int64_t n)
+    {
+        if (e->round_half_away || (reinterpret_cast<uintptr_t>(out) & 15) != 0)
+            return false;
+        if (e->out_type == B200_F32)
+            return n % 4 == 0 && !e->sum_in;
+        return e->out_type != B200_I32 && n % 16 == 0 && (reinterpret_cast<uintptr_t>(e->sum_in) & 15) == 0;
+    }
+
+    // Up to how many tiles a product that would have wider ones is made of 64 columns for a one-shot launch: with a residual, which costs the
+    // persistent kernel more, one per SM, otherwise half as many (64 -> 256 on 56x56, 100 tiles: 3.1 us in 50 wide ones, 3.2 one-shot; with
+    // a residual 3.7 and 3.5).
+    static int one_shot_tiles(const b200_epilogue* e) { return e->sum_in ? num_sms() : num_sms() / 2; }
 
     static void fill_epilogue(ContractParams& p, const b200_epilogue* e, void* out, int a_type)
     {
@@ -2608,9 +2784,25 @@ static int qgemm_impl(const void* A, int a_type, const int8_t* W, bool packed, v
     p.ntaps = 1;
     p.cblocks = int((K + bk - 1) / bk);
     p.tiles_m = int((M + BM - 1) / BM);
-    const int bn = pick_bn(N, p.tiles_m, bk, epilogue && epilogue->sum_in, K);
+    int bn = pick_bn(N, p.tiles_m, bk, epilogue && epilogue->sum_in, K);
+    p.rows = BM;
+    p.split = 1;
+    const bool pieces = one_shot_pieces(epilogue, out, N);
+    const int64_t tiles_n = (N + 63) / 64;
+    if (bn == 64 || (pieces && p.tiles_m * tiles_n <= one_shot_tiles(epilogue)))
+    {
+        const Shape shape = pick_shape(p.tiles_m * tiles_n, (M + 63) / 64 * tiles_n, tiles_n, p.cblocks, four_byte_words(epilogue), pieces, epilogue->out_type == B200_F32);
+        if (shape.one_shot)
+        {
+            bn = 64;
+            p.rows = shape.rows, p.split = shape.split, p.one_shot = 1;
+            p.tiles_m = int((M + p.rows - 1) / p.rows);
+        }
+    }
     p.tiles_n = int((N + bn - 1) / bn);
     p.pair = pick_pair(p.tiles_m, N, bn, bk, p.cblocks, epilogue && epilogue->sum_in, false, epilogue->out_type != B200_F32);
+    if (p.one_shot)
+        p.pair = 1;
 #ifdef B200_PROFILE_WAITS
     if (getenv("B200_FORCE_CTA2") && bn == 256 && N % 256 == 0 && p.tiles_m >= 2 && !(p.tiles_n == 1 && int64_t(p.cblocks) * bn * bk <= B_RESIDENT_MAX))
     {
@@ -2627,7 +2819,7 @@ static int qgemm_impl(const void* A, int a_type, const int8_t* W, bool packed, v
     TensorMaps maps;
     memset(&maps, 0, sizeof(maps));
     uint64_t dims_a[2] = {uint64_t(K), uint64_t(M)}, str[1] = {uint64_t(K)};
-    uint32_t box_a[2] = {uint32_t(bk), uint32_t(BM)};
+    uint32_t box_a[2] = {uint32_t(bk), uint32_t(p.rows)};
     rc = make_map(&maps.a[0], A, 2, dims_a, str, box_a, bk);
     if (rc != B200_OK)
         return rc;
@@ -2722,17 +2914,17 @@ extern "C" int b200_qconv_out_shape(const b200_conv_params* c, int64_t* P, int64
     return B200_OK;
 }
 
-// Chooses the output patch TW x TH x TN (product 128, all powers of two) that wastes the fewest
+// Chooses the output patch TW x TH x TN (product `rows`, all powers of two) that wastes the fewest
 // accumulator rows on positions outside the output.
-static void pick_patch(int64_t NB, int64_t P, int64_t Q, int& TW, int& TH, int& TN)
+static void pick_patch(int64_t NB, int64_t P, int64_t Q, int rows, int& TW, int& TH, int& TN)
 {
     double best = -1.0;
-    for (int tw = 1; tw <= 128; tw *= 2)
-        for (int th = 1; tw * th <= 128; th *= 2)
+    for (int tw = 1; tw <= rows; tw *= 2)
+        for (int th = 1; tw * th <= rows; th *= 2)
         {
-            int tn = 128 / (tw * th);
+            int tn = rows / (tw * th);
             int64_t tiles = ((Q + tw - 1) / tw) * ((P + th - 1) / th) * ((NB + tn - 1) / tn);
-            double eff = double(NB * P * Q) / double(tiles * 128);
+            double eff = double(NB * P * Q) / double(tiles * rows);
             // prefer wider patches on ties (longer contiguous runs for the TMA unit)
             if (eff > best + 1e-9 || (eff > best - 1e-9 && tw * th > TW * TH))
             {
@@ -2810,7 +3002,9 @@ static int qconv_impl(const void* data, int data_type, const int8_t* filters, bo
     p.NB = int(c->N);
     p.P = int(P);
     p.Q = int(Q);
-    pick_patch(c->N, P, Q, p.TW, p.TH, p.TN);
+    p.rows = BM;
+    p.split = 1;
+    pick_patch(c->N, P, Q, BM, p.TW, p.TH, p.TN);
     // Halo mode (stride 1, no dilation, more than one tap, weights small enough to stay in shared memory): a tile is 4
     // rows of 32 positions of which the first 32-(S-1) are output pixels; its input patch, halo included, is loaded ONCE
     // per channel block and every tap reads it through a row-shifted descriptor, instead of one displaced copy per tap.
@@ -2846,6 +3040,25 @@ static int qconv_impl(const void* data, int data_type, const int8_t* filters, bo
                     p.taps[r * c->S + sx].pad = short(r * RW + sx); // row shift of the tap inside the patch
         }
     }
+    auto tiles_of = [&](int TW, int TH, int TN) { return int64_t((Q + TW - 1) / TW) * ((P + TH - 1) / TH) * ((c->N + TN - 1) / TN); };
+    p.tiles_m = int(tiles_of(p.TW, p.TH, p.TN));
+    int bn = pick_bn(c->K, p.tiles_m, bk, epilogue && epilogue->sum_in, c->R * c->S * c->C);
+    const bool pieces = one_shot_pieces(epilogue, out, c->K);
+    const int64_t tiles_n64 = (c->K + 63) / 64;
+    if (!p.halo && (bn == 64 || (pieces && p.tiles_m * tiles_n64 <= one_shot_tiles(epilogue))))
+    {
+        int TW = 1, TH = 1, TN = 1;
+        pick_patch(c->N, P, Q, 64, TW, TH, TN);
+        const Shape shape = pick_shape(p.tiles_m * tiles_n64, tiles_of(TW, TH, TN) * tiles_n64, tiles_n64, int64_t(p.ntaps) * p.cblocks, four_byte_words(epilogue),
+                                       pieces, epilogue->out_type == B200_F32);
+        if (shape.one_shot)
+        {
+            bn = 64;
+            p.rows = shape.rows, p.split = shape.split, p.one_shot = 1;
+            if (p.rows == 64)
+                p.TW = TW, p.TH = TH, p.TN = TN;
+        }
+    }
     if (!p.halo)
         p.RW = p.TW;
     p.sub_w = p.TW < 32 ? p.TW : 32;
@@ -2855,7 +3068,6 @@ static int qconv_impl(const void* data, int data_type, const int8_t* filters, bo
     p.tiles_q = int((Q + p.TW - 1) / p.TW);
     p.tiles_p = int((P + p.TH - 1) / p.TH);
     p.tiles_m = p.tiles_q * p.tiles_p * int((c->N + p.TN - 1) / p.TN);
-    const int bn = pick_bn(c->K, p.tiles_m, bk, epilogue && epilogue->sum_in, c->R * c->S * c->C);
     p.tiles_n = int((c->K + bn - 1) / bn);
     // Row-tile pairs are not taken for convolutions: on the ResNet-50 layers they could apply to (3x3 on 28x28 and 14x14
     // images at batch 128) the halved number of work units costs what the shared weight stages save (measured: 24.8 -> 27 us
@@ -3027,7 +3239,7 @@ extern "C" int b200_qconv_stem(const void* cells, int data_type, const int8_t* p
         p.cells_h = int(Hc);
     }
     else
-        pick_patch(N, P, Q, p.TW, p.TH, p.TN);
+        pick_patch(N, P, Q, BM, p.TW, p.TH, p.TN);
     p.sub_w = p.TW < 32 ? p.TW : 32;
     p.sub_h = (p.TH < 32 / p.sub_w) ? p.TH : 32 / p.sub_w;
     p.tiles_q = int((Q + p.TW - 1) / p.TW);

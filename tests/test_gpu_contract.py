@@ -713,3 +713,50 @@ def test_qgemm_residuals_and_words_off_the_tma_paths(ops, m, n, k):
         o = _at(torch.zeros((m, n), dtype=torch.int32, device="cuda"), at)
         lib.check(lib.LIB.b200_qgemm(a.data_ptr(), lib.I8, w.data_ptr(), o.data_ptr(), m, n, k, ctypes.byref(e), torch.cuda.current_stream().cuda_stream), "raw")
         assert torch.equal(o, acc)
+
+
+# ---------------------------------------------------------------- one tile per CTA
+@pytest.mark.parametrize("m,n,k", [(1, 16, 16), (31, 64, 144), (64, 80, 128), (65, 48, 1040), (129, 208, 272), (600, 256, 2048), (1000, 512, 512), (200, 64, 4096), (160, 512, 2064), (4700, 64, 64)])
+def test_one_shot_products(ops, m, n, k):
+    """tiles of 64 and 128 rows that end early, whole and shared reductions, all results that leave in whole pieces"""
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+
+    def ints(lo, hi, shape, dt):
+        return torch.randint(lo, hi, shape, generator=gen, device="cuda", dtype=torch.int32).to(dt)
+
+    a, w, bias = ints(-128, 128, (m, k), torch.int8), ints(-127, 128, (n, k), torch.int8), ints(-1000, 1001, (n,), torch.int32)
+    scale = torch.rand(n, generator=gen, device="cuda") * 0.01 / k ** 0.5 + 0.005 / k ** 0.5
+    ss = torch.full((1,), 0.37, device="cuda")
+    base = ((a.double() @ w.double().t()).to(torch.int32) + bias).float() * scale
+    res = {torch.uint8: ints(0, 256, (m, n), torch.uint8), torch.int8: ints(-128, 128, (m, n), torch.int8)}
+    for packed in (True, False):
+        for out, relu, r in ((torch.uint8, False, None), (torch.int8, True, None), (torch.int8, False, torch.int8), (torch.uint8, True, torch.uint8), (torch.float32, False, None),
+                             (torch.float32, True, None)):
+            f = base if r is None else base + ss * res[r].float()
+            f = f.clamp(min=0) if relu else f
+            want = f if out == torch.float32 else f.round().clamp(*((0, 255) if out == torch.uint8 else (-128, 127))).to(out)
+            got = ops.qgemm(a, w, scale, out, bias=bias, relu=relu, sum_in=None if r is None else res[r], sum_scale=None if r is None else ss, packed=packed)
+            assert torch.equal(got, want), (out, relu, r, packed)
+
+
+@pytest.mark.parametrize("cfg", [(1, 64, 56, 56, 64, 1, (1, 1)), (1, 128, 14, 13, 80, 3, (1, 1)), (3, 64, 9, 7, 48, 3, (2, 2)), (2, 256, 7, 7, 256, 1, (1, 1)), (1, 64, 31, 30, 256, 1, (1, 1)), (5, 128, 17, 16, 64, 3, (2, 1))])
+@pytest.mark.parametrize("residual", [False, True])
+def test_one_shot_convolutions(ops, cfg, residual):
+    """patches of 64 output pixels over image edges and batches"""
+    n, c, h, w, k, r, stride = cfg
+    rng = np.random.default_rng(sum(cfg[:6]))
+    data = rng.integers(0, 256, size=(n, c, h, w)).astype(np.uint8)
+    filt = rng.integers(-127, 128, size=(k, c, r, r)).astype(np.int8)
+    bias = rng.integers(-1000, 1001, size=k).astype(np.int32)
+    cs = ref.conv_shape(data.shape, filt.shape, stride, (r // 2, r // 2), (r // 2, r // 2), (1, 1))
+    scale = (np.exp(rng.uniform(np.log(0.5), np.log(2.0), size=k)) * 60.0 / (np.sqrt(c * r * r) * 74 * 147)).astype(np.float32)
+    kw = {"sum_in": rng.integers(0, 256, size=(n, k) + tuple(ref.conv_out_hw(cs))).astype(np.uint8), "sum_scale": np.float32(0.61)} if residual else {}
+    for out_dt, relu in ((np.uint8, True), (np.int8, False), (np.float32, False)):
+        if out_dt == np.float32 and residual:
+            continue
+        exp = ref.qconv_fused(data, filt, bias, scale, cs, out_dt, relu=relu, **kw)
+        got = run_conv(ops, data, filt, bias, scale, cs, out_dt, relu, packed=True, **kw)
+        if out_dt == np.float32:
+            same_f32(np.ascontiguousarray(got), exp)
+        else:
+            np.testing.assert_array_equal(got, exp)
