@@ -20,6 +20,7 @@
 #include <math.h>
 #include <algorithm>
 #include <initializer_list>
+#include <type_traits>
 #include "bmm.cuh"
 #include "common.cuh"
 #include "rounded_math.cuh"
@@ -904,35 +905,42 @@ namespace b200
     // src/ngraph/builder/reduce_ops.cpp:68-127), in that order:
     //   mean = KahanSum(x) / N;  var = KahanSum((x - mean) * (x - mean)) / N;  sd = sqrt(var + eps);
     //   y = ((x - mean) / sd) * gamma + beta          (every operation a separate IEEE rounding, no fused multiply-add)
-    // 24576 rows of 768: 197 -> 88 us (226 MB: 35 us); 128 rows: 60 -> 21 us, of which the two chains are 13.
-    template <bool VEC, bool ADDEND>
+    // 24576 rows of 768: 197 -> 88 us (226 MB: 35 us).
+    // FEW: fewer rows than the SMs hold at eight per block (128 rows of 768: 13 of the 21 us that such blocks took were the two chains).
+    // A block has `tile_rows` of them (a power of two below 8), as few as keep every SM busy, and all its threads on each row's loads and
+    // results; while the chains run the other warps bring gamma and beta into L1.
+    template <bool VEC, bool ADDEND, bool FEW>
     __global__ void __launch_bounds__(ROW_THREADS) layer_norm_rows_kernel(const float* __restrict__ in, const float* __restrict__ addend,
                                                                           const float* __restrict__ gamma, const float* __restrict__ beta,
                                                                           float* __restrict__ out, int64_t rows, int L, float count, float eps,
-                                                                          int64_t ahead)
+                                                                          int64_t ahead, int tile_rows)
     {
         if constexpr (ADDEND)
             after_earlier_kernels(in, addend, gamma, beta, out);
         else
             after_earlier_kernels(in, gamma, beta, out);
-        constexpr int R = NORM_ROWS, WARPS = ROW_THREADS / 32;
+        constexpr int WARPS = ROW_THREADS / 32;
+        const int R = FEW ? tile_rows : NORM_ROWS;
         extern __shared__ __align__(16) float tile[];
-        __shared__ float row_mean[R], row_sd[R];
-        const int stride = staged_row_stride(L, VEC), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        __shared__ float row_mean[NORM_ROWS], row_sd[NORM_ROWS];
+        const int stride = staged_row_stride(L, VEC);
+        // rows and columns of a thread: groups of threads (a warp, or more where there are fewer rows than warps) take rows in turn
+        const int groups = FEW ? min(tile_rows, WARPS) : WARPS, per_row = ROW_THREADS / groups;
+        const int warp = threadIdx.x / per_row, lane = threadIdx.x % per_row; // of the group
         const int64_t row0 = int64_t(blockIdx.x) * R;
         const int n_rows = int(min(rows - row0, int64_t(R)));
         in += row0 * L;
         out += row0 * L;
         if (ADDEND)
             addend += row0 * L;
-        for (int r = warp; r < n_rows; r += WARPS)
+        for (int r = warp; r < n_rows; r += groups)
         {
             if (VEC)
             {
                 const float4* x4 = reinterpret_cast<const float4*>(in + int64_t(r) * L);
                 const float4* a4 = reinterpret_cast<const float4*>(addend + int64_t(r) * L);
 #pragma unroll 4
-                for (int c = lane; c < L / 4; c += 32)
+                for (int c = lane; c < L / 4; c += per_row)
                 {
                     float4 v = __ldg(x4 + c);
                     if (ADDEND)
@@ -944,7 +952,7 @@ namespace b200
                 }
             }
             else
-                for (int c = lane; c < L; c += 32)
+                for (int c = lane; c < L; c += per_row)
                     tile[r * stride + c] = ADDEND ? __fadd_rn(in[int64_t(r) * L + c], addend[int64_t(r) * L + c]) : in[int64_t(r) * L + c];
         }
         __syncthreads();
@@ -961,7 +969,16 @@ namespace b200
             row_mean[threadIdx.x] = mean;
             row_sd[threadIdx.x] = __fsqrt_rn(__fadd_rn(var, eps));
         }
-        else if (warp > 0)
+        else if (FEW && threadIdx.x >= 32)
+        {
+            for (int i = threadIdx.x - 32; 32 * i < L; i += ROW_THREADS - 32)
+            {
+                float unused;
+                asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(unused) : "l"(gamma + 32 * i));
+                asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(unused) : "l"(beta + 32 * i));
+            }
+        }
+        else if (threadIdx.x >= 32)
         {
             // the other warps have nothing to do: they bring the rows of the tile that follows this one on the SM into L2, whose
             // loads would otherwise all start when the chains of a whole wave of blocks have ended
@@ -975,12 +992,12 @@ namespace b200
             }
         }
         __syncthreads();
-        for (int r = warp; r < n_rows; r += WARPS)
+        for (int r = warp; r < n_rows; r += groups)
         {
             const float mean = row_mean[r], sd = row_sd[r], y = reciprocal_if_exact(sd);
             if (VEC)
 #pragma unroll 2
-                for (int c = lane; c < L / 4; c += 32)
+                for (int c = lane; c < L / 4; c += per_row)
                 {
                     float4 v = *reinterpret_cast<const float4*>(tile + r * stride + 4 * c);
                     const float4 g = __ldg(reinterpret_cast<const float4*>(gamma) + c), b = __ldg(reinterpret_cast<const float4*>(beta) + c);
@@ -990,7 +1007,7 @@ namespace b200
                     reinterpret_cast<float4*>(out + int64_t(r) * L)[c] = v;
                 }
             else
-                for (int c = lane; c < L; c += 32)
+                for (int c = lane; c < L; c += per_row)
                     out[int64_t(r) * L + c] =
                         __fadd_rn(__fmul_rn(divide_by(__fsub_rn(tile[r * stride + c], mean), sd, y), __ldg(gamma + c)), __ldg(beta + c));
         }
@@ -1683,21 +1700,29 @@ extern "C" int b200_layer_norm_rows_sum_f32(const float* x, const float* addend,
     const bool vec = L % 4 == 0 && all_aligned16({x, addend, gamma, beta, out});
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const float count = static_cast<float>(row_elements);
-    const int64_t grid = (rows + NORM_ROWS - 1) / NORM_ROWS;
+    int tile_rows = NORM_ROWS;
+    while (L >= 32 && tile_rows > 1 && (rows + tile_rows - 1) / tile_rows < sm_count()) // (shorter rows: 2 x 4 1.68 us in eights, 1.88 in twos)
+        tile_rows /= 2;
+    const int64_t grid = (rows + tile_rows - 1) / tile_rows;
     if (grid > 0x7FFFFFFF)
         return B200_ERR_TOO_LARGE;
     auto launch = [&](auto kernel, std::atomic<uint64_t>& told) {
         size_t bytes;
-        if (!staged_bytes(kernel, told, NORM_ROWS, L, vec, bytes))
+        if (!staged_bytes(kernel, told, tile_rows, L, vec, bytes))
             return false;
         // rows that run at the same time: what follows a tile on its SM starts that much further on
         const int64_t resident = std::min<int64_t>(200 * 1024 / int64_t(bytes + 1024), 2048 / ROW_THREADS);
-        b200::launch(kernel, unsigned(grid), ROW_THREADS, bytes, st, x, addend, gamma, beta, out, rows, L, count, epsilon, resident * sm_count() * NORM_ROWS);
+        b200::launch(kernel, unsigned(grid), ROW_THREADS, bytes, st, x, addend, gamma, beta, out, rows, L, count, epsilon, resident * sm_count() * NORM_ROWS, tile_rows);
         return true;
     };
-    static std::atomic<uint64_t> told[4];
-    const bool ok = vec ? (addend ? launch(layer_norm_rows_kernel<true, true>, told[0]) : launch(layer_norm_rows_kernel<true, false>, told[1]))
-                        : (addend ? launch(layer_norm_rows_kernel<false, true>, told[2]) : launch(layer_norm_rows_kernel<false, false>, told[3]));
+    static std::atomic<uint64_t> told[8];
+    auto choose = [&](auto few) {
+        constexpr bool FEW = decltype(few)::value;
+        std::atomic<uint64_t>* const t = told + (FEW ? 4 : 0);
+        return vec ? (addend ? launch(layer_norm_rows_kernel<true, true, FEW>, t[0]) : launch(layer_norm_rows_kernel<true, false, FEW>, t[1]))
+                   : (addend ? launch(layer_norm_rows_kernel<false, true, FEW>, t[2]) : launch(layer_norm_rows_kernel<false, false, FEW>, t[3]));
+    };
+    const bool ok = tile_rows < NORM_ROWS ? choose(std::true_type()) : choose(std::false_type());
     if (!ok)
         return B200_ERR_CUDA;
     return after_launch("b200_layer_norm_rows_f32");
