@@ -127,7 +127,7 @@ namespace b200
                              // as long (free -> landed takes 3 us per 32 KB stage, six stages per 4 us).  Never chosen; the
                              // variant is compiled into instrumented builds only, which can force it.
         int late_successor;  // the stream's next kernel is let in when this one is about done (otherwise: at once)
-        int one_shot;        // one tile of 64 columns, or a part of its reduction, per CTA (see below)
+        int one_shot;        // one tile of 64 columns, or a part of its reduction, per CTA (see below); 2: EPI_ONE_SHOT_ROWS
         int rows;            // rows of a tile: BM, or 64 in one-shot launches (the MMA's other 64 rows compute on what lies there)
         int split;           // CTAs that share one tile's reduction (a thread-block cluster), 1: none
         void* out;
@@ -389,15 +389,15 @@ namespace b200
         }
     }
 
-    // The same 32 columns under the core contract, one-byte output: saturate(half-away(float(acc) * scale) + zero point).
+    // The same columns under the core contract, one-byte output: saturate(half-away(float(acc) * scale) + zero point).
     // floor(RD(|f| + 0.5)), the sum rounded down, is the magnitude of half-away rounding: the exact sum is never below an
     // integer that its rounded value reaches.  zp: |out_zp| <= 2^20 (the caller checks), so that the clamp can come first.
-    template <bool OUT_U8>
-    __device__ __forceinline__ void epilogue_chunk_core(const uint32_t (&v)[32], uint32_t (&w)[8], float scale, int zp)
+    template <bool OUT_U8, int W>
+    __device__ __forceinline__ void epilogue_chunk_core(const uint32_t (&v)[W], uint32_t (&w)[W / 4], float scale, int zp)
     {
         const int lo = (OUT_U8 ? 0 : -128) - zp, hi = (OUT_U8 ? 255 : 127) - zp;
 #pragma unroll
-        for (int j4 = 0; j4 < 8; ++j4)
+        for (int j4 = 0; j4 < W / 4; ++j4)
         {
             int q[4];
 #pragma unroll
@@ -504,7 +504,7 @@ namespace b200
     constexpr int MAX_SPLIT = 8;
     constexpr int SPLIT_EXCHANGE_BYTES = BM * 64 * 4;  // the parts a CTA receives: split x (64 / split) columns x 128 rows
     constexpr int SPLIT_SMEM_LIMIT = 112 * 1024;       // two CTAs per SM
-    constexpr int ONE_SHOT_STAGED_BYTES = EPI_WARPS * 128; // scales and biases of each warp's 16 columns
+    constexpr int ONE_SHOT_STAGED_BYTES = EPI_WARPS * 128 + BM * 64; // scales and biases of each warp's 16 columns, a tile of bytes
 
     // The way out for a CTA whose waits gave up, by all its threads.  Otherwise a CTA leaves when every part has landed and nothing
     // writes to it any more; here parts may still be on their way.  The barrier counts the cluster's threads that have not left:
@@ -520,26 +520,26 @@ namespace b200
         __syncthreads();
     }
 
-    // Row `row` of a one-shot tile: its offset in the result, whether it is inside; returns the column tile.
-    __device__ __forceinline__ int row_of_tile(const ContractParams& p, int tile, int row, bool& valid, int64_t& off)
+    // A one-shot tile: its column tile and where its rows lie in the result
+    struct TileRows
     {
         int tm, tn, q0, p0, n0;
-        decode_tile(p, tile, tm, tn, q0, p0, n0);
-        if (p.conv) // the patch's extents are powers of two
+        __device__ __forceinline__ TileRows(const ContractParams& p, int tile) { decode_tile(p, tile, tm, tn, q0, p0, n0); }
+        // offset of row `row` (of its first column), and whether it is inside
+        __device__ __forceinline__ bool at(const ContractParams& p, int row, int64_t& off) const
         {
-            const int w = __ffs(p.RW) - 1, h = __ffs(p.TH) - 1;
-            const int q = q0 + (row & (p.RW - 1)), pp = p0 + ((row >> w) & (p.TH - 1)), n = n0 + (row >> (w + h));
-            valid = row < p.rows && q < p.Q && pp < p.P && n < p.NB;
-            off = ((int64_t(n) * p.P + pp) * p.Q + q) * p.N;
-        }
-        else
-        {
+            if (p.conv) // the patch's extents are powers of two
+            {
+                const int w = __ffs(p.RW) - 1, h = __ffs(p.TH) - 1;
+                const int q = q0 + (row & (p.RW - 1)), pp = p0 + ((row >> w) & (p.TH - 1)), n = n0 + (row >> (w + h));
+                off = ((int64_t(n) * p.P + pp) * p.Q + q) * p.N;
+                return row < p.rows && q < p.Q && pp < p.P && n < p.NB;
+            }
             const int m = tm * p.rows + row;
-            valid = row < p.rows && m < p.M;
             off = int64_t(m) * p.N;
+            return row < p.rows && m < p.M;
         }
-        return tn;
-    }
+    };
 
     // Four columns of a row, of any contract and type, from their accumulators to memory (element offset `at`, `cols` columns inside;
     // `aligned`: four results may be stored at once).
@@ -620,9 +620,10 @@ namespace b200
                 ptx::store_async(ptx::mapa(dst, uint32_t(owner)), v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3], ptx::mapa(landed, uint32_t(owner)));
             }
         }
-        bool valid;
+        const TileRows rows(p, tile);
         int64_t off;
-        const int tn = row_of_tile(p, tile, row, valid, off);
+        const bool valid = rows.at(p, row, off);
+        const int tn = rows.tn;
         const int first = tn * 64 + rank * quads * 4; // first column finished here
         const bool one_byte = p.out_type == B200_U8 || p.out_type == B200_I8;
         const bool aligned = p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out) & (one_byte ? 3 : 15)) == 0;
@@ -687,19 +688,55 @@ namespace b200
         else
             epilogue_chunk_bytes<SUM, false, false>(v, w, sc, bi, sumw, sum_scale, sum_flip, sum_magic, p.one);
     }
+    // The staged rows of a tile to memory, two at a time per warp, 16 lanes each: the words of a row that are aligned in global memory,
+    // put together from two staged ones, and the up to six bytes before and behind them (as the persistent kernel's rows, but by all
+    // warps: 63 x 65 x 80 4.6 us there, 2.8 so; 300 x 99 x 640 5.5 and 3.8, core contract 6.3 and 4.0).
+    __device__ __forceinline__ void one_shot_rows(const ContractParams& p, const TileRows& rows, uint32_t tile_at, int ew, int lane)
+    {
+        const int col = rows.tn * 64, cols = min(64, p.N - col), k = lane & 15;
+#pragma unroll 1
+        for (int rr = 2 * ew + (lane >> 4); rr < p.rows; rr += 2 * EPI_WARPS)
+        {
+            int64_t off;
+            if (!rows.at(p, rr, off))
+                continue;
+            uint8_t* const dst = static_cast<uint8_t*>(p.out) + off + col;
+            const int head = min(cols, int((0u - uint32_t(reinterpret_cast<uintptr_t>(dst))) & 3u));
+            const int full = (cols - head) >> 2, tail = (cols - head) & 3;
+            const uint32_t row = tile_at + uint32_t(rr) * 64, flip = uint32_t((rr >> 1) & 3) << 4;
+            const uint32_t w0 = uint32_t(k) * 4u, w1 = min(w0 + 4u, 60u);
+            uint32_t a, b;
+            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(a) : "r"(row + (w0 ^ flip)) : "memory");
+            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(b) : "r"(row + (w1 ^ flip)) : "memory");
+            if (k < full)
+                *reinterpret_cast<uint32_t*>(dst + head + 4 * k) = __funnelshift_r(a, b, 8 * head);
+            if (k < head + tail)
+            {
+                const uint32_t byte = k < head ? uint32_t(k) : uint32_t(cols - tail + k - head);
+                uint32_t x;
+                asm volatile("ld.shared.u8 %0, [%1];" : "=r"(x) : "r"(row + (byte ^ flip)) : "memory");
+                dst[byte] = uint8_t(x);
+            }
+        }
+    }
+    template <bool ROWS>
     __device__ __forceinline__ void one_shot_epilogue(const ContractParams& p, int tile, int warp, int lane, uint32_t tmem_base, uint32_t staged, uint32_t tfull, volatile int* abortp,
                                                       int& fail)
     {
         const int quarter = warp & 3, group = (warp - 4) >> 2; // accumulator rows 32 * quarter .. + 31, columns 16 * group .. + 15
-        bool valid;
+        const TileRows rows(p, tile);
         int64_t off;
-        const int col = row_of_tile(p, tile, quarter * 32 + lane, valid, off) * 64 + group * 16, cols = p.N - col;
-        if (quarter * 32 >= p.rows || cols <= 0)
-            return; // warp-uniform; the first warp of the first group always has work, so the CTA stays until its products are complete
+        const bool valid = rows.at(p, quarter * 32 + lane, off);
+        const int col = rows.tn * 64 + group * 16, cols = p.N - col;
+        // one-byte rows that are not whole pieces of 16 leave through shared memory, by all warps
+        const bool ragged = ROWS && (p.out_type == B200_U8 || p.out_type == B200_I8);
+        const bool here = quarter * 32 < p.rows && cols > 0; // warp-uniform
+        if (!here && !ragged)
+            return; // the first warp of the first group always has work, so the CTA stays until its products are complete
         const bool one_byte = p.out_type == B200_U8 || p.out_type == B200_I8;
-        const float sum_scale = p.sum_in ? __ldg(ordered(p.sum_scale)) : 0.0f;
+        const float sum_scale = !ROWS && p.sum_in ? __ldg(ordered(p.sum_scale)) : 0.0f;
         const uint32_t sc = staged + uint32_t(warp - 4) * 128, bi = sc + 64;
-        if (lane < 16)
+        if (lane < 16 && here)
         {
             const float scale = lane < cols ? __ldg(ordered(p.scale) + (p.scale_per_channel ? col + lane : 0)) : 0.0f;
             const int32_t bias = lane < cols && p.bias ? __ldg(ordered(p.bias) + col + lane) : 0;
@@ -707,7 +744,7 @@ namespace b200
             asm volatile("st.shared.b32 [%0], %1;" ::"r"(bi + 4 * lane), "r"(bias) : "memory");
         }
         uint4 sum = make_uint4(0, 0, 0, 0);
-        if (valid && p.sum_in)
+        if (!ROWS && valid && p.sum_in)
             sum = *reinterpret_cast<const uint4*>(ordered(static_cast<const uint8_t*>(p.sum_in)) + off + col);
         if (!__all_sync(0xffffffffu, ptx::mbar_wait(tfull, 0, abortp, 0)))
         {
@@ -724,16 +761,31 @@ namespace b200
             ptx::tmem_ld_wait(v);
             uint32_t w[4];
             const uint32_t sumw[4] = {sum.x, sum.y, sum.z, sum.w};
-            if (p.sum_in)
+            if (ROWS && p.half_away && p.out_type == B200_U8)
+                epilogue_chunk_core<true>(v, w, lds_f4(sc).x, p.out_zp);
+            else if (ROWS && p.half_away)
+                epilogue_chunk_core<false>(v, w, lds_f4(sc).x, p.out_zp);
+            else if (!ROWS && p.sum_in)
                 one_shot_bytes<2>(p, v, w, sc, bi, sumw, sum_scale);
             else
                 one_shot_bytes<0>(p, v, w, sc, bi, sumw, sum_scale);
-            if (valid)
+            if (ragged)
+            {
+                const uint32_t tile_at = staged + EPI_WARPS * 128;
+                if (here) // 64 bytes a row, its four pieces where the lanes of a store meet different banks
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile_at + uint32_t(quarter * 32 + lane) * 64 + ((uint32_t(group) ^ (uint32_t(lane >> 1) & 3)) << 4)),
+                                 "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
+                                 : "memory");
+                asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
+                one_shot_rows(p, rows, tile_at, warp - 4, lane);
+            }
+            else if (valid)
                 *reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.out) + off + col) = make_uint4(w[0], w[1], w[2], w[3]);
             return;
         }
         // f32: four lanes hold eight neighbouring columns of a row, a store writes whole sectors of eight rows
         const int g = lane >> 2, pair_col = 2 * (lane & 3);
+        constexpr bool pairs = !ROWS;
         const uint32_t rows_ok = __ballot_sync(0xffffffffu, valid) >> g;
         ptx::tmem_ld_16x16(t_addr, v, 0);
         ptx::tmem_ld_16x16(t_addr + (16u << 16), v, 8);
@@ -751,8 +803,15 @@ namespace b200
                                        __fmul_rn(__int2float_rn(int32_t(x[1]) + __float_as_int(b2.y)), s2.y));
                 if (p.relu)
                     r = make_float2(fmaxf(r.x, 0.0f), fmaxf(r.y, 0.0f));
-                if (((rows_ok >> (8 * i)) & 1u) != 0 && 8 * j + pair_col < cols)
+                const bool ok = ((rows_ok >> (8 * i)) & 1u) != 0 && 8 * j + pair_col < cols;
+                if (ok && pairs)
                     *reinterpret_cast<float2*>(o + 8 * j) = r;
+                else if (ok)
+                {
+                    o[8 * j] = r.x;
+                    if (8 * j + pair_col + 1 < cols)
+                        o[8 * j + 1] = r.y; // (neighbours' sectors meet in L2)
+                }
             }
         }
     }
@@ -770,7 +829,8 @@ namespace b200
         EPI_SUM,     // one-byte results with a residual that TMA does not bring (or a ring that leaves it no room): the residual into
                      // registers ahead of the accumulator, the stores of EPI_ROWS
         EPI_GENERAL, // everything else: results of any type straight from registers
-        EPI_ONE_SHOT // a kernel of its own: one tile per CTA (one_shot_epilogue)
+        EPI_ONE_SHOT, // kernels of their own, one tile per CTA (one_shot_epilogue): rows of whole pieces, a fused contract;
+        EPI_ONE_SHOT_ROWS // rows that start anywhere, and one-byte results of the core contract
     };
     template <int BN, int BK, bool CTA2 = false, bool SPLITK = false, int EPI = EPI_BYTES>
     __global__ void __launch_bounds__(NUM_THREADS, SPLITK ? 2 : 1)
@@ -778,7 +838,7 @@ namespace b200
     {
         using C = Cfg<BN, BK>;
         constexpr int SPLIT = C::SPLIT, GROUPS = C::GROUPS, NACC = C::NACC;
-        constexpr bool EXCHANGE = SPLITK && EPI != EPI_ONE_SHOT; // the tile's CTAs are a cluster
+        constexpr bool EXCHANGE = SPLITK && EPI != EPI_ONE_SHOT && EPI != EPI_ONE_SHOT_ROWS; // the tile's CTAs are a cluster
         // a split tile has one accumulator: two of these CTAs, of one launch or of consecutive ones, share an SM
         constexpr uint32_t TMEM_COLS = SPLITK ? BN : C::TMEM_COLS;
         // CTA pairs: rank 0 issues the pair's MMAs; a "worker" is what takes units of work in turn (a CTA, or a pair)
@@ -1311,7 +1371,7 @@ namespace b200
             {
                 wait_for_earlier_kernels();
                 if constexpr (!EXCHANGE)
-                    one_shot_epilogue(p, worker, warp, lane, tmem_base, out_base, tfull_bar(0), abortp, fail);
+                    one_shot_epilogue<EPI == EPI_ONE_SHOT_ROWS>(p, worker, warp, lane, tmem_base, out_base, tfull_bar(0), abortp, fail);
                 else
                     split_epilogue(p, worker, split_rank, warp, lane, tmem_base, out_base, tfull_bar(0), sum_bar(0, 0), abortp, fail);
             }
@@ -2176,10 +2236,10 @@ namespace b200
     // [1, 512, 7, 7] 3x3 -> 512: 10.5 us whole, 6.5 in eight; 128 x 1000 x 2048: 17.4 and 6.4; 20 x 2432 x 3072: 8.1 whole, 11.7 in two.
     // `words`: the results are what EPI_WORDS computes, which four of a whole tile's warps take 3 us for.
     //
-    // One-shot launches with whole reductions (`pieces`: the results allow it): tiles of 64 rows while they leave half the SMs to the next
+    // One-shot launches with whole reductions (`form`: the results allow it): tiles of 64 rows while they leave half the SMs to the next
     // launch, which sets up there meanwhile (a k-block takes 0.2 us either way, the tensor pipe's rate at 64 columns; the shorter
     // boxes land 0.15 us earlier), otherwise whole tiles where the reduction is short or the weights are one column tile.  More
-    // k-blocks and tiles run as fast in the persistent kernel (400 x 768 x 768: 3.74 us there, 3.94 one-shot).  Reductions are also shared
+    // k-blocks and tiles run as fast in the persistent kernel (400 x 768 x 768: 3.74 us there, 3.94 one-shot), but for ragged rows of bytes.  Reductions are also shared
     // by tiles of 64 rows, which exchange half as much.  Chains of launches, before and after, us: 128 x 128 x 128 2.69, 2.10;
     // 256 x 1024 x 1024 4.09, 3.91; 128 x 768 x 3072 6.40, 5.12; 64 -> 64 on 56x56 3.16, 2.22; 512 -> 512 3x3 on 7x7 5.64, 4.81;
     // 512 -> 2048 on 7x7 with a residual 3.69, 3.11.  tiles64: 0 where such tiles cannot be had.
@@ -2187,9 +2247,10 @@ namespace b200
     {
         int rows, split, one_shot;
     };
-    static Shape pick_shape(int64_t tiles128, int64_t tiles64, int64_t tiles_n, int64_t nkb, bool words, bool pieces, bool f32)
+    static Shape pick_shape(int64_t tiles128, int64_t tiles64, int64_t tiles_n, int64_t nkb, bool words, int form, bool f32)
     {
-        Shape best{BM, 1, pieces && tiles128 <= (f32 ? num_sms() * 7 / 16 : num_sms()) && (nkb <= 2 || tiles_n == 1)};
+        const bool pieces = form != 0;
+        Shape best{BM, 1, pieces && tiles128 <= (f32 ? num_sms() * 7 / 16 : num_sms()) && (nkb <= 2 || tiles_n == 1 || (form == 2 && !f32))};
         double best_us = 0.19 * double(nkb) * double((tiles128 + num_sms() - 1) / num_sms()) + (words && !best.one_shot ? 3.0 : 0.0);
         for (int r = BM; r >= 64; r -= 64)
         {
@@ -2231,7 +2292,8 @@ namespace b200
             return qcontract_kernel<BN, BK, (BN == 256)>;
 #endif
         return p.split > 1                 ? qcontract_kernel<BN, BK, false, (BN == 64)>
-               : p.one_shot                ? qcontract_kernel<BN, BK, false, (BN == 64), (BN == 64 ? EPI_ONE_SHOT : EPI_BYTES)>
+               : p.one_shot == 1           ? qcontract_kernel<BN, BK, false, (BN == 64), (BN == 64 ? EPI_ONE_SHOT : EPI_BYTES)>
+               : p.one_shot == 2           ? qcontract_kernel<BN, BK, false, (BN == 64), (BN == 64 ? EPI_ONE_SHOT_ROWS : EPI_BYTES)>
                : p.epilogue == EPI_SECTORS ? qcontract_kernel<BN, BK, false, false, EPI_SECTORS>
                : p.epilogue == EPI_BYTES_2 ? qcontract_kernel<BN, BK, false, false, EPI_BYTES_2>
                : p.epilogue == EPI_ROWS    ? qcontract_kernel<BN, BK, false, false, EPI_ROWS>
@@ -2470,20 +2532,24 @@ namespace b200
         return e->round_half_away != 2 && (e->out_type == B200_I32 || (e->out_type == B200_F32 && e->sum_in));
     }
 
-    // what a one-shot launch with a whole reduction writes: a fused contract, results in whole pieces
-    static bool one_shot_pieces(const b200_epilogue* e, const void* out, int64_t n)
+    // Which one-shot kernel writes these results from a whole reduction: 0 none, 1 EPI_ONE_SHOT, 2 EPI_ONE_SHOT_ROWS
+    static int one_shot_form(const b200_epilogue* e, const void* out, int64_t n)
     {
-        if (e->round_half_away || (reinterpret_cast<uintptr_t>(out) & 15) != 0)
-            return false;
+        const uintptr_t at = reinterpret_cast<uintptr_t>(out);
         if (e->out_type == B200_F32)
-            return n % 4 == 0 && !e->sum_in;
-        return e->out_type != B200_I32 && n % 16 == 0 && (reinterpret_cast<uintptr_t>(e->sum_in) & 15) == 0;
+            return e->round_half_away || e->sum_in || (at & 3) ? 0 : n % 2 == 0 && (at & 7) == 0 ? 1 : 2;
+        if (e->out_type != B200_U8 && e->out_type != B200_I8)
+            return 0;
+        const bool pieces = n % 16 == 0 && ((at | reinterpret_cast<uintptr_t>(e->sum_in)) & 15) == 0;
+        if (!e->round_half_away)
+            return pieces ? 1 : e->sum_in ? 0 : 2;
+        return e->round_half_away == 1 && e->out_zero_point >= -(1 << 20) && e->out_zero_point <= (1 << 20) ? 2 : 0;
     }
 
     // Up to how many tiles a product that would have wider ones is made of 64 columns for a one-shot launch: with a residual, which costs the
-    // persistent kernel more, one per SM, otherwise half as many (64 -> 256 on 56x56, 100 tiles: 3.1 us in 50 wide ones, 3.2 one-shot; with
+    // persistent kernel more, and with ragged rows, one per SM, otherwise half as many (64 -> 256 on 56x56, 100 tiles: 3.1 us in 50 wide ones, 3.2 one-shot; with
     // a residual 3.7 and 3.5).
-    static int one_shot_tiles(const b200_epilogue* e) { return e->sum_in ? num_sms() : num_sms() / 2; }
+    static int one_shot_tiles(const b200_epilogue* e, int form) { return form == 0 ? 0 : e->sum_in || form == 2 ? num_sms() : num_sms() / 2; }
 
     static void fill_epilogue(ContractParams& p, const b200_epilogue* e, void* out, int a_type)
     {
@@ -2787,15 +2853,15 @@ static int qgemm_impl(const void* A, int a_type, const int8_t* W, bool packed, v
     int bn = pick_bn(N, p.tiles_m, bk, epilogue && epilogue->sum_in, K);
     p.rows = BM;
     p.split = 1;
-    const bool pieces = one_shot_pieces(epilogue, out, N);
+    const int form = one_shot_form(epilogue, out, N);
     const int64_t tiles_n = (N + 63) / 64;
-    if (bn == 64 || (pieces && p.tiles_m * tiles_n <= one_shot_tiles(epilogue)))
+    if (bn == 64 || p.tiles_m * tiles_n <= one_shot_tiles(epilogue, form))
     {
-        const Shape shape = pick_shape(p.tiles_m * tiles_n, (M + 63) / 64 * tiles_n, tiles_n, p.cblocks, four_byte_words(epilogue), pieces, epilogue->out_type == B200_F32);
+        const Shape shape = pick_shape(p.tiles_m * tiles_n, (M + 63) / 64 * tiles_n, tiles_n, p.cblocks, four_byte_words(epilogue), form, epilogue->out_type == B200_F32);
         if (shape.one_shot)
         {
             bn = 64;
-            p.rows = shape.rows, p.split = shape.split, p.one_shot = 1;
+            p.rows = shape.rows, p.split = shape.split, p.one_shot = shape.split > 1 ? 1 : form;
             p.tiles_m = int((M + p.rows - 1) / p.rows);
         }
     }
@@ -2918,13 +2984,16 @@ extern "C" int b200_qconv_out_shape(const b200_conv_params* c, int64_t* P, int64
 // accumulator rows on positions outside the output.
 static void pick_patch(int64_t NB, int64_t P, int64_t Q, int rows, int& TW, int& TH, int& TN)
 {
+    // (all extents are powers of two: a new argument list pays for this once or twice)
+    const double positions = double(NB * P * Q);
     double best = -1.0;
-    for (int tw = 1; tw <= rows; tw *= 2)
-        for (int th = 1; tw * th <= rows; th *= 2)
+    for (int w = 0; (1 << w) <= rows; ++w)
+        for (int h = 0; (1 << (w + h)) <= rows; ++h)
         {
-            int tn = rows / (tw * th);
-            int64_t tiles = ((Q + tw - 1) / tw) * ((P + th - 1) / th) * ((NB + tn - 1) / tn);
-            double eff = double(NB * P * Q) / double(tiles * rows);
+            const int tw = 1 << w, th = 1 << h, tn = rows >> (w + h);
+            const int n = __builtin_ctz(unsigned(tn));
+            const int64_t tiles = ((Q + tw - 1) >> w) * ((P + th - 1) >> h) * ((NB + tn - 1) >> n);
+            const double eff = positions / double(tiles * rows);
             // prefer wider patches on ties (longer contiguous runs for the TMA unit)
             if (eff > best + 1e-9 || (eff > best - 1e-9 && tw * th > TW * TH))
             {
@@ -3043,18 +3112,18 @@ static int qconv_impl(const void* data, int data_type, const int8_t* filters, bo
     auto tiles_of = [&](int TW, int TH, int TN) { return int64_t((Q + TW - 1) / TW) * ((P + TH - 1) / TH) * ((c->N + TN - 1) / TN); };
     p.tiles_m = int(tiles_of(p.TW, p.TH, p.TN));
     int bn = pick_bn(c->K, p.tiles_m, bk, epilogue && epilogue->sum_in, c->R * c->S * c->C);
-    const bool pieces = one_shot_pieces(epilogue, out, c->K);
+    const int form = one_shot_form(epilogue, out, c->K);
     const int64_t tiles_n64 = (c->K + 63) / 64;
-    if (!p.halo && (bn == 64 || (pieces && p.tiles_m * tiles_n64 <= one_shot_tiles(epilogue))))
+    if (!p.halo && (bn == 64 || p.tiles_m * tiles_n64 <= one_shot_tiles(epilogue, form)))
     {
         int TW = 1, TH = 1, TN = 1;
         pick_patch(c->N, P, Q, 64, TW, TH, TN);
         const Shape shape = pick_shape(p.tiles_m * tiles_n64, tiles_of(TW, TH, TN) * tiles_n64, tiles_n64, int64_t(p.ntaps) * p.cblocks, four_byte_words(epilogue),
-                                       pieces, epilogue->out_type == B200_F32);
+                                       form, epilogue->out_type == B200_F32);
         if (shape.one_shot)
         {
             bn = 64;
-            p.rows = shape.rows, p.split = shape.split, p.one_shot = 1;
+            p.rows = shape.rows, p.split = shape.split, p.one_shot = shape.split > 1 ? 1 : form;
             if (p.rows == 64)
                 p.TW = TW, p.TH = TH, p.TN = TN;
         }

@@ -716,9 +716,11 @@ def test_qgemm_residuals_and_words_off_the_tma_paths(ops, m, n, k):
 
 
 # ---------------------------------------------------------------- one tile per CTA
-@pytest.mark.parametrize("m,n,k", [(1, 16, 16), (31, 64, 144), (64, 80, 128), (65, 48, 1040), (129, 208, 272), (600, 256, 2048), (1000, 512, 512), (200, 64, 4096), (160, 512, 2064), (4700, 64, 64)])
+@pytest.mark.parametrize("m,n,k", [(1, 16, 16), (31, 64, 144), (64, 80, 128), (65, 48, 1040), (129, 208, 272), (600, 256, 2048), (1000, 512, 512), (200, 64, 4096), (160, 512, 2064), (4700, 64, 64),
+                                   (1, 17, 32), (63, 65, 80), (300, 99, 640), (500, 777, 992), (1500, 35, 1040), (129, 130, 208)])
 def test_one_shot_products(ops, m, n, k):
-    """tiles of 64 and 128 rows that end early, whole and shared reductions, all results that leave in whole pieces"""
+    """tiles of 64 and 128 rows that end early, whole and shared reductions, results in whole pieces, in rows that start anywhere and
+    of the core contract"""
     gen = torch.Generator(device="cuda").manual_seed(m + n + k)
 
     def ints(lo, hi, shape, dt):
@@ -727,9 +729,15 @@ def test_one_shot_products(ops, m, n, k):
     a, w, bias = ints(-128, 128, (m, k), torch.int8), ints(-127, 128, (n, k), torch.int8), ints(-1000, 1001, (n,), torch.int32)
     scale = torch.rand(n, generator=gen, device="cuda") * 0.01 / k ** 0.5 + 0.005 / k ** 0.5
     ss = torch.full((1,), 0.37, device="cuda")
-    base = ((a.double() @ w.double().t()).to(torch.int32) + bias).float() * scale
+    acc = (a.double() @ w.double().t()).to(torch.int32)
+    base = (acc + bias).float() * scale
     res = {torch.uint8: ints(0, 256, (m, n), torch.uint8), torch.int8: ints(-128, 128, (m, n), torch.int8)}
+    half_away = (acc.float() * scale[0]).double()
+    half_away = torch.sign(half_away) * (half_away.abs() + 0.5).floor()
     for packed in (True, False):
+        for out, zp in ((torch.int8, 3), (torch.uint8, 128)):
+            want = (half_away + zp).clamp(*((0, 255) if out == torch.uint8 else (-128, 127))).to(out)
+            assert torch.equal(ops.qgemm(a, w, scale[:1], out, core=True, out_zp=zp, packed=packed), want), (out, packed)
         for out, relu, r in ((torch.uint8, False, None), (torch.int8, True, None), (torch.int8, False, torch.int8), (torch.uint8, True, torch.uint8), (torch.float32, False, None),
                              (torch.float32, True, None)):
             f = base if r is None else base + ss * res[r].float()
