@@ -501,7 +501,8 @@ B200_API int b200_qconv_stem_static(const void* in_nchw, int data_type, const in
  *                        shift; every step rounded separately) from one kernel; rows longer than 1535 are unsupported
  *   b200_gelu_f32        op::v0::Gelu as its decomposition computes it (gelu.cpp:46-60): (0.5 * x) * (1 + erf(x / sqrt 2))
  *   b200_bmm_f32         op::v0::BatchMatMul / 2-D op::v0::Dot on f32 (batch_mat_mul.hpp, dot.hpp:108-160): a[b,M,K] x
- *                        b[b,K,N], the sum over k in double, in order, rounded to float once
+ *                        b[b,K,N], the sum over k in double, in order, rounded to float once (large products from exact
+ *                        int8 digit sums, with the same bits)
  *   b200_gather_rows_b32 op::v0::Gather with axis 0 on a 2-D table of 4-byte elements and an i32 / i64 index vector
  *                        (gather.hpp); an index outside the table yields zeros (the reference does not check)
  */

@@ -10,7 +10,7 @@
 //   Max          runtime/reference/max.hpp:32-58     start at -inf, replace when x > max
 //   Broadcast    runtime/reference/broadcast.hpp     output coordinate with the broadcast axes dropped
 //   BatchMatMul  runtime/reference/batch_mat_mul.hpp -> dot.hpp:108-160: the sum over k runs in DOUBLE, in order,
-//                over exact products, and is rounded to float once
+//                over exact products, and is rounded to float once (large products: bmm_digits.cu)
 //   Gather       runtime/reference/gather.hpp        rows of a matrix picked by an index vector
 //   Reshape      runtime/reference/reshape.hpp       axis permutation followed by a free re-interpretation
 //

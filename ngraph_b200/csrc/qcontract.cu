@@ -22,6 +22,8 @@
 //   (one-byte outputs) a swizzled shared-memory staging block of its own -> one TMA store, so
 //   global writes are whole lines and rows/columns outside the tensor are clipped by the TMA
 //   unit.  Ragged widths leave the staging block by plain stores, four-byte outputs go straight from registers.
+// * Launches of few tiles are not persistent: one tile of 64 columns and 64 or 128 rows, or a cluster CTA's part of its
+//   reduction, per CTA, and all 16 epilogue warps write it from registers (ContractParams.one_shot, pick_shape).
 // * Every wait is bounded (ptx::mbar_wait); a timeout sets g_contract_status, the CTA
 //   drains and frees its TMEM, and the host reports B200_ERR_DEVICE_STATUS.
 #include <cuda.h>
